@@ -25,6 +25,7 @@
 #include <mutex>
 #include <string>
 
+#include "canon_math.h"
 #include "nr_device.cuh"
 #include "nr_internal.h"
 
@@ -45,18 +46,18 @@ __device__ __forceinline__ double bond_strain(const EdgeIn &a, int b) {
     const double dyi = a.pos0[2 * i2 + 1] - a.pos0[2 * i1 + 1];
     const double dxf = dxi + a.disp[2 * i2] - a.disp[2 * i1];
     const double dyf = dyi + a.disp[2 * i2 + 1] - a.disp[2 * i1 + 1];
-    const double li = sqrt(dxi * dxi + dyi * dyi);
-    const double lf = sqrt(dxf * dxf + dyf * dyf);
-    return (lf - li) / li;
+    const double li = sqrt_ieee(dxi * dxi + dyi * dyi);
+    const double lf = sqrt_ieee(dxf * dxf + dyf * dyf);
+    return div_ieee(lf - li, li);
 }
 
 __device__ __forceinline__ double axial_term(const EdgeIn &a, int b) {
     const int i1 = a.ij[2 * b], i2 = a.ij[2 * b + 1];
     double dx = a.pos0[2 * i2] + a.width * a.wrap[b] - a.pos0[2 * i1];
     double dy = a.pos0[2 * i2 + 1] - a.pos0[2 * i1 + 1];
-    const double length = sqrt(dx * dx + dy * dy);
-    dx /= length;
-    dy /= length;
+    const double length = sqrt_ieee(dx * dx + dy * dy);
+    dx = div_ieee(dx, length);
+    dy = div_ieee(dy, length);
     const double proj = (a.disp[2 * i2] - a.disp[2 * i1]) * dx + (a.disp[2 * i2 + 1] - a.disp[2 * i1 + 1]) * dy;
     return .5 * proj * proj;
 }

@@ -24,6 +24,8 @@
 
 #include <math.h>
 
+#include "ieee_int.h"
+
 #if defined(__CUDACC__)
 #define NR_HD __host__ __device__ __forceinline__
 #else
@@ -47,17 +49,46 @@ namespace nr {
 #define NR_ATAN_Q9 (0.1999999999999552)
 #define NR_ATAN_Q10 (-0.3333333333333333)
 
+/* IEEE division, square root and 1 / sqrt (two roundings).  On the device
+ * they run on the integer pipe (ieee_int.h): the same bits for a seventh of
+ * the FP64 slots, the bound of every FP64 kernel here. */
+NR_HD double div_ieee(double a, double b) {
+#if defined(__CUDA_ARCH__)
+    return ii_div(a, b);
+#else
+    return a / b;
+#endif
+}
+NR_HD double sqrt_ieee(double q) {
+#if defined(__CUDA_ARCH__)
+    return ii_sqrt(q);
+#else
+    return sqrt(q);
+#endif
+}
+NR_HD double inv_sqrt_ieee(double q) {
+#if defined(__CUDA_ARCH__)
+    return ii_inv_sqrt(q);
+#else
+    return 1.0 / sqrt(q);
+#endif
+}
+
 /* Quadrant/octant reduction, then atan(t) = pi/4 + atan((t-1)/(t+1)) above
  * tan(pi/8), then the polynomial; pi/4, pi/2 and pi are added as two-part
  * constants.  About one ulp for finite non-zero arguments; (0,0) -> 0. */
 NR_HD double atan2_canon(double y, double x) {
     const double ax = fabs(x), ay = fabs(y);
-    const bool swap = ay > ax;
+    /* the comparisons on the operands' bits: an FP64 comparison takes an FP64
+     * slot, and the magnitudes order like their bits (a NaN gives NaN either
+     * way) */
+    const bool swap = ii_bits(ay) > ii_bits(ax);
     const double num = swap ? ax : ay;
     const double den = swap ? ay : ax;
-    const double t = den == 0.0 ? 0.0 : num / den;
-    const bool red = t > 0.41421356237309503;
-    const double u = red ? (t - 1.0) / (t + 1.0) : t;
+    const double t = ii_is_zero(den) ? 0.0 : div_ieee(num, den);
+    const bool red = ii_bits(t) > 0x3fda827999fcef32ULL; /* t > tan(pi / 8) = 0.41421356237309503 */
+    double u = t;
+    if (red) u = div_ieee(t - 1.0, t + 1.0);
     const double z = u * u;
     double q = NR_ATAN_Q0;
     q = fma(q, z, NR_ATAN_Q1);
@@ -73,28 +104,42 @@ NR_HD double atan2_canon(double y, double x) {
     double r = fma(u * z, q, u);
     if (red) r = 0.7853981633974483 + (3.061616997868383e-17 + r);
     if (swap) r = 1.5707963267948966 + (6.123233995736766e-17 - r);
-    if (x < 0.0) r = 3.141592653589793 + (1.2246467991473532e-16 - r);
-    return y < 0.0 ? -r : r;
+    if (ii_negative(x)) r = 3.141592653589793 + (1.2246467991473532e-16 - r);
+    return ii_flip(r, ii_negative(y));
 }
 
 /* Periodic image offset wrap * width; exactly 0.0 for wrap 0. */
 NR_HD double wrap_shift(int wrap, double width) { return wrap ? (double)wrap * width : 0.0; }
+
+/* x + wrap_shift(wrap, width): most arms cross no boundary and take no
+ * operation (x + 0 = x; a -0 stays -0, which no angle or force shows). */
+NR_HD double wrap_add(double x, int wrap, double width) { return wrap ? x + (double)wrap * width : x; }
 
 /* Stretch force on the bond's SECOND end's partner, i.e. the value the
  * reference adds to its first endpoint (large_strain_relax.cu:401-403);
  * the second endpoint receives the negation. */
 NR_HD void bond_force(double x1, double y1, double x2, double y2, double wW, double l0, double k, double &fx,
                       double &fy) {
-    const double rx = (x1 - x2) - wW, ry = y1 - y2;
-    const double inv = 1.0 / sqrt(fma(rx, rx, ry * ry));
-    const double s = k * fma(-l0, inv, 1.0);
-    fx = s * ((x2 + wW) - x1);
-    fy = s * (y2 - y1);
+    double rx = x1 - x2;
+    const double ry = y1 - y2;
+    /* most bonds cross no boundary: then r = (x1 - x2) - 0 and the force's
+     * x2 + 0 - x1 = -(x1 - x2) need no further operation (an exact zero may
+     * change its sign, which no sum that starts from +0 shows) */
+    double dx = -rx;
+    if (!ii_is_zero(wW)) {
+        rx = rx - wW;
+        dx = (x2 + wW) - x1;
+    }
+    const double inv = inv_sqrt_ieee(fma(rx, rx, ry * ry));
+    double s = fma(-l0, inv, 1.0);
+    if (ii_bits(k) != 0x3ff0000000000000ULL) s = k * s; /* k = 1: the usual stiffness */
+    fx = s * dx;
+    fy = s * -ry;
 }
 
 NR_HD double bond_energy(double x1, double y1, double x2, double y2, double wW, double l0, double k) {
     const double rx = (x1 - x2) - wW, ry = y1 - y2;
-    const double dd = sqrt(fma(rx, rx, ry * ry)) - l0;
+    const double dd = sqrt_ieee(fma(rx, rx, ry * ry)) - l0;
     return ((0.5 * k) * dd) * dd;
 }
 
@@ -102,7 +147,8 @@ NR_HD double bond_energy(double x1, double y1, double x2, double y2, double wW, 
 NR_HD double bend_dtheta(double ax, double ay, double bx, double by, double phi0) {
     const double c = fma(ax, by, -(ay * bx));
     const double d = fma(ax, bx, ay * by);
-    return atan2_canon(-c, -d) - phi0;
+    const double th = atan2_canon(-c, -d);
+    return ii_is_zero(phi0) ? th : th - phi0; /* th - 0 = th */
 }
 
 /* Bending forces on j and k (large_strain_relax.cu:453-459); the hinge
@@ -110,8 +156,8 @@ NR_HD double bend_dtheta(double ax, double ay, double bx, double by, double phi0
 NR_HD void bend_force(double ax, double ay, double bx, double by, double kb, double phi0, double &fjx,
                       double &fjy, double &fkx, double &fky) {
     const double g = kb * bend_dtheta(ax, ay, bx, by, phi0);
-    const double g2 = g / fma(ax, ax, ay * ay);
-    const double g3 = g / fma(bx, bx, by * by);
+    const double g2 = div_ieee(g, fma(ax, ax, ay * ay));
+    const double g3 = div_ieee(g, fma(bx, bx, by * by));
     fjx = -ay * g2;
     fjy = ax * g2;
     fkx = by * g3;

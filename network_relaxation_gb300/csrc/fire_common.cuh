@@ -39,21 +39,23 @@ __device__ __forceinline__ double4 gel_terms(const NetDev &d, int e, int r, doub
     const double a = M[2 * r], b = M[2 * r + 1];
     return make_double4(du11 * a, du12 * b, du21 * a, du22 * b);
 }
-__device__ __forceinline__ void gel_du(const NetDev &d, int e, double &du11, double &du12, double &du21,
-                                       double &du22) {
-    double f11, f12, f21, f22;
-    gel_defgrad(d, e, f11, f12, f21, f22);
-    const NetGel &g = *d.gel;
-    const double A = g.elem_area[e];
+__device__ __forceinline__ void gel_du_of(const NetGel &g, double A, double f11, double f12, double f21, double f22,
+                                          double &du11, double &du12, double &du21, double &du22) {
     const double smod = g.smod, bmod = g.bmod, dil = g.gdil;
     const double det = f11 * f22 - f12 * f21;
-    const double coeff1 = -smod * A / det;
-    double coeff2 = bmod * (dil + 1 - det) + smod * (f11 * f11 + f12 * f12 + f21 * f21 + f22 * f22) / (2 * det * det);
+    const double coeff1 = div_ieee(-smod * A, det);
+    double coeff2 = bmod * (dil + 1 - det) + div_ieee(smod * (f11 * f11 + f12 * f12 + f21 * f21 + f22 * f22), 2 * det * det);
     coeff2 *= A;
     du11 = f11 * coeff1 + f22 * coeff2;
     du12 = f12 * coeff1 - f21 * coeff2;
     du21 = f21 * coeff1 - f12 * coeff2;
     du22 = f22 * coeff1 + f11 * coeff2;
+}
+__device__ __forceinline__ void gel_du(const NetDev &d, int e, double &du11, double &du12, double &du21,
+                                       double &du22) {
+    double f11, f12, f21, f22;
+    gel_defgrad(d, e, f11, f12, f21, f22);
+    gel_du_of(*d.gel, d.gel->elem_area[e], f11, f12, f21, f22, du11, du12, du21, du22);
 }
 /* gel_energy (network_mesh_relax.cu:674-699) of element e, as |e| for the
  * cublasDasum the reference sums it with. */
@@ -64,8 +66,8 @@ __device__ __forceinline__ double gel_energy_abs(const NetDev &d, int e) {
     const double A = g.elem_area[e];
     const double smod = g.smod, bmod = g.bmod, dil = g.gdil;
     const double det = f11 * f22 - f12 * f21;
-    double en = smod * A * ((f11 * f11 + f12 * f12 + f21 * f21 + f22 * f22) / det - 2) / 2;
-    en += bmod * A * (det - 1 - dil) * (det - 1 - dil) / 2;
+    double en = smod * A * (div_ieee(f11 * f11 + f12 * f12 + f21 * f21 + f22 * f22, det) - 2) * 0.5;
+    en += bmod * A * (det - 1 - dil) * (det - 1 - dil) * 0.5;
     return fabs(en);
 }
 /* Adds an element's terms to a node's force in the reference's atomicAdd
@@ -114,8 +116,8 @@ __device__ __forceinline__ void node_force_fp64_own(const NetDev &d, int i, doub
             const int4 r = d.tri[t];
             const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
             const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-            const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-            const double bx = (pk.x + wrap_shift(wk, W)) - ph.x, by = pk.y - ph.y;
+            const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+            const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
             const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
             const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
             double fjx, fjy, fkx, fky;
@@ -185,8 +187,8 @@ __device__ inline void items_pass(const NetDev &d, int first, int stride) {
             const int4 r = d.tri[t];
             const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
             const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-            const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-            const double bx = (pk.x + wrap_shift(wk, W)) - ph.x, by = pk.y - ph.y;
+            const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+            const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
             const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
             const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
             double fjx, fjy, fkx, fky;
@@ -264,21 +266,21 @@ struct Scal {
 };
 
 __device__ __forceinline__ bool crit_met(const FireParamsDev &p, double fmag, double maxf, double sqrt_dof) {
-    return p.criterion == 1 ? (maxf < p.fcut) : (fmag / sqrt_dof < p.fcut);
+    return p.criterion == 1 ? (maxf < p.fcut) : (div_ieee(fmag, sqrt_dof) < p.fcut);
 }
 
 /* State at the top of run_fire_md (large_strain_relax.cu:616-643). */
 __device__ inline void scal_init(Scal &s, const FireParamsDev &p, double F2, double M2, double sqrt_dof) {
     s.alpha = p.alpha0;
     s.dt = p.dt_max;
-    s.dtsq = .5 * s.dt * s.dt / p.mass;
-    s.dtm = .5 * s.dt / p.mass;
+    s.dtsq = div_ieee(.5 * s.dt * s.dt, p.mass);
+    s.dtm = div_ieee(.5 * s.dt, p.mass);
     s.mix_na = 0.0;
     s.mix_a = 0.0;
     s.power = 0.0;
     s.vmag = 0.0;
-    s.fmag = sqrt(F2);
-    s.maxf = sqrt(M2);
+    s.fmag = sqrt_ieee(F2);
+    s.maxf = sqrt_ieee(M2);
     s.mix_pending = 0;
     s.zero_v = 0;
     s.since = 0;
@@ -295,26 +297,26 @@ __device__ inline void scal_step(Scal &s, const FireParamsDev &p, double P, doub
                           double sqrt_dof) {
     s.step++;
     s.power = P;
-    s.vmag = sqrt(V2);
-    s.fmag = sqrt(F2);
-    s.maxf = sqrt(M2);
-    s.mix_a = s.alpha * s.vmag / s.fmag;
+    s.vmag = sqrt_ieee(V2);
+    s.fmag = sqrt_ieee(F2);
+    s.maxf = sqrt_ieee(M2);
+    s.mix_a = div_ieee(s.alpha * s.vmag, s.fmag);
     s.mix_na = -s.alpha;
     s.mix_pending = 1;
     if (P > 0) {
         s.since++;
         if (s.since > p.nmin) {
             s.dt = fmin(s.dt * p.finc, p.dt_max);
-            s.dtm = .5 * s.dt / p.mass;
-            s.dtsq = .5 * s.dt * s.dt / p.mass;
+            s.dtm = div_ieee(.5 * s.dt, p.mass);
+            s.dtsq = div_ieee(.5 * s.dt * s.dt, p.mass);
             s.alpha *= p.falpha;
         }
         s.zero_v = 0;
     } else {
         s.since = 0;
         s.dt *= p.fdec;
-        s.dtm = .5 * s.dt / p.mass;
-        s.dtsq = s.dt * s.dt * .5 / p.mass;
+        s.dtm = div_ieee(.5 * s.dt, p.mass);
+        s.dtsq = div_ieee(s.dt * s.dt * .5, p.mass);
         s.alpha = p.alpha0;
         s.zero_v = 1;
     }
@@ -380,8 +382,8 @@ __device__ inline void energy_tiles(const NetDev &d, int t0, int tstride, double
                 const int4 r = d.tri[item];
                 const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
                 const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-                const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-                const double bx = (pk.x + wrap_shift(wk, W)) - ph.x, by = pk.y - ph.y;
+                const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+                const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
                 const double kb = d.tri_kb ? d.tri_kb[item] : d.kb;
                 const double phi0 = d.tri_phi0 ? d.tri_phi0[item] : 0.0;
                 e = bend_energy(ax, ay, bx, by, kb, phi0);

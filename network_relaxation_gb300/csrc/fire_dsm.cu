@@ -97,7 +97,7 @@ static __device__ __noinline__ void anchor_eval_dsm(const NetDev &d, const NetDs
             const double k = d.bond_k ? d.bond_k[b] : d.ks;
             const float hx = (float)rx, hy = (float)ry;
             const float4 rec = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
-            const float2 sk = make_float2((float)(sqrt(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)k);
+            const float2 sk = make_float2((float)(sqrt_ieee(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)k);
             d.mb_data[sl] = rec;
             d.mb_sk[sl] = sk;
             if (res.mb) {
@@ -111,8 +111,8 @@ static __device__ __noinline__ void anchor_eval_dsm(const NetDev &d, const NetDs
             const int4 r = __ldg(d.tri + t);
             const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
             const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-            const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-            const double bx = (pk.x + wrap_shift(wk, W)) - ph.x, by = pk.y - ph.y;
+            const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+            const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
             const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
             const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
             const float4 arms = make_float4((float)ax, (float)ay, (float)bx, (float)by);

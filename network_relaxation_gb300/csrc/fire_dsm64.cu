@@ -82,7 +82,7 @@ __host__ __device__ inline Dsm64Layout dsm64_layout(const Dsm64Sizes &z) {
 
 constexpr int kDsm64Threads = 256;
 
-__global__ void __launch_bounds__(kDsm64Threads, 1)
+__global__ void __launch_bounds__(kDsm64Threads, 2)
     k_fire_dsm64(const NetDev *nets, const NetDsm *dsms, int n_nets, FireParamsDev p, int *queue, const int *order,
                  Dsm64Sizes z) {
     namespace cg = cooperative_groups;

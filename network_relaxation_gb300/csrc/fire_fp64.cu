@@ -376,8 +376,8 @@ __global__ void k_affine(double2 *x, int n, double miny, double yrange, double x
     if (i >= n) return;
     double2 p = x[i];
     const double dy = p.y - miny;
-    p.x = p.x + xdisp * dy / yrange;
-    p.y = p.y + ydisp * dy / yrange;
+    p.x = p.x + div_ieee(xdisp * dy, yrange);
+    p.y = p.y + div_ieee(ydisp * dy, yrange);
     x[i] = p;
 }
 
@@ -420,8 +420,8 @@ __global__ void k_affine_batch(const NetDev *nets, const double4 *prm) {
     for (int i = threadIdx.x; i < d.n; i += blockDim.x) {
         double2 p = d.x[i];
         const double dy = p.y - q.x;
-        p.x = p.x + q.z * dy / q.y;
-        p.y = p.y + q.w * dy / q.y;
+        p.x = p.x + div_ieee(q.z * dy, q.y);
+        p.y = p.y + div_ieee(q.w * dy, q.y);
         d.x[i] = p;
     }
 }

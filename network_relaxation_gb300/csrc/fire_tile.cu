@@ -244,7 +244,7 @@ static __device__ __noinline__ void tile_anchor_eval(const NetDev &d, const NetT
                 const double kk = d.bond_k ? d.bond_k[b] : d.ks;
                 const float hx = (float)rx, hy = (float)ry;
                 mb[k] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
-                sk[k] = make_float2((float)(sqrt(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)kk);
+                sk[k] = make_float2((float)(sqrt_ieee(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)kk);
             }
         if (d.use_triples)
             for (int k = threadIdx.x; k < td.nt; k += blockDim.x) {
@@ -252,8 +252,8 @@ static __device__ __noinline__ void tile_anchor_eval(const NetDev &d, const NetT
                 const int4 r = d.tri[tt];
                 const double2 ph = d.x[r.x], pj = d.x[r.y], pkk = d.x[r.z];
                 const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-                const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-                const double bx = (pkk.x + wrap_shift(wk, W)) - ph.x, by = pkk.y - ph.y;
+                const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+                const double bx = wrap_add(pkk.x, wk, W) - ph.x, by = pkk.y - ph.y;
                 const double kb = d.tri_kb ? d.tri_kb[tt] : d.kb;
                 const double phi0 = d.tri_phi0 ? d.tri_phi0[tt] : 0.0;
                 arms[k] = make_float4((float)ax, (float)ay, (float)bx, (float)by);

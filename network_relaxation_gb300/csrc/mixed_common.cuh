@@ -455,8 +455,8 @@ __device__ __forceinline__ bool need_anchor(const MixScal &s, const MixParams &q
  * reference always takes a first step). */
 __device__ __forceinline__ void mix_certify(MixScal &s, const FireParamsDev &p, double sqrt_dof, double F2,
                                             double M2) {
-    s.fmag = sqrt(F2);
-    s.maxf = sqrt(M2);
+    s.fmag = sqrt_ieee(F2);
+    s.maxf = sqrt_ieee(M2);
     s.m2_anchor = (float)M2;
     s.n_anchor++;
     s.converged = crit_met(p, s.fmag, s.maxf, sqrt_dof);
@@ -549,15 +549,15 @@ static __device__ __noinline__ void anchor_eval(const NetDev &d, const Team &tm,
             const double k = d.bond_k ? d.bond_k[b] : d.ks;
             const float hx = (float)rx, hy = (float)ry;
             d.mb_data[b] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
-            d.mb_sk[b] = make_float2((float)(sqrt(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)k);
+            d.mb_sk[b] = make_float2((float)(sqrt_ieee(fma(rx, rx, ry * ry)) - d.bond_l0[b]), (float)k);
         }
     if (d.use_triples)
         for (int t = tm.first(); t < d.n_triples; t += tm.stride()) {
             const int4 r = d.tri[t];
             const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
             const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-            const double ax = (pj.x + wrap_shift(wj, W)) - ph.x, ay = pj.y - ph.y;
-            const double bx = (pk.x + wrap_shift(wk, W)) - ph.x, by = pk.y - ph.y;
+            const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+            const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
             const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
             const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
             d.mt_arms[t] = make_float4((float)ax, (float)ay, (float)bx, (float)by);
