@@ -77,8 +77,29 @@ NR_HD double inv_sqrt_ieee(double q) {
 /* Quadrant/octant reduction, then atan(t) = pi/4 + atan((t-1)/(t+1)) above
  * tan(pi/8), then the polynomial; pi/4, pi/2 and pi are added as two-part
  * constants.  About one ulp for finite non-zero arguments; (0,0) -> 0. */
-NR_HD double atan2_canon(double y, double x) {
-    const double ax = fabs(x), ay = fabs(y);
+/* Rare cases as functions of their own, called, not inlined: an inlined
+ * branch becomes predicated instructions, and a predicated-off FP64
+ * instruction takes its slot all the same (measured). */
+#if defined(__CUDACC__)
+#define NR_RARE static __host__ __device__ __noinline__
+#else
+#define NR_RARE static inline
+#endif
+NR_RARE double atan2_octant(double r, bool red, bool swap, bool xneg) {
+    if (red) r = 0.7853981633974483 + (3.061616997868383e-17 + r);
+    if (swap) r = 1.5707963267948966 + (6.123233995736766e-17 - r);
+    if (xneg) r = 3.141592653589793 + (1.2246467991473532e-16 - r);
+    return r;
+}
+NR_RARE double wrap_product(int wrap, double width) { return (double)wrap * width; }
+NR_RARE double wrap_sum(double x, int wrap, double width) { return x + (double)wrap * width; }
+/* (x1 - x2) - wW */
+NR_RARE double wrap_gap(double x1, double x2, double wW) { return (x1 - x2) - wW; }
+/* (x2 + wW) - x1 */
+NR_RARE double wrap_reach(double x1, double x2, double wW) { return (x2 + wW) - x1; }
+
+/* atan2 from the operands' magnitudes and signs (negative: below zero). */
+NR_HD double atan2_parts(double ay, double ax, bool yneg, bool xneg) {
     /* the comparisons on the operands' bits: an FP64 comparison takes an FP64
      * slot, and the magnitudes order like their bits (a NaN gives NaN either
      * way) */
@@ -102,18 +123,26 @@ NR_HD double atan2_canon(double y, double x) {
     q = fma(q, z, NR_ATAN_Q9);
     q = fma(q, z, NR_ATAN_Q10);
     double r = fma(u * z, q, u);
-    if (red) r = 0.7853981633974483 + (3.061616997868383e-17 + r);
-    if (swap) r = 1.5707963267948966 + (6.123233995736766e-17 - r);
-    if (ii_negative(x)) r = 3.141592653589793 + (1.2246467991473532e-16 - r);
-    return ii_flip(r, ii_negative(y));
+    /* nearly straight triples, the usual ones, need none of these */
+    if (red || swap || xneg) r = atan2_octant(r, red, swap, xneg);
+    return ii_flip(r, yneg);
+}
+NR_HD double atan2_canon(double y, double x) {
+    return atan2_parts(ii_abs(y), ii_abs(x), ii_negative(y), ii_negative(x));
 }
 
 /* Periodic image offset wrap * width; exactly 0.0 for wrap 0. */
-NR_HD double wrap_shift(int wrap, double width) { return wrap ? (double)wrap * width : 0.0; }
+NR_HD double wrap_shift(int wrap, double width) {
+    if (wrap == 0) return 0.0;
+    return wrap_product(wrap, width);
+}
 
 /* x + wrap_shift(wrap, width): most arms cross no boundary and take no
  * operation (x + 0 = x; a -0 stays -0, which no angle or force shows). */
-NR_HD double wrap_add(double x, int wrap, double width) { return wrap ? x + (double)wrap * width : x; }
+NR_HD double wrap_add(double x, int wrap, double width) {
+    if (wrap != 0) x = wrap_sum(x, wrap, width);
+    return x;
+}
 
 /* Stretch force on the bond's SECOND end's partner, i.e. the value the
  * reference adds to its first endpoint (large_strain_relax.cu:401-403);
@@ -125,16 +154,15 @@ NR_HD void bond_force(double x1, double y1, double x2, double y2, double wW, dou
     /* most bonds cross no boundary: then r = (x1 - x2) - 0 and the force's
      * x2 + 0 - x1 = -(x1 - x2) need no further operation (an exact zero may
      * change its sign, which no sum that starts from +0 shows) */
-    double dx = -rx;
+    double dx = ii_flip(rx, true);
     if (!ii_is_zero(wW)) {
-        rx = rx - wW;
-        dx = (x2 + wW) - x1;
+        rx = wrap_gap(x1, x2, wW);
+        dx = wrap_reach(x1, x2, wW);
     }
     const double inv = inv_sqrt_ieee(fma(rx, rx, ry * ry));
-    double s = fma(-l0, inv, 1.0);
-    if (ii_bits(k) != 0x3ff0000000000000ULL) s = k * s; /* k = 1: the usual stiffness */
+    const double s = k * fma(-l0, inv, 1.0);
     fx = s * dx;
-    fy = s * -ry;
+    fy = s * ii_flip(ry, true);
 }
 
 NR_HD double bond_energy(double x1, double y1, double x2, double y2, double wW, double l0, double k) {
@@ -147,8 +175,8 @@ NR_HD double bond_energy(double x1, double y1, double x2, double y2, double wW, 
 NR_HD double bend_dtheta(double ax, double ay, double bx, double by, double phi0) {
     const double c = fma(ax, by, -(ay * bx));
     const double d = fma(ax, bx, ay * by);
-    const double th = atan2_canon(-c, -d);
-    return ii_is_zero(phi0) ? th : th - phi0; /* th - 0 = th */
+    /* atan2(-c, -d): the signs taken from the bits */
+    return atan2_parts(ii_abs(c), ii_abs(d), ii_positive(c), ii_positive(d)) - phi0;
 }
 
 /* Bending forces on j and k (large_strain_relax.cu:453-459); the hinge
@@ -158,10 +186,10 @@ NR_HD void bend_force(double ax, double ay, double bx, double by, double kb, dou
     const double g = kb * bend_dtheta(ax, ay, bx, by, phi0);
     const double g2 = div_ieee(g, fma(ax, ax, ay * ay));
     const double g3 = div_ieee(g, fma(bx, bx, by * by));
-    fjx = -ay * g2;
+    fjx = ii_flip(ay * g2, true);
     fjy = ax * g2;
     fkx = by * g3;
-    fky = -bx * g3;
+    fky = ii_flip(bx * g3, true);
 }
 
 NR_HD double bend_energy(double ax, double ay, double bx, double by, double kb, double phi0) {
