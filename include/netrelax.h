@@ -560,6 +560,16 @@ int nr_network_plan(nr_network *dnet, int precision, char *buf, size_t cap);
  * the builder's error (NR_ERR_CAPACITY, NR_ERR_INVALID). */
 int nr_tile_layout_check(const nr_host_network *net, int ctas, int target_nodes, long long stats[6]);
 
+/* No reference counterpart; host only: builds the resident FP64 kernel's
+ * layout of this network (triples and gel elements included) for at most
+ * `ctas` CTAs of `smem_limit` bytes of shared memory each and checks every
+ * invariant the kernel relies on (each node owned once, every local
+ * reference, incidence entry, wrap and rest length equal to the network's,
+ * halo nodes published by their owners).  stats[0..5]: tiles, chunks per
+ * unit, largest shared memory (bytes), items over all tiles, halo nodes over
+ * all tiles, violations found.  Returns NR_OK or the builder's error. */
+int nr_res64_layout_check(const nr_host_network *net, int ctas, long long smem_limit, long long stats[6]);
+
 /* No reference counterpart; host only: builds the sub-block layout of the
  * thread-block-cluster kernels for this network and checks it: every node
  * in exactly one gather record of its own sub-block, records ordered by

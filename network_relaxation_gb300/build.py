@@ -34,6 +34,7 @@ CUDA_UNITS = [
     ("fire_dsm.cu", ["--fmad=false"]),
     ("fire_tile.cu", ["--fmad=false"]),
     ("fire_dsm64.cu", ["--fmad=false"]),
+    ("fire_res64.cu", ["--fmad=false"]),
     ("api.cu", []),
     ("tuning.cu", []),
     ("noalloc.cu", ["--fmad=false"]),

@@ -113,6 +113,10 @@ struct DeviceSet {
     char *tile_mem = nullptr;
     int tile_ctas = 0;
     int tile_threads = 512;
+    /* resident FP64 layout of a single network (fire_res64.cu); n_ctas = 0:
+     * none */
+    Res64Dev res{};
+    size_t res_smem = 0;
     ~DeviceSet() {
         if (tile_mem) cudaFree(tile_mem);
         if (arena) cudaFree(arena);
@@ -319,6 +323,61 @@ static int build_tile_set(const nr_host_network &h, const Incidence &inc, const 
     return NR_OK;
 }
 
+/* NR_FP64_KERNEL: res (default), dsm, l2 or grid. */
+enum { kFp64Res, kFp64Dsm, kFp64L2, kFp64Grid };
+static int fp64_kernel_choice() {
+    const char *env = knob("NR_FP64_KERNEL");
+    if (env && strcmp(env, "dsm") == 0) return kFp64Dsm;
+    if (env && strcmp(env, "l2") == 0) return kFp64L2;
+    if (env && strcmp(env, "grid") == 0) return kFp64Grid;
+    return kFp64Res;
+}
+
+/* FP64, one network: networks of at most NR_FP64_CLUSTER_NODES nodes relax
+ * on the on-chip kernels (NR_FP64_KERNEL), larger ones, and those that fit
+ * none, on the cooperative grid kernel.  All give the same bits.  The
+ * resident kernel takes whatever fits the SMs' shared memory (about 130 000
+ * nodes of a p = 0.65 lattice); a cluster of NR_FP64_CLUSTER CTAs (default
+ * 16) has the FP64 pipes of 16 SMs and beats the grid kernel up to
+ * kFp64DsmNodes. */
+constexpr int kFp64DsmNodes = 4096;
+static int fp64_cluster_nodes() {
+    const char *env = knob("NR_FP64_CLUSTER_NODES");
+    return env ? std::max(0, atoi(env)) : 1 << 30;
+}
+
+/* Offsets of the resident FP64 layout in a network's image. */
+struct ResOff {
+    size_t desc, ro, vf[2], part[2], maxp[2], bar;
+};
+
+/* Adds the resident FP64 layout of the (single) network h to the image; false
+ * when it does not fit. */
+static bool add_res_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
+                           bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
+                           const std::vector<int> &partner, Image &img, ResOff &o, Res64Host &L) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (build_res64_layout(h, inc, fcodes, use_bonds, use_triples, eptr, eent, partner, sms, res64_smem_limit(), L) !=
+        NR_OK)
+        return false;
+    if (!res64_fits(L.n_ctas, false, L.max_smem) || (h.n_facets() > 0 && !res64_fits(L.n_ctas, true, L.max_smem)))
+        return false;
+    o.desc = img.put(L.desc.data(), L.desc.size());
+    o.ro = img.put(L.ro.data(), L.ro.size());
+    for (int c = 0; c < 2; ++c) {
+        o.vf[c] = img.add(sizeof(double2) * 2 * (size_t)h.n_points);
+        o.part[c] = img.add(sizeof(double) * 3 * (size_t)L.n_units);
+        o.maxp[c] = img.add(sizeof(unsigned long long) * (size_t)L.n_ctas);
+    }
+    o.bar = img.add(sizeof(unsigned long long));
+    return true;
+}
+
 static int build_set(int n, const nr_host_network *const *nets, const double *ks, const double *kb,
                      const unsigned char *const *fcodes_in, cudaStream_t stream, DeviceSet &S) {
     if (n <= 0) return fail(NR_ERR_INVALID, "network count must be positive");
@@ -355,8 +414,12 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     S.gel.assign(n, NetGel{});
     std::vector<NetOff> off(n);
     const bool want_tile = n == 1 && nets[0]->n_points >= tile_min_nodes();
+    const bool want_res = n == 1 && fp64_kernel_choice() == kFp64Res && nets[0]->n_points <= fp64_cluster_nodes();
     Incidence inc0;
     std::vector<unsigned char> fc0;
+    bool have_res = false;
+    ResOff res_off{};
+    Res64Host res_host;
     for (int i = 0; i < n; ++i) {
         const nr_host_network &h = *nets[i];
         memcpy(img.bytes.data() + x_off + sizeof(double2) * S.node_off[i], h.points.data(),
@@ -403,24 +466,8 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         const int nf = h.n_facets();
         std::vector<int4> elem(nf);
         for (int f = 0; f < nf; ++f) elem[f] = make_int4(h.facets[3 * f], h.facets[3 * f + 1], h.facets[3 * f + 2], 0);
-        std::vector<int> eptr((size_t)h.n_points + 1, 0), eent(3 * (size_t)nf), partner(h.n_points, -1);
-        for (int v : h.facets) eptr[v + 1]++;
-        for (int v = 0; v < h.n_points; ++v) eptr[v + 1] += eptr[v];
-        {
-            std::vector<int> fill(eptr.begin(), eptr.end() - 1);
-            for (int f = 0; f < nf; ++f)
-                for (int r = 0; r < 3; ++r) eent[fill[h.facets[3 * f + r]]++] = 3 * f + r;
-        }
-        bool pairs_ok = true;
-        for (int q = 0; q < h.n_mesh_pairs(); ++q) {
-            const int a = h.mesh_pairs[2 * q], b = h.mesh_pairs[2 * q + 1];
-            if (a == b || partner[a] >= 0 || partner[b] >= 0) {
-                pairs_ok = false;
-                continue;
-            }
-            partner[a] = b;
-            partner[b] = a;
-        }
+        std::vector<int> eptr, eent, partner;
+        const bool pairs_ok = element_incidence(h, eptr, eent, partner);
         S.gel_ok.push_back(pairs_ok);
         S.minx.push_back(h.minx);
         o.elem = img.put(elem.data(), elem.size());
@@ -431,6 +478,9 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         o.eent = img.put(eent.data(), eent.size());
         o.partner = img.put(partner.data(), partner.size());
         build_dsm_layout(h, inc, fc.data(), img, o, S.dsm[i]);
+        if (want_res && i == 0)
+            have_res = add_res_layout(h, inc, fc.data(), ks[i] > 0, kb[i] > 0, eptr, eent, partner, img, res_off,
+                                      res_host);
         if (want_tile && i == 0) {
             inc0 = std::move(inc);
             fc0 = fc;
@@ -549,6 +599,21 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         NR_CUDA_TRY(launch_inv_mats((const double *)S.dev[i].x, (const int *)S.gel[i].elem, 4, S.dev[i].n_elems,
                                     S.gel[i].elem_inv, stream));
     NR_CUDA_TRY(cudaStreamSynchronize(stream));
+    if (have_res) {
+        Res64Dev &r = S.res;
+        r.sub = res_host.sub;
+        r.n_units = res_host.n_units;
+        r.desc = (const Res64Desc *)(base + res_off.desc);
+        r.ro = (const unsigned char *)(base + res_off.ro);
+        for (int c = 0; c < 2; ++c) {
+            r.vf[c] = (double2 *)(base + res_off.vf[c]);
+            r.part[c] = (double *)(base + res_off.part[c]);
+            r.maxp[c] = (unsigned long long *)(base + res_off.maxp[c]);
+        }
+        r.bar = (unsigned long long *)(base + res_off.bar);
+        S.res_smem = res_host.max_smem;
+        r.n_ctas = res_host.n_ctas;
+    }
     if (want_tile) return build_tile_set(*nets[0], inc0, fc0.data(), S, stream);
     return NR_OK;
 }
@@ -625,6 +690,10 @@ struct GridPlan {
     bool dsm64;
     const NetDsm *m_dev;
     int bmax, emax, tmax;
+    /* FP64: the resident kernel */
+    bool res;
+    Res64Dev rd;
+    size_t res_smem;
 };
 
 /* Per-CTA maxima of the FP64 distributed-shared-memory kernel for clusters
@@ -656,30 +725,11 @@ static bool fp64_dsm_plan(const DeviceSet &S, int C, int &bmax, int &emax, int &
     return true;
 }
 
-/* NR_FP64_KERNEL: dsm (default), l2 (k_fire_cluster) or grid. */
-static int fp64_kernel_choice() {
-    const char *env = knob("NR_FP64_KERNEL");
-    if (env && strcmp(env, "l2") == 0) return 1;
-    if (env && strcmp(env, "grid") == 0) return 2;
-    return 0;
-}
-
 /* Mixed precision, one network: up to kMixedCtaNodes nodes the whole
  * relaxation runs in one CTA with u in shared memory (no grid barriers);
  * larger networks use the cooperative kernel over the whole GPU. */
 constexpr int kMixedCtaNodes = 4096;
 
-/* FP64, one network: networks of at most NR_FP64_CLUSTER_NODES nodes
- * (default 16384) relax on one thread-block cluster of NR_FP64_CLUSTER CTAs
- * (default 16; hardware cluster barriers), larger ones on the cooperative
- * grid kernel over the whole GPU.  Both give the same bits.  On small
- * networks the grid kernel's step is bound by the latency of its software
- * grid barriers; beyond about ten thousand nodes the FP64 work of the step
- * needs more than 16 SMs. */
-static int fp64_cluster_nodes() {
-    const char *env = knob("NR_FP64_CLUSTER_NODES");
-    return env ? std::max(0, atoi(env)) : 16384;
-}
 static int fp64_cluster_ctas() {
     const char *env = knob("NR_FP64_CLUSTER");
     const int c = env ? atoi(env) : 16;
@@ -696,6 +746,7 @@ static int grid_plan(const DeviceSet &S, int i, bool mixed, GridPlan &g) {
     g.dsm64 = false;
     g.m_dev = S.dsm_array + i;
     g.bmax = g.emax = g.tmax = 0;
+    g.res = false;
     const int sms = sm_count();
     const char *mk = knob("NR_MIX_KERNEL");
     if (mixed && S.tile_ctas > 0 && !(mk && strcmp(mk, "grid") == 0)) {
@@ -709,10 +760,16 @@ static int grid_plan(const DeviceSet &S, int i, bool mixed, GridPlan &g) {
         if ((size_t)5 * g.blocks > (size_t)4 * g.d.n_tiles * 8) return fail(NR_ERR_CAPACITY, "reduction scratch too small");
     } else {
         const int choice = fp64_kernel_choice();
-        if (g.d.n <= fp64_cluster_nodes() && choice != 2) {
+        const bool on_chip = g.d.n <= fp64_cluster_nodes() && choice != kFp64Grid;
+        if (on_chip && choice == kFp64Res && S.res.n_ctas > 0 && !(g.d.use_gel && g.d.n_elems == 0)) {
+            g.res = true;
+            g.rd = S.res;
+            g.res_smem = S.res_smem;
+            g.blocks = S.res.n_ctas;
+        } else if (on_chip && (choice != kFp64Res || g.d.n <= kFp64DsmNodes)) {
             int c = fp64_cluster_ctas(), active = 0;
             const std::vector<int> one{i};
-            if (choice == 0 && fp64_dsm_plan(S, c, g.bmax, g.emax, g.tmax, &one)) {
+            if (choice != kFp64L2 && fp64_dsm_plan(S, c, g.bmax, g.emax, g.tmax, &one)) {
                 g.dsm64 = true;
             } else {
                 while (c > 1 && (fp64_cluster_max_active(c, g.d.use_gel != 0, &active) != cudaSuccess || active < 1)) {
@@ -745,6 +802,8 @@ static int enqueue_grid(const GridPlan &g, const nr_fire_params &prm, cudaStream
         NR_CUDA_TRY(
             launch_mixed_tile(g.d, g.tl, to_dev(prm), g.blocks, g.tile_threads, barrier_budget_ns(), stream));
     else if (g.mixed) NR_CUDA_TRY(launch_mixed_grid(g.d, to_dev(prm), g.blocks, barrier_budget_ns(), stream));
+    else if (g.res)
+        NR_CUDA_TRY(launch_fp64_res(g.d, g.rd, to_dev(prm), g.res_smem, barrier_budget_ns(), stream));
     else if (g.cluster > 0) {
         /* the cluster kernels take their energies themselves */
         if (g.dsm64)
@@ -1043,7 +1102,7 @@ static int enqueue_set_batch(DeviceSet &S, const nr_fire_params &prm, cudaStream
     } else {
         const int c = fp64_batch_cluster(S.max_nodes);
         int bmax = 0, emax = 0, tmax = 0;
-        if (c > 1 && fp64_kernel_choice() == 0 && fp64_dsm_plan(S, c, bmax, emax, tmax)) {
+        if (c > 1 && fp64_kernel_choice() <= kFp64Dsm && fp64_dsm_plan(S, c, bmax, emax, tmax)) {
             NR_CUDA_TRY(launch_fp64_dsm(S.dev_array, S.dsm_array, S.n_nets, c, bmax, emax, tmax, to_dev(prm), S.queue,
                                         S.order, stream));
         } else if (c > 1) {
@@ -1610,6 +1669,7 @@ int nr_network_plan(nr_network *d, int precision, char *buf, size_t cap) {
             snprintf(out, sizeof out, "k_fire_tile_mixed ctas=%d threads=%d tiles=%d max_tile_nodes=%d", g.blocks,
                      g.tile_threads, g.tl.n_tiles, g.tl.max_nodes);
         else if (g.mixed) snprintf(out, sizeof out, "k_fire_grid_mixed ctas=%d", g.blocks);
+        else if (g.res) snprintf(out, sizeof out, "k_fire_res64 ctas=%d sub=%d smem=%zu", g.blocks, g.rd.sub, g.res_smem);
         else if (g.cluster > 0) snprintf(out, sizeof out, "%s cluster=%d", g.dsm64 ? "k_fire_dsm64" : "k_fire_cluster", g.cluster);
         else snprintf(out, sizeof out, "k_fire_grid ctas=%d sub=%d", g.blocks, g.d.sub);
     }
@@ -1642,7 +1702,7 @@ int nr_batch_plan(nr_batch *b, int precision, char *buf, size_t cap) {
     } else {
         const int c = fp64_batch_cluster(S.max_nodes);
         int bmax = 0, emax = 0, tmax = 0;
-        if (c > 1 && fp64_kernel_choice() == 0 && fp64_dsm_plan(S, c, bmax, emax, tmax))
+        if (c > 1 && fp64_kernel_choice() <= kFp64Dsm && fp64_dsm_plan(S, c, bmax, emax, tmax))
             snprintf(out, sizeof out, "k_fire_dsm64 cluster=%d", c);
         else if (c > 1) snprintf(out, sizeof out, "k_fire_cluster cluster=%d", c);
         else snprintf(out, sizeof out, "k_fire_batch (one CTA per network)");

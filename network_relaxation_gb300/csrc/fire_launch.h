@@ -55,6 +55,24 @@ cudaError_t dsm64_max_active(int cluster, int bmax, int emax, int tmax, int *out
 cudaError_t launch_fp64_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, int cluster, int bmax,
                             int emax, int tmax, const FireParamsDev &p, int *queue_dev, const int *order_dev,
                             cudaStream_t stream);
+/* Host arrays of a Res64 layout (fire_res64.cu) and the resident FP64
+ * kernel: layout (eptr / eent: per-node element entries 3 e + vertex;
+ * partner: duplicate vertex or -1), shared-memory limit, co-residency and
+ * launch.  The same bits as launch_fp64_grid. */
+struct Res64Host {
+    int n_ctas = 0, sub = 1, n_units = 0;
+    size_t max_smem = 0;
+    std::vector<Res64Desc> desc;
+    std::vector<unsigned char> ro;
+};
+struct Incidence;
+int build_res64_layout(const ::nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
+                       bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
+                       const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out);
+size_t res64_smem_limit();
+bool res64_fits(int ctas, bool gel, size_t smem);
+cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
+                            unsigned long long budget_ns, cudaStream_t stream);
 cudaError_t launch_forces(const NetDev &d, cudaStream_t stream);
 cudaError_t launch_affine(double2 *x, int n, double miny, double yrange, double xdisp, double ydisp,
                           cudaStream_t stream);

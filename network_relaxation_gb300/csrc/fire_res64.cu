@@ -1,0 +1,1136 @@
+/*
+ * Plain FP64 FIRE (the run_fire_md arithmetic, bit-identical to the oracle)
+ * of one network held on chip by the whole GPU, with ONE grid barrier per
+ * FIRE step.
+ *
+ * What bounds an FP64 step.  The FP64 pipe issues 1.7 lanes per clock and SM
+ * (a warp instruction every 19 clocks, 64 clocks apart on one scheduler), so
+ * a step costs about 110 FP64 slots per node after ieee_int.h took the
+ * divisions and roots off that pipe; the cooperative grid kernel
+ * (fire_fp64.cu) adds three software grid barriers, a last CTA that reduces
+ * and advances the scalars alone while the others wait, and L2 round trips
+ * for every position, incidence entry and item force.  Here each CTA keeps a
+ * spatial tile of the network in shared memory for the whole relaxation:
+ *   - own nodes' x, v, F, the halo's x, every item (bond, triple, gel
+ *     element) that touches an own node, its topology, its forces;
+ *   - per step only the boundary nodes' {v, F} and the reduction partials
+ *     cross CTAs (through L2);
+ *   - pass A (mixing, drift, half kick) of the halo is recomputed from the
+ *     owner's published v and F with the owner's operations: same bits, no
+ *     barrier between drift and forces; items on a tile boundary are
+ *     evaluated by each tile they touch (7 % more bonds, 13 % more triples on
+ *     32 x 13 node tiles);
+ *   - every CTA combines the partials itself, in the canonical order, and
+ *     advances its own copy of the FIRE scalars: no second barrier.
+ * Tiles are made of whole reduction units (`sub` chunks of 32 consecutive
+ * nodes, 256-node tiles of the canonical sum cut in 8 / sub units), so the
+ * chunk butterflies stay inside a warp.
+ *
+ * FP64 work per step and tile: the three sums of a chunk share one butterfly
+ * (6 additions for 3 x 5: once xor 16 and 8 have left each sum in fewer
+ * lanes, other sums use the free ones), maxima run on the integer pipe, a
+ * triple's hinge force is formed once instead of at each of its three
+ * entries, and the nodes are gathered in the order of their list lengths, one
+ * thread per node and component.
+ *
+ * Measured per FIRE step (us): 1 024 nodes 22.5 (cluster of 16) -> 8.4; 9 991
+ * nodes 40 (grid kernel) -> 10.9; 65 536 nodes 77 -> 23.1, 90 000 nodes 36.7;
+ * Mikado of 50 306 nodes 26; gel of 27 792 nodes 67 -> 27.6.  Of the 23.1 us:
+ * items 10.7, passes over nodes and the gather 7.1, barrier and imbalance 1.7,
+ * totals and scalars 3.9; the FP64 pipe is active for 17.  512 threads: 768
+ * and 1024 measured 3 to 9 % slower.
+ *
+ * Compiled with --fmad=false: the same bits as the oracle.
+ */
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstring>
+#include <thread>
+#include <vector>
+
+#include "fire_common.cuh"
+#include "fire_launch.h"
+#include "nr_internal.h"
+
+namespace nr {
+
+/* ----- device helpers ----- */
+
+/* Butterfly of three values at once: lane 0 gets sum(P), lane 16 sum(V),
+ * lane 8 sum(F), each with the bits of warp_sum (an xor butterfly's lanes all
+ * hold the same commutative sums, so half of them may work for another
+ * value). */
+__device__ __forceinline__ double warp_sum3(double P, double V, double F, int lane) {
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
+    double a = b4 ? V : P;
+    a = a + __shfl_xor_sync(kFull, b4 ? P : V, 16);
+    F = F + __shfl_xor_sync(kFull, F, 16);
+    double c = b3 ? F : a;
+    c = c + __shfl_xor_sync(kFull, b3 ? a : F, 8);
+    c = c + __shfl_xor_sync(kFull, c, 4);
+    c = c + __shfl_xor_sync(kFull, c, 2);
+    return c + __shfl_xor_sync(kFull, c, 1);
+}
+
+/* Largest of the lanes' non-negative doubles, compared as integers (a NaN
+ * counts as 0, as fmax drops it). */
+__device__ __forceinline__ unsigned long long max_bits(double v) {
+    const unsigned long long u = ii_bits(v);
+    return u > 0x7ff0000000000000ULL ? 0ULL : u;
+}
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long u) {
+    const unsigned hi = (unsigned)(u >> 32), mh = __reduce_max_sync(kFull, hi);
+    const unsigned ml = __reduce_max_sync(kFull, hi == mh ? (unsigned)u : 0u);
+    return ((unsigned long long)mh << 32) | ml;
+}
+
+/* Grid barrier number `epoch` of the launch: thread 0 arrives with release
+ * semantics on a monotonic counter and polls it (2.1 us over 152 CTAs
+ * against 2.4 for fence + atomic + volatile poll with naps).  False when the
+ * wait ran out of its budget or another CTA gave up. */
+__device__ __forceinline__ bool res_barrier(unsigned long long *bar, FireState *st, unsigned long long target,
+                                            unsigned long long budget_ns, unsigned site, int *s_ok) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(bar) : "memory");
+        int ok = 1;
+        unsigned spins = 0;
+        unsigned long long t0 = 0, c;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(bar) : "memory");
+            if (c >= target) break;
+            if ((++spins & 63u) != 0) continue;
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (*(volatile unsigned *)&st->abort_flag) {
+                ok = 0;
+                break;
+            }
+            if (now - t0 > budget_ns) {
+                atomicExch(&st->abort_flag, 1u);
+                atomicExch(&st->timeout_site, site);
+                ok = 0;
+                break;
+            }
+        }
+        *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
+/* Tree of the eight lane-group sums w[0..8), of which the first `ng` can be
+ * nonzero (x + 0 = x). */
+__device__ __forceinline__ double tree8_n(const double *w, int ng) {
+    if (ng <= 1) return w[0];
+    if (ng <= 2) return w[0] + w[1];
+    if (ng <= 4) return (w[0] + w[1]) + (w[2] + w[3]);
+    return tree8(w);
+}
+
+static __device__ __noinline__ double res_fmin(double a, double b) { return fmin(a, b); }
+static __device__ __noinline__ double res_half_slow(double v) { return .5 * v; }
+/* v / 2 by the exponent. */
+__device__ __forceinline__ double res_half(double v) {
+    const unsigned e = (unsigned)(ii_bits(v) >> 52) & 0x7ffu;
+    return e - 2u < 2045u ? ii_double(ii_bits(v) - 0x0010000000000000ULL) : res_half_slow(v);
+}
+/* a < b for a >= 0 or NaN. */
+__device__ __forceinline__ bool res_less(double a, double b) {
+    return ii_positive(b) && ii_bits(b) <= 0x7ff0000000000000ULL && ii_abs_bits(a) < ii_bits(b);
+}
+
+/* scal_init / scal_step (fire_common.cuh) by one warp: the lanes of one
+ * instruction stream take the three trees, the three roots and the four
+ * quotients side by side, so the serial chain is a third of one thread's.
+ * tot: [P, V2, F2] x 8 group sums; m2: bits of max|F|^2. */
+__device__ __forceinline__ void scal_warp(Scal &s, const FireParamsDev &p, const double *tot, int ng,
+                                          unsigned long long m2, double sqrt_dof, bool init) {
+    const int lane = threadIdx.x & 31;
+    double t = ii_double(m2);
+    if (lane < 3) t = tree8_n(tot + 8 * lane, ng);
+    const double root = sqrt_ieee(lane == 0 ? 1.0 : t);
+    const double P = __shfl_sync(kFull, t, 0);
+    const double vmag = __shfl_sync(kFull, root, 1), fmag = __shfl_sync(kFull, root, 2),
+                 maxf = __shfl_sync(kFull, root, 3);
+    const double dt_old = s.dt, alpha_old = s.alpha;
+    int since = s.since;
+    /* P > 0: neither sign bit nor zero nor NaN */
+    const unsigned long long pb = ii_bits(P);
+    const bool up = pb != 0ULL && pb <= 0x7ff0000000000000ULL;
+    /* dt finc | dt fdec | alpha falpha on lanes 0 | 1 | 2 */
+    const double pr = (lane == 2 ? alpha_old : dt_old) * (lane == 0 ? p.finc : lane == 1 ? p.fdec : p.falpha);
+    const double grown = __shfl_sync(kFull, pr, 0), shrunk = __shfl_sync(kFull, pr, 1),
+                 cooled = __shfl_sync(kFull, pr, 2);
+    double dt = p.dt_max, alpha = p.alpha0;
+    int zero_v = 0;
+    if (init) {
+        since = 0;
+    } else if (up) {
+        dt = dt_old;
+        alpha = alpha_old;
+        if (++since > p.nmin) {
+            /* fmin of two non-negative numbers by their bits */
+            const unsigned long long gb = ii_bits(grown);
+            dt = gb <= 0x7ff0000000000000ULL ? (gb < ii_bits(p.dt_max) ? grown : p.dt_max) : res_fmin(grown, p.dt_max);
+            alpha = cooled;
+        }
+    } else {
+        since = 0;
+        dt = shrunk;
+        zero_v = 1;
+    }
+    /* alpha |v| on lane 0, dt / 2 on lane 1, dt^2 / 2 on lane 2 (halving is
+     * exact, so the order of the reference's factors does not matter) */
+    const double hdt = res_half(dt);
+    double num = (lane == 0 ? alpha_old : lane == 1 ? 1.0 : hdt) * (lane == 0 ? vmag : lane == 1 ? hdt : dt);
+    double den = p.mass;
+    if (lane == 0) den = init ? 1.0 : fmag;
+    if (lane == 3) {
+        num = fmag;
+        den = sqrt_dof;
+    }
+    const double q = div_ieee(num, den);
+    const double dtm = __shfl_sync(kFull, q, 1), dtsq = __shfl_sync(kFull, q, 2), rms = __shfl_sync(kFull, q, 3);
+    const bool finite = (ii_bits(fmag) & 0x7ff0000000000000ULL) != 0x7ff0000000000000ULL;
+    __syncwarp();
+    if (lane == 0) {
+        s.dt = dt;
+        s.dtm = dtm;
+        s.dtsq = dtsq;
+        s.alpha = alpha;
+        s.since = since;
+        s.fmag = fmag;
+        s.maxf = maxf;
+        s.zero_v = zero_v;
+        s.converged = res_less(p.criterion == 1 ? maxf : rms, p.fcut);
+        if (init) {
+            s.mix_na = 0.0;
+            s.mix_a = 0.0;
+            s.power = 0.0;
+            s.vmag = 0.0;
+            s.mix_pending = 0;
+            s.step = 0;
+            s.status = finite ? 0 : NR_ERR_NONFINITE;
+            s.done = p.max_steps <= 0 || s.status != 0;
+        } else {
+            s.step++;
+            s.power = P;
+            s.vmag = vmag;
+            s.mix_a = q;
+            s.mix_na = -alpha_old;
+            s.mix_pending = 1;
+            if (!finite || (pb & 0x7ff0000000000000ULL) == 0x7ff0000000000000ULL) s.status = NR_ERR_NONFINITE;
+            s.done = s.converged || s.step >= p.max_steps || s.status != 0;
+        }
+    }
+}
+
+/* Pass A of one node (pass_a_node's operations, fire_fp64.cu). */
+__device__ __forceinline__ void res_mix(const Scal &s, double2 &v, const double2 f) {
+    if (s.mix_pending) {
+        v.x = fma(s.mix_na, v.x, v.x);
+        v.y = fma(s.mix_na, v.y, v.y);
+        v.x = fma(s.mix_a, f.x, v.x);
+        v.y = fma(s.mix_a, f.y, v.y);
+        if (s.zero_v) v = make_double2(0.0, 0.0);
+    }
+}
+__device__ __forceinline__ void res_drift(const Scal &s, double2 &x, const double2 v, const double2 f) {
+    x.x = fma(s.dt, v.x, x.x);
+    x.y = fma(s.dt, v.y, x.y);
+    x.x = fma(s.dtsq, f.x, x.x);
+    x.y = fma(s.dtsq, f.y, x.y);
+}
+
+/* Tile sum from its unit partials (tile_from_units with wide loads). */
+__device__ __forceinline__ double res_tile_sum(const double *p, int sub) {
+    if (sub == 8) return __ldcg(p);
+    const double2 *q = reinterpret_cast<const double2 *>(p);
+    const double2 a = __ldcg(q);
+    if (sub == 4) return a.x + a.y;
+    const double2 b = __ldcg(q + 1);
+    if (sub == 2) return (a.x + a.y) + (b.x + b.y);
+    const double2 c = __ldcg(q + 2), e = __ldcg(q + 3);
+    return ((a.x + a.y) + (b.x + b.y)) + ((c.x + c.y) + (e.x + e.y));
+}
+
+constexpr int kResThreads = 512;
+
+/* One tile of the network per CTA (Res64Desc / Res64Segs, nr_device.cuh).
+ * kGel: the network carries a gel; its elements, their reference inverses
+ * and the duplicate vertices join the tile. */
+template <bool kGel>
+__global__ void __launch_bounds__(kResThreads, 1)
+    k_fire_res64(NetDev d, Res64Dev r, FireParamsDev p, unsigned long long budget_ns) {
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    __shared__ Scal s_sc;
+    __shared__ double s_tot[24];
+    __shared__ unsigned long long s_max[kResThreads / 32];
+    __shared__ unsigned long long s_m2;
+    __shared__ int s_ok;
+    const Res64Desc td = r.desc[blockIdx.x];
+    const Res64Segs g = res64_segs(td);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NT = kResThreads, NW = kResThreads / 32;
+    const int sub = r.sub, un = kChunk * sub; /* nodes of a unit */
+    const int no = td.nu * un;                /* own local indices (the last unit may be padded) */
+    /* the tile's record, then the working arrays */
+    {
+        const int4 *src = reinterpret_cast<const int4 *>(r.ro + td.ro_off);
+        int4 *dst = reinterpret_cast<int4 *>(s_raw);
+        for (unsigned k = tid; k < g.rec / 16u; k += NT) dst[k] = __ldg(src + k);
+    }
+    const int *units = reinterpret_cast<const int *>(s_raw + g.units);
+    const int *halo = reinterpret_cast<const int *>(s_raw + g.halo);
+    const double *bl0 = reinterpret_cast<const double *>(s_raw + g.bl0);
+    const double *bk = reinterpret_cast<const double *>(s_raw + g.bk);
+    const unsigned *bref = reinterpret_cast<const unsigned *>(s_raw + g.bref);
+    const signed char *bwrap = reinterpret_cast<const signed char *>(s_raw + g.bwrap);
+    const uint2 *tref = reinterpret_cast<const uint2 *>(s_raw + g.tref);
+    const double *tkb = reinterpret_cast<const double *>(s_raw + g.tkb);
+    const double *tphi = reinterpret_cast<const double *>(s_raw + g.tphi);
+    const uint2 *eref = reinterpret_cast<const uint2 *>(s_raw + g.eref);
+    const int *eid = reinterpret_cast<const int *>(s_raw + g.eid);
+    const uint2 *grec = reinterpret_cast<const uint2 *>(s_raw + g.grec);
+    const unsigned short *inc = reinterpret_cast<const unsigned short *>(s_raw + g.inc);
+    const unsigned short *part = reinterpret_cast<const unsigned short *>(s_raw + g.partner);
+    const unsigned char *pub = s_raw + g.pub;
+    const unsigned short *grp = reinterpret_cast<const unsigned short *>(s_raw + g.grp);
+    double2 *s_x = reinterpret_cast<double2 *>(s_raw + g.x);
+    double2 *s_v = reinterpret_cast<double2 *>(s_raw + g.v);
+    double2 *s_f = reinterpret_cast<double2 *>(s_raw + g.f);   /* own force sums (gel: before the partner's) */
+    double2 *s_ff = kGel ? reinterpret_cast<double2 *>(s_raw + g.ff) : s_f; /* forces */
+    double2 *s_bf = reinterpret_cast<double2 *>(s_raw + g.bf);
+    double2 *s_tf = reinterpret_cast<double2 *>(s_raw + g.tf); /* per triple: hinge, j, k */
+    double *s_M = reinterpret_cast<double *>(s_raw + g.eM);    /* per element: 6 inverse entries, area, - */
+    double *s_du = reinterpret_cast<double *>(s_raw + g.du);   /* per element: dU/dF11, F12, F21, F22 */
+    __syncthreads();
+    auto node_of = [&](int li) { return units[li / un] * un + li % un; };
+    for (int li = tid; li < no; li += NT) {
+        const int i = node_of(li);
+        s_x[li] = i < d.n ? d.x[i] : make_double2(0.0, 0.0);
+        s_v[li] = make_double2(0.0, 0.0);
+        s_ff[li] = make_double2(0.0, 0.0);
+    }
+    for (int h = tid; h < td.nh; h += NT) s_x[no + h] = d.x[halo[h]];
+    const int nel = kGel ? td.nel : 0;
+    if (kGel)
+        for (int e = tid; e < nel; e += NT) {
+            const double *M = d.gel->elem_inv + 6 * (size_t)eid[e];
+            for (int c = 0; c < 6; ++c) s_M[8 * e + c] = M[c];
+            s_M[8 * e + 6] = d.gel->elem_area[eid[e]];
+        }
+    const double W = d.width;
+    const int nb = d.use_bonds ? td.nb : 0, nt = d.use_triples ? td.nt : 0;
+    const int ngrp = (int)res64_groups(td);
+    const int n_units = r.n_units, upt = 8 / sub;
+    const int ng = min(8, (d.n_tiles + 31) / 32); /* lane groups of the canonical sum that hold a tile */
+    unsigned long long epoch = 0;
+    int par = 0;
+    bool init = true;
+    /* v and F of the thread's first halo node, loaded while the totals and
+     * the scalars are computed */
+    double2 hv = make_double2(0.0, 0.0), hf = hv;
+    for (;;) {
+        if (!init) {
+            const Scal &s = s_sc;
+            if (s.done) break;
+            for (int li = tid; li < no; li += NT) {
+                double2 x = s_x[li], v = s_v[li];
+                const double2 f = s_ff[li];
+                res_mix(s, v, f);
+                res_drift(s, x, v, f);
+                s_x[li] = x;
+                v.x = fma(s.dtm, f.x, v.x);
+                v.y = fma(s.dtm, f.y, v.y);
+                s_v[li] = v;
+            }
+            for (int h = tid; h < td.nh; h += NT) {
+                if (h != tid) {
+                    const double2 *q = r.vf[par ^ 1] + 2 * (size_t)halo[h];
+                    hv = __ldcg(q);
+                    hf = __ldcg(q + 1);
+                }
+                double2 x = s_x[no + h];
+                res_mix(s, hv, hf);
+                res_drift(s, x, hv, hf);
+                s_x[no + h] = x;
+            }
+        }
+        __syncthreads();
+        /* items, 32 to a warp */
+        for (int w = warp; w < ngrp; w += NW) {
+            const int code = grp[w], kind = code >> 14, item = 32 * (code & 0x3fff) + lane;
+            if (kGel && kind == 2) {
+                const int e = item;
+                if (e < nel) {
+                    const uint2 q = eref[e];
+                    const double2 p1 = s_x[q.x & 0xffffu], p2 = s_x[q.x >> 16], p3 = s_x[q.y];
+                    const double *M = s_M + 8 * e;
+                    const double f11 = p1.x * M[0] + p2.x * M[2] + p3.x * M[4];
+                    const double f12 = p1.x * M[1] + p2.x * M[3] + p3.x * M[5];
+                    const double f21 = p1.y * M[0] + p2.y * M[2] + p3.y * M[4];
+                    const double f22 = p1.y * M[1] + p2.y * M[3] + p3.y * M[5];
+                    double *du = s_du + 4 * e;
+                    gel_du_of(*d.gel, M[6], f11, f12, f21, f22, du[0], du[1], du[2], du[3]);
+                }
+            } else if (kind == 1) {
+                const int t = item;
+                if (t < nt) {
+                    const uint2 q = tref[t];
+                    const double2 ph = s_x[q.x & 0xffffu], pj = s_x[q.x >> 16], pk = s_x[q.y & 0xffffu];
+                    const int wj = (signed char)(q.y >> 16), wk = (signed char)(q.y >> 24);
+                    const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+                    const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
+                    double fjx, fjy, fkx, fky;
+                    bend_force(ax, ay, bx, by, td.has_kb ? tkb[t] : d.kb, td.has_phi ? tphi[t] : 0.0, fjx, fjy, fkx,
+                               fky);
+                    /* the hinge's (-F_j) - F_k */
+                    s_tf[3 * t] = make_double2(ii_flip(fjx, true) - fkx, ii_flip(fjy, true) - fky);
+                    s_tf[3 * t + 1] = make_double2(fjx, fjy);
+                    s_tf[3 * t + 2] = make_double2(fkx, fky);
+                }
+            } else if (kind == 0) {
+                const int b = item;
+                if (b < nb) {
+                    const unsigned q = bref[b];
+                    const double2 p1 = s_x[q & 0xffffu], p2 = s_x[q >> 16];
+                    double fx, fy;
+                    bond_force(p1.x, p1.y, p2.x, p2.y, wrap_shift(bwrap[b], W), bl0[b], td.has_k ? bk[b] : d.ks, fx,
+                               fy);
+                    s_bf[b] = make_double2(fx, fy);
+                }
+            }
+        }
+        __syncthreads();
+        /* gather in canonical order, one thread per node and component */
+        {
+            const double *bfd = reinterpret_cast<const double *>(s_bf);
+            const double *tfd = reinterpret_cast<const double *>(s_tf);
+            double *fd = reinterpret_cast<double *>(s_f);
+            for (int k = tid; k < 2 * td.ngather; k += NT) {
+                const uint2 q = grec[k >> 1];
+                const int c = k & 1;
+                const unsigned short *e = inc + (q.y & 0xffffu);
+                double f = 0.0;
+                if ((q.y >> (24 + c)) & 1u) {
+                    if (d.use_bonds) {
+                        const int m = (int)((q.x >> 16) & 0xffu);
+#pragma unroll 4
+                        for (int a = 0; a < m; ++a) {
+                            const unsigned code = e[a];
+                            f = f + ii_flip(bfd[(code & ~1u) + c], (code & 1u) != 0);
+                        }
+                        e += m;
+                    }
+                    if (d.use_triples) {
+                        const int m = (int)(q.x >> 24);
+#pragma unroll 4
+                        for (int a = 0; a < m; ++a) f = f + tfd[2 * e[a] + c];
+                        e += m;
+                    }
+                    if (kGel) {
+                        const int m = (int)((q.y >> 16) & 0xffu);
+                        for (int a = 0; a < m; ++a) {
+                            const int el = e[a] / 3, v = e[a] - 3 * el;
+                            const double *M = s_M + 8 * el + 2 * v;
+                            f = f + s_du[4 * el + 2 * c] * M[0];
+                            f = f + s_du[4 * el + 2 * c + 1] * M[1];
+                        }
+                    }
+                }
+                fd[2 * (q.x & 0xffffu) + c] = f;
+            }
+        }
+        __syncthreads();
+        /* half kick, publication, the chunks' partial sums in node order */
+        const double dtm = init ? 0.0 : s_sc.dtm;
+        unsigned long long mx = 0ULL;
+        double2 *vf = r.vf[par];
+        double *pt = r.part[par];
+        for (int u = warp; u < td.nu; u += NW) {
+            const int unit = units[u];
+            double acc = 0.0, acc2 = 0.0, acc4 = 0.0;
+            for (int c = 0; c < sub; ++c) {
+                const int li = u * un + c * kChunk + lane, i = unit * un + c * kChunk + lane;
+                double tP = 0.0, tV = 0.0, tF = 0.0;
+                if (i < d.n) {
+                    double2 f = s_f[li];
+                    if (kGel) {
+                        const unsigned q = part[li];
+                        if (q != 0xffffu) {
+                            const double2 o = s_f[q];
+                            f.x = f.x + o.x;
+                            f.y = f.y + o.y;
+                        }
+                        s_ff[li] = f;
+                    }
+                    double2 v = make_double2(0.0, 0.0);
+                    if (!init) {
+                        v = s_v[li];
+                        v.x = fma(dtm, f.x, v.x);
+                        v.y = fma(dtm, f.y, v.y);
+                        s_v[li] = v;
+                    }
+                    if (pub[li]) {
+                        vf[2 * (size_t)i] = v;
+                        vf[2 * (size_t)i + 1] = f;
+                    }
+                    tP = dot2(v.x, v.y, f.x, f.y);
+                    tV = dot2(v.x, v.y, v.x, v.y);
+                    tF = dot2(f.x, f.y, f.x, f.y);
+                }
+                mx = max(mx, max_bits(tF));
+                const double cs = warp_sum3(tP, tV, tF, lane);
+                /* the lower levels of tree8 over the unit's chunks */
+                if (sub == 1) {
+                    acc4 = cs;
+                } else if ((c & 1) == 0) {
+                    acc = cs;
+                } else {
+                    const double p2 = acc + cs;
+                    if (sub == 2) acc4 = p2;
+                    else if ((c & 2) == 0) acc2 = p2;
+                    else {
+                        const double p4 = acc2 + p2;
+                        if (sub == 4) acc4 = p4;
+                        else if ((c & 4) == 0) acc4 = p4;
+                        else acc4 = acc4 + p4;
+                    }
+                }
+            }
+            if ((lane & 7) == 0 && lane != 24) pt[(size_t)(lane == 0 ? 0 : lane == 16 ? 1 : 2) * n_units + unit] = acc4;
+        }
+        mx = warp_max_bits(mx);
+        if (lane == 0) s_max[warp] = mx;
+        __syncthreads();
+        if (warp == 0) {
+            const unsigned long long m = warp_max_bits(lane < NW ? s_max[lane] : 0ULL);
+            if (lane == 0) r.maxp[par][blockIdx.x] = m;
+        }
+        ++epoch;
+        if (!res_barrier(r.bar, d.st, epoch * (unsigned long long)gridDim.x, budget_ns, 31, &s_ok)) return;
+        if (tid < td.nh) {
+            const double2 *q = vf + 2 * (size_t)halo[tid];
+            hv = __ldcg(q);
+            hf = __ldcg(q + 1);
+        }
+        /* the canonical totals.  Up to four lane groups: a warp each for
+         * every sum (the shortest chain); more: warp k sums the tiles of lane
+         * group k for all three (the fewest FP64 slots) */
+        if (ng <= 4) {
+            if (warp < 3 * ng) {
+                const int q = warp / ng, grp = warp - q * ng, t = 32 * grp + lane;
+                double a = t < d.n_tiles ? res_tile_sum(pt + (size_t)q * n_units + (size_t)t * upt, sub) : 0.0;
+                a = warp_sum(a);
+                if (lane == 0) s_tot[8 * q + grp] = a;
+            } else if (warp == 12) {
+                if (lane < 24 && (lane & 7) >= ng) s_tot[lane] = 0.0;
+            } else if (warp == 13) {
+                unsigned long long m = 0ULL;
+                for (unsigned b = lane; b < gridDim.x; b += 32) m = max(m, __ldcg(r.maxp[par] + b));
+                m = warp_max_bits(m);
+                if (lane == 0) s_m2 = m;
+            }
+        } else if (warp < ng) {
+            const int k = 32 * warp + lane;
+            double a[3] = {0.0, 0.0, 0.0};
+            if (k < d.n_tiles) {
+#pragma unroll
+                for (int q = 0; q < 3; ++q) a[q] = res_tile_sum(pt + (size_t)q * n_units + (size_t)k * upt, sub);
+                for (int t = k + kTile; t < d.n_tiles; t += kTile)
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+                        a[q] = a[q] + res_tile_sum(pt + (size_t)q * n_units + (size_t)t * upt, sub);
+            }
+            const double c = warp_sum3(a[0], a[1], a[2], lane);
+            if ((lane & 7) == 0 && lane != 24) s_tot[8 * (lane == 0 ? 0 : lane == 16 ? 1 : 2) + warp] = c;
+        } else if (warp < 8) {
+            if (lane < 3) s_tot[8 * lane + warp] = 0.0;
+        } else if (warp == 8) {
+            unsigned long long m = 0ULL;
+            for (unsigned b = lane; b < gridDim.x; b += 32) m = max(m, __ldcg(r.maxp[par] + b));
+            m = warp_max_bits(m);
+            if (lane == 0) s_m2 = m;
+        }
+        __syncthreads();
+        if (warp == 0) scal_warp(s_sc, p, s_tot, ng, s_m2, d.sqrt_dof, init);
+        __syncthreads();
+        init = false;
+        par ^= 1;
+    }
+    /* the last pass A only mixes v */
+    for (int li = tid; li < no; li += NT) {
+        const int i = node_of(li);
+        if (i >= d.n) continue;
+        double2 v = s_v[li];
+        const double2 f = s_ff[li];
+        res_mix(s_sc, v, f);
+        d.x[i] = s_x[li];
+        d.v[i] = v;
+        d.f[i] = f;
+    }
+    if (blockIdx.x == 0 && tid == 0) scal_store(d.st, s_sc);
+}
+
+static const void *res_kernel(bool gel) {
+    return gel ? (const void *)k_fire_res64<true> : (const void *)k_fire_res64<false>;
+}
+
+/* Largest dynamic shared memory of the kernel on this device. */
+size_t res64_smem_limit() {
+    int dev = 0, optin = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, res_kernel(true)) != cudaSuccess) return 0;
+    return optin > (int)fa.sharedSizeBytes ? (size_t)(optin - (int)fa.sharedSizeBytes) : 0;
+}
+
+/* Whether `ctas` CTAs of the kernel are co-resident. */
+bool res64_fits(int ctas, bool gel, size_t smem) {
+    int dev = 0, sms = 0, per_sm = 0;
+    const void *k = res_kernel(gel);
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResThreads, smem) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return ctas <= per_sm * sms;
+}
+
+cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
+                            unsigned long long budget_ns, cudaStream_t stream) {
+    const void *k = res_kernel(d.use_gel != 0);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(r.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
+    NetDev dd = d;
+    Res64Dev rr = r;
+    FireParamsDev pp = p;
+    unsigned long long bb = budget_ns;
+    void *args[] = {&dd, &rr, &pp, &bb};
+    return launch_cooperative(k, r.n_ctas, kResThreads, args, smem, stream);
+}
+
+/* ------------------------------------------------------------------ */
+/* Host side: the layout                                                */
+/* ------------------------------------------------------------------ */
+
+namespace {
+
+/* Runs f(k, scratch) for k < n, on a few host threads when `items` items of
+ * work repay their start; every thread has its own Scratch. */
+template <class Scratch, class F>
+void parallel_for(int n, long items, F f) {
+    const int nt = std::max(1, std::min({n, (int)std::thread::hardware_concurrency(), 16, (int)(items / 20000)}));
+    std::atomic<int> next{0};
+    auto work = [&] {
+        Scratch s;
+        for (int k; (k = next.fetch_add(1)) < n;) f(k, s);
+    };
+    std::vector<std::thread> ts;
+    for (int t = 1; t < nt; ++t) ts.emplace_back(work);
+    work();
+    for (auto &t : ts) t.join();
+}
+
+struct NoScratch {};
+/* Local index of every node, slot of every item in the tile at hand (-1). */
+struct TileScratch {
+    std::vector<int> loc, bslot, tslot, eslot;
+};
+
+}  // namespace
+
+/* Tiles of whole reduction units (Res64Host).  Units are dealt to tiles in
+ * strips of y and columns of x; of several unit sizes and column counts the
+ * one whose largest tile takes the fewest FP64 slots is taken: row-ordered
+ * lattices get blocks (256 x 256: 152 tiles of 32 x 13 or 14 nodes that
+ * evaluate 12 % more items than the network has), networks numbered by y
+ * bands.  NR_ERR_CAPACITY when a tile exceeds the 16-bit local encoding or
+ * smem_limit, or when boundary items make the largest tile's work more than
+ * 2.5 times an even share (the numbering then has no locality, and the
+ * kernels that evaluate every item once are faster). */
+int build_res64_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
+                       bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
+                       const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out) {
+    const int n = h.n_points, ne = use_bonds ? h.n_edges() : 0, nt = use_triples ? h.n_triples() : 0;
+    const int nel = h.n_facets();
+    if (n <= 0 || max_ctas < 1) return NR_ERR_INVALID;
+    /* duplicate vertices without elements: the other kernels */
+    if (nel == 0 && h.n_mesh_pairs() > 0) return NR_ERR_CAPACITY;
+    /* about 230 bytes of shared memory a node at the least */
+    if ((size_t)n * 230 > (size_t)max_ctas * smem_limit) return NR_ERR_CAPACITY;
+    /* candidates: units of `sub` chunks dealt to S strips of y, each cut in
+     * c columns of x.  Cuts move by up to a tenth of a strip (column) to the
+     * widest gap nearby, so that strips end between rows and columns between
+     * the chunks of a row. */
+    struct Cand {
+        int sub, c, T;
+        std::vector<int> tile; /* of every unit */
+        double cost;
+    };
+    auto snap = [](auto at, int target, int win, int lo, int hi) {
+        int best = target;
+        double gap = -1.0;
+        for (int k = 0; k <= 2 * win; ++k) {
+            const int i = target + (k & 1 ? (k + 1) / 2 : -(k / 2));
+            if (i <= lo || i >= hi) continue;
+            const double g = at(i) - at(i - 1);
+            if (g > 1.5 * gap + 1e-12) {
+                gap = g;
+                best = i;
+            }
+        }
+        return std::min(std::max(best, lo), hi);
+    };
+    const double W = std::max(h.offset, 1e-300), H = std::max(h.maxy - h.miny, 1e-300);
+    auto units_of = [&](int sub) { return (n + kChunk * sub - 1) / (kChunk * sub); };
+    auto deal = [&](Cand &q, const std::vector<double> &ux, const std::vector<double> &uy, const std::vector<int> &by_y) {
+        const int U = (int)by_y.size(), S = std::max(1, std::min(U, max_ctas / q.c));
+        std::vector<int> idx(by_y);
+        q.tile.assign(U, 0);
+        q.T = 0;
+        for (int st = 0, lo = 0; st < S; ++st) {
+            const int hi = st == S - 1 ? U
+                                       : snap([&](int i) { return uy[idx[i]]; }, (int)((long)U * (st + 1) / S),
+                                              std::max(1, U / S / 10), lo, U);
+            if (q.c > 1)
+                std::stable_sort(idx.begin() + lo, idx.begin() + hi, [&](int a, int b) { return ux[a] < ux[b]; });
+            const int m = hi - lo;
+            for (int k = 0, l = 0; k < q.c; ++k) {
+                const int r = k == q.c - 1 ? m
+                                           : snap([&](int i) { return ux[idx[lo + i]]; }, (int)((long)m * (k + 1) / q.c),
+                                                  std::max(1, m / q.c / 10), l, m);
+                if (r > l) {
+                    for (int i = l; i < r; ++i) q.tile[idx[lo + i]] = q.T;
+                    q.T++;
+                }
+                l = r;
+            }
+            lo = hi;
+        }
+    };
+    /* FP64 slots of the largest tile's step (per warp of items: bonds 8,
+     * triples 33, elements 45; nodes 45 a chunk) and of the totals that every
+     * CTA takes from the unit partials */
+    auto cost = [&](Cand &q) {
+        const int sh = __builtin_ctz((unsigned)(kChunk * q.sub)); /* a power of two */
+        std::vector<int> nb(q.T, 0), nt3(q.T, 0), ne3(q.T, 0), nu(q.T, 0);
+        auto of = [&](int i) { return q.tile[i >> sh]; };
+        for (int b = 0; b < ne; ++b) {
+            const int x = of(h.edge_ij[2 * b]), y = of(h.edge_ij[2 * b + 1]);
+            nb[x]++;
+            if (y != x) nb[y]++;
+        }
+        auto three = [&](const int *v, std::vector<int> &cnt) {
+            const int x = of(v[0]), y = of(v[1]), z = of(v[2]);
+            cnt[x]++;
+            if (y != x) cnt[y]++;
+            if (z != x && z != y) cnt[z]++;
+        };
+        for (int t = 0; t < nt; ++t) three(&h.tri_hjk[3 * t], nt3);
+        for (int e = 0; e < nel; ++e) three(&h.facets[3 * e], ne3);
+        for (int t : q.tile) nu[t]++;
+        double worst = 0.0;
+        for (int t = 0; t < q.T; ++t)
+            worst = std::max(worst, 8 * std::ceil(nb[t] / 32.0) + 33 * std::ceil(nt3[t] / 32.0) +
+                                        45 * std::ceil(ne3[t] / 32.0) + 45.0 * nu[t] * q.sub);
+        q.cost = worst + 3.0 * (8 / q.sub - 1) * ((n + kTile - 1) / kTile) / 32.0;
+    };
+    const long items = (long)ne + nt + nel;
+    std::vector<Cand> cand;
+    std::vector<std::vector<double>> uxs(9), uys(9);
+    std::vector<std::vector<int>> order(9);
+    for (int sub : {1, 2, 4, 8}) {
+        const int U = units_of(sub), un = kChunk * sub;
+        if (sub > 1 && (U < max_ctas || n < 16 * kTile)) break; /* fewer partials only matter when there are many */
+        std::vector<double> &ux = uxs[sub], &uy = uys[sub];
+        ux.assign(U, 0.0);
+        uy.assign(U, 0.0);
+        for (int u = 0; u < U; ++u) {
+            const int i0 = u * un, i1 = std::min(n, i0 + un);
+            for (int i = i0; i < i1; ++i) {
+                ux[u] += h.points[2 * i];
+                uy[u] += h.points[2 * i + 1];
+            }
+            ux[u] /= i1 - i0;
+            uy[u] /= i1 - i0;
+        }
+        std::vector<int> &o = order[sub];
+        o.resize(U);
+        for (int u = 0; u < U; ++u) o[u] = u;
+        std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return uy[a] < uy[b]; });
+        /* columns: bands (c = 1), and around square tiles */
+        const int G = std::min(U, max_ctas), sq = std::max(1, (int)std::lround(std::sqrt(G * W / H)));
+        std::vector<int> cs{1};
+        for (int c : {sq / 3, sq / 2, 2 * sq / 3, 3 * sq / 4, sq}) cs.push_back(std::max(1, std::min(G, c)));
+        std::sort(cs.begin(), cs.end());
+        cs.erase(std::unique(cs.begin(), cs.end()), cs.end());
+        for (int c : cs) cand.push_back(Cand{sub, c, 0, {}, 1e300});
+    }
+    parallel_for<NoScratch>((int)cand.size(), items, [&](int k, NoScratch &) {
+        deal(cand[k], uxs[cand[k].sub], uys[cand[k].sub], order[cand[k].sub]);
+        cost(cand[k]);
+    });
+    const Cand &best = *std::min_element(cand.begin(), cand.end(),
+                                         [](const Cand &a, const Cand &b) { return a.cost < b.cost; });
+    const int sub = best.sub, un = kChunk * sub, U = units_of(sub), T = best.T;
+    const std::vector<int> &tile = best.tile;
+    out = Res64Host();
+    out.sub = sub;
+    out.n_ctas = T;
+    out.n_units = (n + kTile - 1) / kTile * (8 / sub);
+    /* every item once, shared by all SMs, against the largest tile (small
+     * networks are bound by latency and may do more) */
+    if (best.cost > 2.5 * (8.0 * ne + 33.0 * nt + 45.0 * nel + 45.0 * n) / 32.0 / max_ctas + 2000.0)
+        return NR_ERR_CAPACITY;
+    std::vector<std::vector<int>> tu(T);
+    for (int u = 0; u < U; ++u) tu[tile[u]].push_back(u);
+    out.desc.assign(T, Res64Desc{});
+    std::vector<std::vector<unsigned char>> rec(T);
+    std::vector<std::vector<int>> halos(T);
+    std::vector<char> failed(T, 0);
+    const bool has_k = !h.bond_k.empty(), has_kb = !h.tri_kb.empty(), has_phi = !h.tri_phi0.empty();
+    parallel_for<TileScratch>(T, items, [&](int t, TileScratch &sc) {
+        if (sc.loc.empty()) {
+            sc.loc.assign(n, -1);
+            sc.bslot.assign(ne, -1);
+            sc.tslot.assign(nt, -1);
+            sc.eslot.assign(nel, -1);
+        }
+        const std::vector<int> &un_of = tu[t];
+        const int no = (int)un_of.size() * un;
+        /* nodes gathered here: the own ones and other tiles' duplicate
+         * partners of own ones */
+        std::vector<int> gn, ghosts;
+        for (int u : un_of)
+            for (int i = u * un; i < std::min(n, (u + 1) * un); ++i) {
+                gn.push_back(i);
+                if (partner[i] >= 0 && tile[partner[i] / un] != t) ghosts.push_back(partner[i]);
+            }
+        std::sort(ghosts.begin(), ghosts.end());
+        ghosts.erase(std::unique(ghosts.begin(), ghosts.end()), ghosts.end());
+        gn.insert(gn.end(), ghosts.begin(), ghosts.end());
+        std::vector<int> bl, tl, el, hal(ghosts);
+        /* the items of the gathered nodes, each once, in index order */
+        auto add = [](std::vector<int> &list, std::vector<int> &slot, int q) {
+            if (slot[q] < 0) {
+                slot[q] = 0;
+                list.push_back(q);
+            }
+        };
+        for (int i : gn) {
+            if (use_bonds)
+                for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e) add(bl, sc.bslot, inc.bent[e] >> 1);
+            if (use_triples)
+                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e) add(tl, sc.tslot, inc.tent[e] >> 2);
+            for (int e = eptr[i]; e < eptr[i + 1]; ++e) add(el, sc.eslot, eent[e] / 3);
+        }
+        auto number = [](std::vector<int> &list, std::vector<int> &slot) {
+            std::sort(list.begin(), list.end());
+            for (size_t k = 0; k < list.size(); ++k) slot[list[k]] = (int)k;
+        };
+        number(bl, sc.bslot);
+        number(tl, sc.tslot);
+        number(el, sc.eslot);
+        for (size_t u = 0; u < un_of.size(); ++u)
+            for (int i = un_of[u] * un; i < std::min(n, (un_of[u] + 1) * un); ++i)
+                sc.loc[i] = (int)u * un + i % un;
+        for (int i : ghosts) sc.loc[i] = 0;
+        auto touch = [&](int i) {
+            if (sc.loc[i] < 0) {
+                sc.loc[i] = 0;
+                hal.push_back(i);
+            }
+        };
+        for (int b : bl) {
+            touch(h.edge_ij[2 * b]);
+            touch(h.edge_ij[2 * b + 1]);
+        }
+        for (int q : tl)
+            for (int r = 0; r < 3; ++r) touch(h.tri_hjk[3 * q + r]);
+        for (int q : el)
+            for (int r = 0; r < 3; ++r) touch(h.facets[3 * q + r]);
+        std::sort(hal.begin(), hal.end());
+        for (size_t k = 0; k < hal.size(); ++k) sc.loc[hal[k]] = no + (int)k;
+        struct Reset {
+            TileScratch &sc;
+            const std::vector<int> &gn, &hal, &bl, &tl, &el;
+            ~Reset() {
+                for (int i : gn) sc.loc[i] = -1;
+                for (int i : hal) sc.loc[i] = -1;
+                for (int q : bl) sc.bslot[q] = -1;
+                for (int q : tl) sc.tslot[q] = -1;
+                for (int q : el) sc.eslot[q] = -1;
+            }
+        } reset{sc, gn, hal, bl, tl, el};
+        auto local = [&](int i) { return sc.loc[i]; };
+        if (no + hal.size() > 0xffff || bl.size() > 0x7fff || 3 * tl.size() > 0xffff || 3 * el.size() > 0xffff) {
+            failed[t] = 1;
+            return;
+        }
+        /* the longest lists first: the lanes of a warp gather equally many */
+        auto nbe = [&](int i) { return use_bonds ? inc.bptr[i + 1] - inc.bptr[i] : 0; };
+        auto nte = [&](int i) { return use_triples ? inc.tptr[i + 1] - inc.tptr[i] : 0; };
+        auto nee = [&](int i) { return eptr[i + 1] - eptr[i]; };
+        std::stable_sort(gn.begin(), gn.end(), [&](int a, int b) {
+            if (nee(a) != nee(b)) return nee(a) > nee(b);
+            return nte(a) != nte(b) ? nte(a) > nte(b) : nbe(a) > nbe(b);
+        });
+        std::vector<unsigned short> incv;
+        std::vector<uint2> grec;
+        for (int i : gn) {
+            if (nbe(i) > 255 || nte(i) > 255 || nee(i) > 255 || incv.size() > 0xffff) {
+                failed[t] = 1;
+                return;
+            }
+            grec.push_back(make_uint2((unsigned)local(i) | (unsigned)nbe(i) << 16 | (unsigned)nte(i) << 24,
+                                      (unsigned)incv.size() | (unsigned)nee(i) << 16 | (unsigned)(fcodes[i] & 3u) << 24));
+            if (use_bonds)
+                for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e)
+                    incv.push_back((unsigned short)(sc.bslot[inc.bent[e] >> 1] << 1 | (inc.bent[e] & 1)));
+            if (use_triples)
+                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e)
+                    incv.push_back((unsigned short)(3 * sc.tslot[inc.tent[e] >> 2] + (inc.tent[e] & 3)));
+            for (int e = eptr[i]; e < eptr[i + 1]; ++e)
+                incv.push_back((unsigned short)(3 * sc.eslot[eent[e] / 3] + eent[e] % 3));
+        }
+        Res64Desc &td = out.desc[t];
+        td.nu = (int)un_of.size();
+        td.no = no;
+        td.nh = (int)hal.size();
+        td.nb = (int)bl.size();
+        td.nt = (int)tl.size();
+        td.nel = (int)el.size();
+        td.ngather = (int)gn.size();
+        td.ni = (int)incv.size();
+        td.has_k = has_k;
+        td.has_kb = has_kb;
+        td.has_phi = has_phi;
+        td.has_gel = nel > 0;
+        const Res64Segs g = res64_segs(td);
+        if (g.total > smem_limit) {
+            failed[t] = 1;
+            return;
+        }
+        std::vector<unsigned char> &o = rec[t];
+        o.assign(g.rec, 0);
+        auto put = [&](unsigned off, const void *src, size_t bytes) {
+            if (bytes) memcpy(o.data() + off, src, bytes);
+        };
+        put(g.units, un_of.data(), 4 * un_of.size());
+        put(g.halo, hal.data(), 4 * hal.size());
+        for (size_t k = 0; k < bl.size(); ++k) {
+            const int b = bl[k];
+            const unsigned q = (unsigned)local(h.edge_ij[2 * b]) | (unsigned)local(h.edge_ij[2 * b + 1]) << 16;
+            put(g.bref + 4 * k, &q, 4);
+            put(g.bl0 + 8 * k, &h.edge_l0[b], 8);
+            if (has_k) put(g.bk + 8 * k, &h.bond_k[b], 8);
+            o[g.bwrap + k] = (unsigned char)h.edge_wrap[b];
+        }
+        for (size_t k = 0; k < tl.size(); ++k) {
+            const int q = tl[k];
+            const uint2 w = make_uint2((unsigned)local(h.tri_hjk[3 * q]) | (unsigned)local(h.tri_hjk[3 * q + 1]) << 16,
+                                       (unsigned)local(h.tri_hjk[3 * q + 2]) |
+                                           (unsigned)(unsigned char)h.tri_wrap[2 * q] << 16 |
+                                           (unsigned)(unsigned char)h.tri_wrap[2 * q + 1] << 24);
+            put(g.tref + 8 * k, &w, 8);
+            if (has_kb) put(g.tkb + 8 * k, &h.tri_kb[q], 8);
+            if (has_phi) put(g.tphi + 8 * k, &h.tri_phi0[q], 8);
+        }
+        for (size_t k = 0; k < el.size(); ++k) {
+            const int *f = &h.facets[3 * (size_t)el[k]];
+            const uint2 w = make_uint2((unsigned)local(f[0]) | (unsigned)local(f[1]) << 16, (unsigned)local(f[2]));
+            put(g.eref + 8 * k, &w, 8);
+            put(g.eid + 4 * k, &el[k], 4);
+        }
+        put(g.grec, grec.data(), 8 * grec.size());
+        /* groups of 32 items in the order the warps take them: four of one
+         * kind (one for each scheduler), then four of the other, so that a
+         * scheduler's warps are not all in their FP64 or all in their integer
+         * part at once; what is left over last, the short bonds */
+        std::vector<unsigned short> heavy, light, grp;
+        for (int k = 0; k < (td.nel + 31) / 32; ++k) heavy.push_back((unsigned short)(2 << 14 | k));
+        for (int k = 0; k < (td.nt + 31) / 32; ++k) heavy.push_back((unsigned short)(1 << 14 | k));
+        for (int k = 0; k < (td.nb + 31) / 32; ++k) light.push_back((unsigned short)k);
+        for (size_t a = 0, b = 0; a < heavy.size() || b < light.size();) {
+            for (int k = 0; k < 4 && a < heavy.size(); ++k) grp.push_back(heavy[a++]);
+            for (int k = 0; k < 4 && b < light.size(); ++k) grp.push_back(light[b++]);
+        }
+        put(g.grp, grp.data(), 2 * grp.size());
+        put(g.inc, incv.data(), 2 * incv.size());
+        if (td.has_gel)
+            for (int u = 0; u < td.nu; ++u)
+                for (int k = 0; k < un; ++k) {
+                    const int i = un_of[u] * un + k;
+                    const unsigned short q = i < n && partner[i] >= 0 ? (unsigned short)local(partner[i]) : 0xffff;
+                    put(g.partner + 2 * (unsigned)(u * un + k), &q, 2);
+                }
+        halos[t] = hal;
+    });
+    for (char f : failed)
+        if (f) return NR_ERR_CAPACITY;
+    /* own nodes in other tiles' halos are published every step */
+    std::vector<unsigned char> wanted(n, 0);
+    for (const auto &hal : halos)
+        for (int i : hal) wanted[i] = 1;
+    for (int t = 0; t < T; ++t) {
+        const Res64Segs g = res64_segs(out.desc[t]);
+        for (int u = 0; u < out.desc[t].nu; ++u)
+            for (int k = 0; k < un; ++k) {
+                const int i = tu[t][u] * un + k;
+                rec[t][g.pub + (unsigned)(u * un + k)] = i < n ? wanted[i] : 0;
+            }
+        out.desc[t].ro_off = (long long)out.ro.size();
+        out.ro.insert(out.ro.end(), rec[t].begin(), rec[t].end());
+        out.max_smem = std::max(out.max_smem, (size_t)g.total);
+    }
+    return NR_OK;
+}
+
+}  // namespace nr
+
+extern "C" int nr_res64_layout_check(const nr_host_network *h, int ctas, long long smem_limit, long long stats[6]) {
+    using namespace nr;
+    if (!h || !stats || ctas < 1 || smem_limit < 1) return NR_ERR_INVALID;
+    for (int k = 0; k < 6; ++k) stats[k] = 0;
+    const int n = h->n_points;
+    Incidence inc;
+    build_incidence(n, h->edge_ij.data(), h->n_edges(), h->tri_hjk.data(), h->n_triples(), true, true, inc);
+    std::vector<int> eptr, eent, partner;
+    element_incidence(*h, eptr, eent, partner);
+    std::vector<unsigned char> fc(n);
+    nr_host_network_fcodes(h, fc.data());
+    Res64Host L;
+    const int rc = build_res64_layout(*h, inc, fc.data(), true, true, eptr, eent, partner, ctas, (size_t)smem_limit, L);
+    if (rc != NR_OK) return rc;
+    const int un = kChunk * L.sub;
+    long long bad = 0, items = 0, halo = 0;
+    std::vector<int> owned(n, 0), wanted(n, 0), published(n, 0);
+    if (L.n_ctas > ctas || (int)L.desc.size() != L.n_ctas) ++bad;
+    for (const Res64Desc &td : L.desc) {
+        const Res64Segs g = res64_segs(td);
+        if (td.ro_off % 16 || td.ro_off + (long long)g.rec > (long long)L.ro.size() || g.total > (unsigned)smem_limit ||
+            g.total > L.max_smem || td.no != td.nu * un) {
+            ++bad;
+            continue;
+        }
+        const unsigned char *rec = L.ro.data() + td.ro_off;
+        auto at = [&](unsigned off, auto &v) { memcpy(&v, rec + off, sizeof v); };
+        /* node id of a local index, -1 when it is none */
+        auto node = [&](unsigned l) -> int {
+            int id = -1;
+            if (l < (unsigned)td.no) {
+                at(g.units + 4 * (l / un), id);
+                id = id * un + (int)(l % un);
+                return id < n ? id : -1;
+            }
+            if (l < (unsigned)(td.no + td.nh)) at(g.halo + 4 * (l - td.no), id);
+            return id >= 0 && id < n ? id : -1;
+        };
+        for (int l = 0; l < td.no; ++l) {
+            const int i = node(l);
+            if (i < 0) continue;
+            owned[i]++;
+            published[i] = rec[g.pub + l];
+            if (td.has_gel) {
+                unsigned short q;
+                at(g.partner + 2 * l, q);
+                if ((q == 0xffff) != (partner[i] < 0) || (q != 0xffff && node(q) != partner[i])) ++bad;
+            }
+        }
+        for (int k = 0; k < td.nh; ++k) {
+            const int i = node(td.no + k);
+            if (i < 0) ++bad;
+            else wanted[i] = 1;
+        }
+        std::vector<int> bid(td.nb, -1), tid(td.nt, -1), els(td.nel, -1);
+        std::vector<unsigned short> codes(res64_groups(td));
+        for (size_t k = 0; k < codes.size(); ++k) at(g.grp + 2 * (unsigned)k, codes[k]);
+        std::sort(codes.begin(), codes.end());
+        for (size_t k = 0; k < codes.size(); ++k) {
+            const size_t gb = (size_t)(td.nb + 31) / 32, gt = (size_t)(td.nt + 31) / 32;
+            const size_t want = k < gb ? k : k < gb + gt ? (1u << 14 | (k - gb)) : (2u << 14 | (k - gb - gt));
+            bad += codes[k] != want;
+        }
+        for (int k = 0; k < td.nel; ++k) {
+            uint2 w;
+            at(g.eid + 4 * k, els[k]);
+            at(g.eref + 8 * k, w);
+            const int *f = els[k] >= 0 && els[k] < h->n_facets() ? &h->facets[3 * (size_t)els[k]] : nullptr;
+            if (!f || node(w.x & 0xffff) != f[0] || node(w.x >> 16) != f[1] || node(w.y) != f[2]) ++bad;
+        }
+        int gathered = 0;
+        for (int k = 0; k < td.ngather; ++k) {
+            uint2 w;
+            at(g.grec + 8 * k, w);
+            const int i = node(w.x & 0xffff);
+            const int nbn = (w.x >> 16) & 255, ntn = w.x >> 24, nen = (w.y >> 16) & 255, e0 = w.y & 0xffff;
+            if (i < 0 || (w.y >> 24) != (fc[i] & 3u) || e0 + nbn + ntn + nen > td.ni || nbn != inc.bptr[i + 1] - inc.bptr[i] ||
+                ntn != inc.tptr[i + 1] - inc.tptr[i] || nen != eptr[i + 1] - eptr[i]) {
+                ++bad;
+                continue;
+            }
+            gathered += (w.x & 0xffff) < (unsigned)td.no;
+            for (int a = 0; a < nbn + ntn + nen; ++a) {
+                unsigned short c;
+                at(g.inc + 2 * (e0 + a), c);
+                if (a < nbn) {
+                    const int b = inc.bent[inc.bptr[i] + a] >> 1;
+                    unsigned q;
+                    double l0;
+                    if ((c >> 1) >= td.nb || (c & 1) != (inc.bent[inc.bptr[i] + a] & 1)) {
+                        ++bad;
+                        continue;
+                    }
+                    at(g.bref + 4 * (c >> 1), q);
+                    at(g.bl0 + 8 * (c >> 1), l0);
+                    if (node(q & 0xffff) != h->edge_ij[2 * b] || node(q >> 16) != h->edge_ij[2 * b + 1] ||
+                        l0 != h->edge_l0[b] || (signed char)rec[g.bwrap + (c >> 1)] != h->edge_wrap[b])
+                        ++bad;
+                    if (bid[c >> 1] >= 0 && bid[c >> 1] != b) ++bad;
+                    bid[c >> 1] = b;
+                } else if (a < nbn + ntn) {
+                    const int e = inc.tent[inc.tptr[i] + a - nbn], t = e >> 2;
+                    uint2 q;
+                    if (c / 3 >= td.nt || c % 3 != (e & 3)) {
+                        ++bad;
+                        continue;
+                    }
+                    at(g.tref + 8 * (c / 3), q);
+                    if (node(q.x & 0xffff) != h->tri_hjk[3 * t] || node(q.x >> 16) != h->tri_hjk[3 * t + 1] ||
+                        node(q.y & 0xffff) != h->tri_hjk[3 * t + 2] ||
+                        (signed char)(q.y >> 16) != h->tri_wrap[2 * t] || (signed char)(q.y >> 24) != h->tri_wrap[2 * t + 1])
+                        ++bad;
+                    if (tid[c / 3] >= 0 && tid[c / 3] != t) ++bad;
+                    tid[c / 3] = t;
+                } else {
+                    const int e = eent[eptr[i] + a - nbn - ntn];
+                    if (c / 3 >= td.nel || els[c / 3] != e / 3 || c % 3 != e % 3) ++bad;
+                }
+            }
+        }
+        int own_nodes = 0;
+        for (int l = 0; l < td.no; ++l) own_nodes += node(l) >= 0;
+        if (gathered != own_nodes) ++bad;
+        for (int b : bid) bad += b < 0;
+        for (int t : tid) bad += t < 0;
+        items += td.nb + td.nt + td.nel;
+        halo += td.nh;
+    }
+    for (int i = 0; i < n; ++i) bad += owned[i] != 1 || wanted[i] != published[i];
+    stats[0] = L.n_ctas;
+    stats[1] = L.sub;
+    stats[2] = (long long)L.max_smem;
+    stats[3] = items;
+    stats[4] = halo;
+    stats[5] = bad;
+    return NR_OK;
+}

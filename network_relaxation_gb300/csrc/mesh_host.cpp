@@ -40,6 +40,30 @@ struct MeshPointLess {
  * equivalent to an earlier one is not inserted) and pairs every map entry
  * with x < minx + 1e-10, in map order, with the entry found at
  * (x + offset, y). */
+bool element_incidence(const nr_host_network &h, std::vector<int> &eptr, std::vector<int> &eent,
+                       std::vector<int> &partner) {
+    const int n = h.n_points, nf = h.n_facets();
+    eptr.assign((size_t)n + 1, 0);
+    eent.assign(3 * (size_t)nf, 0);
+    partner.assign(n, -1);
+    for (int v : h.facets) eptr[v + 1]++;
+    for (int v = 0; v < n; ++v) eptr[v + 1] += eptr[v];
+    std::vector<int> fill(eptr.begin(), eptr.end() - 1);
+    for (int f = 0; f < nf; ++f)
+        for (int r = 0; r < 3; ++r) eent[fill[h.facets[3 * f + r]]++] = 3 * f + r;
+    bool ok = true;
+    for (int q = 0; q < h.n_mesh_pairs(); ++q) {
+        const int a = h.mesh_pairs[2 * q], b = h.mesh_pairs[2 * q + 1];
+        if (a == b || partner[a] >= 0 || partner[b] >= 0) {
+            ok = false;
+            continue;
+        }
+        partner[a] = b;
+        partner[b] = a;
+    }
+    return ok;
+}
+
 void find_mesh_pairs(const std::vector<double> &points, double offset, double minx, std::vector<int> &pairs) {
     /* The same red-black tree as std::map (hence the same answers on
      * near-duplicates, where PointComp is not a strict order), with its

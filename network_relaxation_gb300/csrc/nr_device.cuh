@@ -237,6 +237,83 @@ struct NetTile {
     unsigned long long *bar;             /* grid barrier counter (monotonic) */
 };
 
+/* Layout of one network for the resident FP64 kernel (fire_res64.cu): one
+ * tile of whole reduction units per CTA, everything the tile needs in shared
+ * memory for the whole relaxation.  Local nodes: own ones (unit slot x unit
+ * size + index; units[] names the units, so own node ids need no list), then
+ * the halo (halo[] = node ids).  The record (segments up to `rec`) is copied
+ * from global memory at the start, the working arrays follow it:
+ *   bref u32    local i | local j << 16     bwrap i8, bl0 f64, bk f64 (if any)
+ *   tref uint2  {local h | local j << 16, local k | wrap j << 16 | wrap k << 24}
+ *   tkb, tphi   f64 (if any)
+ *   eref uint2  {local v1 | v2 << 16, v3}   eid i32 element ids (gel)
+ *   grec uint2  gather records, longest lists first: {local | bonds << 16 |
+ *               triples << 24, first entry | elements << 16 | fcode << 24}
+ *   inc  u16    entries in canonical order: bond slot << 1 | role, 3 x triple
+ *               slot + role, 3 x element slot + vertex
+ *   partner u16 local duplicate vertex of each own node (gel; 0xffff none)
+ *   pub  u8     own nodes that other tiles hold in their halos
+ *   grp  u16    the warps' groups of 32 items, in the order they are taken:
+ *               kind << 14 | group (kinds: 0 bonds, 1 triples, 2 elements) */
+struct Res64Desc {
+    long long ro_off;
+    int nu, no, nh, nb, nt, nel, ngather, ni;
+    int has_k, has_kb, has_phi, has_gel; /* of the network: the same in every tile */
+};
+struct Res64Segs {
+    unsigned units, halo, bl0, bk, tkb, tphi, tref, eref, grec, bref, eid, inc, partner, grp, bwrap, pub, rec;
+    unsigned x, v, f, ff, bf, tf, eM, du, total;
+};
+__host__ __device__ inline unsigned res64_groups(const Res64Desc &t) {
+    return (unsigned)((t.nb + 31) / 32 + (t.nt + 31) / 32 + (t.nel + 31) / 32);
+}
+__host__ __device__ inline Res64Segs res64_segs(const Res64Desc &t) {
+    Res64Segs g;
+    unsigned o = 0;
+    auto seg = [&o](unsigned bytes) {
+        const unsigned at = o;
+        o += tile_pad16(bytes);
+        return at;
+    };
+    g.units = seg(4u * t.nu);
+    g.halo = seg(4u * t.nh);
+    g.bl0 = seg(8u * t.nb);
+    g.bk = seg(t.has_k ? 8u * t.nb : 0u);
+    g.tkb = seg(t.has_kb ? 8u * t.nt : 0u);
+    g.tphi = seg(t.has_phi ? 8u * t.nt : 0u);
+    g.tref = seg(8u * t.nt);
+    g.eref = seg(8u * t.nel);
+    g.grec = seg(8u * t.ngather);
+    g.bref = seg(4u * t.nb);
+    g.eid = seg(4u * t.nel);
+    g.inc = seg(2u * t.ni);
+    g.partner = seg(t.has_gel ? 2u * t.no : 0u);
+    g.grp = seg(2u * res64_groups(t));
+    g.bwrap = seg(1u * t.nb);
+    g.pub = seg(1u * t.no);
+    g.rec = o;
+    const unsigned local = (unsigned)(t.no + t.nh);
+    g.x = seg(16u * local);
+    g.v = seg(16u * t.no);
+    g.f = seg(16u * (t.has_gel ? local : (unsigned)t.no));
+    g.ff = seg(t.has_gel ? 16u * t.no : 0u);
+    g.bf = seg(16u * t.nb);
+    g.tf = seg(48u * t.nt);
+    g.eM = seg(64u * t.nel);
+    g.du = seg(32u * t.nel);
+    g.total = o;
+    return g;
+}
+struct Res64Dev {
+    int n_ctas, sub, n_units;       /* CTAs (tiles); chunks per unit; units, padded to whole 256-node tiles */
+    const Res64Desc *desc;
+    const unsigned char *ro;
+    double2 *vf[2];                 /* published {v, F} per node, by step parity */
+    double *part[2];                /* unit partials of P, |v|^2, |F|^2 (units past the end stay 0) */
+    unsigned long long *maxp[2];    /* per CTA: bits of max |F|^2 */
+    unsigned long long *bar;        /* grid barrier counter (monotonic) */
+};
+
 /* ----- reductions ----- */
 
 __device__ __forceinline__ double warp_sum(double v) {

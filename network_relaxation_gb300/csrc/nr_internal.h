@@ -52,6 +52,12 @@ struct Incidence {
 void build_incidence(int n_points, const int *edge_ij, int n_edges, const int *tri_hjk, int n_triples, bool use_bonds,
                      bool use_triples, Incidence &inc);
 
+/* Per-node gel element entries 3 e + vertex, elements in index order
+ * (eptr[N + 1], eent[3F]), and each node's duplicate partner (-1: none).
+ * False when a vertex is in more than one pair (or paired with itself). */
+bool element_incidence(const nr_host_network &h, std::vector<int> &eptr, std::vector<int> &eent,
+                       std::vector<int> &partner);
+
 /* Min/max y in the reader's convention (min starts at FLT_MAX, max at
  * FLT_MIN). */
 void y_range(const std::vector<double> &points, double &miny, double &maxy);
