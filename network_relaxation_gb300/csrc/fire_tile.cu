@@ -10,10 +10,12 @@
  * barriers.  Here one CTA per SM takes whole tiles (NetTile, nr_device.cuh)
  * and does a tile's whole step on chip:
  *   0. the tile's record (item references, anchor records, incidence,
- *      fcodes, halo list: one contiguous block) arrives in shared memory by
- *      one cp.async.bulk, issued while the previous tile computes (two
- *      stage buffers, an mbarrier each);
- *   1. u, v, F of the own nodes (contiguous in tile order) and of the halo;
+ *      fcodes, halo list: one contiguous block) and its own nodes' state
+ *      (contiguous in tile order) arrive in shared memory by cp.async.bulk,
+ *      issued while the previous tile computes, the first tile's during the
+ *      grid barrier (two stage buffers, an mbarrier each); a CTA with a
+ *      single tile keeps it in shared memory between anchors;
+ *   1. u, v, F of the halo (cp.async once the record's halo list is in);
  *   2. pass A (mixing, drift, half kick) for own AND halo nodes: the halo's
  *      drift is recomputed from the same inputs with the same operations as
  *      its owner's, so it has the same bits and needs no barrier;
@@ -28,6 +30,15 @@
  * the same sum in the same order as in the other mixed kernels.  Anchors
  * (rare) take two more barriers: X += u, then the FP64 force and the tile
  * records' anchor data.
+ *
+ * What bounds a step (65 536 nodes, one tile per SM, 6.4 us): items 1.2 us,
+ * gather 1.4, pass A and halo 0.8, totals and scalars 1.2, barrier 1.7; the
+ * step took 8.3 us when every step loaded the record and the own state again,
+ * the totals' loads came in five dependent rounds, each triple entry of the
+ * gather selected its share, and the item loops ended in nearly empty rounds.
+ * 16 384 nodes 6.7 -> 4.9, 262 144 nodes 19.1 -> 17.1, 1 048 576 nodes 58.2 ->
+ * 56.5 us: there 14 tiles a step pass through the SM, whose warps issue on
+ * 32 % of the cycles and wait mostly at the barriers between the phases.
  *
  * Every wait is bounded: the grid barrier by a %globaltimer budget, the
  * mbarrier waits by the same budget; a wait that runs out sets the
@@ -49,43 +60,50 @@ namespace nr {
 
 /* ----- grid barrier: a monotonic counter, every CTA waits for all ----- */
 
-/* Arrives at barrier number `epoch` (1, 2, ...) of the launch and waits
- * until all G CTAs have; false when the wait exceeded budget_ns or another
- * CTA gave up (st->abort_flag); every thread of the CTA sees the same
- * result. */
-__device__ inline bool tile_barrier(const NetTile &tl, FireState *st, unsigned G, unsigned long long epoch,
-                                    unsigned long long budget_ns, unsigned site) {
-    __shared__ int s_ok;
-    __syncthreads();
+/* Thread 0: arrives at the grid barrier, with release semantics, for a CTA
+ * that has synchronised. */
+__device__ __forceinline__ void tile_arrive(const NetTile &tl) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(tl.bar) : "memory");
+}
+/* Waits until all G CTAs have arrived at barrier number `epoch` (1, 2, ...)
+ * of the launch; false when the wait exceeded budget_ns or another CTA gave
+ * up (st->abort_flag); every thread of the CTA sees the same result. */
+__device__ __forceinline__ bool tile_wait(const NetTile &tl, FireState *st, unsigned G, unsigned long long epoch,
+                                          unsigned long long budget_ns, unsigned site, int *s_ok) {
     if (threadIdx.x == 0) {
         int ok = 1;
-        __threadfence();
-        atomicAdd(tl.bar, 1ULL);
         const unsigned long long target = epoch * (unsigned long long)G;
-        volatile unsigned long long *bar = tl.bar;
-        volatile unsigned *abort_flag = &st->abort_flag;
-        const unsigned long long t0 = global_ns();
+        unsigned long long t0 = 0, c;
         unsigned spins = 0;
-        while (*bar < target) {
-            if (*abort_flag) {
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(tl.bar) : "memory");
+            if (c >= target) break;
+            if ((++spins & 63u) != 0) continue;
+            if (*(volatile unsigned *)&st->abort_flag) {
                 ok = 0;
                 break;
             }
-            if ((++spins & 63u) == 0 && global_ns() - t0 > budget_ns) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > budget_ns) {
                 atomicExch(&st->abort_flag, 1u);
                 atomicExch(&st->timeout_site, site);
                 ok = 0;
                 break;
             }
-            __nanosleep(32);
         }
-        __threadfence();
-        s_ok = ok;
+        *s_ok = ok;
     }
     __syncthreads();
-    const int ok = s_ok;
+    return *s_ok != 0;
+}
+
+/* The CTA's own barrier, then the grid's. */
+__device__ __forceinline__ bool tile_barrier(const NetTile &tl, FireState *st, unsigned G, unsigned long long epoch,
+                                             unsigned long long budget_ns, unsigned site, int *s_ok) {
     __syncthreads();
-    return ok != 0;
+    if (threadIdx.x == 0) tile_arrive(tl);
+    return tile_wait(tl, st, G, epoch, budget_ns, site, s_ok);
 }
 
 /* ----- TMA bulk copy into shared memory, completion on an mbarrier ----- */
@@ -96,12 +114,14 @@ __device__ __forceinline__ void mbar_init(unsigned long long *mbar) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)));
 }
 
-/* One thread: expect `bytes` and copy them from global src to shared dst
- * (both 16-byte aligned, bytes a multiple of 16: the host checks the
- * layout). */
-__device__ __forceinline__ void tma_load(void *dst, const void *src, unsigned bytes, unsigned long long *mbar) {
+/* One thread: announce `bytes` of copies on the mbarrier's current phase. */
+__device__ __forceinline__ void mbar_expect(unsigned long long *mbar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(mbar)), "r"(bytes)
                  : "memory");
+}
+/* One thread: copy `bytes` (announced) from global src to shared dst (both
+ * 16-byte aligned, bytes a multiple of 16: the host checks the layout). */
+__device__ __forceinline__ void tma_copy(void *dst, const void *src, unsigned bytes, unsigned long long *mbar) {
     asm volatile(
         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
         "l"(src), "r"(bytes), "r"(smem_u32(mbar))
@@ -134,11 +154,6 @@ __device__ inline bool mbar_wait(unsigned long long *mbar, unsigned parity, unsi
 __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 /* ----- per-tile pieces ----- */
@@ -163,14 +178,17 @@ __device__ inline TileState tile_state_at(unsigned char *base, int max_nodes, in
     return t;
 }
 
-/* Starts the copies of tile td's own state (state copy `cur`). */
-__device__ __forceinline__ void issue_own(const NetTile &tl, const TileDesc &td, int cur, const TileState &ts) {
-    for (int k = threadIdx.x; k < td.no; k += blockDim.x) {
-        const int p = td.own_pos + k;
-        cp_async16(ts.u + k, tl.u[cur] + p);
-        cp_async16(ts.vf + k, tl.vf[cur] + p);
-        cp_async16(ts.fa + k, tl.fa + p);
-    }
+/* One thread: starts the bulk copies of tile td's record and own state
+ * (state copy `cur`) into a stage buffer and a state buffer.  Own state is
+ * contiguous in tile order; own_pos is a multiple of 16, a node 16 bytes. */
+__device__ __forceinline__ void load_tile(const NetTile &tl, const TileDesc &td, int cur, unsigned char *rec,
+                                          const TileState &ts, unsigned long long *mbar) {
+    const unsigned total = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh).total, own = 16u * (unsigned)td.no;
+    mbar_expect(mbar, total + 3u * own);
+    tma_copy(rec, tl.ro + td.ro_off, total, mbar);
+    tma_copy(ts.u, tl.u[cur] + td.own_pos, own, mbar);
+    tma_copy(ts.vf, tl.vf[cur] + td.own_pos, own, mbar);
+    tma_copy(ts.fa, tl.fa + td.own_pos, own, mbar);
 }
 /* Starts the copies of tile td's halo state (its record already in shared
  * memory). */
@@ -281,8 +299,11 @@ static __device__ __noinline__ void tile_anchor_totals(const NetTile &tl, int G,
  * with two CTAs per SM (smaller tiles; one CTA's barriers overlap the
  * other's work). */
 
-/* Dynamic shared memory of a CTA: two record buffers of max_ro bytes, two
- * node-state buffers, the item results of one tile. */
+/* Dynamic shared memory of a CTA: two record buffers of max_ro bytes and two
+ * node-state buffers.  The tile size is chosen as if the item results had
+ * arrays of their own (16 B a triple, 8 B a bond; they now overwrite the
+ * record), so that the tiles, and with them the order of the sums, stay what
+ * they were. */
 __host__ __device__ inline size_t tile_smem_bytes(unsigned max_ro, int max_nodes, int max_own, int max_bonds,
                                                   int max_tris) {
     return 2 * (size_t)max_ro + 2 * tile_state_bytes(max_nodes, max_own) + 16 * (size_t)max_tris +
@@ -291,13 +312,28 @@ __host__ __device__ inline size_t tile_smem_bytes(unsigned max_ro, int max_nodes
 
 constexpr int kDescCache = 32;
 
+/* A wait that ran out: record the timeout, let every copy in flight land
+ * (bounded waits; n0, n1: loads issued into each buffer that were not waited
+ * for).  Kept out of line: captured by reference, the counters and with them
+ * the buffers' addresses would live in local memory. */
+static __device__ __noinline__ void tile_abort(FireState *st, unsigned long long *mbar, bool n0, unsigned par0, bool n1,
+                                               unsigned par1, unsigned long long budget_ns) {
+    if (threadIdx.x == 0) {
+        atomicExch(&st->abort_flag, 1u);
+        atomicExch(&st->timeout_site, 25u);
+    }
+    cp_async_wait_all();
+    if (n0) mbar_wait(&mbar[0], par0, budget_ns);
+    if (n1) mbar_wait(&mbar[1], par1, budget_ns);
+}
+
 template <int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     k_fire_tile_mixed(NetDev d, NetTile tl, FireParamsDev p, unsigned long long budget_ns) {
     extern __shared__ float4 s_dyn[];
     __shared__ MixShared sh;
     __shared__ __align__(8) unsigned long long s_mbar[2];
-    __shared__ int s_fail;
+    __shared__ int s_fail, s_ok;
     /* FIRE scalars, advanced by thread 0 of every CTA (identical copies) */
     __shared__ MixScal s;
     __shared__ MixParams q;
@@ -309,13 +345,11 @@ __global__ void __launch_bounds__(NT, MINB)
     const size_t sbytes = tile_state_bytes(tl.max_nodes, tl.max_own);
     const TileState ts0 = tile_state_at(dyn + 2 * (size_t)tl.max_ro, tl.max_nodes, tl.max_own);
     const TileState ts1 = tile_state_at(dyn + 2 * (size_t)tl.max_ro + sbytes, tl.max_nodes, tl.max_own);
-    float4 *s_tdf = reinterpret_cast<float4 *>(dyn + 2 * (size_t)tl.max_ro + 2 * sbytes);
-    float2 *s_bdf = reinterpret_cast<float2 *>(s_tdf + tl.max_tris);
     const unsigned G = gridDim.x;
     FireState *st = d.st;
     unsigned long long epoch = 0;
     unsigned uses0 = 0u, uses1 = 0u; /* completed phases of each stage buffer's mbarrier */
-    unsigned iss0 = 0u, iss1 = 0u;   /* record copies issued into each stage buffer */
+    unsigned iss0 = 0u, iss1 = 0u;   /* loads issued into each stage buffer */
     if (threadIdx.x == 0) {
         q = mix_params(p, d.sqrt_dof);
         mbar_init(&s_mbar[0]);
@@ -335,7 +369,7 @@ __global__ void __launch_bounds__(NT, MINB)
         tl.dpart[2 * blockIdx.x] = tF2;
         tl.dpart[2 * blockIdx.x + 1] = tM2;
     }
-    if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 21)) return;
+    if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 21, &s_ok)) return;
     if (threadIdx.x == 0) {
         double F2, M2;
         tile_anchor_totals(tl, G, F2, M2);
@@ -347,7 +381,14 @@ __global__ void __launch_bounds__(NT, MINB)
     const int n_mine = (int)blockIdx.x < tl.n_tiles ? (tl.n_tiles - 1 - (int)blockIdx.x) / (int)G + 1 : 0;
     for (int k = threadIdx.x; k < min(n_mine, kDescCache); k += NT) s_desc[k] = tl.desc[blockIdx.x + k * G];
     __syncthreads();
+    /* the gather's threads: the order of the sums does not depend on NT */
+    constexpr int NG = NT < 512 ? NT : 512;
     auto desc = [&](int k) -> TileDesc { return k < kDescCache ? s_desc[k] : tl.desc[blockIdx.x + k * G]; };
+    /* One tile per CTA: record and own state stay in shared memory between
+     * anchors, a step reads only the halo.  The item results then go to the
+     * second stage buffer; a streamed record is overwritten in place. */
+    const bool resident = tl.n_tiles <= (int)G;
+    bool loaded = false; /* tile 0 is in buffer 0, or its load in flight */
     for (;;) {
         const Coef &c = sh.coef;
         if (c.done) {
@@ -366,97 +407,107 @@ __global__ void __launch_bounds__(NT, MINB)
         }
         const int nxt = cur ^ 1;
         float P = 0.f, V2 = 0.f, Fs = 0.f, M2f = 0.f, A = 0.f;
-        /* the pipeline: the record (TMA) and the node state (cp.async) of
-         * tile k + 1 are in flight while tile k computes */
+        /* the pipeline: the record and own state (TMA) of tile k + 1 are in
+         * flight while tile k computes, its halo state (cp.async) from the
+         * moment the record is in */
         if (n_mine > 0) {
             const TileDesc td0 = desc(0);
-            if (threadIdx.x == 0)
-                tma_load(stage0, tl.ro + td0.ro_off, tile_segs(td0.nb, td0.nt, td0.no, td0.ni, td0.nh).total,
-                         &s_mbar[0]);
-            ++iss0;
-            issue_own(tl, td0, cur, ts0);
-            cp_async_commit();
-            if (mbar_wait(&s_mbar[0], uses0 & 1u, budget_ns)) {
-                ++uses0;
-                issue_halo(tl, td0, stage0, cur, ts0); /* only from a record that arrived */
-            } else {
-                s_fail = 1;
+            if (!loaded) {
+                if (threadIdx.x == 0) {
+                    /* what other CTAs wrote at the anchor and its barrier
+                     * made visible, before bulk copies read it */
+                    asm volatile("fence.proxy.async;" ::: "memory");
+                    load_tile(tl, td0, cur, stage0, ts0, &s_mbar[0]);
+                }
+                ++iss0;
+                loaded = true;
             }
-            cp_async_commit();
+            bool in = true;
+            if (iss0 > uses0) {
+                in = mbar_wait(&s_mbar[0], uses0 & 1u, budget_ns);
+                if (in) ++uses0;
+                else s_fail = 1;
+            }
+            if (in) issue_halo(tl, td0, stage0, cur, ts0); /* only from a record that arrived */
+            if (!resident) loaded = false;
         }
-        /* a wait that ran out: record the timeout, let every copy in flight
-         * land (record copies: bounded waits), leave */
-        auto abort_tiles = [&]() {
-            if (threadIdx.x == 0) {
-                atomicExch(&st->abort_flag, 1u);
-                atomicExch(&st->timeout_site, 25u);
-            }
-            cp_async_wait_all();
-            if (iss0 > uses0) mbar_wait(&s_mbar[0], uses0 & 1u, budget_ns);
-            if (iss1 > uses1) mbar_wait(&s_mbar[1], uses1 & 1u, budget_ns);
-        };
         for (int k = 0; k < n_mine; ++k) {
             const int b = k & 1;
             const TileDesc td = desc(k);
             const bool more = k + 1 < n_mine;
             const TileDesc tn = more ? desc(k + 1) : td;
-            const TileState &sc = b ? ts1 : ts0, &sn = b ? ts0 : ts1;
+            float4 *const sc_u = b ? ts1.u : ts0.u, *const sc_vf = b ? ts1.vf : ts0.vf, *const sc_fa = b ? ts1.fa : ts0.fa;
+            const TileState sn{b ? ts0.u : ts1.u, b ? ts0.vf : ts1.vf, b ? ts0.fa : ts1.fa};
             unsigned char *const rec_n = b ? stage0 : stage1;
-            __syncthreads();
+            cp_async_wait_all(); /* this tile's halo state (its own part: mbarrier) */
+            __syncthreads();     /* and the previous tile's gather is done with the other buffers */
             if (s_fail) {
-                abort_tiles();
+                tile_abort(st, s_mbar, iss0 > uses0, uses0 & 1u, iss1 > uses1, uses1 & 1u, budget_ns);
                 return;
             }
             if (more) {
-                if (threadIdx.x == 0)
-                    tma_load(rec_n, tl.ro + tn.ro_off, tile_segs(tn.nb, tn.nt, tn.no, tn.ni, tn.nh).total,
-                             &s_mbar[b ^ 1]);
+                if (threadIdx.x == 0) load_tile(tl, tn, cur, rec_n, sn, &s_mbar[b ^ 1]);
                 if (b) ++iss0;
                 else ++iss1;
-                issue_own(tl, tn, cur, sn);
             }
-            cp_async_commit();
-            cp_async_wait1(); /* this tile's own and halo state is in */
-            __syncthreads();
             const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
             const int no = td.no, nn = no + td.nh, op = td.own_pos;
-            const unsigned char *rec = b ? stage1 : stage0;
+            unsigned char *const rec = b ? stage1 : stage0;
+            unsigned char *const out = resident ? stage1 : rec;
             /* pass A of own and halo nodes, in place */
             for (int kk = threadIdx.x; kk < nn; kk += NT) {
-                float4 w = sc.u[kk];
-                const float4 q = sc.vf[kk];
+                float4 w = sc_u[kk];
+                const float4 q = sc_vf[kk];
                 float2 v = make_float2(q.x, q.y);
                 tile_pass_a(c, w, v, make_float2(q.z, q.w));
-                sc.u[kk] = w;
-                sc.vf[kk] = make_float4(v.x, v.y, q.z, q.w);
+                sc_u[kk] = w;
+                sc_vf[kk] = make_float4(v.x, v.y, q.z, q.w);
             }
             __syncthreads();
-            /* item pass into shared memory */
-            if (d.use_bonds) {
+            /* item pass: groups of 32 triples, then of 32 bonds, dealt to the
+             * warps in one sequence, so that no warp idles in a last round of
+             * either.  A result replaces the anchor data it came from:
+             *   bond    sk    force change on node i
+             *   triple  arms  {dF_j, dF_k};  pk  the hinge's -(dF_j + dF_k);
+             *           tref  the hinge's sum of |components| (first word)
+             * so that the gather adds what it loads, without a select per
+             * role (30 instructions an entry before). */
+            {
+                const int lane = threadIdx.x & 31, ntg = d.use_triples ? (td.nt + 31) >> 5 : 0,
+                          nbg = d.use_bonds ? (td.nb + 31) >> 5 : 0;
                 const unsigned *bref = reinterpret_cast<const unsigned *>(rec + g.bref);
                 const float4 *mb = reinterpret_cast<const float4 *>(rec + g.mb);
                 const float2 *sk = reinterpret_cast<const float2 *>(rec + g.sk);
-                for (int kk = threadIdx.x; kk < td.nb; kk += NT) {
-                    const unsigned r = bref[kk];
-                    const float4 ui = sc.u[r & 0xffffu], uj = sc.u[r >> 16];
-                    float2 dh, dlo;
-                    u_diff2(make_float2(uj.x, uj.y), make_float2(uj.z, uj.w), make_float2(ui.x, ui.y),
-                            make_float2(ui.z, ui.w), dh, dlo);
-                    s_bdf[kk] = bond_dforce(mb[kk], sk[kk], dh, dlo);
-                }
-            }
-            if (d.use_triples) {
                 const uint2 *tref = reinterpret_cast<const uint2 *>(rec + g.tref);
                 const float4 *arms = reinterpret_cast<const float4 *>(rec + g.arms);
                 const float2 *pk = reinterpret_cast<const float2 *>(rec + g.pk);
-                for (int kk = threadIdx.x; kk < td.nt; kk += NT) {
-                    const uint2 r = tref[kk];
-                    const float4 uh = sc.u[r.x & 0xffffu], uj = sc.u[r.x >> 16], uk = sc.u[r.y];
-                    const float2 hh = make_float2(uh.x, uh.y), hl = make_float2(uh.z, uh.w);
-                    float2 dFj, dFk;
-                    tri_dforce(arms[kk], pk[kk], u_diff(make_float2(uj.x, uj.y), make_float2(uj.z, uj.w), hh, hl),
-                               u_diff(make_float2(uk.x, uk.y), make_float2(uk.z, uk.w), hh, hl), dFj, dFk);
-                    s_tdf[kk] = make_float4(dFj.x, dFj.y, dFk.x, dFk.y);
+                float2 *o_b = reinterpret_cast<float2 *>(out + g.sk);
+                float4 *o_t = reinterpret_cast<float4 *>(out + g.arms);
+                float2 *o_h = reinterpret_cast<float2 *>(out + g.pk);
+                float2 *o_m = reinterpret_cast<float2 *>(out + g.tref);
+                for (int w = threadIdx.x >> 5; w < ntg + nbg; w += NT / 32) {
+                    if (w < ntg) {
+                        const int kk = 32 * w + lane;
+                        if (kk >= td.nt) continue;
+                        const uint2 r = tref[kk];
+                        const float4 uh = sc_u[r.x & 0xffffu], uj = sc_u[r.x >> 16], uk = sc_u[r.y];
+                        const float2 hh = make_float2(uh.x, uh.y), hl = make_float2(uh.z, uh.w);
+                        float2 dFj, dFk;
+                        tri_dforce(arms[kk], pk[kk], u_diff(make_float2(uj.x, uj.y), make_float2(uj.z, uj.w), hh, hl),
+                                   u_diff(make_float2(uk.x, uk.y), make_float2(uk.z, uk.w), hh, hl), dFj, dFk);
+                        o_t[kk] = make_float4(dFj.x, dFj.y, dFk.x, dFk.y);
+                        o_h[kk] = make_float2(-(dFj.x + dFk.x), -(dFj.y + dFk.y));
+                        o_m[kk].x = ((fabsf(dFj.x) + fabsf(dFj.y)) + fabsf(dFk.x)) + fabsf(dFk.y);
+                    } else {
+                        const int kk = 32 * (w - ntg) + lane;
+                        if (kk >= td.nb) continue;
+                        const unsigned r = bref[kk];
+                        const float4 ui = sc_u[r & 0xffffu], uj = sc_u[r >> 16];
+                        float2 dh, dlo;
+                        u_diff2(make_float2(uj.x, uj.y), make_float2(uj.z, uj.w), make_float2(ui.x, ui.y),
+                                make_float2(ui.z, ui.w), dh, dlo);
+                        o_b[kk] = bond_dforce(mb[kk], sk[kk], dh, dlo);
+                    }
                 }
             }
             /* the next tile's record is in by now (bounded wait): start its
@@ -470,10 +521,9 @@ __global__ void __launch_bounds__(NT, MINB)
                     s_fail = 1;
                 }
             }
-            cp_async_commit();
             __syncthreads();
             if (s_fail) {
-                abort_tiles();
+                tile_abort(st, s_mbar, iss0 > uses0, uses0 & 1u, iss1 > uses1, uses1 & 1u, budget_ns);
                 return;
             }
             /* gather of the own nodes, half kick, the next step's state */
@@ -481,37 +531,55 @@ __global__ void __launch_bounds__(NT, MINB)
             const unsigned short *ibe = reinterpret_cast<const unsigned short *>(rec + g.ibe);
             const unsigned short *inc = reinterpret_cast<const unsigned short *>(rec + g.inc);
             const unsigned char *fcode = rec + g.fcode;
-            for (int kk = threadIdx.x; kk < no; kk += NT) {
+            const int to_mag = (int)g.tref - (int)g.pk;
+            for (int kk = threadIdx.x; (int)threadIdx.x < NG && kk < no; kk += NG) {
                 const unsigned fc = fcode[kk];
                 const int e0 = iptr[kk], eb = ibe[kk], e1 = iptr[kk + 1];
-                const float4 fa = sc.fa[kk];
+                const float4 fa = sc_fa[kk];
                 const float2 ah = make_float2(fa.x, fa.y), al = make_float2(fa.z, fa.w);
                 float2 F = make_float2(0.f, 0.f);
                 if (fc != 0) {
                     /* the node's bond entries, then its triple entries (the
-                     * canonical order), each list without a branch per
-                     * entry; own nodes are ordered by list lengths */
+                     * canonical order), four loads at a time; own nodes are
+                     * ordered by list lengths */
                     float2 dF = make_float2(0.f, 0.f);
                     float mag = 0.f;
-#pragma unroll 4
-                    for (int e = e0; e < eb; ++e) {
-                        const unsigned code = inc[e];
-                        float2 df = s_bdf[code >> 1];
-                        df = neg_if(df, code);
-                        dF.x += df.x;
-                        dF.y += df.y;
-                        mag += fabsf(df.x) + fabsf(df.y);
+                    for (int e = e0; e < eb; e += 4) {
+                        float2 df[4];
+                        unsigned code[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, eb - 1)];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) df[j] = *reinterpret_cast<const float2 *>(out + 8u * (code[j] & 0x7fffu));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (e + j < eb) {
+                                df[j] = neg_if(df[j], code[j] >> 15);
+                                dF.x += df[j].x;
+                                dF.y += df[j].y;
+                                mag += fabsf(df[j].x) + fabsf(df[j].y);
+                            }
                     }
-#pragma unroll 4
-                    for (int e = eb; e < e1; ++e) {
-                        const unsigned code = inc[e];
-                        const int role = code & 3;
-                        const float4 qv = s_tdf[(code & 0x7fffu) >> 2];
-                        float gx, gy, mg;
-                        tri_entry(qv, role, gx, gy, mg);
-                        dF.x += gx;
-                        dF.y += gy;
-                        mag += mg;
+                    for (int e = eb; e < e1; e += 4) {
+                        float2 df[4];
+                        float mg[4];
+                        unsigned code[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, e1 - 1)];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const unsigned char *at = out + 8u * (code[j] & 0x7fffu);
+                            df[j] = *reinterpret_cast<const float2 *>(at);
+                            mg[j] = fabsf(df[j].x) + fabsf(df[j].y);
+                            if (code[j] >> 15) mg[j] = *reinterpret_cast<const float *>(at + to_mag);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            if (e + j < e1) {
+                                dF.x += df[j].x;
+                                dF.y += df[j].y;
+                                mag += mg[j];
+                            }
                     }
                     A = fmaxf(A, mag);
                     F.x = ah.x + (al.x + dF.x);
@@ -519,50 +587,80 @@ __global__ void __launch_bounds__(NT, MINB)
                     if (!(fc & 1)) F.x = 0.f;
                     if (!(fc & 2)) F.y = 0.f;
                 }
-                const float4 q = sc.vf[kk];
+                const float4 q = sc_vf[kk];
                 float2 v = make_float2(q.x, q.y);
                 v.x = fmaf(c.dtm, F.x, v.x);
                 v.y = fmaf(c.dtm, F.y, v.y);
-                tl.u[nxt][op + kk] = sc.u[kk];
-                tl.vf[nxt][op + kk] = make_float4(v.x, v.y, F.x, F.y);
+                const float4 vf = make_float4(v.x, v.y, F.x, F.y);
+                tl.u[nxt][op + kk] = sc_u[kk];
+                tl.vf[nxt][op + kk] = vf;
+                if (resident) sc_vf[kk] = vf;
                 P += fmaf(v.x, F.x, v.y * F.y);
                 V2 += fmaf(v.x, v.x, v.y * v.y);
                 const float f2 = fmaf(F.x, F.x, F.y * F.y);
                 Fs += f2;
                 M2f = fmaxf(M2f, f2);
             }
-            /* the next tile's first barrier orders this gather's reads of the
-             * stage and state buffers before they are refilled */
+            /* the shared memory written here, before bulk copies (the async
+             * proxy) overwrite it; the next tile's first barrier orders the
+             * rest */
+            if (!resident) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
-        cp_async_wait_all();
+        /* the next state just written, before bulk copies read it */
+        if (!resident) asm volatile("fence.proxy.async.global;" ::: "memory");
         warp_part(Part{P, V2, Fs, M2f, A}, sh.slots);
         __syncthreads();
         if (threadIdx.x < 32) {
             const Part t = block_totals(sh.slots);
-            if (threadIdx.x == 0) {
+            if (threadIdx.x < 5) {
                 /* two copies by step parity: a CTA that runs ahead into the
                  * next step writes the other copy while the rest still read
                  * this one */
-                float *cp = tl.cpart + 5 * ((size_t)cur * G + blockIdx.x);
-                cp[0] = t.P;
-                cp[1] = t.V2;
-                cp[2] = t.F2;
-                cp[3] = t.M2;
-                cp[4] = t.A;
+                float v = t.P;
+                if (threadIdx.x == 1) v = t.V2;
+                if (threadIdx.x == 2) v = t.F2;
+                if (threadIdx.x == 3) v = t.M2;
+                if (threadIdx.x == 4) v = t.A;
+                tl.cpart[(5 * (size_t)cur + threadIdx.x) * G + blockIdx.x] = v;
             }
         }
-        if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 22)) return;
+        /* the first tile's record and own state (written by this CTA) of the
+         * next step travel during the barrier and the totals */
+        const bool ahead = !resident && n_mine > 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            tile_arrive(tl);
+            if (ahead) load_tile(tl, s_desc[0], nxt, stage0, ts0, &s_mbar[0]);
+        }
+        if (!tile_wait(tl, st, G, ++epoch, budget_ns, 22, &s_ok)) {
+            if (ahead) mbar_wait(&s_mbar[0], uses0 & 1u, budget_ns);
+            return;
+        }
+        if (ahead) {
+            ++iss0;
+            loaded = true;
+        }
         if (threadIdx.x < 32) {
             /* lane l accumulates CTAs l, l + 32, ... in order, then the
-             * butterfly: the same totals in every CTA */
+             * butterfly: the same totals in every CTA.  160 CTAs' loads are
+             * in flight at once (a loop paid an L2 round trip per 32) */
             Part t{0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int kk = threadIdx.x; kk < (int)G; kk += 32) {
-                const float *cp = tl.cpart + 5 * ((size_t)cur * G + kk);
-                t.P += __ldcg(cp);
-                t.V2 += __ldcg(cp + 1);
-                t.F2 += __ldcg(cp + 2);
-                t.M2 = fmaxf(t.M2, __ldcg(cp + 3));
-                t.A = fmaxf(t.A, __ldcg(cp + 4));
+            const float *cp = tl.cpart + 5 * (size_t)cur * G;
+            for (int k0 = threadIdx.x; k0 < (int)G; k0 += 160) {
+                float v[5][5];
+#pragma unroll
+                for (int r = 0; r < 5; ++r)
+#pragma unroll
+                    for (int w = 0; w < 5; ++w) v[r][w] = __ldcg(cp + w * G + min(k0 + 32 * r, (int)G - 1));
+#pragma unroll
+                for (int r = 0; r < 5; ++r)
+                    if (k0 + 32 * r < (int)G) {
+                        t.P += v[r][0];
+                        t.V2 += v[r][1];
+                        t.F2 += v[r][2];
+                        t.M2 = fmaxf(t.M2, v[r][3]);
+                        t.A = fmaxf(t.A, v[r][4]);
+                    }
             }
             t = warp_reduce(t);
             if (threadIdx.x == 0) {
@@ -573,6 +671,16 @@ __global__ void __launch_bounds__(NT, MINB)
         __syncthreads();
         cur = nxt;
         if (sh.coef.anchor) {
+            /* the load under way, or the resident tile, will be stale */
+            if (iss0 > uses0) {
+                if (!mbar_wait(&s_mbar[0], uses0 & 1u, budget_ns)) {
+                    tile_abort(st, s_mbar, iss0 > uses0, uses0 & 1u, iss1 > uses1, uses1 & 1u, budget_ns);
+                    return;
+                }
+                ++uses0;
+            }
+            loaded = false;
+            asm volatile("fence.proxy.async;" ::: "memory"); /* the buffers are loaded again */
             /* X += u (FP64), u = 0, then the FP64 anchor */
             for (int pp = blockIdx.x * NT + threadIdx.x; pp < tl.n_pos; pp += G * NT) {
                 const int i = tl.node_of_pos[pp];
@@ -584,13 +692,13 @@ __global__ void __launch_bounds__(NT, MINB)
                 d.x[i] = x;
                 tl.u[cur][pp] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
-            if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 23)) return;
+            if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 23, &s_ok)) return;
             tile_anchor_eval(d, tl, cur, sh.dslots, tF2, tM2);
             if (threadIdx.x == 0) {
                 tl.dpart[2 * blockIdx.x] = tF2;
                 tl.dpart[2 * blockIdx.x + 1] = tM2;
             }
-            if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 24)) return;
+            if (!tile_barrier(tl, st, G, ++epoch, budget_ns, 24, &s_ok)) return;
             if (threadIdx.x == 0) {
                 double F2, M2;
                 tile_anchor_totals(tl, G, F2, M2);
@@ -764,7 +872,10 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
         }
         for (size_t k = 0; k < bl.size(); ++k) bslot[bl[k]] = (int)k;
         for (size_t k = 0; k < tlist.size(); ++k) tslot[tlist[k]] = (int)k;
-        /* incidence of the own nodes, canonical order: bonds, then triples */
+        /* incidence of the own nodes, canonical order: bonds, then triples;
+         * an entry is where its result will lie in the record (these
+         * segments' offsets do not depend on the incidence) */
+        const TileSegs at = tile_segs((int)bl.size(), (int)tlist.size(), (int)o.size(), 0, 0);
         iptr.clear();
         ibe.clear();
         incv.clear();
@@ -772,11 +883,15 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
             iptr.push_back((unsigned short)incv.size());
             if (use_bonds)
                 for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e)
-                    incv.push_back((unsigned short)((bslot[inc.bent[e] >> 1] << 1) | (inc.bent[e] & 1)));
+                    incv.push_back((unsigned short)(((inc.bent[e] & 1) << 15) | (at.sk / 8 + bslot[inc.bent[e] >> 1])));
             ibe.push_back((unsigned short)incv.size());
             if (use_triples)
                 for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e)
-                    incv.push_back((unsigned short)(0x8000 | (tslot[inc.tent[e] >> 2] << 2) | (inc.tent[e] & 3)));
+{
+                    const int sl = tslot[inc.tent[e] >> 2], role = inc.tent[e] & 3;
+                    incv.push_back((unsigned short)(role == 0 ? 0x8000 | (at.pk / 8 + sl)
+                                                              : at.arms / 8 + 2 * sl + (role == 2)));
+                }
             if (incv.size() > 0xffff) {
                 reset();
                 return NR_ERR_CAPACITY;
@@ -903,10 +1018,12 @@ extern "C" int nr_tile_layout_check(const nr_host_network *h, int ctas, int targ
             for (int x = a; x < e; ++x) {
                 unsigned short c;
                 memcpy(&c, rec + g.inc + 2 * x, 2);
-                const bool tri = (c & 0x8000u) != 0;
-                if (tri != (x >= b)) ++bad;
-                if (!tri && (c >> 1) >= (unsigned)td.nb) ++bad;
-                if (tri && (((c & 0x7fffu) >> 2) >= (unsigned)td.nt || (c & 3u) > 2u)) ++bad;
+                /* where the entry's result lies: sk, pk (hinges) or arms */
+                const unsigned at = c & 0x7fffu, flag = c >> 15;
+                const unsigned lo = x < b ? g.sk / 8 : flag ? g.pk / 8 : g.arms / 8;
+                const unsigned cnt = x < b ? td.nb : flag ? td.nt : 2 * td.nt;
+                if (g.total > 8u * 0x8000u) continue; /* larger than any shared memory: never launched */
+                if (at < lo || at >= lo + cnt) ++bad;
             }
         }
         halo_total += td.nh;

@@ -184,8 +184,10 @@ struct NetDsm {
  *   ibe   no x u16      end of each own node's bond entries (its triple
  *                       entries follow up to the next iptr)
  *   inc   ni x u16      entries in the canonical order (bonds, then
- *                       triples): bond slot << 1 | role, triple 0x8000 |
- *                       slot << 2 | role
+ *                       triples): byte offset / 8 of the item's result in the
+ *                       record (bond: its sk, 0x8000 set for the second node;
+ *                       triple: its arms, first half for j, second for k, or
+ *                       0x8000 | its pk for the hinge)
  *   fcode no x u8
  *   halo  nh x i32      tile-order position of each halo node
  * (local node k < no: own node k; no + h: halo node h).  The anchor records
