@@ -152,6 +152,10 @@ __device__ __forceinline__ T ldro(const T *p) {
     else return __ldg(p);
 }
 
+/* dF + (code's sign bit ? -g : g): the product is exact, so this is the sum. */
+__device__ __forceinline__ float signed_add(float sg, float g, float dF) { return fmaf(sg, g, dF); }
+__device__ __forceinline__ float sign_of(unsigned code) { return (code & 1u) ? -1.0f : 1.0f; }
+
 template <int NT, bool RES>
 __global__ void __launch_bounds__(NT, 1)
     k_fire_dsm_mixed(const NetDev *nets, const NetDsm *dsms, int n_nets, const int *n_dev, FireParamsDev p,
@@ -236,25 +240,57 @@ __global__ void __launch_bounds__(NT, 1)
         const int t0 = m.to[rank * spr], t1 = m.to[(rank + 1) * spr];
         const int eb0 = m.be[rank * spr], eb1 = m.be[(rank + 1) * spr];
         const int et0 = m.te[rank * spr], et1 = m.te[(rank + 1) * spr];
-        if (R) { /* the CTA's read-only slices into shared memory */
+        if (R) /* the CTA's read-only slices into shared memory */
             for (int k = threadIdx.x; k < nloc; k += NT) s_grec[k] = m.grec[n0 + k];
-            for (int k = threadIdx.x; k < eb1 - eb0; k += NT) s_bent[k] = m.bent[eb0 + k];
-            for (int k = threadIdx.x; k < et1 - et0; k += NT) s_tent[k] = m.tent[et0 + k];
-            if (d.use_bonds)
-                for (int k = threadIdx.x; k < b1 - b0; k += NT) s_bref[k] = m.bref[b0 + k];
-            if (d.use_triples)
-                for (int k = threadIdx.x; k < t1 - t0; k += NT) s_tref[k] = m.tref[t0 + k];
+        /* Node references and incidence entries resolved, once per network
+         * and launch, to the shared::cluster addresses of this cluster size:
+         * decoding owner, slot and role of every entry took two thirds of the
+         * gather's instructions.  In the shared copies, else in the network's
+         * scratch of the global-memory and FP64 kernels (same sizes: 8 B a
+         * bond, 16 B a triple, 8 of 16 B, 12 of 32 B).
+         *   bond item    addresses of u_i, u_j
+         *   triple item  addresses of u_h, u_j, u_k
+         *   bond entry   address of the force change | 1 on the second node
+         *   triple entry address of {dF_j, dF_k}, for k of its second half,
+         *                | 1 on the hinge: minus the sum of both halves */
+        uint2 *const xb = R ? reinterpret_cast<uint2 *>(s_bref) : reinterpret_cast<uint2 *>(d.bdf) + b0;
+        int4 *const xt = R ? s_tref : reinterpret_cast<int4 *>(d.tdf) + t0;
+        unsigned *const xbe = R ? reinterpret_cast<unsigned *>(s_bent) : reinterpret_cast<unsigned *>(d.bfrc) + eb0;
+        unsigned *const xte = R ? reinterpret_cast<unsigned *>(s_tent) : reinterpret_cast<unsigned *>(d.tfrc) + et0;
+        if (d.use_bonds) {
+            for (int k = threadIdx.x; k < b1 - b0; k += NT) {
+                const int2 r = __ldg(m.bref + b0 + k);
+                xb[k] = make_uint2(u_addr(s_au, r.x, lg, bsub), u_addr(s_au, r.y, lg, bsub));
+            }
+            for (int k = threadIdx.x; k < eb1 - eb0; k += NT) {
+                const unsigned code = (unsigned)__ldg(m.bent + eb0 + k);
+                const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 1) & 0x7ffffffu) - m.bo[r * spr];
+                xbe[k] = (s_ab[r] + 8u * (unsigned)ls) | (code & 1u);
+            }
+        }
+        if (d.use_triples) {
+            for (int k = threadIdx.x; k < t1 - t0; k += NT) {
+                const int4 r = __ldg(m.tref + t0 + k);
+                xt[k] = make_int4((int)u_addr(s_au, r.x, lg, bsub), (int)u_addr(s_au, r.y, lg, bsub),
+                                  (int)u_addr(s_au, r.z, lg, bsub), r.w);
+            }
+            for (int k = threadIdx.x; k < et1 - et0; k += NT) {
+                const unsigned code = (unsigned)__ldg(m.tent + et0 + k);
+                const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 2) & 0x3ffffffu) - m.to[r * spr];
+                const unsigned role = code & 3u;
+                xte[k] = (s_at[r] + 16u * (unsigned)ls + (role == 2u ? 8u : 0u)) | (role == 0u ? 1u : 0u);
+            }
         }
         /* item and node data for the step loops: shared copies or global */
-        const int2 *Bref = R ? s_bref : m.bref + b0;
+        const uint2 *Bref = xb;
         const float4 *Mb = R ? res.mb : d.mb_data + b0;
         const float2 *Sk = R ? res.sk : d.mb_sk + b0;
-        const int4 *Tref = R ? s_tref : m.tref + t0;
+        const int4 *Tref = xt;
         const float4 *Arms = R ? res.arms : d.mt_arms + t0;
         const float2 *Pk = R ? res.pk : d.mt_pk + t0;
         const int4 *Gr = R ? s_grec : m.grec + n0;
-        const int *Be = R ? s_bent : m.bent + eb0;
-        const int *Te = R ? s_tent : m.tent + et0;
+        const unsigned *Be = xbe;
+        const unsigned *Te = xte;
         const float2 *FaH = R ? res.fahi : d.fa_hi + n0;
         const float2 *FaL = R ? res.falo : d.fa_lo + n0;
         if (threadIdx.x == 0) s_flag = ((volatile FireState *)d.st)->yielded;
@@ -349,18 +385,17 @@ __global__ void __launch_bounds__(NT, 1)
                 const int nb = b1 - b0;
                 int sl = threadIdx.x;
                 if (sl < nb) {
-                    int2 r = ldro<RES>(Bref + sl);
+                    uint2 r = Bref[sl];
                     float4 ra = Mb[sl];
                     float2 sk = Sk[sl];
                     for (;;) {
-                        const float4 ui = dsm_ld4(u_addr(s_au, r.x, lg, bsub));
-                        const float4 uj = dsm_ld4(u_addr(s_au, r.y, lg, bsub));
+                        const float4 ui = dsm_ld4(r.x), uj = dsm_ld4(r.y);
                         const int nx = sl + NT;
-                        int2 rn = r;
+                        uint2 rn = r;
                         float4 ran = ra;
                         float2 skn = sk;
                         if (nx < nb) {
-                            rn = ldro<RES>(Bref + nx);
+                            rn = Bref[nx];
                             ran = Mb[nx];
                             skn = Sk[nx];
                         }
@@ -380,19 +415,18 @@ __global__ void __launch_bounds__(NT, 1)
                 const int nt = t1 - t0;
                 int sl = threadIdx.x;
                 if (sl < nt) {
-                    int4 r = ldro<RES>(Tref + sl);
+                    int4 r = Tref[sl];
                     float4 arms = Arms[sl];
                     float2 pk = Pk[sl];
                     for (;;) {
-                        const float4 uh = dsm_ld4(u_addr(s_au, r.x, lg, bsub));
-                        const float4 uj = dsm_ld4(u_addr(s_au, r.y, lg, bsub));
-                        const float4 uk = dsm_ld4(u_addr(s_au, r.z, lg, bsub));
+                        const float4 uh = dsm_ld4((unsigned)r.x), uj = dsm_ld4((unsigned)r.y),
+                                     uk = dsm_ld4((unsigned)r.z);
                         const int nx = sl + NT;
                         int4 rn = r;
                         float4 armsn = arms;
                         float2 pkn = pk;
                         if (nx < nt) {
-                            rn = ldro<RES>(Tref + nx);
+                            rn = Tref[nx];
                             armsn = Arms[nx];
                             pkn = Pk[nx];
                         }
@@ -433,31 +467,45 @@ __global__ void __launch_bounds__(NT, 1)
                     float2 dF = make_float2(0.f, 0.f);
                     float mag = 0.f;
                     if (d.use_bonds) {
-#pragma unroll 4
-                        for (int e = bq0; e < bq1; ++e) {
-                            const unsigned code = (unsigned)ldro<RES>(Be + e);
-                            const int r = (int)(code >> 28) >> lg;
-                            const int ls = (int)((code >> 1) & 0x7ffffffu) - s_m.bo[r * spr];
-                            float2 df = dsm_ld2(s_ab[r] + 8u * (unsigned)ls);
-                            df = neg_if(df, code);
-                            dF.x += df.x;
-                            dF.y += df.y;
-                            mag += fabsf(df.x) + fabsf(df.y);
+                        for (int e = bq0; e < bq1; e += 4) {
+                            unsigned code[4];
+                            float2 df[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) code[j] = Be[min(e + j, bq1 - 1)];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) df[j] = dsm_ld2(code[j] & ~1u);
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (e + j < bq1) {
+                                    const float sg = sign_of(code[j]);
+                                    dF.x = signed_add(sg, df[j].x, dF.x);
+                                    dF.y = signed_add(sg, df[j].y, dF.y);
+                                    mag += fabsf(df[j].x) + fabsf(df[j].y);
+                                }
                         }
                     }
                     if (d.use_triples) {
-#pragma unroll 4
-                        for (int e = tq0; e < tq1; ++e) {
-                            const unsigned code = (unsigned)ldro<RES>(Te + e);
-                            const int r = (int)(code >> 28) >> lg;
-                            const int role = code & 3;
-                            const int ls = (int)((code >> 2) & 0x3ffffffu) - s_m.to[r * spr];
-                            const float4 qv = dsm_ld4(s_at[r] + 16u * (unsigned)ls);
-                            float gx, gy, mg;
-                            tri_entry(qv, role, gx, gy, mg);
-                            dF.x += gx;
-                            dF.y += gy;
-                            mag += mg;
+                        for (int e = tq0; e < tq1; e += 4) {
+                            unsigned code[4];
+                            float2 df[4], dk[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) code[j] = Te[min(e + j, tq1 - 1)];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                df[j] = dsm_ld2(code[j] & ~1u);
+                                dk[j] = make_float2(0.f, 0.f);
+                                if (code[j] & 1u) dk[j] = dsm_ld2((code[j] & ~1u) + 8u);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (e + j < tq1) {
+                                    /* tri_entry's values: dF_j, dF_k (plus an
+                                     * exact 0) or -(dF_j + dF_k) */
+                                    const float sg = sign_of(code[j]);
+                                    dF.x = signed_add(sg, df[j].x + dk[j].x, dF.x);
+                                    dF.y = signed_add(sg, df[j].y + dk[j].y, dF.y);
+                                    mag += ((fabsf(df[j].x) + fabsf(df[j].y)) + fabsf(dk[j].x)) + fabsf(dk[j].y);
+                                }
                         }
                     }
                     A = fmaxf(A, mag);
