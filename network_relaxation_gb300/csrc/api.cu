@@ -67,7 +67,7 @@ struct Image {
 
 struct NetOff {
     size_t mb_data, mb_sk, bdf, mt_arms, mt_pk, tdf, bfrc, tfrc;
-    size_t dsm_bref, dsm_bidx, dsm_tref, dsm_bent, dsm_tent, dsm_grec;
+    size_t dsm_bref, dsm_bidx, dsm_tref, dsm_bent, dsm_tent, dsm_grec, dsm_xrec, dsm_xent;
     size_t fcode, bond, bond_l0, bond_k, tri, tri_kb, tri_phi0, bptr, bent, tptr, tent, part, epart;
     size_t elem, elem_inv, elem_area, efrc, eptr, eent, partner;
     bool has_bond_k, has_tri_kb, has_tri_phi0;
@@ -145,7 +145,8 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
     auto ref = [&](int v) { return (part(v) << 16) | (v % bsub); };
     std::vector<int2> bref(fits ? ne : 0);
     std::vector<int> bidx(fits ? ne : 0), bslot(fits ? ne : 0), dbent(fits ? inc.bent.size() : 0);
-    std::vector<int4> tref(fits ? nt : 0), grec(fits ? n : 0);
+    std::vector<int4> tref(fits ? nt : 0), grec(fits ? n : 0), xrec(fits ? n : 0);
+    size_t quads = 0;
     std::vector<int> tslot(fits ? nt : 0), dtent(fits ? inc.tent.size() : 0);
     if (fits) {
         int cnt[kDsmParts + 1] = {0};
@@ -202,6 +203,15 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
                 grec[v0 + k] = make_int4(v | ((int)(fcodes[v] & 3u) << 28), inc.bptr[v], nbe(v) | (nte(v) << 16),
                                          inc.tptr[v]);
             }
+            /* bsub is a multiple of 32: the groups of a sub-block are the
+             * groups a warp gathers */
+            for (int k0 = 0; k0 < v1 - v0; k0 += 32) {
+                const int k1 = std::min(v1 - v0, k0 + 32);
+                int nq = 0;
+                for (int k = k0; k < k1; ++k) nq = std::max(nq, (nbe(ord[k]) + nte(ord[k]) + 3) / 4);
+                for (int k = k0; k < k1; ++k) xrec[v0 + k] = make_int4(grec[v0 + k].x, (int)quads, nq, 0);
+                quads += (size_t)32 * nq;
+            }
         }
         m.bsub = bsub;
     }
@@ -211,6 +221,8 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
     o.dsm_bent = img.put(dbent.data(), dbent.size());
     o.dsm_tent = img.put(dtent.data(), dtent.size());
     o.dsm_grec = img.put(grec.data(), grec.size());
+    o.dsm_xrec = img.put(xrec.data(), xrec.size());
+    o.dsm_xent = img.add(sizeof(uint4) * quads);
 }
 
 /* Networks of at least NR_TILE_MIN_NODES nodes (default 131072) relaxed
@@ -588,6 +600,8 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         m.bent = (const int *)(base + o.dsm_bent);
         m.tent = (const int *)(base + o.dsm_tent);
         m.grec = (const int4 *)(base + o.dsm_grec);
+        m.xrec = (const int4 *)(base + o.dsm_xrec);
+        m.xent = (uint4 *)(base + o.dsm_xent);
     }
     S.dsm_array = (NetDsm *)(base + dsm_off);
     memcpy(img.bytes.data() + dsm_off, S.dsm.data(), sizeof(NetDsm) * n);
@@ -2130,6 +2144,8 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
     const int *bent = (const int *)(base + o.dsm_bent);
     const int *tent = (const int *)(base + o.dsm_tent);
     const int4 *grec = (const int4 *)(base + o.dsm_grec);
+    const int4 *xrec = (const int4 *)(base + o.dsm_xrec);
+    const long long xquads = (long long)(img.bytes.size() - o.dsm_xent) / (long long)sizeof(uint4);
     const int bsub = m.bsub;
     long long bad = 0;
     auto ref_of = [&](int v) { return ((v / bsub) << 16) | (v % bsub); };
@@ -2141,6 +2157,12 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
         for (int k = v0; k < v1; ++k) {
             const int4 r = grec[k];
             const int v = r.x & 0x0fffffff, f = (int)((unsigned)r.x >> 28);
+            /* the group's record: the same node, room for its entries, the
+             * same place for all 32 lanes and no other group's */
+            const int4 xr = xrec[k], x0 = xrec[k - (k - v0) % 32];
+            if (xr.x != r.x || xr.y != x0.y || xr.z != x0.z || 4 * xr.z < (r.z & 0xffff) + (int)((unsigned)r.z >> 16) ||
+                xr.y + 32LL * xr.z > xquads || (k > v0 && (k - v0) % 32 == 0 && xr.y < xrec[k - 1].y + 32 * xrec[k - 1].z))
+                ++bad;
             if (v < v0 || v >= v1) {
                 ++bad;
                 continue;

@@ -21,6 +21,15 @@
  * 32 B per owned node + 8 B per owned bond + 16 B per owned triple; the
  * host uses this kernel when the largest network of the batch fits.
  *
+ * What bounds a step (8100 nodes on 4 CTAs, read-only data in global memory;
+ * cycles): items 10 100, gather 10 000 to 13 500, pass A 2 200, three cluster
+ * barriers with the wait for the slowest CTA 8 000, totals and scalars 4 500.
+ * The gather took 16 200 while it decoded every entry and loaded it from L2 as
+ * it went: entries are addresses now, a warp's lie in quads side by side, and
+ * the next quad travels while one is added.  192-network batch of 600 steps:
+ * 47.2 -> 36.8 ms, one network of 2491 nodes on 4 resident CTAs 7.5 -> 6.8 us
+ * per step.
+ *
  * Compiled with --fmad=false; FP32 expressions use explicit fmaf().
  */
 #include "mixed_common.cuh"
@@ -152,9 +161,37 @@ __device__ __forceinline__ T ldro(const T *p) {
     else return __ldg(p);
 }
 
-/* dF + (code's sign bit ? -g : g): the product is exact, so this is the sum. */
-__device__ __forceinline__ float signed_add(float sg, float g, float dF) { return fmaf(sg, g, dF); }
-__device__ __forceinline__ float sign_of(unsigned code) { return (code & 1u) ? -1.0f : 1.0f; }
+/* Four entries of a node's gather: addresses with flags (see the kernel),
+ * their force changes, added in order.  tri_entry's values: dF_j or dF_k
+ * (plus an exact 0), or -(dF_j + dF_k). */
+struct GatherQuad {
+    unsigned c[4];
+    float2 a[4], b[4];
+    __device__ __forceinline__ void load(uint4 code) {
+        c[0] = code.x;
+        c[1] = code.y;
+        c[2] = code.z;
+        c[3] = code.w;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[j] = dsm_ld2(c[j] & ~3u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            b[j] = make_float2(0.f, 0.f);
+            if (c[j] & 2u) b[j] = dsm_ld2((c[j] & ~3u) + 8u);
+        }
+    }
+    /* The first `n` entries; the product with the sign is exact. */
+    __device__ __forceinline__ void add(int n, float2 &dF, float &mag) const {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < n) {
+                const float sg = (c[j] & 1u) ? -1.0f : 1.0f;
+                dF.x = fmaf(sg, a[j].x + b[j].x, dF.x);
+                dF.y = fmaf(sg, a[j].y + b[j].y, dF.y);
+                mag += ((fabsf(a[j].x) + fabsf(a[j].y)) + fabsf(b[j].x)) + fabsf(b[j].y);
+            }
+    }
+};
 
 template <int NT, bool RES>
 __global__ void __launch_bounds__(NT, 1)
@@ -179,12 +216,12 @@ __global__ void __launch_bounds__(NT, 1)
     int4 *s_tref = reinterpret_cast<int4 *>(dyn + L.tref);
     int2 *s_bref = reinterpret_cast<int2 *>(dyn + L.bref);
     int4 *s_grec = reinterpret_cast<int4 *>(dyn + L.grec);
-    int *s_bent = reinterpret_cast<int *>(dyn + L.bent);
-    int *s_tent = reinterpret_cast<int *>(dyn + L.tent);
+    unsigned *s_ent = reinterpret_cast<unsigned *>(dyn + L.bent); /* bond and triple entries: L.tent follows */
     __shared__ MixShared sh;
     __shared__ NetDev s_d;
     __shared__ NetDsm s_m;
     __shared__ int s_slot;
+    __shared__ float4 s_zero; /* what padding entries add */
     /* every CTA's step totals and rank 0's escalation flag, pushed into
      * every CTA of the cluster before the barrier that ends the step: each
      * CTA then reads them from its own shared memory */
@@ -195,6 +232,7 @@ __global__ void __launch_bounds__(NT, 1)
     __shared__ unsigned s_au[kDsmParts], s_ab[kDsmParts], s_at[kDsmParts];
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const int spr = kDsmParts / C, lg = __ffs(spr) - 1; /* sub-blocks per CTA, log2 */
+    if (threadIdx.x == 0) s_zero = make_float4(0.f, 0.f, 0.f, 0.f);
     if ((int)threadIdx.x < C) {
         s_au[threadIdx.x] = dsm_addr(s_u, threadIdx.x);
         s_ab[threadIdx.x] = dsm_addr(s_bdf, threadIdx.x);
@@ -245,40 +283,54 @@ __global__ void __launch_bounds__(NT, 1)
         /* Node references and incidence entries resolved, once per network
          * and launch, to the shared::cluster addresses of this cluster size:
          * decoding owner, slot and role of every entry took two thirds of the
-         * gather's instructions.  In the shared copies, else in the network's
-         * scratch of the global-memory and FP64 kernels (same sizes: 8 B a
-         * bond, 16 B a triple, 8 of 16 B, 12 of 32 B).
+         * gather's instructions.  References go to the shared copies, or to
+         * idle scratch (the force changes of the global-memory kernels: 8 B a
+         * bond, 16 B a triple):
          *   bond item    addresses of u_i, u_j
          *   triple item  addresses of u_h, u_j, u_k
-         *   bond entry   address of the force change | 1 on the second node
-         *   triple entry address of {dF_j, dF_k}, for k of its second half,
-         *                | 1 on the hinge: minus the sum of both halves */
+         * A node's entries, bonds then triples, lie together (shared copies:
+         * by node; else in the quads of NetDsm.xent, padded with s_zero):
+         *   bond    address of the force change | 1 on the second node
+         *   triple  address of {dF_j, dF_k}, for k of its second half, for
+         *           the hinge | 3: minus the sum of both halves */
         uint2 *const xb = R ? reinterpret_cast<uint2 *>(s_bref) : reinterpret_cast<uint2 *>(d.bdf) + b0;
         int4 *const xt = R ? s_tref : reinterpret_cast<int4 *>(d.tdf) + t0;
-        unsigned *const xbe = R ? reinterpret_cast<unsigned *>(s_bent) : reinterpret_cast<unsigned *>(d.bfrc) + eb0;
-        unsigned *const xte = R ? reinterpret_cast<unsigned *>(s_tent) : reinterpret_cast<unsigned *>(d.tfrc) + et0;
-        if (d.use_bonds) {
+        auto bond_entry = [&](int e) -> unsigned {
+            const unsigned code = (unsigned)__ldg(m.bent + e);
+            const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 1) & 0x7ffffffu) - m.bo[r * spr];
+            return (s_ab[r] + 8u * (unsigned)ls) | (code & 1u);
+        };
+        auto triple_entry = [&](int e) -> unsigned {
+            const unsigned code = (unsigned)__ldg(m.tent + e);
+            const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 2) & 0x3ffffffu) - m.to[r * spr];
+            const unsigned role = code & 3u;
+            return (s_at[r] + 16u * (unsigned)ls + (role == 2u ? 8u : 0u)) | (role == 0u ? 3u : 0u);
+        };
+        if (d.use_bonds)
             for (int k = threadIdx.x; k < b1 - b0; k += NT) {
                 const int2 r = __ldg(m.bref + b0 + k);
                 xb[k] = make_uint2(u_addr(s_au, r.x, lg, bsub), u_addr(s_au, r.y, lg, bsub));
             }
-            for (int k = threadIdx.x; k < eb1 - eb0; k += NT) {
-                const unsigned code = (unsigned)__ldg(m.bent + eb0 + k);
-                const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 1) & 0x7ffffffu) - m.bo[r * spr];
-                xbe[k] = (s_ab[r] + 8u * (unsigned)ls) | (code & 1u);
-            }
-        }
-        if (d.use_triples) {
+        if (d.use_triples)
             for (int k = threadIdx.x; k < t1 - t0; k += NT) {
                 const int4 r = __ldg(m.tref + t0 + k);
                 xt[k] = make_int4((int)u_addr(s_au, r.x, lg, bsub), (int)u_addr(s_au, r.y, lg, bsub),
                                   (int)u_addr(s_au, r.z, lg, bsub), r.w);
             }
-            for (int k = threadIdx.x; k < et1 - et0; k += NT) {
-                const unsigned code = (unsigned)__ldg(m.tent + et0 + k);
-                const int r = (int)(code >> 28) >> lg, ls = (int)((code >> 2) & 0x3ffffffu) - m.to[r * spr];
-                const unsigned role = code & 3u;
-                xte[k] = (s_at[r] + 16u * (unsigned)ls + (role == 2u ? 8u : 0u)) | (role == 0u ? 1u : 0u);
+        const unsigned zero_at = dsm_addr(&s_zero, (unsigned)rank);
+        for (int k = threadIdx.x; k < nloc; k += NT) {
+            const int4 g = __ldg(m.grec + n0 + k);
+            const int nb = d.use_bonds ? g.z & 0xffff : 0, nt = d.use_triples ? (int)((unsigned)g.z >> 16) : 0;
+            if (R) {
+                unsigned *const p = s_ent + (g.y - eb0) + (g.w - et0);
+                for (int e = 0; e < nb; ++e) p[e] = bond_entry(g.y + e);
+                for (int e = 0; e < nt; ++e) p[nb + e] = triple_entry(g.w + e);
+            } else {
+                const int4 x = __ldg(m.xrec + n0 + k);
+                unsigned *const p = reinterpret_cast<unsigned *>(m.xent + x.y + (k & 31));
+                for (int e = 0; e < 4 * x.z; ++e)
+                    p[128 * (e >> 2) + (e & 3)] =
+                        e < nb ? bond_entry(g.y + e) : e < nb + nt ? triple_entry(g.w + e - nb) : zero_at;
             }
         }
         /* item and node data for the step loops: shared copies or global */
@@ -288,9 +340,7 @@ __global__ void __launch_bounds__(NT, 1)
         const int4 *Tref = xt;
         const float4 *Arms = R ? res.arms : d.mt_arms + t0;
         const float2 *Pk = R ? res.pk : d.mt_pk + t0;
-        const int4 *Gr = R ? s_grec : m.grec + n0;
-        const unsigned *Be = xbe;
-        const unsigned *Te = xte;
+        const int4 *Gr = R ? s_grec : m.xrec + n0;
         const float2 *FaH = R ? res.fahi : d.fa_hi + n0;
         const float2 *FaL = R ? res.falo : d.fa_lo + n0;
         if (threadIdx.x == 0) s_flag = ((volatile FireState *)d.st)->yielded;
@@ -454,60 +504,47 @@ __global__ void __launch_bounds__(NT, 1)
             int idle = 0;
             if (rank == 0 && threadIdx.x == 0 && yield_at > 0) idle = *(volatile int *)(queue + 1);
             for (int k = threadIdx.x; k < nloc; k += NT) {
-                /* one record load gives the node, its fcode and both entry
-                 * ranges */
+                /* one record load gives the node, its fcode and its entries */
                 const int4 g = ldro<RES>(Gr + k);
                 const int li = (g.x & 0x0fffffff) - n0;
                 const unsigned fc = (unsigned)g.x >> 28;
-                const int bq0 = g.y - eb0, bq1 = bq0 + (g.z & 0xffff);
-                const int tq0 = g.w - et0, tq1 = tq0 + ((unsigned)g.z >> 16);
                 const float2 ah = FaH[li], al = FaL[li];
                 float2 F = make_float2(0.f, 0.f);
+                float2 dF = make_float2(0.f, 0.f);
+                float mag = 0.f;
+                if constexpr (RES) {
+                    /* the entries' loads one quad ahead of their sums */
+                    const int cnt = (d.use_bonds ? g.z & 0xffff : 0) + (d.use_triples ? (int)((unsigned)g.z >> 16) : 0);
+                    const unsigned *const p = s_ent + (g.y - eb0) + (g.w - et0);
+                    if (fc != 0 && cnt > 0) {
+                        GatherQuad q, qn;
+                        q.load(make_uint4(p[0], p[min(1, cnt - 1)], p[min(2, cnt - 1)], p[min(3, cnt - 1)]));
+                        for (int e = 0;;) {
+                            const int en = e + 4;
+                            if (en < cnt)
+                                qn.load(make_uint4(p[en], p[min(en + 1, cnt - 1)], p[min(en + 2, cnt - 1)],
+                                                   p[min(en + 3, cnt - 1)]));
+                            q.add(cnt - e, dF, mag);
+                            if (en >= cnt) break;
+                            e = en;
+                            q = qn;
+                        }
+                    }
+                } else {
+                    /* quads of the whole group, the next one's addresses on
+                     * their way from L2 while this one is added; padding
+                     * entries add 0 */
+                    const uint4 *const p = m.xent + g.y + (k & 31);
+                    uint4 code = g.z > 0 ? p[0] : make_uint4(zero_at, zero_at, zero_at, zero_at);
+                    for (int i = 0; i < g.z; ++i) {
+                        const uint4 next = p[32 * min(i + 1, g.z - 1)];
+                        GatherQuad q;
+                        q.load(code);
+                        q.add(4, dF, mag);
+                        code = next;
+                    }
+                }
                 if (fc != 0) {
-                    float2 dF = make_float2(0.f, 0.f);
-                    float mag = 0.f;
-                    if (d.use_bonds) {
-                        for (int e = bq0; e < bq1; e += 4) {
-                            unsigned code[4];
-                            float2 df[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) code[j] = Be[min(e + j, bq1 - 1)];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) df[j] = dsm_ld2(code[j] & ~1u);
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                if (e + j < bq1) {
-                                    const float sg = sign_of(code[j]);
-                                    dF.x = signed_add(sg, df[j].x, dF.x);
-                                    dF.y = signed_add(sg, df[j].y, dF.y);
-                                    mag += fabsf(df[j].x) + fabsf(df[j].y);
-                                }
-                        }
-                    }
-                    if (d.use_triples) {
-                        for (int e = tq0; e < tq1; e += 4) {
-                            unsigned code[4];
-                            float2 df[4], dk[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) code[j] = Te[min(e + j, tq1 - 1)];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                df[j] = dsm_ld2(code[j] & ~1u);
-                                dk[j] = make_float2(0.f, 0.f);
-                                if (code[j] & 1u) dk[j] = dsm_ld2((code[j] & ~1u) + 8u);
-                            }
-#pragma unroll
-                            for (int j = 0; j < 4; ++j)
-                                if (e + j < tq1) {
-                                    /* tri_entry's values: dF_j, dF_k (plus an
-                                     * exact 0) or -(dF_j + dF_k) */
-                                    const float sg = sign_of(code[j]);
-                                    dF.x = signed_add(sg, df[j].x + dk[j].x, dF.x);
-                                    dF.y = signed_add(sg, df[j].y + dk[j].y, dF.y);
-                                    mag += ((fabsf(df[j].x) + fabsf(df[j].y)) + fabsf(dk[j].x)) + fabsf(dk[j].y);
-                                }
-                        }
-                    }
                     A = fmaxf(A, mag);
                     F.x = ah.x + (al.x + dF.x);
                     F.y = ah.y + (al.y + dF.y);
@@ -604,7 +641,7 @@ __global__ void __launch_bounds__(NT, 1)
         }
         cl.sync();
         if (rank == 0) {
-            mixed_energies(d, sh.red);
+            mixed_energies(d, sh.dslots);
             if (threadIdx.x == 0) {
                 mix_report(d.st, s);
                 d.st->yielded = 0;
@@ -619,14 +656,18 @@ size_t dsm_smem_bytes(int bmax, int emax, int tmax, int ebmax, int etmax, int re
     return dsm_layout(DsmSizes{bmax, emax, tmax, ebmax, etmax, resident}).total;
 }
 
+constexpr int kDsmStatic = 3024;
 /* Largest dynamic shared memory the kernel may use on this device. */
 size_t dsm_smem_limit() {
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    /* (at least kDsmStatic of it static: the plans, and with them the order
+     * of the sums, do not move with the kernel's static arrays) */
     cudaFuncAttributes fa;
     if (cudaFuncGetAttributes(&fa, (const void *)k_fire_dsm_mixed<512, true>) != cudaSuccess) return 0;
-    return optin > (int)fa.sharedSizeBytes ? (size_t)(optin - (int)fa.sharedSizeBytes) : 0;
+    const int fixed = std::max((int)fa.sharedSizeBytes, kDsmStatic);
+    return optin > fixed ? (size_t)(optin - fixed) : 0;
 }
 
 template <int NT, bool RES>

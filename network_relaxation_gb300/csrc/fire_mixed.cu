@@ -63,7 +63,7 @@ __device__ void relax_network_cta_mixed(const NetDev &d, const FireParamsDev &p,
     }
     mixed_finish(d, tm);
     __syncthreads();
-    mixed_energies(d, sh.red);
+    mixed_energies(d, sh.dslots);
     if (threadIdx.x == 0) mix_report(d.st, s);
     __syncthreads();
 }
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(NT, 1) k_fire_cluster_mixed(const NetDev *nets
         mixed_finish(d, tm);
         cl.sync();
         if (rank == 0) {
-            mixed_energies(d, sh.red);
+            mixed_energies(d, sh.dslots);
             if (threadIdx.x == 0) mix_report(d.st, s);
         }
         cl.sync();

@@ -647,8 +647,7 @@ static __device__ void mixed_finish(const NetDev &d, const Team &tm) {
 
 struct MixShared {
     float slots[5 * 32];
-    double dslots[64];
-    double red[32];
+    double dslots[64]; /* anchor totals; the final energies' 32 doubles */
     Coef coef;
 };
 

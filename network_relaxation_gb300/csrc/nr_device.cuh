@@ -156,6 +156,12 @@ struct NetDsm {
      * first bond entry, bond entries | triple entries << 16, first triple
      * entry} (entries: indices into bent / tent) */
     const int4 *grec;
+    /* the same nodes in groups of 32 gather records (a warp's): {node |
+     * fcode << 28, the group's first quad in xent, quads a lane, 0}, and the
+     * room for their entries, bonds then triples, four to a quad, quad q of
+     * lane l at first + 32 q + l (written by the kernel as addresses) */
+    const int4 *xrec;
+    uint4 *xent;
 };
 
 /* Layout of one large network for the tiled mixed-precision kernel
