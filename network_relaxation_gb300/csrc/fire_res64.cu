@@ -85,41 +85,6 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long u
     return ((unsigned long long)mh << 32) | ml;
 }
 
-/* Grid barrier number `epoch` of the launch: thread 0 arrives with release
- * semantics on a monotonic counter and polls it (2.1 us over 152 CTAs
- * against 2.4 for fence + atomic + volatile poll with naps).  False when the
- * wait ran out of its budget or another CTA gave up. */
-__device__ __forceinline__ bool res_barrier(unsigned long long *bar, FireState *st, unsigned long long target,
-                                            unsigned long long budget_ns, unsigned site, int *s_ok) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(bar) : "memory");
-        int ok = 1;
-        unsigned spins = 0;
-        unsigned long long t0 = 0, c;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(bar) : "memory");
-            if (c >= target) break;
-            if ((++spins & 63u) != 0) continue;
-            const unsigned long long now = global_ns();
-            if (t0 == 0) t0 = now;
-            if (*(volatile unsigned *)&st->abort_flag) {
-                ok = 0;
-                break;
-            }
-            if (now - t0 > budget_ns) {
-                atomicExch(&st->abort_flag, 1u);
-                atomicExch(&st->timeout_site, site);
-                ok = 0;
-                break;
-            }
-        }
-        *s_ok = ok;
-    }
-    __syncthreads();
-    return *s_ok != 0;
-}
-
 /* Tree of the eight lane-group sums w[0..8), of which the first `ng` can be
  * nonzero (x + 0 = x). */
 __device__ __forceinline__ double tree8_n(const double *w, int ng) {
@@ -511,7 +476,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
             if (lane == 0) r.maxp[par][blockIdx.x] = m;
         }
         ++epoch;
-        if (!res_barrier(r.bar, d.st, epoch * (unsigned long long)gridDim.x, budget_ns, 31, &s_ok)) return;
+        if (!epoch_barrier(r.bar, d.st, epoch * (unsigned long long)gridDim.x, budget_ns, 31, &s_ok)) return;
         if (tid < td.nh) {
             const double2 *q = vf + 2 * (size_t)halo[tid];
             hv = __ldcg(q);

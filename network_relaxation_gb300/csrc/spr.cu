@@ -15,15 +15,17 @@
  *    reference's and the oracle's.
  *  - The reduced system lives on the device in SELL-32 (rows in slices of
  *    32, each slice padded to its longest row, column-major inside the
- *    slice): a warp reads a slice's values and columns coalesced.  Rows are
- *    sorted by length inside windows of 256 (SELL-C-sigma), so slices pad
- *    little.
+ *    slice): a warp reads a slice's values and columns coalesced.  The free
+ *    nodes are cut into compact parts, one for each CTA of the solver, and
+ *    sorted by row length inside a part (SELL-C-sigma), so slices pad little.
  *  - bc is linear in (compression, shear), so the protocol needs two
  *    solves: the unit compression and the unit shear loads, solved
  *    together (one matrix read per iteration for both) by a conjugate
  *    gradient with a 2x2 block-Jacobi (per node) preconditioner, in its
- *    single-reduction form (two grid barriers per iteration), in one
- *    persistent cooperative kernel with budgeted grid barriers.  Every protocol point is then a
+ *    single-reduction form, in one persistent cooperative kernel with
+ *    budgeted grid barriers (k_spr_res: one barrier per iteration, the part
+ *    of each CTA in shared memory; k_spr_pcg, two barriers and everything in
+ *    L2, for systems too large for that).  Every protocol point is then a
  *    linear combination, checked by its own residual ||rhs - K_ff u||
  *    (one SpMV) and followed by the energies (canonical tile sums).
  *  - On a rank-deficient system (floppy modes) CG from zero returns the
@@ -51,7 +53,7 @@ namespace {
 constexpr double kSprDrop = 1e-10; /* FLT_TOL, sparse_relax.cpp:45 */
 constexpr int kSprThreads = 512;
 constexpr int kSlice = 32;
-constexpr int kSigma = 256; /* rows sorted by length within windows of this size */
+constexpr int kPartNodes = 64; /* nodes of a part while the GPU has SMs left: a slice for each scheduler */
 
 /* ------------------------------------------------------------ assembly */
 
@@ -425,6 +427,320 @@ __global__ void __launch_bounds__(kSprThreads) k_spr_pcg(SprDev d, double tol, i
     }
 }
 
+/* The parts of k_spr_res: part g owns slices [sl0[g], sl0[g + 1]) and reads
+ * the halo nodes hnode[h0[g] .. h0[g + 1]) (their columns, owned by other
+ * parts). lcol: each entry's column as the part's local row (own rows, then
+ * two per halo node), at the positions of SprDev.val. */
+struct SprRes {
+    const int *sl0, *h0, *hnode;
+    const unsigned short *lcol;
+    double2 *pub[2]; /* s = K z of every row, by the iteration's parity */
+    double *part;    /* [parity][part][kParts] */
+    unsigned long long *count;
+};
+
+/* Largest part: rows, halo rows, entries (0 where they stay in global). */
+struct SprResSizes {
+    int rows, hrows, entries;
+};
+
+/* Shared memory of a CTA. mode 0: everything; 1: without the matrix; 2: own
+ * vectors and preconditioner in global memory too. */
+struct SprResLayout {
+    size_t z, hr, hq, hs, hm, ho, hn, sl, r, p, q, x, s, m, o, val, col, total;
+};
+__host__ __device__ inline SprResLayout spr_res_layout(int mode, const SprResSizes &z) {
+    SprResLayout L{};
+    const size_t R = (size_t)z.rows, H = (size_t)z.hrows;
+    size_t o = 0;
+    L.z = o, o += 16 * (R + H);
+    L.hr = o, o += 16 * H;
+    L.hq = o, o += 16 * H;
+    L.hs = o, o += 16 * H;
+    L.hm = o, o += 8 * H;
+    if (mode < 2) {
+        L.r = o, o += 16 * R;
+        L.p = o, o += 16 * R;
+        L.q = o, o += 16 * R;
+        L.x = o, o += 16 * R;
+        L.s = o, o += 16 * R;
+        L.m = o, o += 8 * R;
+        L.o = o, o += 4 * R;
+    }
+    L.sl = o, o += 8 * (R / kSlice);
+    if (mode < 1) {
+        L.val = o, o += 8 * (size_t)z.entries;
+        L.col = o, o += 2 * (size_t)z.entries;
+    }
+    L.ho = o = (o + 15) / 16 * 16, o += 4 * H;
+    L.hn = o, o += 2 * H;
+    L.total = (o + 15) / 16 * 16;
+    return L;
+}
+
+/* Six warp sums at once (8 additions where one by one take 30): after xor
+ * 16, 8 and 4 every lane carries one sum. Lanes with (lane & 3) == 0 hold sum
+ * spr_sum_of(lane). */
+__device__ __forceinline__ double spr_sum6(const double *v, int lane) {
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0, b2 = (lane & 4) != 0;
+    double a = b4 ? v[1] : v[0], b = b4 ? v[3] : v[2], c = b4 ? v[5] : v[4];
+    a = a + __shfl_xor_sync(kFull, b4 ? v[0] : v[1], 16);
+    b = b + __shfl_xor_sync(kFull, b4 ? v[2] : v[3], 16);
+    c = c + __shfl_xor_sync(kFull, b4 ? v[4] : v[5], 16);
+    double e = b3 ? b : a;
+    e = e + __shfl_xor_sync(kFull, b3 ? a : b, 8);
+    c = c + __shfl_xor_sync(kFull, c, 8);
+    double f = b2 ? c : e;
+    f = f + __shfl_xor_sync(kFull, b2 ? e : c, 4);
+    f = f + __shfl_xor_sync(kFull, f, 2);
+    return f + __shfl_xor_sync(kFull, f, 1);
+}
+__device__ __forceinline__ int spr_sum_of(int lane) {
+    const int b4 = lane >> 4 & 1, b3 = lane >> 3 & 1, b2 = lane >> 2 & 1;
+    return b2 ? 4 + b4 : 2 * b3 + b4;
+}
+
+/* The two rows of a node sit in neighbouring lanes: this lane's row of
+ * z = M^-1 r (precond), both right-hand sides. */
+__device__ __forceinline__ double2 precond_row(double2 m, double o, double2 r, int lane) {
+    const double ox = __shfl_xor_sync(kFull, r.x, 1), oy = __shfl_xor_sync(kFull, r.y, 1);
+    const bool odd = lane & 1;
+    const double a = odd ? o : m.x, b = odd ? m.y : o;
+    return make_double2(fma(a, odd ? ox : r.x, b * (odd ? r.x : ox)), fma(a, odd ? oy : r.y, b * (odd ? r.y : oy)));
+}
+
+/* The same iteration as k_spr_pcg with one grid barrier: each CTA keeps
+ * its part's vectors, its halo's r, q and z and, where they fit, its rows of
+ * the matrix in shared memory. After the barrier every CTA sums the partials
+ * itself, advances its own copy of the scalars, and repeats the owners' vector
+ * pass for its halo (q, r and z from the owners' published s: their bits), so
+ * that nothing has to cross CTAs between the vector pass and the SpMV.
+ *
+ * What bounds an iteration: the FP64 pipe (a warp instruction every 19 clocks
+ * and SM): 2 per matrix entry and 18 per row; then the barrier (2.1 us over
+ * 152 CTAs) and the partials' and the halo's way through L2.
+ * Measured per iteration, this kernel against k_spr_pcg (two barriers with a
+ * last CTA working alone, all vectors through L2, 40 additions a warp for the
+ * sums): 96 rows 7.0 us (31), 3 040 rows 8.1 (41), 50 560 rows 13.1 (46),
+ * 124 000 rows 20.0 (48, matrix in global memory), 318 400 rows 39.6 (74,
+ * mode 2). */
+constexpr int kResSprThreads = 512;
+
+template <int MODE>
+__global__ void __launch_bounds__(kResSprThreads, 1) k_spr_res(SprDev d, SprRes e, SprResSizes z, double tol,
+                                                               int max_iter, unsigned long long budget_ns) {
+    extern __shared__ double2 s_spr[];
+    constexpr int NT = kResSprThreads, NW = NT / 32, kSums = 6;
+    __shared__ double s_red[NW * kParts], s_tot[kParts], s_al[2], s_be[2];
+    __shared__ int s_done, s_ok;
+    unsigned char *dyn = reinterpret_cast<unsigned char *>(s_spr);
+    const SprResLayout L = spr_res_layout(MODE, z);
+    const int G = (int)gridDim.x, g = (int)blockIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int sl0 = e.sl0[g], nsl = e.sl0[g + 1] - sl0, R = kSlice * nsl, row0 = kSlice * sl0;
+    const int h0 = e.h0[g], HR = 2 * (e.h0[g + 1] - h0), nhu = (HR + 31) / 32;
+    double2 *const s_z = reinterpret_cast<double2 *>(dyn + L.z);
+    double2 *const s_hr = reinterpret_cast<double2 *>(dyn + L.hr);
+    double2 *const s_hq = reinterpret_cast<double2 *>(dyn + L.hq);
+    double2 *const s_hs = reinterpret_cast<double2 *>(dyn + L.hs);
+    double2 *const s_hm = reinterpret_cast<double2 *>(dyn + L.hm);
+    double *const s_ho = reinterpret_cast<double *>(dyn + L.ho);
+    int *const s_hn = reinterpret_cast<int *>(dyn + L.hn);
+    int2 *const s_sl = reinterpret_cast<int2 *>(dyn + L.sl);
+    constexpr bool own = MODE < 2;
+    double2 *const v_r = own ? reinterpret_cast<double2 *>(dyn + L.r) : d.r + row0;
+    double2 *const v_p = own ? reinterpret_cast<double2 *>(dyn + L.p) : d.p + row0;
+    double2 *const v_q = own ? reinterpret_cast<double2 *>(dyn + L.q) : d.q + row0;
+    double2 *const v_x = own ? reinterpret_cast<double2 *>(dyn + L.x) : d.x + row0;
+    double2 *const s_s = reinterpret_cast<double2 *>(dyn + L.s);
+    const double2 *const v_m = own ? reinterpret_cast<double2 *>(dyn + L.m) : d.mdiag + row0 / 2;
+    const double *const v_o = own ? reinterpret_cast<double *>(dyn + L.o) : d.moff + row0 / 2;
+    const long e0 = d.slice_ptr[sl0];
+    const double *const v_val = MODE < 1 ? reinterpret_cast<double *>(dyn + L.val) : d.val + e0;
+    const unsigned short *const v_col = MODE < 1 ? reinterpret_cast<unsigned short *>(dyn + L.col) : e.lcol + e0;
+    const double2 zero = make_double2(0.0, 0.0);
+    /* x = p = q = 0, r = b; with z = s = 0 and alpha = beta = 0 the first pass
+     * below leaves them and forms z = M^-1 r and b.b */
+    for (int i = tid; i < R; i += NT) {
+        s_z[i] = zero;
+        v_r[i] = d.b[row0 + i];
+        v_p[i] = v_q[i] = v_x[i] = zero;
+        if (own) {
+            s_s[i] = zero;
+            if (i & 1) {
+                const_cast<double *>(v_o)[i >> 1] = d.moff[(row0 + i) >> 1];
+                const_cast<double2 *>(v_m)[i >> 1] = d.mdiag[(row0 + i) >> 1];
+            }
+        } else {
+            e.pub[1][row0 + i] = zero;
+        }
+    }
+    for (int j = tid; j < HR; j += NT) {
+        const int node = e.hnode[h0 + (j >> 1)];
+        s_hr[j] = d.b[2 * node + (j & 1)];
+        s_hq[j] = s_hs[j] = zero;
+        if (j & 1) {
+            s_hn[j >> 1] = node;
+            s_hm[j >> 1] = d.mdiag[node];
+            s_ho[j >> 1] = d.moff[node];
+        }
+    }
+    for (int u = tid; u < nsl; u += NT) s_sl[u] = make_int2((int)(d.slice_ptr[sl0 + u] - e0), d.slice_w[sl0 + u]);
+    if (MODE < 1) {
+        const int ne = (int)(d.slice_ptr[sl0 + nsl] - e0);
+        for (int k = tid; k < ne; k += NT) {
+            const_cast<double *>(v_val)[k] = d.val[e0 + k];
+            const_cast<unsigned short *>(v_col)[k] = e.lcol[e0 + k];
+        }
+    }
+    if (tid < 2) s_al[tid] = s_be[tid] = 0.0;
+    /* scalars of right-hand side `lane` (warp 0, lanes 0 and 1) */
+    double k_rho = 0.0, k_alpha = 0.0, k_bb = 0.0, k_rr = 0.0;
+    int k_active = 0, k_iters = 0;
+    unsigned long long target = 0;
+    __syncthreads();
+    for (int it = 0;; ++it) {
+        const int par = it & 1;
+        double2 *const pub = e.pub[par];
+        const double al0 = s_al[0], al1 = s_al[1], be0 = s_be[0], be1 = s_be[1];
+        double acc[kSums] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}; /* r.z, z.s, r.r of both */
+        /* vector pass: own slices, then the halo, dealt to the warps */
+        for (int u = warp; u < nsl + nhu; u += NW) {
+            if (u < nsl) {
+                const int i = kSlice * u + lane;
+                const double2 zv = s_z[i], sv = own ? s_s[i] : e.pub[par ^ 1][row0 + i];
+                double2 pv = v_p[i], qv = v_q[i], xv = v_x[i], rv = v_r[i];
+                pv.x = fma(be0, pv.x, zv.x);
+                pv.y = fma(be1, pv.y, zv.y);
+                qv.x = fma(be0, qv.x, sv.x);
+                qv.y = fma(be1, qv.y, sv.y);
+                xv.x = fma(al0, pv.x, xv.x);
+                xv.y = fma(al1, pv.y, xv.y);
+                rv.x = fma(-al0, qv.x, rv.x);
+                rv.y = fma(-al1, qv.y, rv.y);
+                v_p[i] = pv;
+                v_q[i] = qv;
+                v_x[i] = xv;
+                v_r[i] = rv;
+                acc[4] = fma(rv.x, rv.x, acc[4]);
+                acc[5] = fma(rv.y, rv.y, acc[5]);
+                s_z[i] = precond_row(v_m[i >> 1], v_o[i >> 1], rv, lane);
+            } else {
+                const int j = kSlice * (u - nsl) + lane;
+                const int jc = min(j, HR - 2 + (lane & 1)); /* the last warp's spare lanes repeat the last node */
+                const double2 sv = s_hs[jc];
+                double2 qv = s_hq[jc], rv = s_hr[jc];
+                qv.x = fma(be0, qv.x, sv.x);
+                qv.y = fma(be1, qv.y, sv.y);
+                rv.x = fma(-al0, qv.x, rv.x);
+                rv.y = fma(-al1, qv.y, rv.y);
+                const double2 zv = precond_row(s_hm[jc >> 1], s_ho[jc >> 1], rv, lane);
+                __syncwarp();
+                if (j < HR) {
+                    s_hq[j] = qv;
+                    s_hr[j] = rv;
+                    s_z[R + j] = zv;
+                }
+            }
+        }
+        __syncthreads();
+        /* s = K z */
+        for (int u = warp; u < nsl; u += NW) {
+            const int2 sl = s_sl[u];
+            const double *val = v_val + sl.x + lane;
+            const unsigned short *col = v_col + sl.x + lane;
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll 4
+            for (int k = 0; k < sl.y; ++k) {
+                const double m = val[k * kSlice];
+                const double2 pv = s_z[col[k * kSlice]];
+                a0 = fma(m, pv.x, a0);
+                a1 = fma(m, pv.y, a1);
+            }
+            const int i = kSlice * u + lane;
+            pub[row0 + i] = make_double2(a0, a1);
+            if (own) s_s[i] = make_double2(a0, a1);
+            const double2 rv = v_r[i], zv = s_z[i];
+            acc[0] = fma(rv.x, zv.x, acc[0]);
+            acc[1] = fma(rv.y, zv.y, acc[1]);
+            acc[2] = fma(zv.x, a0, acc[2]);
+            acc[3] = fma(zv.y, a1, acc[3]);
+        }
+        const double sum = spr_sum6(acc, lane);
+        if ((lane & 3) == 0) s_red[warp * kParts + spr_sum_of(lane)] = sum;
+        __syncthreads();
+        double *const part = e.part + (size_t)par * G * kParts;
+        if (warp < kSums) {
+            double t = lane < NW ? s_red[lane * kParts + warp] : 0.0;
+            for (int x = NW / 2; x > 0; x >>= 1) t = t + __shfl_xor_sync(kFull, t, x);
+            if (lane == 0) part[g * kParts + warp] = t;
+        }
+        if (G > 1) {
+            target += (unsigned long long)G;
+            if (!epoch_barrier(e.count, d.bar, target, budget_ns, 25, &s_ok)) return;
+        } else {
+            __syncthreads();
+        }
+        /* totals, a warp per sum; meanwhile the halo's s */
+        if (warp < kSums) {
+            double t = 0.0;
+            for (int b = lane; b < G; b += 32) t = t + __ldcg(part + b * kParts + warp);
+            t = warp_sum(t);
+            if (lane == 0) s_tot[warp] = t;
+        } else {
+            for (int j = tid - 32 * kSums; j < HR; j += NT - 32 * kSums)
+                s_hs[j] = __ldcg(pub + 2 * s_hn[j >> 1] + (j & 1));
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const int k = lane & 1;
+            const double rho = s_tot[k], mu = s_tot[2 + k], rr = s_tot[4 + k];
+            double alpha = 0.0, beta = 0.0;
+            bool stop;
+            if (it == 0) {
+                k_bb = k_rr = rr;
+                k_active = rr > 0 && rho != 0 && mu != 0;
+                if (k_active) alpha = rho / mu;
+                k_rho = rho;
+                stop = max_iter <= 0;
+            } else {
+                if (k_active) {
+                    k_iters++;
+                    k_rr = rr;
+                    beta = rho / k_rho;
+                    const double den = mu - beta * rho / k_alpha;
+                    if (!(rr > tol * tol * k_bb) || rho == 0 || !(den != 0) || !isfinite(den)) {
+                        k_active = 0;
+                        beta = 0.0;
+                    } else {
+                        alpha = rho / den;
+                        k_rho = rho;
+                    }
+                }
+                stop = k_iters >= max_iter;
+            }
+            k_alpha = alpha;
+            const bool done = !__any_sync(kFull, k_active) || __any_sync(kFull, stop);
+            if (lane < 2) {
+                s_al[k] = alpha;
+                s_be[k] = beta;
+            }
+            if (lane == 0) s_done = done;
+        }
+        __syncthreads();
+        if (s_done) break;
+    }
+    if (own)
+        for (int i = tid; i < R; i += NT) d.x[row0 + i] = v_x[i];
+    if (g == 0 && tid < 2) {
+        SprScal *sc = d.sc;
+        sc->rr[tid] = k_rr;
+        sc->bb[tid] = k_bb;
+        sc->iters[tid] = k_iters;
+        sc->active[tid] = k_active;
+    }
+}
+
 /* ---------------------------------------------- per protocol point */
 
 struct SprPointDev {
@@ -593,6 +909,12 @@ using namespace nr;
             return fail(NR_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));     \
     } while (0)
 
+/* Barrier words of a solve, zeroed before it. */
+struct SprBar {
+    FireState st;
+    unsigned long long count;
+};
+
 struct nr_spr {
     int n = 0, nr = 0, n_slices = 0;
     long nnz_upper = 0, sell_len = 0;
@@ -614,6 +936,10 @@ struct nr_spr {
     double *d_u_red = nullptr, *d_rpart = nullptr, *d_scalar = nullptr, *d_epart = nullptr;
     double2 *d_u_final = nullptr;
     int e_stride = 1;
+    int parts = 1;        /* grid of k_spr_res */
+    int mode = -1;        /* its template argument; -1: k_spr_pcg */
+    SprRes res{};
+    SprResSizes rsz{};
     int rpart_blocks = 1; /* capacity of d_rpart in blocks */
     int pcg_blocks = 1;   /* grid of k_spr_pcg (capacity of dev.part) */
     ~nr_spr() {
@@ -676,6 +1002,58 @@ struct Img {
         return off;
     }
 };
+
+/* Cuts nodes idx[b, e) into parts [g0, g0 + P) by recursive coordinate
+ * bisection along the longer side, in whole units of 16 nodes (a slice of 32
+ * rows); start[g]: a part's first node. */
+void spr_parts(const std::vector<double> &px, const std::vector<double> &py, int *idx, int b, int e, int g0, int P,
+               int *start) {
+    if (P == 1) {
+        start[g0] = b;
+        return;
+    }
+    double x0 = DBL_MAX, x1 = -DBL_MAX, y0 = DBL_MAX, y1 = -DBL_MAX;
+    for (int k = b; k < e; ++k) {
+        x0 = std::min(x0, px[idx[k]]);
+        x1 = std::max(x1, px[idx[k]]);
+        y0 = std::min(y0, py[idx[k]]);
+        y1 = std::max(y1, py[idx[k]]);
+    }
+    const std::vector<double> &key = x1 - x0 > y1 - y0 ? px : py;
+    const int units = (e - b + kSlice / 2 - 1) / (kSlice / 2), left = P / 2;
+    const int mid = std::min(e, b + kSlice / 2 * (int)(((long)units * left + P / 2) / P));
+    if (mid > b && mid < e)
+        std::nth_element(idx + b, idx + mid, idx + e,
+                         [&](int a, int c) { return key[a] != key[c] ? key[a] < key[c] : a < c; });
+    spr_parts(px, py, idx, b, mid, g0, left, start);
+    spr_parts(px, py, idx, mid, e, g0 + left, P - left, start);
+}
+
+const void *spr_res_kernel(int mode) {
+    return mode == 0 ? (const void *)k_spr_res<0> : mode == 1 ? (const void *)k_spr_res<1> : (const void *)k_spr_res<2>;
+}
+
+/* The first mode of k_spr_res whose parts fit a CTA's shared memory
+ * (NR_SPR_SMEM: bytes to stay below), or -1. */
+int spr_res_mode(const SprResSizes &z, bool narrow, int *mode) {
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const char *env = getenv("NR_SPR_SMEM");
+    const double cap = env ? atof(env) : 1e9;
+    *mode = -1;
+    for (int m = 0; narrow && m < 3 && *mode < 0 && e == cudaSuccess; ++m) {
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, spr_res_kernel(m));
+        const size_t need = spr_res_layout(m, z).total;
+        if (e != cudaSuccess || need + fa.sharedSizeBytes > (size_t)optin || (double)need > cap) continue;
+        e = cudaFuncSetAttribute(spr_res_kernel(m), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 optin - (int)fa.sharedSizeBytes);
+        *mode = m;
+    }
+    if (e != cudaSuccess) return fail(NR_ERR_CUDA, std::string("k_spr_res: ") + cudaGetErrorString(e));
+    return NR_OK;
+}
 
 int spr_blocks(int *blocks) {
     int per_sm = 0;
@@ -742,7 +1120,9 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
             S->dof_map[2 * i + 1] = S->nr++;
         }
     }
-    /* reduced full-symmetric rows, columns ascending */
+    /* reduced full-symmetric rows, columns ascending: the upper triangle is
+     * walked by rows, so a row gets its transposed entries (smaller columns)
+     * in order before its own */
     std::vector<long> rcnt(S->nr + 1, 0);
     const UpperK &K = S->K;
     for (long r = 0; r < K.n_dof; ++r)
@@ -774,79 +1154,99 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
                     diag[rr] = K.val[q];
                 }
             }
-        std::vector<std::pair<int, double>> tmp;
-        for (int r = 0; r < S->nr; ++r) {
-            tmp.clear();
-            for (long q = rcnt[r]; q < rcnt[r + 1]; ++q) tmp.push_back({rcol[q], rval[q]});
-            std::sort(tmp.begin(), tmp.end(), [](const std::pair<int, double> &a, const std::pair<int, double> &b) {
-                return a.first < b.first;
-            });
-            for (size_t k = 0; k < tmp.size(); ++k) {
-                rcol[rcnt[r] + k] = tmp[k].first;
-                rval[rcnt[r] + k] = tmp[k].second;
-            }
-        }
     }
-    /* SELL-32 with nodes sorted by row length inside windows of kSigma rows
-     * (SELL-C-sigma): slices of rows of similar length pad little, the
-     * window keeps neighbouring nodes together for the gathers, and a
-     * node's x and y rows stay adjacent (rows 2k, 2k + 1 of device node k)
-     * for the 2x2 block preconditioner.  perm: device row -> reduced row;
-     * columns are renumbered; each row keeps its column order, so its sum
-     * is unchanged. */
+    /* SELL-32 over the parts of the solver (spr_parts): nodes sorted by row
+     * length inside a part, a part's slices its own (its last one filled up
+     * with null rows: perm -1, no entries), a node's x and y rows adjacent
+     * (rows 2k, 2k + 1 of device node k) for the 2x2 block preconditioner.
+     * perm: device row -> reduced row; columns are renumbered; each row keeps
+     * its column order, so its sum is unchanged. */
     const int nn = S->nr / 2;
-    const auto row_len = [&](int r) { return rcnt[r + 1] - rcnt[r]; };
-    std::vector<int> pnode(nn);
+    const auto row_len = [&](int r) { return r < 0 ? 0L : rcnt[r + 1] - rcnt[r]; };
+    const int P = std::max(1, std::min(sm_count_spr(), (nn + kPartNodes - 1) / kPartNodes));
+    std::vector<double> px(nn), py(nn);
+    for (int i = 0; i < S->n; ++i)
+        if (S->dof_map[2 * i] >= 0) {
+            const double x = h.points[2 * i], y = h.points[2 * i + 1];
+            px[S->dof_map[2 * i] / 2] = std::isfinite(x) ? x : 0.0; /* any order will do, but an order */
+            py[S->dof_map[2 * i] / 2] = std::isfinite(y) ? y : 0.0;
+        }
+    std::vector<int> pnode(nn), sl0, perm;
     for (int j = 0; j < nn; ++j) pnode[j] = j;
-    const int wnodes = kSigma / 2;
-    for (int w0 = 0; w0 < nn; w0 += wnodes) {
-        const int w1 = std::min(nn, w0 + wnodes);
-        std::stable_sort(pnode.begin() + w0, pnode.begin() + w1, [&](int a, int b) {
-            return std::max(row_len(2 * a), row_len(2 * a + 1)) > std::max(row_len(2 * b), row_len(2 * b + 1));
+    std::vector<int> part0(P + 1, 0);
+    spr_parts(px, py, pnode.data(), 0, nn, 0, P, part0.data());
+    part0[P] = nn;
+    for (int g = 0; g < P; ++g) {
+        sl0.push_back((int)(perm.size() / kSlice));
+        std::sort(pnode.begin() + part0[g], pnode.begin() + part0[g + 1], [&](int a, int b) {
+            const long la = std::max(row_len(2 * a), row_len(2 * a + 1)), lb = std::max(row_len(2 * b), row_len(2 * b + 1));
+            return la != lb ? la > lb : a < b;
         });
+        for (int k = part0[g]; k < part0[g + 1]; ++k) {
+            perm.push_back(2 * pnode[k]);
+            perm.push_back(2 * pnode[k] + 1);
+        }
+        while (perm.size() % kSlice) perm.push_back(-1);
     }
-    std::vector<int> perm(S->nr), inv(S->nr);
-    for (int k = 0; k < nn; ++k) {
-        perm[2 * k] = 2 * pnode[k];
-        perm[2 * k + 1] = 2 * pnode[k] + 1;
-    }
-    for (int k = 0; k < S->nr; ++k) inv[perm[k]] = k;
+    const int nrp = (int)perm.size(); /* device rows */
+    sl0.push_back(nrp / kSlice);
+    std::vector<int> inv(S->nr);
+    for (int k = 0; k < nrp; ++k)
+        if (perm[k] >= 0) inv[perm[k]] = k;
     S->perm = perm;
-    S->n_slices = (S->nr + kSlice - 1) / kSlice;
+    S->n_slices = nrp / kSlice;
     std::vector<long> slice_ptr(S->n_slices + 1, 0);
     std::vector<int> slice_w(S->n_slices, 0);
     for (int sl = 0; sl < S->n_slices; ++sl) {
         int w = 0;
-        for (int l = 0; l < kSlice; ++l) {
-            const int k = sl * kSlice + l;
-            if (k < S->nr) w = std::max(w, (int)row_len(perm[k]));
-        }
+        for (int l = 0; l < kSlice; ++l) w = std::max(w, (int)row_len(perm[sl * kSlice + l]));
         slice_w[sl] = w;
         slice_ptr[sl + 1] = slice_ptr[sl] + (long)w * kSlice;
     }
     S->sell_len = slice_ptr[S->n_slices];
-    std::vector<int> scol(S->sell_len, 0);
+    std::vector<int> scol(S->sell_len, 0), h0(1, 0), hnode, local(nrp / 2, -1);
+    std::vector<unsigned short> lcol(S->sell_len, 0);
     std::vector<double> sval(S->sell_len, 0.0);
-    for (int sl = 0; sl < S->n_slices; ++sl)
-        for (int l = 0; l < kSlice; ++l) {
-            const int k = sl * kSlice + l;
-            const int r = k < S->nr ? perm[k] : -1;
-            for (int q = 0; q < slice_w[sl]; ++q) {
-                const long at = slice_ptr[sl] + (long)q * kSlice + l;
-                if (r >= 0 && q < row_len(r)) {
-                    scol[at] = inv[rcol[rcnt[r] + q]];
-                    sval[at] = rval[rcnt[r] + q];
-                } else {
-                    scol[at] = k < S->nr ? k : 0; /* padding: a valid index, value 0 */
+    SprResSizes &rz = S->rsz;
+    bool narrow = true; /* local rows in 16 bits */
+    for (int g = 0; g < P; ++g) {
+        const int r0 = sl0[g] * kSlice, R = (sl0[g + 1] - sl0[g]) * kSlice;
+        for (int sl = sl0[g]; sl < sl0[g + 1]; ++sl)
+            for (int l = 0; l < kSlice; ++l) {
+                const int k = sl * kSlice + l, r = perm[k];
+                for (int q = 0; q < slice_w[sl]; ++q) {
+                    const long at = slice_ptr[sl] + (long)q * kSlice + l;
+                    int c = k; /* padding: a valid index, value 0 */
+                    if (q < row_len(r)) {
+                        c = inv[rcol[rcnt[r] + q]];
+                        sval[at] = rval[rcnt[r] + q];
+                    }
+                    int lc = c - r0;
+                    if (lc < 0 || lc >= R) {
+                        int &m = local[c / 2];
+                        if (m < h0[g]) { /* the part's first use of this node */
+                            m = (int)hnode.size();
+                            hnode.push_back(c / 2);
+                        }
+                        lc = R + 2 * (m - h0[g]) + (c & 1);
+                    }
+                    narrow = narrow && lc < 65536;
+                    scol[at] = c;
+                    lcol[at] = (unsigned short)lc;
                 }
             }
-        }
+        h0.push_back((int)hnode.size());
+        rz.rows = std::max(rz.rows, R);
+        rz.hrows = std::max(rz.hrows, 2 * (h0[g + 1] - h0[g]));
+        rz.entries = std::max(rz.entries, (int)std::min(slice_ptr[sl0[g + 1]] - slice_ptr[sl0[g]], 1L << 28));
+    }
     /* inverse of each node's 2x2 diagonal block (scalar Jacobi when the
      * block is singular or nearly so) */
-    std::vector<double2> mdiag(std::max(1, nn));
-    std::vector<double> moff(std::max(1, nn));
-    for (int k = 0; k < nn; ++k) {
+    std::vector<double2> mdiag(std::max(1, nrp / 2), make_double2(0.0, 0.0));
+    std::vector<double> moff(std::max(1, nrp / 2), 0.0);
+    for (int k = 0; k < nrp / 2; ++k) {
         const int rx = perm[2 * k];
+        if (rx < 0) continue;
         const double kxx = diag[rx], kyy = diag[rx + 1];
         double kxy = 0.0;
         for (long q = rcnt[rx]; q < rcnt[rx + 1]; ++q)
@@ -888,6 +1288,12 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
         delete S;
         return rc;
     }
+    S->parts = P;
+    rc = spr_res_mode(rz, narrow, &S->mode);
+    if (rc != NR_OK) {
+        delete S;
+        return rc;
+    }
     const int tb = (S->n_edges + kTile - 1) / kTile, tt = (S->n_triples + kTile - 1) / kTile;
     S->e_stride = std::max(1, std::max(tb, tt));
     Img img;
@@ -897,22 +1303,26 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     const size_t o_val = img.put(sval.data(), sval.size());
     const size_t o_md = img.put(mdiag.data(), mdiag.size());
     const size_t o_mo = img.put(moff.data(), moff.size());
-    const size_t o_b = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_x = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_r = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_p = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_q = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_z = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_s = img.add(sizeof(double2) * (S->nr + 1));
-    const size_t o_part = img.add(sizeof(double) * kParts * (size_t)blocks);
+    const size_t o_b = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_x = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_r = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_p = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_q = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_z = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_s = img.add(sizeof(double2) * (nrp + 1));
+    const size_t o_part = img.add(sizeof(double) * kParts * (size_t)std::max(blocks, 2 * P));
     S->pcg_blocks = blocks;
     S->rpart_blocks = 4 * sm_count_spr(); /* k_spr_residual's largest grid */
     const size_t o_rpart = img.add(sizeof(double) * kParts * (size_t)S->rpart_blocks);
     const size_t o_sc = img.add(sizeof(SprScal));
-    const size_t o_bar = img.add(sizeof(FireState));
+    const size_t o_bar = img.add(sizeof(SprBar));
+    const size_t o_sl0 = img.put(sl0.data(), sl0.size());
+    const size_t o_h0 = img.put(h0.data(), h0.size());
+    const size_t o_hn = img.put(hnode.data(), hnode.size());
+    const size_t o_lcol = img.put(lcol.data(), lcol.size());
     const size_t o_map = img.put(dof_dev.data(), dof_dev.size());
     const size_t o_top = img.put(S->top.data(), S->top.size());
-    const size_t o_ured = img.add(sizeof(double) * (S->nr + 1));
+    const size_t o_ured = img.add(sizeof(double) * (nrp + 1));
     const size_t o_uf = img.add(sizeof(double2) * (size_t)S->n);
     const size_t o_pos = img.put((const double2 *)h.points.data(), (size_t)S->n);
     const size_t o_bond = img.put(bond.data(), bond.size());
@@ -929,7 +1339,7 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     }
     char *base = S->arena;
     SprDev &d = S->dev;
-    d.nr = S->nr;
+    d.nr = nrp;
     d.n_slices = S->n_slices;
     d.slice_ptr = (const long *)(base + o_sp);
     d.slice_w = (const int *)(base + o_sw);
@@ -946,7 +1356,15 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     d.s = (double2 *)(base + o_s);
     d.part = (double *)(base + o_part);
     d.sc = (SprScal *)(base + o_sc);
-    d.bar = (FireState *)(base + o_bar);
+    d.bar = &((SprBar *)(base + o_bar))->st;
+    S->res.sl0 = (const int *)(base + o_sl0);
+    S->res.h0 = (const int *)(base + o_h0);
+    S->res.hnode = (const int *)(base + o_hn);
+    S->res.lcol = (const unsigned short *)(base + o_lcol);
+    S->res.pub[0] = d.s;
+    S->res.pub[1] = d.z;
+    S->res.part = d.part;
+    S->res.count = &((SprBar *)(base + o_bar))->count;
     S->d_rpart = (double *)(base + o_rpart);
     S->d_dof_map = (int *)(base + o_map);
     S->d_top = (unsigned char *)(base + o_top);
@@ -1008,18 +1426,18 @@ int nr_spr_solve(nr_spr *S, int affine, double tol, int max_iter, void *stream) 
         S->rel_residual[0] = S->rel_residual[1] = 0;
         return NR_OK;
     }
-    std::vector<double> rhs2, rhs_dev(2 * (size_t)S->nr);
+    std::vector<double> rhs2, rhs_dev(2 * S->perm.size(), 0.0);
     unit_rhs(*S, affine, rhs2);
-    for (int k = 0; k < S->nr; ++k) { /* device order */
-        rhs_dev[2 * (size_t)k] = rhs2[2 * (size_t)S->perm[k]];
-        rhs_dev[2 * (size_t)k + 1] = rhs2[2 * (size_t)S->perm[k] + 1];
+    for (size_t k = 0; k < S->perm.size(); ++k) { /* device order */
+        if (S->perm[k] < 0) continue;
+        rhs_dev[2 * k] = rhs2[2 * (size_t)S->perm[k]];
+        rhs_dev[2 * k + 1] = rhs2[2 * (size_t)S->perm[k] + 1];
     }
     SPR_TRY(cudaMemcpyAsync((void *)S->dev.b, rhs_dev.data(), sizeof(double) * rhs_dev.size(), cudaMemcpyHostToDevice,
                             s));
     SPR_TRY(cudaStreamSynchronize(s)); /* rhs_dev is a local */
     SPR_TRY(cudaMemsetAsync(S->dev.sc, 0, sizeof(SprScal), s));
-    SPR_TRY(cudaMemsetAsync(S->dev.bar, 0, sizeof(FireState), s));
-    const int blocks = S->pcg_blocks;
+    SPR_TRY(cudaMemsetAsync(S->dev.bar, 0, sizeof(SprBar), s));
     SprDev dd = S->dev;
     double tt = tol;
     int mi = max_iter;
@@ -1027,8 +1445,16 @@ int nr_spr_solve(nr_spr *S, int affine, double tol, int max_iter, void *stream) 
     double ms = env ? atof(env) : 2000.0;
     if (!(ms > 0)) ms = 2000.0;
     unsigned long long budget = (unsigned long long)(ms * 1e6);
-    void *args[] = {&dd, &tt, &mi, &budget};
-    SPR_TRY(cudaLaunchCooperativeKernel((const void *)k_spr_pcg, dim3(blocks), dim3(kSprThreads), args, 0, s));
+    if (S->mode >= 0) {
+        SprRes re = S->res;
+        SprResSizes rz = S->rsz;
+        void *args[] = {&dd, &re, &rz, &tt, &mi, &budget};
+        SPR_TRY(cudaLaunchCooperativeKernel(spr_res_kernel(S->mode), dim3(S->parts), dim3(kResSprThreads), args,
+                                            spr_res_layout(S->mode, rz).total, s));
+    } else {
+        void *args[] = {&dd, &tt, &mi, &budget};
+        SPR_TRY(cudaLaunchCooperativeKernel((const void *)k_spr_pcg, dim3(S->pcg_blocks), dim3(kSprThreads), args, 0, s));
+    }
     SprScal sc;
     FireState bar;
     SPR_TRY(cudaMemcpyAsync(&sc, S->dev.sc, sizeof(sc), cudaMemcpyDeviceToHost, s));
