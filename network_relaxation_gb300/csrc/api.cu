@@ -348,8 +348,8 @@ static int fp64_kernel_choice() {
 /* FP64, one network: networks of at most NR_FP64_CLUSTER_NODES nodes relax
  * on the on-chip kernels (NR_FP64_KERNEL), larger ones, and those that fit
  * none, on the cooperative grid kernel.  All give the same bits.  The
- * resident kernel takes whatever fits the SMs' shared memory (about 130 000
- * nodes of a p = 0.65 lattice); a cluster of NR_FP64_CLUSTER CTAs (default
+ * resident kernel takes whatever fits the SMs' shared memory in one of its
+ * modes (about 200 000 nodes of a p = 0.65 lattice); a cluster of NR_FP64_CLUSTER CTAs (default
  * 16) has the FP64 pipes of 16 SMs and beats the grid kernel up to
  * kFp64DsmNodes. */
 constexpr int kFp64DsmNodes = 4096;
@@ -377,7 +377,8 @@ static bool add_res_layout(const nr_host_network &h, const Incidence &inc, const
     if (build_res64_layout(h, inc, fcodes, use_bonds, use_triples, eptr, eent, partner, sms, res64_smem_limit(), L) !=
         NR_OK)
         return false;
-    if (!res64_fits(L.n_ctas, false, L.max_smem) || (h.n_facets() > 0 && !res64_fits(L.n_ctas, true, L.max_smem)))
+    if (!res64_fits(L.n_ctas, false, L.mode, L.max_smem) ||
+        (h.n_facets() > 0 && !res64_fits(L.n_ctas, true, L.mode, L.max_smem)))
         return false;
     o.desc = img.put(L.desc.data(), L.desc.size());
     o.ro = img.put(L.ro.data(), L.ro.size());
@@ -617,6 +618,7 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         Res64Dev &r = S.res;
         r.sub = res_host.sub;
         r.n_units = res_host.n_units;
+        r.mode = res_host.mode;
         r.desc = (const Res64Desc *)(base + res_off.desc);
         r.ro = (const unsigned char *)(base + res_off.ro);
         for (int c = 0; c < 2; ++c) {
@@ -1683,7 +1685,9 @@ int nr_network_plan(nr_network *d, int precision, char *buf, size_t cap) {
             snprintf(out, sizeof out, "k_fire_tile_mixed ctas=%d threads=%d tiles=%d max_tile_nodes=%d", g.blocks,
                      g.tile_threads, g.tl.n_tiles, g.tl.max_nodes);
         else if (g.mixed) snprintf(out, sizeof out, "k_fire_grid_mixed ctas=%d", g.blocks);
-        else if (g.res) snprintf(out, sizeof out, "k_fire_res64 ctas=%d sub=%d smem=%zu", g.blocks, g.rd.sub, g.res_smem);
+        else if (g.res) 
+            snprintf(out, sizeof out, "k_fire_res64 ctas=%d sub=%d smem=%zu%s", g.blocks, g.rd.sub, g.res_smem,
+                     g.rd.mode == kResPairs ? " pairs" : g.rd.mode == kResStream ? " stream" : "");
         else if (g.cluster > 0) snprintf(out, sizeof out, "%s cluster=%d", g.dsm64 ? "k_fire_dsm64" : "k_fire_cluster", g.cluster);
         else snprintf(out, sizeof out, "k_fire_grid ctas=%d sub=%d", g.blocks, g.d.sub);
     }

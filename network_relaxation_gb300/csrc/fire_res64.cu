@@ -40,11 +40,20 @@
  * totals and scalars 3.9; the FP64 pipe is active for 17.  512 threads: 768
  * and 1024 measured 3 to 9 % slower.
  *
+ * Tiles that do not fit whole (from about 125 000 nodes of a p = 0.65 lattice) are
+ * still twice as fast as the grid kernel with their topology, v and F in L2
+ * (res64_segs): 160 000 nodes 128 -> 57 us a step, a gel of 90 300 nodes 115 ->
+ * 77, and with two forces a triple instead of three in shared memory Mikado of
+ * 197 246 nodes 136 -> 77 (numbered by y bands: boundary items add 27 %; the
+ * FP64 pipe's share of that tile is 58).  The streamed reads are in order, a
+ * warp's line at a time, and hide behind the FP64 work of the other 15 warps.
+ *
  * Compiled with --fmad=false: the same bits as the oracle.
  */
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <thread>
 #include <vector>
@@ -225,8 +234,11 @@ constexpr int kResThreads = 512;
 
 /* One tile of the network per CTA (Res64Desc / Res64Segs, nr_device.cuh).
  * kGel: the network carries a gel; its elements, their reference inverses
- * and the duplicate vertices join the tile. */
-template <bool kGel>
+ * and the duplicate vertices join the tile.  kMode other than
+ * kResWhole: tiles too large to be held whole; topology, v and F are read from
+ * L2 in order, and what is reached at random (x, the items' forces) is in
+ * shared memory. */
+template <bool kGel, int kMode>
 __global__ void __launch_bounds__(kResThreads, 1)
     k_fire_res64(NetDev d, Res64Dev r, FireParamsDev p, unsigned long long budget_ns) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -236,33 +248,37 @@ __global__ void __launch_bounds__(kResThreads, 1)
     __shared__ unsigned long long s_m2;
     __shared__ int s_ok;
     const Res64Desc td = r.desc[blockIdx.x];
-    const Res64Segs g = res64_segs(td);
+    const Res64Segs g = res64_segs(td, kMode);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr bool kStream = kMode != kResWhole, kPairs = kMode == kResPairs;
     constexpr int NT = kResThreads, NW = kResThreads / 32;
-    const int sub = r.sub, un = kChunk * sub; /* nodes of a unit */
+    const int sub = r.sub, un = kChunk * sub; /* nodes of a unit, a power of two */
+    const int lg_un = 31 - __clz(un);
     const int no = td.nu * un;                /* own local indices (the last unit may be padded) */
     /* the tile's record, then the working arrays */
+    const unsigned char *const rec = kStream ? r.ro + td.ro_off : s_raw;
     {
         const int4 *src = reinterpret_cast<const int4 *>(r.ro + td.ro_off);
         int4 *dst = reinterpret_cast<int4 *>(s_raw);
-        for (unsigned k = tid; k < g.rec / 16u; k += NT) dst[k] = __ldg(src + k);
+        const unsigned bytes = kStream ? tile_pad16(4u * td.nu) : g.rec; /* the unit numbers come first */
+        for (unsigned k = tid; k < bytes / 16u; k += NT) dst[k] = __ldg(src + k);
     }
     const int *units = reinterpret_cast<const int *>(s_raw + g.units);
-    const int *halo = reinterpret_cast<const int *>(s_raw + g.halo);
-    const double *bl0 = reinterpret_cast<const double *>(s_raw + g.bl0);
-    const double *bk = reinterpret_cast<const double *>(s_raw + g.bk);
-    const unsigned *bref = reinterpret_cast<const unsigned *>(s_raw + g.bref);
-    const signed char *bwrap = reinterpret_cast<const signed char *>(s_raw + g.bwrap);
-    const uint2 *tref = reinterpret_cast<const uint2 *>(s_raw + g.tref);
-    const double *tkb = reinterpret_cast<const double *>(s_raw + g.tkb);
-    const double *tphi = reinterpret_cast<const double *>(s_raw + g.tphi);
-    const uint2 *eref = reinterpret_cast<const uint2 *>(s_raw + g.eref);
-    const int *eid = reinterpret_cast<const int *>(s_raw + g.eid);
-    const uint2 *grec = reinterpret_cast<const uint2 *>(s_raw + g.grec);
-    const unsigned short *inc = reinterpret_cast<const unsigned short *>(s_raw + g.inc);
-    const unsigned short *part = reinterpret_cast<const unsigned short *>(s_raw + g.partner);
-    const unsigned char *pub = s_raw + g.pub;
-    const unsigned short *grp = reinterpret_cast<const unsigned short *>(s_raw + g.grp);
+    const int *halo = reinterpret_cast<const int *>(rec + g.halo);
+    const double *bl0 = reinterpret_cast<const double *>(rec + g.bl0);
+    const double *bk = reinterpret_cast<const double *>(rec + g.bk);
+    const unsigned *bref = reinterpret_cast<const unsigned *>(rec + g.bref);
+    const signed char *bwrap = reinterpret_cast<const signed char *>(rec + g.bwrap);
+    const uint2 *tref = reinterpret_cast<const uint2 *>(rec + g.tref);
+    const double *tkb = reinterpret_cast<const double *>(rec + g.tkb);
+    const double *tphi = reinterpret_cast<const double *>(rec + g.tphi);
+    const uint2 *eref = reinterpret_cast<const uint2 *>(rec + g.eref);
+    const int *eid = reinterpret_cast<const int *>(rec + g.eid);
+    const uint2 *grec = reinterpret_cast<const uint2 *>(rec + g.grec);
+    const unsigned short *inc = reinterpret_cast<const unsigned short *>(rec + g.inc);
+    const unsigned short *part = reinterpret_cast<const unsigned short *>(rec + g.partner);
+    const unsigned char *pub = rec + g.pub;
+    const unsigned short *grp = reinterpret_cast<const unsigned short *>(rec + g.grp);
     double2 *s_x = reinterpret_cast<double2 *>(s_raw + g.x);
     double2 *s_v = reinterpret_cast<double2 *>(s_raw + g.v);
     double2 *s_f = reinterpret_cast<double2 *>(s_raw + g.f);   /* own force sums (gel: before the partner's) */
@@ -272,16 +288,18 @@ __global__ void __launch_bounds__(kResThreads, 1)
     double *s_M = reinterpret_cast<double *>(s_raw + g.eM);    /* per element: 6 inverse entries, area, - */
     double *s_du = reinterpret_cast<double *>(s_raw + g.du);   /* per element: dU/dF11, F12, F21, F22 */
     __syncthreads();
-    auto node_of = [&](int li) { return units[li / un] * un + li % un; };
+    auto node_of = [&](int li) { return (units[li >> lg_un] << lg_un) + (li & (un - 1)); };
     for (int li = tid; li < no; li += NT) {
         const int i = node_of(li);
         s_x[li] = i < d.n ? d.x[i] : make_double2(0.0, 0.0);
-        s_v[li] = make_double2(0.0, 0.0);
-        s_ff[li] = make_double2(0.0, 0.0);
+        if (!kStream) {
+            s_v[li] = make_double2(0.0, 0.0);
+            s_ff[li] = make_double2(0.0, 0.0);
+        }
     }
     for (int h = tid; h < td.nh; h += NT) s_x[no + h] = d.x[halo[h]];
     const int nel = kGel ? td.nel : 0;
-    if (kGel)
+    if (kGel && !kStream)
         for (int e = tid; e < nel; e += NT) {
             const double *M = d.gel->elem_inv + 6 * (size_t)eid[e];
             for (int c = 0; c < 6; ++c) s_M[8 * e + c] = M[c];
@@ -303,14 +321,17 @@ __global__ void __launch_bounds__(kResThreads, 1)
             const Scal &s = s_sc;
             if (s.done) break;
             for (int li = tid; li < no; li += NT) {
-                double2 x = s_x[li], v = s_v[li];
-                const double2 f = s_ff[li];
+                const int i = kStream ? node_of(li) : 0;
+                if (kStream && i >= d.n) continue;
+                double2 *const pv = kStream ? d.v + i : s_v + li;
+                double2 x = s_x[li], v = *pv;
+                const double2 f = kStream ? d.f[i] : s_ff[li];
                 res_mix(s, v, f);
                 res_drift(s, x, v, f);
                 s_x[li] = x;
                 v.x = fma(s.dtm, f.x, v.x);
                 v.y = fma(s.dtm, f.y, v.y);
-                s_v[li] = v;
+                *pv = v;
             }
             for (int h = tid; h < td.nh; h += NT) {
                 if (h != tid) {
@@ -333,13 +354,14 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 if (e < nel) {
                     const uint2 q = eref[e];
                     const double2 p1 = s_x[q.x & 0xffffu], p2 = s_x[q.x >> 16], p3 = s_x[q.y];
-                    const double *M = s_M + 8 * e;
+                    const double *M = kStream ? d.gel->elem_inv + 6 * (size_t)eid[e] : s_M + 8 * e;
+                    const double area = kStream ? d.gel->elem_area[eid[e]] : M[6];
                     const double f11 = p1.x * M[0] + p2.x * M[2] + p3.x * M[4];
                     const double f12 = p1.x * M[1] + p2.x * M[3] + p3.x * M[5];
                     const double f21 = p1.y * M[0] + p2.y * M[2] + p3.y * M[4];
                     const double f22 = p1.y * M[1] + p2.y * M[3] + p3.y * M[5];
                     double *du = s_du + 4 * e;
-                    gel_du_of(*d.gel, M[6], f11, f12, f21, f22, du[0], du[1], du[2], du[3]);
+                    gel_du_of(*d.gel, area, f11, f12, f21, f22, du[0], du[1], du[2], du[3]);
                 }
             } else if (kind == 1) {
                 const int t = item;
@@ -352,10 +374,15 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     double fjx, fjy, fkx, fky;
                     bend_force(ax, ay, bx, by, td.has_kb ? tkb[t] : d.kb, td.has_phi ? tphi[t] : 0.0, fjx, fjy, fkx,
                                fky);
-                    /* the hinge's (-F_j) - F_k */
-                    s_tf[3 * t] = make_double2(ii_flip(fjx, true) - fkx, ii_flip(fjy, true) - fky);
-                    s_tf[3 * t + 1] = make_double2(fjx, fjy);
-                    s_tf[3 * t + 2] = make_double2(fkx, fky);
+                    if (kPairs) {
+                        s_tf[2 * t] = make_double2(fjx, fjy);
+                        s_tf[2 * t + 1] = make_double2(fkx, fky);
+                    } else {
+                        /* the hinge's (-F_j) - F_k */
+                        s_tf[3 * t] = make_double2(ii_flip(fjx, true) - fkx, ii_flip(fjy, true) - fky);
+                        s_tf[3 * t + 1] = make_double2(fjx, fjy);
+                        s_tf[3 * t + 2] = make_double2(fkx, fky);
+                    }
                 }
             } else if (kind == 0) {
                 const int b = item;
@@ -374,7 +401,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
         {
             const double *bfd = reinterpret_cast<const double *>(s_bf);
             const double *tfd = reinterpret_cast<const double *>(s_tf);
-            double *fd = reinterpret_cast<double *>(s_f);
+            double *fd = reinterpret_cast<double *>(kStream && !kGel ? d.f : s_f);
             for (int k = tid; k < 2 * td.ngather; k += NT) {
                 const uint2 q = grec[k >> 1];
                 const int c = k & 1;
@@ -393,20 +420,31 @@ __global__ void __launch_bounds__(kResThreads, 1)
                     if (d.use_triples) {
                         const int m = (int)(q.x >> 24);
 #pragma unroll 4
-                        for (int a = 0; a < m; ++a) f = f + tfd[2 * e[a] + c];
+                        for (int a = 0; a < m; ++a) {
+                            if (kPairs) {
+                                const unsigned code = e[a], t = code / 3u, role = code - 3u * t;
+                                const double u = tfd[4 * t + (role == 2u ? 2u : 0u) + c];
+                                f = f + (role == 0u ? ii_flip(u, true) - tfd[4 * t + 2u + c] : u);
+                            } else {
+                                f = f + tfd[2 * e[a] + c];
+                            }
+                        }
                         e += m;
                     }
                     if (kGel) {
                         const int m = (int)((q.y >> 16) & 0xffu);
                         for (int a = 0; a < m; ++a) {
                             const int el = e[a] / 3, v = e[a] - 3 * el;
-                            const double *M = s_M + 8 * el + 2 * v;
+                            const double *M =
+                                (kStream ? d.gel->elem_inv + 6 * (size_t)eid[el] : s_M + 8 * el) + 2 * v;
                             f = f + s_du[4 * el + 2 * c] * M[0];
                             f = f + s_du[4 * el + 2 * c + 1] * M[1];
                         }
                     }
                 }
-                fd[2 * (q.x & 0xffffu) + c] = f;
+                const int li = (int)(q.x & 0xffffu);
+                if (!kStream || kGel) fd[2 * li + c] = f;
+                else if (li < no) fd[2 * (size_t)node_of(li) + c] = f; /* a gel that is not set: no use for other tiles' duplicates */
             }
         }
         __syncthreads();
@@ -422,7 +460,7 @@ __global__ void __launch_bounds__(kResThreads, 1)
                 const int li = u * un + c * kChunk + lane, i = unit * un + c * kChunk + lane;
                 double tP = 0.0, tV = 0.0, tF = 0.0;
                 if (i < d.n) {
-                    double2 f = s_f[li];
+                    double2 f = kStream && !kGel ? d.f[i] : s_f[li];
                     if (kGel) {
                         const unsigned q = part[li];
                         if (q != 0xffffu) {
@@ -430,15 +468,17 @@ __global__ void __launch_bounds__(kResThreads, 1)
                             f.x = f.x + o.x;
                             f.y = f.y + o.y;
                         }
-                        s_ff[li] = f;
+                        if (kStream) d.f[i] = f;
+                        else s_ff[li] = f;
                     }
                     double2 v = make_double2(0.0, 0.0);
                     if (!init) {
-                        v = s_v[li];
+                        v = kStream ? d.v[i] : s_v[li];
                         v.x = fma(dtm, f.x, v.x);
                         v.y = fma(dtm, f.y, v.y);
-                        s_v[li] = v;
                     }
+                    if (kStream) d.v[i] = v;
+                    else if (!init) s_v[li] = v;
                     if (pub[li]) {
                         vf[2 * (size_t)i] = v;
                         vf[2 * (size_t)i + 1] = f;
@@ -530,35 +570,41 @@ __global__ void __launch_bounds__(kResThreads, 1)
     for (int li = tid; li < no; li += NT) {
         const int i = node_of(li);
         if (i >= d.n) continue;
-        double2 v = s_v[li];
-        const double2 f = s_ff[li];
+        double2 v = kStream ? d.v[i] : s_v[li];
+        const double2 f = kStream ? d.f[i] : s_ff[li];
         res_mix(s_sc, v, f);
         d.x[i] = s_x[li];
         d.v[i] = v;
-        d.f[i] = f;
+        if (!kStream) d.f[i] = f;
     }
     if (blockIdx.x == 0 && tid == 0) scal_store(d.st, s_sc);
 }
 
-static const void *res_kernel(bool gel) {
-    return gel ? (const void *)k_fire_res64<true> : (const void *)k_fire_res64<false>;
+static const void *res_kernel(bool gel, int mode) {
+    if (mode == kResPairs) return gel ? (const void *)k_fire_res64<true, kResPairs> : (const void *)k_fire_res64<false, kResPairs>;
+    if (mode == kResStream)
+        return gel ? (const void *)k_fire_res64<true, kResStream> : (const void *)k_fire_res64<false, kResStream>;
+    return gel ? (const void *)k_fire_res64<true, kResWhole> : (const void *)k_fire_res64<false, kResWhole>;
 }
 
-/* Largest dynamic shared memory of the kernel on this device. */
+/* Largest dynamic shared memory of the kernel on this device (NR_RES64_SMEM:
+ * bytes to stay below). */
 size_t res64_smem_limit() {
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return 0;
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, res_kernel(true)) != cudaSuccess) return 0;
-    return optin > (int)fa.sharedSizeBytes ? (size_t)(optin - (int)fa.sharedSizeBytes) : 0;
+    if (cudaFuncGetAttributes(&fa, res_kernel(true, kResStream)) != cudaSuccess) return 0;
+    const size_t most = optin > (int)fa.sharedSizeBytes ? (size_t)(optin - (int)fa.sharedSizeBytes) : 0;
+    const char *env = getenv("NR_RES64_SMEM");
+    return env ? std::min(most, (size_t)std::max(0, atoi(env))) : most;
 }
 
 /* Whether `ctas` CTAs of the kernel are co-resident. */
-bool res64_fits(int ctas, bool gel, size_t smem) {
+bool res64_fits(int ctas, bool gel, int mode, size_t smem) {
     int dev = 0, sms = 0, per_sm = 0;
-    const void *k = res_kernel(gel);
+    const void *k = res_kernel(gel, mode);
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
@@ -571,7 +617,7 @@ bool res64_fits(int ctas, bool gel, size_t smem) {
 
 cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
                             unsigned long long budget_ns, cudaStream_t stream) {
-    const void *k = res_kernel(d.use_gel != 0);
+    const void *k = res_kernel(d.use_gel != 0, r.mode);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(r.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
@@ -630,8 +676,8 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
     if (n <= 0 || max_ctas < 1) return NR_ERR_INVALID;
     /* duplicate vertices without elements: the other kernels */
     if (nel == 0 && h.n_mesh_pairs() > 0) return NR_ERR_CAPACITY;
-    /* about 230 bytes of shared memory a node at the least */
-    if ((size_t)n * 230 > (size_t)max_ctas * smem_limit) return NR_ERR_CAPACITY;
+    /* shared memory at the least: x, the bonds' and triples' forces */
+    if (16.0 * n + 16.0 * ne + 32.0 * nt + 32.0 * nel > (double)max_ctas * smem_limit) return NR_ERR_CAPACITY;
     /* candidates: units of `sub` chunks dealt to S strips of y, each cut in
      * c columns of x.  Cuts move by up to a tenth of a strip (column) to the
      * widest gap nearby, so that strips end between rows and columns between
@@ -880,8 +926,8 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
         td.has_kb = has_kb;
         td.has_phi = has_phi;
         td.has_gel = nel > 0;
-        const Res64Segs g = res64_segs(td);
-        if (g.total > smem_limit) {
+        const Res64Segs g = res64_segs(td, kResWhole);
+        if (res64_segs(td, kResPairs).total > smem_limit) {
             failed[t] = 1;
             return;
         }
@@ -947,7 +993,7 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
     for (const auto &hal : halos)
         for (int i : hal) wanted[i] = 1;
     for (int t = 0; t < T; ++t) {
-        const Res64Segs g = res64_segs(out.desc[t]);
+        const Res64Segs g = res64_segs(out.desc[t], kResWhole);
         for (int u = 0; u < out.desc[t].nu; ++u)
             for (int k = 0; k < un; ++k) {
                 const int i = tu[t][u] * un + k;
@@ -955,7 +1001,11 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
             }
         out.desc[t].ro_off = (long long)out.ro.size();
         out.ro.insert(out.ro.end(), rec[t].begin(), rec[t].end());
-        out.max_smem = std::max(out.max_smem, (size_t)g.total);
+    }
+    for (out.mode = kResWhole;; ++out.mode) {
+        out.max_smem = 0;
+        for (const Res64Desc &td : out.desc) out.max_smem = std::max(out.max_smem, (size_t)res64_segs(td, out.mode).total);
+        if (out.max_smem <= smem_limit) break; /* at kResPairs at the latest (above) */
     }
     return NR_OK;
 }
@@ -981,7 +1031,7 @@ extern "C" int nr_res64_layout_check(const nr_host_network *h, int ctas, long lo
     std::vector<int> owned(n, 0), wanted(n, 0), published(n, 0);
     if (L.n_ctas > ctas || (int)L.desc.size() != L.n_ctas) ++bad;
     for (const Res64Desc &td : L.desc) {
-        const Res64Segs g = res64_segs(td);
+        const Res64Segs g = res64_segs(td, L.mode);
         if (td.ro_off % 16 || td.ro_off + (long long)g.rec > (long long)L.ro.size() || g.total > (unsigned)smem_limit ||
             g.total > L.max_smem || td.no != td.nu * un) {
             ++bad;

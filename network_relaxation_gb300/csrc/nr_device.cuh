@@ -275,7 +275,14 @@ struct Res64Segs {
 __host__ __device__ inline unsigned res64_groups(const Res64Desc &t) {
     return (unsigned)((t.nb + 31) / 32 + (t.nt + 31) / 32 + (t.nel + 31) / 32);
 }
-__host__ __device__ inline Res64Segs res64_segs(const Res64Desc &t) {
+/* Where a tile lives. kResStream: the record stays in global memory but for
+ * the unit numbers, and so do v, F and the elements' reference inverses; the
+ * working arrays the items and the gather reach at random share what that
+ * frees. kResPairs: as well, a triple's hinge force is formed by the gather
+ * from the other two instead of being kept beside them. */
+enum { kResWhole, kResStream, kResPairs, kResModes };
+__host__ __device__ inline Res64Segs res64_segs(const Res64Desc &t, int mode) {
+    const bool stream = mode != kResWhole;
     Res64Segs g;
     unsigned o = 0;
     auto seg = [&o](unsigned bytes) {
@@ -300,20 +307,22 @@ __host__ __device__ inline Res64Segs res64_segs(const Res64Desc &t) {
     g.bwrap = seg(1u * t.nb);
     g.pub = seg(1u * t.no);
     g.rec = o;
-    const unsigned local = (unsigned)(t.no + t.nh);
+    if (stream) o = tile_pad16(4u * t.nu);
+    const unsigned local = (unsigned)(t.no + t.nh), own = stream ? 0u : (unsigned)t.no;
     g.x = seg(16u * local);
-    g.v = seg(16u * t.no);
-    g.f = seg(16u * (t.has_gel ? local : (unsigned)t.no));
-    g.ff = seg(t.has_gel ? 16u * t.no : 0u);
+    g.v = seg(16u * own);
+    g.f = seg(16u * (t.has_gel ? local : own));
+    g.ff = seg(t.has_gel ? 16u * own : 0u);
     g.bf = seg(16u * t.nb);
-    g.tf = seg(48u * t.nt);
-    g.eM = seg(64u * t.nel);
+    g.tf = seg((mode == kResPairs ? 32u : 48u) * t.nt);
+    g.eM = seg(stream ? 0u : 64u * t.nel);
     g.du = seg(32u * t.nel);
     g.total = o;
     return g;
 }
 struct Res64Dev {
     int n_ctas, sub, n_units;       /* CTAs (tiles); chunks per unit; units, padded to whole 256-node tiles */
+    int mode;                       /* which k_fire_res64 (res64_segs) */
     const Res64Desc *desc;
     const unsigned char *ro;
     double2 *vf[2];                 /* published {v, F} per node, by step parity */
