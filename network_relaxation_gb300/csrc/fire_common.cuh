@@ -79,10 +79,8 @@ __device__ __forceinline__ void gel_add(double4 t, double &fx, double &fy) {
     fy = fy + t.w;
 }
 
-/* Masked force on node i from its bonds, triples and (kGel) gel elements,
- * in the canonical order.  The mixed-precision kernels never carry a gel
- * and instantiate kGel = false. */
-template <bool kGel = true>
+/* Masked force on node i from its bonds and triples, in the canonical order
+ * (the anchors of the mixed-precision kernels, which never carry a gel). */
 __device__ __forceinline__ void node_force_fp64_own(const NetDev &d, int i, double &fx, double &fy) {
     fx = 0.0;
     fy = 0.0;
@@ -134,35 +132,8 @@ __device__ __forceinline__ void node_force_fp64_own(const NetDev &d, int i, doub
             }
         }
     }
-    if (kGel && d.use_gel) {
-        const NetGel &g = *d.gel;
-        const int e1 = g.eptr[i + 1];
-        for (int e = g.eptr[i]; e < e1; ++e) {
-            const int code = g.eent[e];
-            const int el = code / 3, r = code - 3 * el;
-            double du11, du12, du21, du22;
-            gel_du(d, el, du11, du12, du21, du22);
-            gel_add(gel_terms(d, el, r, du11, du12, du21, du22), fx, fy);
-        }
-    }
     if (!(c & 1)) fx = 0.0;
     if (!(c & 2)) fy = 0.0;
-}
-
-/* Force on node i: its own masked sum plus, for a duplicate mesh vertex,
- * its partner's (duplicate_forces, network_mesh_relax.cu:754-780, unmasked;
- * a + b and b + a round alike, so both vertices get the same value). */
-__device__ __forceinline__ void node_force_fp64(const NetDev &d, int i, double &fx, double &fy) {
-    node_force_fp64_own(d, i, fx, fy);
-    if (d.use_gel) {
-        const int q = d.gel->partner[i];
-        if (q >= 0) {
-            double gx, gy;
-            node_force_fp64_own(d, q, gx, gy);
-            fx = fx + gx;
-            fy = fy + gy;
-        }
-    }
 }
 
 /* Item pass of the FP64 force: every bond force (the value its first
@@ -170,37 +141,40 @@ __device__ __forceinline__ void node_force_fp64(const NetDev &d, int i, double &
  * scratch, items b = first, first + stride, ...  GB300's FP64 pipe is the
  * bound of the plain path, and the per-node gather below would otherwise
  * evaluate each bond twice and each triple three times. */
+__device__ __forceinline__ void bond_item(const NetDev &d, int b) {
+    const int4 r = d.bond[b];
+    const double2 p1 = d.x[r.x], p2 = d.x[r.y];
+    const double k = d.bond_k ? d.bond_k[b] : d.ks;
+    double fx, fy;
+    bond_force(p1.x, p1.y, p2.x, p2.y, wrap_shift(r.z, d.width), d.bond_l0[b], k, fx, fy);
+    d.bfrc[b] = make_double2(fx, fy);
+}
+__device__ __forceinline__ void triple_item(const NetDev &d, int t) {
+    const double W = d.width;
+    const int4 r = d.tri[t];
+    const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
+    const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
+    const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
+    const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
+    const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
+    const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
+    double fjx, fjy, fkx, fky;
+    bend_force(ax, ay, bx, by, kb, phi0, fjx, fjy, fkx, fky);
+    d.tfrc[t] = make_double4(fjx, fjy, fkx, fky);
+}
+__device__ __forceinline__ void gel_item(const NetDev &d, int e) {
+    double du11, du12, du21, du22;
+    gel_du(d, e, du11, du12, du21, du22);
+    for (int r = 0; r < 3; ++r) d.gel->efrc[3 * (size_t)e + r] = gel_terms(d, e, r, du11, du12, du21, du22);
+}
 template <bool kGel>
 __device__ inline void items_pass(const NetDev &d, int first, int stride) {
-    const double W = d.width;
     if (d.use_bonds)
-        for (int b = first; b < d.n_edges; b += stride) {
-            const int4 r = d.bond[b];
-            const double2 p1 = d.x[r.x], p2 = d.x[r.y];
-            const double k = d.bond_k ? d.bond_k[b] : d.ks;
-            double fx, fy;
-            bond_force(p1.x, p1.y, p2.x, p2.y, wrap_shift(r.z, W), d.bond_l0[b], k, fx, fy);
-            d.bfrc[b] = make_double2(fx, fy);
-        }
+        for (int b = first; b < d.n_edges; b += stride) bond_item(d, b);
     if (d.use_triples)
-        for (int t = first; t < d.n_triples; t += stride) {
-            const int4 r = d.tri[t];
-            const double2 ph = d.x[r.x], pj = d.x[r.y], pk = d.x[r.z];
-            const int wj = (signed char)(r.w & 0xff), wk = (signed char)((r.w >> 8) & 0xff);
-            const double ax = wrap_add(pj.x, wj, W) - ph.x, ay = pj.y - ph.y;
-            const double bx = wrap_add(pk.x, wk, W) - ph.x, by = pk.y - ph.y;
-            const double kb = d.tri_kb ? d.tri_kb[t] : d.kb;
-            const double phi0 = d.tri_phi0 ? d.tri_phi0[t] : 0.0;
-            double fjx, fjy, fkx, fky;
-            bend_force(ax, ay, bx, by, kb, phi0, fjx, fjy, fkx, fky);
-            d.tfrc[t] = make_double4(fjx, fjy, fkx, fky);
-        }
+        for (int t = first; t < d.n_triples; t += stride) triple_item(d, t);
     if (kGel && d.use_gel)
-        for (int e = first; e < d.n_elems; e += stride) {
-            double du11, du12, du21, du22;
-            gel_du(d, e, du11, du12, du21, du22);
-            for (int r = 0; r < 3; ++r) d.gel->efrc[3 * (size_t)e + r] = gel_terms(d, e, r, du11, du12, du21, du22);
-        }
+        for (int e = first; e < d.n_elems; e += stride) gel_item(d, e);
 }
 
 /* Per-node gather of the item forces in the canonical order; the same bits
@@ -243,8 +217,10 @@ __device__ __forceinline__ void node_force_items_own(const NetDev &d, int i, dou
     if (!(c & 2)) fy = 0.0;
 }
 
-/* node_force_fp64 from the item scratch.  kGel = false compiles the gel
- * terms out (networks without a gel). */
+/* Force on node i: its own masked sum plus, for a duplicate mesh vertex,
+ * its partner's (duplicate_forces, network_mesh_relax.cu:754-780, unmasked;
+ * a + b and b + a round alike, so both vertices get the same value).  kGel =
+ * false compiles the gel terms out (networks without a gel). */
 template <bool kGel>
 __device__ __forceinline__ void node_force_items(const NetDev &d, int i, double &fx, double &fy) {
     node_force_items_own<kGel>(d, i, fx, fy);
@@ -393,16 +369,8 @@ __device__ inline void energy_tiles(const NetDev &d, int t0, int tstride, double
             }
         }
         if (in_tile) { /* warp-uniform: kTile is a multiple of 32 */
-            e = warp_sum(e);
-            wxx = warp_sum(wxx);
-            wyy = warp_sum(wyy);
-            wxy = warp_sum(wxy);
-            if (lane == 0) {
-                s_red[warp] = e;
-                s_red[8 + warp] = wxx;
-                s_red[16 + warp] = wyy;
-                s_red[24 + warp] = wxy;
-            }
+            const double w = warp_sum4(e, wxx, wyy, wxy, lane);
+            if ((lane & 7) == 0) s_red[8 * ((lane >> 4) | (lane >> 2 & 2)) + warp] = w;
         }
         __syncthreads();
         if (threadIdx.x < 4 && (cat < 2 || threadIdx.x == 0)) {
@@ -416,25 +384,49 @@ __device__ inline void energy_tiles(const NetDev &d, int t0, int tstride, double
 /* Totals of the energy pass: energies and the virial {W_xx, W_yy, W_xy}
  * (bond sum + triple sum; the gel contributes no virial). */
 __device__ inline void energy_final(const NetDev &d, double *s_red, double &es, double &eb, double &eg,
-                                    double *vir = nullptr) {
+                                    double *vir) {
     const int tb = (d.n_edges + kTile - 1) / kTile, tt = (d.n_triples + kTile - 1) / kTile;
     const int tg = (d.n_elems + kTile - 1) / kTile;
     const size_t M = (size_t)energy_stride(d);
-    es = 0.0;
-    eb = 0.0;
-    eg = 0.0;
-    double wb[3] = {0.0, 0.0, 0.0}, wt[3] = {0.0, 0.0, 0.0};
-    const bool bonds = d.use_bonds && d.n_edges > 0, tris = d.use_triples && d.n_triples > 0;
-    if (bonds) es = final_sum(d.epart, tb, 8, s_red);
-    if (tris) eb = final_sum(d.epart + 4 * M, tt, 8, s_red);
-    if (d.use_gel && d.n_elems > 0) eg = final_sum(d.epart + 8 * M, tg, 8, s_red);
-    if (vir) {
-        for (int c = 0; c < 3; ++c) {
-            if (bonds) wb[c] = final_sum(d.epart + (1 + c) * M, tb, 8, s_red);
-            if (tris) wt[c] = final_sum(d.epart + (5 + c) * M, tt, 8, s_red);
-            vir[c] = wb[c] + wt[c];
+    /* four lists at a time: a warp for every list and lane group of the
+     * canonical sum (final_sum), then a lane for every list's tree */
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double w[kEpartLists];
+#pragma unroll
+    for (int q0 = 0; q0 < kEpartLists; q0 += 4) {
+        const int n_tiles = q0 == 0 ? (d.use_bonds ? tb : 0) : q0 == 4 ? (d.use_triples ? tt : 0) : (d.use_gel ? tg : 0);
+        const int lists = min(4, kEpartLists - q0);
+        for (int c = warp; c < 8 * lists; c += nw) {
+            const double *p = d.epart + (size_t)(q0 + (c >> 3)) * M;
+            const int k = 32 * (c & 7) + lane;
+            double acc = 0.0;
+            if (32 * (c & 7) < n_tiles) {
+                if (k < n_tiles) {
+                    acc = __ldcg(p + k);
+                    for (int t = k + kTile; t < n_tiles; t += kTile) acc = acc + __ldcg(p + t);
+                }
+                acc = warp_sum(acc);
+            }
+            if (lane == 0) s_red[c] = acc;
         }
+        __syncthreads();
+        double t = 0.0;
+        if (warp == 0 && n_tiles > 0) {
+            if (lane < lists) t = tree8(s_red + 8 * lane);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (q0 + c < kEpartLists) w[q0 + c] = __shfl_sync(kFull, t, c);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (q0 + c < kEpartLists) w[q0 + c] = 0.0;
+        }
+        __syncthreads();
     }
+    es = w[0];
+    eb = w[4];
+    eg = w[8];
+    for (int c = 0; c < 3; ++c) vir[c] = w[1 + c] + w[5 + c];
 }
 
 }  // namespace nr

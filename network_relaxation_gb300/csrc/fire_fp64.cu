@@ -179,13 +179,22 @@ __global__ void k_fire_grid(NetDev d, FireParamsDev p, unsigned long long budget
     }
 }
 
-__global__ void k_energy_tiles(NetDev d) {
-    __shared__ double s_red[32]; /* one slot per warp, up to 1024 threads */
+/* Energies and virial of one network: the tiles' partials, then the last CTA
+ * takes the totals.  Bound by latency (a chain of FP64 operations at 64
+ * clocks each): a kernel for the tiles and one for the totals, one list after
+ * the other by all threads alike, took 10 and 12 us at 1 024 nodes; a call of
+ * nr_energies 41 -> 28 us there, 200 -> 101 at 250 000 nodes. */
+__global__ void __launch_bounds__(kTile) k_energies(NetDev d) {
+    __shared__ double s_red[32];
+    __shared__ int s_last;
     energy_tiles(d, blockIdx.x, gridDim.x, s_red);
-}
-
-__global__ void k_energy_final(NetDev d) {
-    __shared__ double s_red[32]; /* one slot per warp, up to 1024 threads */
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicInc(&d.st->energy_count, gridDim.x - 1) == gridDim.x - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
     double es, eb, eg, vir[3];
     energy_final(d, s_red, es, eb, eg, vir);
     if (threadIdx.x == 0) {
@@ -361,12 +370,78 @@ __global__ void __launch_bounds__(kTile, 1)
     }
 }
 
-__global__ void k_forces(NetDev d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+/* Forces at the current positions: every item once (a thread each, small
+ * CTAs, so that a small network's items meet on few FP64 pipes), then the
+ * nodes' sums.  A thread per node that evaluated the node's items itself (each
+ * bond twice, each triple three times, one after the other) took 36 us of
+ * device time at 1 024 nodes on four SMs, these two 14; a call of nr_forces 53
+ * -> 30 us there, 100 at 250 000 nodes (a good part of it the copy to the
+ * host). */
+constexpr int kForceThreads = 64;
+template <bool kGel>
+__global__ void __launch_bounds__(kForceThreads) k_force_items(NetDev d, int bt, int be) {
+    int b = (int)blockIdx.x;
+    if (b < bt) { /* triples first: the longest */
+        const int t = b * kForceThreads + threadIdx.x;
+        if (t < d.n_triples) triple_item(d, t);
+        return;
+    }
+    b -= bt;
+    if (kGel && b < be) {
+        const int e = b * kForceThreads + threadIdx.x;
+        if (e < d.n_elems) gel_item(d, e);
+        return;
+    }
+    b = (b - be) * kForceThreads + threadIdx.x;
+    if (b < d.n_edges) bond_item(d, b);
+}
+/* Component c of node i's own masked force (node_force_items_own's sum). */
+template <bool kGel>
+__device__ __forceinline__ double force_component(const NetDev &d, int i, int c) {
+    double f = 0.0;
+    if (!(d.fcode[i] >> c & 1)) return f;
+    if (d.use_bonds) {
+        const double *bf = reinterpret_cast<const double *>(d.bfrc);
+        const int e1 = d.bptr[i + 1];
+#pragma unroll 4
+        for (int e = d.bptr[i]; e < e1; ++e) {
+            const int code = d.bent[e];
+            f = f + ii_flip(bf[2 * (size_t)(code >> 1) + c], (code & 1) != 0);
+        }
+    }
+    if (d.use_triples) {
+        const int e1 = d.tptr[i + 1];
+#pragma unroll 4
+        for (int e = d.tptr[i]; e < e1; ++e) {
+            const int code = d.tent[e], role = code & 3;
+            const double *tf = reinterpret_cast<const double *>(d.tfrc) + 4 * (size_t)(code >> 2) + c;
+            const double u = tf[role == 2 ? 2 : 0], w = tf[2];
+            f = f + (role == 0 ? ii_flip(u, true) - w : u);
+        }
+    }
+    if (kGel && d.use_gel) {
+        const NetGel &g = *d.gel;
+        const int e1 = g.eptr[i + 1];
+        for (int e = g.eptr[i]; e < e1; ++e) {
+            const double2 t = reinterpret_cast<const double2 *>(g.efrc + g.eent[e])[c];
+            f = f + t.x;
+            f = f + t.y;
+        }
+    }
+    return f;
+}
+/* A thread per node and component: the chain of sums is what bounds it. */
+template <bool kGel>
+__global__ void __launch_bounds__(kForceThreads) k_force_nodes(NetDev d) {
+    const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(k >> 1), c = (int)(k & 1);
     if (i >= d.n) return;
-    double fx, fy;
-    node_force_fp64(d, i, fx, fy);
-    d.f[i] = make_double2(fx, fy);
+    double f = force_component<kGel>(d, i, c);
+    if (kGel && d.use_gel) {
+        const int q = d.gel->partner[i];
+        if (q >= 0) f = f + force_component<kGel>(d, q, c);
+    }
+    reinterpret_cast<double *>(d.f)[2 * (size_t)i + c] = f;
 }
 
 /* affine_displace (large_strain_relax.cu:527-537) over N nodes; with
@@ -457,8 +532,7 @@ cudaError_t launch_fp64_grid(const NetDev &d, const FireParamsDev &p, int blocks
 }
 
 cudaError_t launch_energies(const NetDev &d, int blocks, cudaStream_t stream) {
-    k_energy_tiles<<<blocks, kTile, 0, stream>>>(d);
-    k_energy_final<<<1, kTile, 0, stream>>>(d);
+    k_energies<<<blocks, kTile, 0, stream>>>(d);
     return cudaGetLastError();
 }
 
@@ -529,7 +603,15 @@ cudaError_t launch_fp64_cluster(const NetDev *nets_dev, int n_nets, int cluster,
 }
 
 cudaError_t launch_forces(const NetDev &d, cudaStream_t stream) {
-    k_forces<<<(d.n + 255) / 256, 256, 0, stream>>>(d);
+    auto blocks = [](int n) { return (n + kForceThreads - 1) / kForceThreads; };
+    const int bt = d.use_triples ? blocks(d.n_triples) : 0, be = d.use_gel ? blocks(d.n_elems) : 0,
+              bb = d.use_bonds ? blocks(d.n_edges) : 0, bn = (int)(((long)2 * d.n + kForceThreads - 1) / kForceThreads);
+    if (bt + be + bb > 0) {
+        if (d.use_gel) k_force_items<true><<<bt + be + bb, kForceThreads, 0, stream>>>(d, bt, be);
+        else k_force_items<false><<<bt + bb, kForceThreads, 0, stream>>>(d, bt, 0);
+    }
+    if (d.use_gel) k_force_nodes<true><<<bn, kForceThreads, 0, stream>>>(d);
+    else k_force_nodes<false><<<bn, kForceThreads, 0, stream>>>(d);
     return cudaGetLastError();
 }
 

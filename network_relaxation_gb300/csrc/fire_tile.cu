@@ -233,7 +233,7 @@ static __device__ __noinline__ void tile_anchor_eval(const NetDev &d, const NetT
         const int i = tl.node_of_pos[p];
         if (i < 0) continue;
         double fx, fy;
-        node_force_fp64_own<false>(d, i, fx, fy);
+        node_force_fp64_own(d, i, fx, fy);
         d.f[i] = make_double2(fx, fy);
         const float hx = (float)fx, hy = (float)fy;
         tl.fa[p] = make_float4(hx, hy, (float)(fx - (double)hx), (float)(fy - (double)hy));

@@ -565,7 +565,7 @@ static __device__ __noinline__ void anchor_eval(const NetDev &d, const Team &tm,
         }
     for (int i = tm.first(); i < d.n; i += tm.stride()) {
         double fx, fy;
-        node_force_fp64_own<false>(d, i, fx, fy);
+        node_force_fp64_own(d, i, fx, fy);
         d.f[i] = make_double2(fx, fy);
         const float hx = (float)fx, hy = (float)fy;
         d.fa_hi[i] = make_float2(hx, hy);

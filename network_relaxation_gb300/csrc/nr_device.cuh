@@ -76,7 +76,8 @@ struct __align__(128) FireState {
     double vir[3];  /* virial {W_xx, W_yy, W_xy} of the stretch and bending forces */
     int pad[2];
     unsigned int bar_count, bar_gen, abort_flag, timeout_site;
-    unsigned int pad2[28];
+    unsigned int energy_count; /* CTAs of k_energies that are done; back to 0 with the last */
+    unsigned int pad2[27];
 };
 
 struct NetDev {
@@ -337,6 +338,20 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_xor_sync(kFull, v, off);
     return v;
+}
+/* Four warp sums (warp_sum's order each) in 6 additions where one by one take
+ * 20: after xor 16 and 8 every lane carries one sum, number (lane >> 4) |
+ * (lane >> 2 & 2). */
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double e, int lane) {
+    const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
+    double u = b4 ? b : a, v = b4 ? e : c;
+    u = u + __shfl_xor_sync(kFull, b4 ? a : b, 16);
+    v = v + __shfl_xor_sync(kFull, b4 ? c : e, 16);
+    double w = b3 ? v : u;
+    w = w + __shfl_xor_sync(kFull, b3 ? u : v, 8);
+    w = w + __shfl_xor_sync(kFull, w, 4);
+    w = w + __shfl_xor_sync(kFull, w, 2);
+    return w + __shfl_xor_sync(kFull, w, 1);
 }
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
