@@ -10,7 +10,8 @@
  * value a step writes and reads back is on chip:
  *   per node (owner CTA)   x, v, F (double2 each)
  *   per item (owner CTA)   the bond's force on its node i (double2), the
- *                          triple's forces on j and k (double4)
+ *                          triple's forces on hinge, j and k (three double2;
+ *                          two, j and k, where three do not fit)
  *   per 32-node chunk      its partial sums of P, |v|^2, |F|^2, max |F|^2
  * A CTA reads other CTAs' positions (item pass), item forces (gather) and
  * chunk partials (reduction) with ld.shared::cluster after the hardware
@@ -24,14 +25,24 @@
  * references, rest length, stiffness, wraps, incidence range) is loaded
  * once per relaxation into registers.
  *
+ * What bounds it: a step of a small network the chain of FP64 operations (64
+ * clocks each for a lone warp) and remote loads, about 11 us; a full GPU the
+ * FP64 pipes.  So the sums of a chunk share one butterfly (6 additions instead
+ * of 15, and the maxima as integers), a triple's hinge force is formed once
+ * instead of at each of its entries, only the lane groups of the canonical sum
+ * that hold a tile are summed (the others cost 250 FP64 instructions a CTA and
+ * step), a tile's partials and four entries of the gather are loaded at once,
+ * and a warp advances the scalars (scal_warp).  100 steps of 64 lattices of 16^2
+ * to 96^2 nodes 16.3 -> 10.8 ms, of 9 of up to 33^2 2.2 -> 1.35 ms.
+ *
  * Compiled with --fmad=false: the same bits as the oracle.
  */
 #include <cooperative_groups.h>
 
 #include <algorithm>
 
-#include "fire_common.cuh"
 #include "fire_launch.h"
+#include "fp64_step.cuh"
 
 namespace nr {
 
@@ -53,16 +64,18 @@ __device__ __forceinline__ double cl_ld1d(unsigned a) {
     asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
     return v;
 }
-__device__ __forceinline__ double4 cl_ld4d(unsigned a) {
-    const double2 lo = cl_ld2d(a), hi = cl_ld2d(a + 16u);
-    return make_double4(lo.x, lo.y, hi.x, hi.y);
+__device__ __forceinline__ unsigned long long cl_ld1u(unsigned a) {
+    unsigned long long v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a));
+    return v;
 }
 
 }  // namespace
 
-/* Per-CTA maxima of a launch: nodes, bond slots, triple slots. */
+/* Per-CTA maxima of a launch: nodes, bond slots, triple slots; pairs: two
+ * forces a triple (j, k) instead of three, where three do not fit. */
 struct Dsm64Sizes {
-    int bmax, emax, tmax;
+    int bmax, emax, tmax, pairs;
 };
 struct Dsm64Layout {
     size_t x, v, f, bf, tf, part, total;
@@ -74,7 +87,7 @@ __host__ __device__ inline Dsm64Layout dsm64_layout(const Dsm64Sizes &z) {
     L.v = o;  o += 16 * (size_t)z.bmax;
     L.f = o;  o += 16 * (size_t)z.bmax;
     L.bf = o; o += 16 * (size_t)z.emax;
-    L.tf = o; o += 32 * (size_t)z.tmax;
+    L.tf = o; o += (z.pairs ? 32 : 48) * (size_t)z.tmax;
     L.part = o; o += 4 * 8 * (size_t)((z.bmax + kChunk - 1) / kChunk);
     L.total = o;
     return L;
@@ -82,6 +95,7 @@ __host__ __device__ inline Dsm64Layout dsm64_layout(const Dsm64Sizes &z) {
 
 constexpr int kDsm64Threads = 256;
 
+template <bool kPairs>
 __global__ void __launch_bounds__(kDsm64Threads, 2)
     k_fire_dsm64(const NetDev *nets, const NetDsm *dsms, int n_nets, FireParamsDev p, int *queue, const int *order,
                  Dsm64Sizes z) {
@@ -94,7 +108,7 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
     double2 *s_v = reinterpret_cast<double2 *>(dyn + L.v);
     double2 *s_f = reinterpret_cast<double2 *>(dyn + L.f);
     double2 *s_bf = reinterpret_cast<double2 *>(dyn + L.bf);
-    double4 *s_tf = reinterpret_cast<double4 *>(dyn + L.tf);
+    double2 *s_tf = reinterpret_cast<double2 *>(dyn + L.tf); /* hinge (not kPairs), j, k of every triple */
     double *s_part = reinterpret_cast<double *>(dyn + L.part); /* [q * umax + local chunk] */
     const int umax = (z.bmax + kChunk - 1) / kChunk;
     __shared__ NetDev s_d;
@@ -102,9 +116,11 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
     __shared__ Scal s_sc;
     __shared__ int s_slot;
     __shared__ double s_red[32];
+    __shared__ unsigned long long s_wmax[kDsm64Threads / 32]; /* bits of max |F|^2 */
     __shared__ unsigned s_ax[kDsmParts], s_abf[kDsmParts], s_atf[kDsmParts], s_apt[kDsmParts];
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const int spr = kDsmParts / C, lg = __ffs(spr) - 1;
+    constexpr int NW = kDsm64Threads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)threadIdx.x < C) {
         s_ax[threadIdx.x] = cl_addr(s_x, threadIdx.x);
@@ -131,7 +147,6 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
         const int b0 = m.bo[rank * spr], b1 = m.bo[(rank + 1) * spr];
         const int t0 = m.to[rank * spr], t1 = m.to[(rank + 1) * spr];
         const double W = d.width;
-        const int n_units = d.n_tiles * 8;
         /* positions in */
         for (int li = threadIdx.x; li < nloc; li += blockDim.x) s_x[li] = d.x[n0 + li];
         /* the thread's first bond and triple, cached for the relaxation */
@@ -171,13 +186,16 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
             bond_force(p1.x, p1.y, p2.x, p2.y, wW, l0, k, fx, fy);
             return make_double2(fx, fy);
         };
-        auto tri_item = [&](int rh, int rj, int rk, double wj, double wk, double kb, double phi0) -> double4 {
+        auto tri_item = [&](int k, int rh, int rj, int rk, double wj, double wk, double kb, double phi0) {
             const double2 ph = cl_ld2d(xaddr(rh)), pj = cl_ld2d(xaddr(rj)), pk = cl_ld2d(xaddr(rk));
             const double ax = (pj.x + wj) - ph.x, ay = pj.y - ph.y;
             const double bx = (pk.x + wk) - ph.x, by = pk.y - ph.y;
             double fjx, fjy, fkx, fky;
             bend_force(ax, ay, bx, by, kb, phi0, fjx, fjy, fkx, fky);
-            return make_double4(fjx, fjy, fkx, fky);
+            double2 *const out = s_tf + (kPairs ? 2 * k : 3 * k + 1);
+            out[0] = make_double2(fjx, fjy);
+            out[1] = make_double2(fkx, fky);
+            if (!kPairs) out[-1] = make_double2(ii_flip(fjx, true) - fkx, ii_flip(fjy, true) - fky);
         };
         bool init = true;
         for (;;) {
@@ -187,18 +205,9 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
                 for (int li = threadIdx.x; li < nloc; li += blockDim.x) {
                     double2 xi = s_x[li], vi = s_v[li];
                     const double2 fi = s_f[li];
-                    if (s.mix_pending) {
-                        vi.x = fma(s.mix_na, vi.x, vi.x);
-                        vi.y = fma(s.mix_na, vi.y, vi.y);
-                        vi.x = fma(s.mix_a, fi.x, vi.x);
-                        vi.y = fma(s.mix_a, fi.y, vi.y);
-                        if (s.zero_v) vi = make_double2(0.0, 0.0);
-                    }
+                    res_mix(s, vi, fi);
                     if (!s.done) {
-                        xi.x = fma(s.dt, vi.x, xi.x);
-                        xi.y = fma(s.dt, vi.y, xi.y);
-                        xi.x = fma(s.dtsq, fi.x, xi.x);
-                        xi.y = fma(s.dtsq, fi.y, xi.y);
+                        res_drift(s, xi, vi, fi);
                         vi.x = fma(s.dtm, fi.x, vi.x);
                         vi.y = fma(s.dtm, fi.y, vi.y);
                         s_x[li] = xi;
@@ -216,13 +225,13 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
                 s_bf[k] = bond_item(r.x, r.y, wrap_shift(__ldg(&d.bond[b].z), W), __ldg(d.bond_l0 + b),
                                     d.bond_k ? __ldg(d.bond_k + b) : d.ks);
             }
-            if ((int)threadIdx.x < nt) s_tf[threadIdx.x] = tri_item(ct_h, ct_j, ct_k, ct_wj, ct_wk, ct_kb, ct_phi);
+            if ((int)threadIdx.x < nt) tri_item(threadIdx.x, ct_h, ct_j, ct_k, ct_wj, ct_wk, ct_kb, ct_phi);
             for (int k = threadIdx.x + blockDim.x; k < nt; k += blockDim.x) {
                 const int4 r = __ldg(m.tref + t0 + k);
                 const int w = __ldg(&d.tri[r.w].w);
-                s_tf[k] = tri_item(r.x, r.y, r.z, wrap_shift((signed char)(w & 0xff), W),
-                                   wrap_shift((signed char)((w >> 8) & 0xff), W), d.tri_kb ? __ldg(d.tri_kb + r.w) : d.kb,
-                                   d.tri_phi0 ? __ldg(d.tri_phi0 + r.w) : 0.0);
+                tri_item(k, r.x, r.y, r.z, wrap_shift((signed char)(w & 0xff), W),
+                         wrap_shift((signed char)((w >> 8) & 0xff), W), d.tri_kb ? __ldg(d.tri_kb + r.w) : d.kb,
+                         d.tri_phi0 ? __ldg(d.tri_phi0 + r.w) : 0.0);
             }
             cl.sync();
             /* gather, half kick (v = 0 at the start), chunk partials; warp w
@@ -238,30 +247,40 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
                     if (fc != 0) {
                         if (d.use_bonds) {
                             const int e1 = __ldg(d.bptr + i + 1);
+#pragma unroll 4
                             for (int e = __ldg(d.bptr + i); e < e1; ++e) {
                                 const unsigned code = (unsigned)__ldg(m.bent + e);
                                 const int r = (int)(code >> 28) >> lg;
                                 const int ls = (int)((code >> 1) & 0x7ffffffu) - m.bo[r * spr];
                                 const double2 f = cl_ld2d(s_abf[r] + 16u * (unsigned)ls);
-                                /* a select, not a branch: the same sum */
-                                fx = fx + ((code & 1) ? -f.x : f.x);
-                                fy = fy + ((code & 1) ? -f.y : f.y);
+                                fx = fx + ii_flip(f.x, (code & 1) != 0);
+                                fy = fy + ii_flip(f.y, (code & 1) != 0);
                             }
                         }
                         if (d.use_triples) {
                             const int e1 = __ldg(d.tptr + i + 1);
+#pragma unroll 4
                             for (int e = __ldg(d.tptr + i); e < e1; ++e) {
                                 const unsigned code = (unsigned)__ldg(m.tent + e);
                                 const int r = (int)(code >> 28) >> lg;
-                                const int role = code & 3;
                                 const int ls = (int)((code >> 2) & 0x3ffffffu) - m.to[r * spr];
-                                const double4 f = cl_ld4d(s_atf[r] + 32u * (unsigned)ls);
-                                /* selects, not a branch per role: the same
-                                 * operands and operations as the oracle's
-                                 * case-by-case sum */
-                                const double hx = (-f.x) - f.z, hy = (-f.y) - f.w;
-                                fx = fx + (role == 0 ? hx : (role == 1 ? f.x : f.z));
-                                fy = fy + (role == 0 ? hy : (role == 1 ? f.y : f.w));
+                                const unsigned role = code & 3u;
+                                if (kPairs) {
+                                    const unsigned at = s_atf[r] + 32u * (unsigned)ls;
+                                    const double2 f = cl_ld2d(at + (role == 2u ? 16u : 0u));
+                                    if (role == 0u) {
+                                        const double2 fk = cl_ld2d(at + 16u);
+                                        fx = fx + (ii_flip(f.x, true) - fk.x);
+                                        fy = fy + (ii_flip(f.y, true) - fk.y);
+                                    } else {
+                                        fx = fx + f.x;
+                                        fy = fy + f.y;
+                                    }
+                                } else {
+                                    const double2 f = cl_ld2d(s_atf[r] + 16u * (3u * (unsigned)ls + role));
+                                    fx = fx + f.x;
+                                    fy = fy + f.y;
+                                }
                             }
                         }
                         if (!(fc & 1)) fx = 0.0;
@@ -281,47 +300,60 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
                     tV = dot2(vi.x, vi.y, vi.x, vi.y);
                     tF = dot2(fx, fy, fx, fy);
                 }
-                const double sP = warp_sum(tP), sV = warp_sum(tV), sF = warp_sum(tF), sM = warp_max(tF);
-                if (lane == 0) {
-                    s_part[c] = sP;
-                    s_part[umax + c] = sV;
-                    s_part[2 * umax + c] = sF;
-                    s_part[3 * umax + c] = sM;
-                }
+                const double sum = warp_sum3(tP, tV, tF, lane);
+                const unsigned long long most = warp_max_bits(max_bits(tF));
+                if ((lane & 7) == 0) /* lanes 0, 16, 8: P, |v|^2, |F|^2; lane 24: max |F|^2 */
+                    s_part[(lane == 0 ? 0 : lane == 16 ? 1 : lane == 8 ? 2 : 3) * umax + c] =
+                        lane == 24 ? ii_double(most) : sum;
             }
             cl.sync();
             /* every CTA: the canonical totals over all chunks (units of one
-             * chunk, padded with zeros to whole 256-node tiles), then the
-             * FIRE scalars in thread 0 */
-            auto unit = [&](int q, int u) -> double {
-                if (u * kChunk >= d.n) return 0.0;
-                const int r = (u * kChunk) / per, lc = u - r * (per / kChunk);
-                return cl_ld1d(s_apt[r] + 8u * (unsigned)(q * umax + lc));
-            };
-            double tot[3];
-            for (int q = 0; q < 3; ++q) {
-                double acc = 0.0;
-                const int k = 32 * warp + lane; /* 8 warps: lane sums of tiles k, k + 256, ... */
+             * chunk, padded with zeros to whole 256-node tiles), all of a
+             * tile's loads in flight at once; then the FIRE scalars */
+            const int ng = min(8, (d.n_tiles + 31) / 32); /* lane groups that hold a tile */
+            unsigned long long mx = 0ULL;
+            if (warp < ng) { /* lane sums of tiles k, k + 256, ... */
+                const int k = 32 * warp + lane, cpr = per / kChunk;
+                double acc[3] = {0.0, 0.0, 0.0};
                 for (int t = k; t < d.n_tiles; t += kTile) {
-                    double u8[8];
-                    for (int j = 0; j < 8; ++j) u8[j] = unit(q, 8 * t + j);
-                    const double ts = ((u8[0] + u8[1]) + (u8[2] + u8[3])) + ((u8[4] + u8[5]) + (u8[6] + u8[7]));
-                    acc = t == k ? ts : acc + ts;
+                    int r = 8 * t / cpr, lc = 8 * t - r * cpr;
+                    double u8[3][8];
+                    unsigned long long m8[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        u8[0][j] = u8[1][j] = u8[2][j] = 0.0;
+                        m8[j] = 0ULL;
+                        if ((8 * t + j) * kChunk < d.n) {
+                            const unsigned at = s_apt[r] + 8u * (unsigned)lc;
+#pragma unroll
+                            for (int q = 0; q < 3; ++q) u8[q][j] = cl_ld1d(at + 8u * (unsigned)(q * umax));
+                            m8[j] = cl_ld1u(at + 24u * (unsigned)umax);
+                        }
+                        if (++lc == cpr) {
+                            lc = 0;
+                            ++r;
+                        }
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) mx = max(mx, m8[j]);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+                        const double *u = u8[q];
+                        const double ts = ((u[0] + u[1]) + (u[2] + u[3])) + ((u[4] + u[5]) + (u[6] + u[7]));
+                        acc[q] = t == k ? ts : acc[q] + ts;
+                    }
                 }
-                acc = warp_sum(acc);
-                if (lane == 0) s_red[8 * q + warp] = acc;
+                const double sum = warp_sum3(acc[0], acc[1], acc[2], lane);
+                if ((lane & 7) == 0 && lane != 24) s_red[8 * (lane == 0 ? 0 : lane == 16 ? 1 : 2) + warp] = sum;
+            } else if (lane < 3) {
+                s_red[8 * lane + warp] = 0.0;
             }
-            double mx = 0.0;
-            for (int u = threadIdx.x; u < n_units; u += blockDim.x) mx = fmax(mx, unit(3, u));
-            mx = warp_max(mx);
-            if (lane == 0) s_red[24 + warp] = mx;
+            mx = warp_max_bits(mx);
+            if (lane == 0) s_wmax[warp] = mx;
             __syncthreads();
-            if (threadIdx.x == 0) {
-                for (int q = 0; q < 3; ++q) tot[q] = tree8(s_red + 8 * q);
-                double M2 = s_red[24];
-                for (int w = 1; w < 8; ++w) M2 = fmax(M2, s_red[24 + w]);
-                if (init) scal_init(s_sc, p, tot[2], M2, d.sqrt_dof);
-                else scal_step(s_sc, p, tot[0], tot[1], tot[2], M2, d.sqrt_dof);
+            if (warp == 0) {
+                const unsigned long long most = warp_max_bits(lane < NW ? s_wmax[lane] : 0ULL);
+                scal_warp(s_sc, p, s_red, ng, most, d.sqrt_dof, init);
             }
             __syncthreads();
             init = false;
@@ -350,54 +382,75 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
     }
 }
 
-size_t dsm64_smem_bytes(int bmax, int emax, int tmax) { return dsm64_layout(Dsm64Sizes{bmax, emax, tmax}).total; }
+static const void *dsm64_kernel(bool pairs) {
+    return pairs ? (const void *)k_fire_dsm64<true> : (const void *)k_fire_dsm64<false>;
+}
 
-static cudaError_t dsm64_config(int cluster, size_t smem, cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr,
+/* The launch of a batch: three forces a triple, unless two leave room for
+ * more clusters on the GPU. */
+static cudaError_t dsm64_config(int cluster, Dsm64Sizes &z, cudaLaunchConfig_t &cfg, cudaLaunchAttribute *attr,
                                 int *max_clusters) {
     cudaError_t e;
-    int dev, sms;
+    int dev, sms, best = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_fire_dsm64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-        return e;
-    if (cluster > 8 &&
-        (e = cudaFuncSetAttribute(k_fire_dsm64, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
-        return e;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg = cudaLaunchConfig_t{};
     cfg.blockDim = dim3(kDsm64Threads);
-    cfg.dynamicSmemBytes = smem;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cfg.gridDim = dim3((sms / cluster) * cluster);
     *max_clusters = 0;
-    return cudaOccupancyMaxActiveClusters(max_clusters, (void *)k_fire_dsm64, &cfg);
+    cudaError_t failed = cudaSuccess;
+    for (int pairs = 0; pairs < 2; ++pairs) {
+        const void *k = dsm64_kernel(pairs != 0);
+        Dsm64Sizes y = z;
+        y.pairs = pairs;
+        cfg.dynamicSmemBytes = dsm64_layout(y).total;
+        int n = 0;
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            failed = e;
+        } else if (n > *max_clusters) {
+            *max_clusters = n;
+            best = pairs;
+        }
+    }
+    z.pairs = best;
+    cfg.dynamicSmemBytes = dsm64_layout(z).total;
+    return *max_clusters > 0 ? cudaSuccess : failed;
 }
 
 cudaError_t dsm64_max_active(int cluster, int bmax, int emax, int tmax, int *out) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    return dsm64_config(cluster, dsm64_smem_bytes(bmax, emax, tmax), cfg, attr, out);
+    Dsm64Sizes z{bmax, emax, tmax, 0};
+    return dsm64_config(cluster, z, cfg, attr, out);
 }
 
 cudaError_t launch_fp64_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, int cluster, int bmax,
                             int emax, int tmax, const FireParamsDev &p, int *queue_dev, const int *order_dev,
                             cudaStream_t stream) {
     if (cluster < 1 || cluster > kDsmParts || (kDsmParts % cluster) != 0) return cudaErrorInvalidValue;
-    const Dsm64Sizes z{std::max(bmax, 1), std::max(emax, 1), std::max(tmax, 1)};
+    Dsm64Sizes z{std::max(bmax, 1), std::max(emax, 1), std::max(tmax, 1), 0};
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     int max_clusters = 0;
-    cudaError_t e = dsm64_config(cluster, dsm64_layout(z).total, cfg, attr, &max_clusters);
+    cudaError_t e = dsm64_config(cluster, z, cfg, attr, &max_clusters);
     if (e != cudaSuccess) return e;
     if (max_clusters < 1) return cudaErrorLaunchOutOfResources;
     cfg.gridDim = dim3(std::max(1, std::min(n_nets, max_clusters)) * cluster);
     cfg.stream = stream;
     if ((e = cudaMemsetAsync(queue_dev, 0, sizeof(int), stream)) != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, k_fire_dsm64, nets_dev, dsm_dev, n_nets, p, queue_dev, order_dev, z);
+    FireParamsDev pp = p;
+    void *args[] = {&nets_dev, &dsm_dev, &n_nets, &pp, &queue_dev, &order_dev, &z};
+    return cudaLaunchKernelExC(&cfg, dsm64_kernel(z.pairs != 0), args);
 }
 
 }  // namespace nr
