@@ -268,26 +268,31 @@ static int build_tile_set(const nr_host_network &h, const Incidence &inc, const 
     NetTile &tl = S.tile;
     bool ok = false;
     for (int target = tile_target_nodes(); target >= 64 && !ok; target = target * 4 / 5) {
-        if (build_tile_layout(h, inc, fcodes, d.use_bonds != 0, d.use_triples != 0, per_sm * sms, target, th) !=
-            NR_OK)
-            return NR_OK;
-        tl = NetTile{};
-        tl.n_tiles = th.n_tiles;
-        tl.n_pos = th.n_pos;
-        tl.max_nodes = th.max_nodes;
-        tl.max_bonds = th.max_bonds;
-        tl.max_tris = th.max_tris;
-        tl.max_own = th.max_own;
-        tl.max_ro = th.max_ro;
-        ok = tile_smem(tl) <= limit;
+        for (const bool quads : {true, false}) {
+            if (build_tile_layout(h, inc, fcodes, d.use_bonds != 0, d.use_triples != 0, per_sm * sms, target, quads, th) !=
+                NR_OK)
+                return NR_OK;
+            tl = NetTile{};
+            tl.n_tiles = th.n_tiles;
+            tl.n_pos = th.n_pos;
+            tl.max_nodes = th.max_nodes;
+            tl.max_bonds = th.max_bonds;
+            tl.max_tris = th.max_tris;
+            tl.max_own = th.max_own;
+            tl.max_ro = th.max_ro;
+            tl.quads = quads;
+            ok = tile_plan_smem(th) <= limit;
+            /* quads that do not fit (a hub's list fills up 31 others') */
+            if (!ok || tile_smem(tl) <= limit) break;
+        }
     }
     if (!ok) return NR_OK;
     /* every tile record is a whole number of 16-byte units at a 16-byte
      * offset, as cp.async.bulk requires */
     for (const TileDesc &td : th.desc)
-        if (td.ro_off % 16 != 0 || tile_segs(td.nb, td.nt, td.no, td.ni, td.nh).total % 16 != 0)
+        if (td.ro_off % 16 != 0 || tile_segs(td).total % 16 != 0)
             return fail(NR_ERR_INVALID, "tile layout: record not 16-byte aligned");
-    const int ctas = tile_grid_ctas(tile_smem(tl), threads);
+    const int ctas = tile_grid_ctas(tl, threads);
     if (ctas < 1) {
         cudaGetLastError();
         return NR_OK;

@@ -112,7 +112,7 @@ cudaError_t dsm_max_active(int cluster, int bmax, int emax, int tmax, int ebmax,
 /* Host arrays of a NetTile layout (fire_tile.cu). */
 struct TileHost {
     int n_tiles = 0, n_pos = 0, max_nodes = 0, max_bonds = 0, max_tris = 0, max_own = 0;
-    unsigned max_ro = 0;
+    unsigned max_ro = 0, max_plain = 0; /* largest record; the same with the entries not in quads */
     std::vector<TileDesc> desc;
     std::vector<unsigned char> ro;
     std::vector<int> node_of_pos, bid, tid;
@@ -121,9 +121,10 @@ struct Incidence;
 /* The tiled mixed-precision kernel for one large network: layout, launch
  * width (co-resident CTAs for its shared memory) and launch. */
 int build_tile_layout(const ::nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
-                      bool use_triples, int ctas, int target_nodes, TileHost &out);
+                      bool use_triples, int ctas, int target_nodes, bool quads, TileHost &out);
+size_t tile_plan_smem(const TileHost &th);
 size_t tile_smem(const NetTile &tl);
-int tile_grid_ctas(size_t smem, int threads);
+int tile_grid_ctas(const NetTile &tl, int threads);
 cudaError_t launch_mixed_tile(const NetDev &d, const NetTile &tl, const FireParamsDev &p, int ctas, int threads,
                               unsigned long long budget_ns, cudaStream_t stream);
 int mixed_grid_blocks(int n);

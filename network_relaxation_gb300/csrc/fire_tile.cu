@@ -15,7 +15,7 @@
  *      issued while the previous tile computes, the first tile's during the
  *      grid barrier (two stage buffers, an mbarrier each); a CTA with a
  *      single tile keeps it in shared memory between anchors;
- *   1. u, v, F of the halo (cp.async once the record's halo list is in);
+ *   1. u, v, F of the halo (cp.async during the previous tile's gather);
  *   2. pass A (mixing, drift, half kick) for own AND halo nodes: the halo's
  *      drift is recomputed from the same inputs with the same operations as
  *      its owner's, so it has the same bits and needs no barrier;
@@ -31,14 +31,19 @@
  * (rare) take two more barriers: X += u, then the FP64 force and the tile
  * records' anchor data.
  *
- * What bounds a step (65 536 nodes, one tile per SM, 6.4 us): items 1.2 us,
- * gather 1.4, pass A and halo 0.8, totals and scalars 1.2, barrier 1.7; the
+ * What bounds a step (65 536 nodes, one tile per SM, 6.3 us): items 1.2 us,
+ * gather 1.3, pass A and halo 0.8, totals and scalars 1.2, barrier 1.7; the
  * step took 8.3 us when every step loaded the record and the own state again,
  * the totals' loads came in five dependent rounds, each triple entry of the
  * gather selected its share, and the item loops ended in nearly empty rounds.
- * 16 384 nodes 6.7 -> 4.9, 262 144 nodes 19.1 -> 17.1, 1 048 576 nodes 58.2 ->
- * 56.5 us: there 14 tiles a step pass through the SM, whose warps issue on
- * 32 % of the cycles and wait mostly at the barriers between the phases.
+ * 16 384 nodes 6.7 -> 4.8, 262 144 nodes 19.1 -> 15.6, 1 048 576 nodes 58.2 ->
+ * 50.8 us: there 14 tiles a step pass through the SM, whose warps issue on
+ * 45 % of the cycles and wait for shared memory (3.3 wavefronts a load) and at
+ * the barriers between the phases.  Of the last 5.8 us, 2.4 came from the
+ * gather's entries in quads (four 2-byte loads of scattered addresses before),
+ * 3.4 from pass A following the previous tile's gather without a barrier.  Two
+ * groups of 512 threads with a tile each were slower (62 us): with one buffer
+ * a group the loads are exposed, and the phases share the same pipes.
  *
  * Every wait is bounded: the grid barrier by a %globaltimer budget, the
  * mbarrier waits by the same budget; a wait that runs out sets the
@@ -183,7 +188,7 @@ __device__ inline TileState tile_state_at(unsigned char *base, int max_nodes, in
  * contiguous in tile order; own_pos is a multiple of 16, a node 16 bytes. */
 __device__ __forceinline__ void load_tile(const NetTile &tl, const TileDesc &td, int cur, unsigned char *rec,
                                           const TileState &ts, unsigned long long *mbar) {
-    const unsigned total = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh).total, own = 16u * (unsigned)td.no;
+    const unsigned total = tile_segs(td).total, own = 16u * (unsigned)td.no;
     mbar_expect(mbar, total + 3u * own);
     tma_copy(rec, tl.ro + td.ro_off, total, mbar);
     tma_copy(ts.u, tl.u[cur] + td.own_pos, own, mbar);
@@ -194,8 +199,7 @@ __device__ __forceinline__ void load_tile(const NetTile &tl, const TileDesc &td,
  * memory). */
 __device__ __forceinline__ void issue_halo(const NetTile &tl, const TileDesc &td, const unsigned char *rec, int cur,
                                            const TileState &ts) {
-    const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
-    const int *halo = reinterpret_cast<const int *>(rec + g.halo);
+    const int *halo = reinterpret_cast<const int *>(rec + tile_segs(td).halo);
     for (int h = threadIdx.x; h < td.nh; h += blockDim.x) {
         const int pp = halo[h];
         cp_async16(ts.u + td.no + h, tl.u[cur] + pp);
@@ -217,6 +221,20 @@ __device__ __forceinline__ void tile_pass_a(const Coef &c, float4 &w, float2 &v,
         df_add(w.y, w.w, fmaf(c.dt, v.y, c.dtsq * F.y));
         v.x = fmaf(c.dtm, F.x, v.x);
         v.y = fmaf(c.dtm, F.y, v.y);
+    }
+}
+
+/* Pass A of local nodes first, first + NT, ... < end of a state buffer, in
+ * place. */
+template <int NT>
+__device__ __forceinline__ void tile_pass_range(const Coef &c, const TileState &ts, int first, int end) {
+    for (int k = first; k < end; k += NT) {
+        float4 w = ts.u[k];
+        const float4 q = ts.vf[k];
+        float2 v = make_float2(q.x, q.y);
+        tile_pass_a(c, w, v, make_float2(q.z, q.w));
+        ts.u[k] = w;
+        ts.vf[k] = make_float4(v.x, v.y, q.z, q.w);
     }
 }
 
@@ -247,7 +265,7 @@ static __device__ __noinline__ void tile_anchor_eval(const NetDev &d, const NetT
     }
     for (int t = blockIdx.x; t < tl.n_tiles; t += G) {
         const TileDesc td = tl.desc[t];
-        const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
+        const TileSegs g = tile_segs(td);
         unsigned char *rec = tl.ro + td.ro_off;
         float4 *mb = reinterpret_cast<float4 *>(rec + g.mb);
         float2 *sk = reinterpret_cast<float2 *>(rec + g.sk);
@@ -299,15 +317,13 @@ static __device__ __noinline__ void tile_anchor_totals(const NetTile &tl, int G,
  * with two CTAs per SM (smaller tiles; one CTA's barriers overlap the
  * other's work). */
 
-/* Dynamic shared memory of a CTA: two record buffers of max_ro bytes and two
- * node-state buffers.  The tile size is chosen as if the item results had
- * arrays of their own (16 B a triple, 8 B a bond; they now overwrite the
- * record), so that the tiles, and with them the order of the sums, stay what
- * they were. */
-__host__ __device__ inline size_t tile_smem_bytes(unsigned max_ro, int max_nodes, int max_own, int max_bonds,
-                                                  int max_tris) {
-    return 2 * (size_t)max_ro + 2 * tile_state_bytes(max_nodes, max_own) + 16 * (size_t)max_tris +
-           8 * (size_t)max_bonds;
+/* Shared memory by which the tile size is chosen: records with the entries not
+ * in quads, and item results with arrays of their own (16 B a triple, 8 B a
+ * bond; they now overwrite the record), so that the tiles, and with them the
+ * order of the sums, stay what they were. */
+size_t tile_plan_smem(const TileHost &th) {
+    return 2 * (size_t)th.max_plain + 2 * tile_state_bytes(th.max_nodes, th.max_own) + 16 * (size_t)th.max_tris +
+           8 * (size_t)th.max_bonds;
 }
 
 constexpr int kDescCache = 32;
@@ -327,7 +343,11 @@ static __device__ __noinline__ void tile_abort(FireState *st, unsigned long long
     if (n1) mbar_wait(&mbar[1], par1, budget_ns);
 }
 
-template <int NT, int MINB>
+/* resident: one tile per CTA at most.  Its record and own state stay in shared
+ * memory between anchors, a step reads only the halo; the item results then go
+ * to the second stage buffer (a streamed record is overwritten in place).
+ * quads: the layout of the incidence entries (NetTile). */
+template <int NT, int MINB, bool resident, bool quads>
 __global__ void __launch_bounds__(NT, MINB)
     k_fire_tile_mixed(NetDev d, NetTile tl, FireParamsDev p, unsigned long long budget_ns) {
     extern __shared__ float4 s_dyn[];
@@ -384,11 +404,9 @@ __global__ void __launch_bounds__(NT, MINB)
     /* the gather's threads: the order of the sums does not depend on NT */
     constexpr int NG = NT < 512 ? NT : 512;
     auto desc = [&](int k) -> TileDesc { return k < kDescCache ? s_desc[k] : tl.desc[blockIdx.x + k * G]; };
-    /* One tile per CTA: record and own state stay in shared memory between
-     * anchors, a step reads only the halo.  The item results then go to the
-     * second stage buffer; a streamed record is overwritten in place. */
-    const bool resident = tl.n_tiles <= (int)G;
     bool loaded = false; /* tile 0 is in buffer 0, or its load in flight */
+    if (resident && quads && n_mine > 0 && threadIdx.x < 4) /* ordered by the barriers before the first gather */
+        reinterpret_cast<float *>(stage1 + tile_segs(s_desc[0]).zero)[threadIdx.x] = 0.f;
     for (;;) {
         const Coef &c = sh.coef;
         if (c.done) {
@@ -407,9 +425,13 @@ __global__ void __launch_bounds__(NT, MINB)
         }
         const int nxt = cur ^ 1;
         float P = 0.f, V2 = 0.f, Fs = 0.f, M2f = 0.f, A = 0.f;
-        /* the pipeline: the record and own state (TMA) of tile k + 1 are in
-         * flight while tile k computes, its halo state (cp.async) from the
-         * moment the record is in */
+        /* the pipeline, two barriers a streamed tile: the record and own state (TMA)
+         * of tile k + 1 are in flight while tile k's items and gather run, its
+         * halo state (cp.async) during the gather, and its pass A follows the
+         * gather directly: a thread waits only for what it reads, the bulk
+         * copies (own nodes) and its own halo copies (the same thread's
+         * nodes), so that the threads without a node to gather start it while
+         * the others sum */
         if (n_mine > 0) {
             const TileDesc td0 = desc(0);
             if (!loaded) {
@@ -429,6 +451,18 @@ __global__ void __launch_bounds__(NT, MINB)
                 else s_fail = 1;
             }
             if (in) issue_halo(tl, td0, stage0, cur, ts0); /* only from a record that arrived */
+            if (resident) {
+                /* nothing else to do meanwhile: own and halo nodes in one
+                 * sequence over the threads (5.0 us a step against 5.3 at
+                 * 22 500 nodes) */
+                cp_async_wait_all();
+                __syncthreads();
+                if (in) tile_pass_range<NT>(c, ts0, threadIdx.x, td0.no + td0.nh);
+            } else if (in) {
+                tile_pass_range<NT>(c, ts0, threadIdx.x, td0.no);
+                cp_async_wait_all();
+                tile_pass_range<NT>(c, ts0, td0.no + threadIdx.x, td0.no + td0.nh);
+            }
             if (!resident) loaded = false;
         }
         for (int k = 0; k < n_mine; ++k) {
@@ -439,31 +473,25 @@ __global__ void __launch_bounds__(NT, MINB)
             float4 *const sc_u = b ? ts1.u : ts0.u, *const sc_vf = b ? ts1.vf : ts0.vf, *const sc_fa = b ? ts1.fa : ts0.fa;
             const TileState sn{b ? ts0.u : ts1.u, b ? ts0.vf : ts1.vf, b ? ts0.fa : ts1.fa};
             unsigned char *const rec_n = b ? stage0 : stage1;
-            cp_async_wait_all(); /* this tile's halo state (its own part: mbarrier) */
-            __syncthreads();     /* and the previous tile's gather is done with the other buffers */
+            __syncthreads(); /* this tile's pass A; the previous tile's gather is done with the other buffers */
             if (s_fail) {
                 tile_abort(st, s_mbar, iss0 > uses0, uses0 & 1u, iss1 > uses1, uses1 & 1u, budget_ns);
                 return;
             }
+            /* the next tile: its halo list straight from memory (no anchor
+             * changes it), before its record is here */
+            const int *const halo_n = reinterpret_cast<const int *>(tl.ro + tn.ro_off + tile_segs(tn).halo);
+            int hp = 0;
             if (more) {
                 if (threadIdx.x == 0) load_tile(tl, tn, cur, rec_n, sn, &s_mbar[b ^ 1]);
                 if (b) ++iss0;
                 else ++iss1;
+                if ((int)threadIdx.x < tn.nh) hp = __ldg(halo_n + threadIdx.x);
             }
-            const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
-            const int no = td.no, nn = no + td.nh, op = td.own_pos;
+            const TileSegs g = tile_segs(td);
+            const int no = td.no, op = td.own_pos;
             unsigned char *const rec = b ? stage1 : stage0;
             unsigned char *const out = resident ? stage1 : rec;
-            /* pass A of own and halo nodes, in place */
-            for (int kk = threadIdx.x; kk < nn; kk += NT) {
-                float4 w = sc_u[kk];
-                const float4 q = sc_vf[kk];
-                float2 v = make_float2(q.x, q.y);
-                tile_pass_a(c, w, v, make_float2(q.z, q.w));
-                sc_u[kk] = w;
-                sc_vf[kk] = make_float4(v.x, v.y, q.z, q.w);
-            }
-            __syncthreads();
             /* item pass: groups of 32 triples, then of 32 bonds, dealt to the
              * warps in one sequence, so that no warp idles in a last round of
              * either.  A result replaces the anchor data it came from:
@@ -510,31 +538,23 @@ __global__ void __launch_bounds__(NT, MINB)
                     }
                 }
             }
-            /* the next tile's record is in by now (bounded wait): start its
-             * halo state */
-            if (more) {
-                if (mbar_wait(&s_mbar[b ^ 1], (b ? uses0 : uses1) & 1u, budget_ns)) {
-                    if (b) ++uses0;
-                    else ++uses1;
-                    issue_halo(tl, tn, rec_n, cur, sn); /* only from a record that arrived */
-                } else {
-                    s_fail = 1;
+            if (more)
+                for (int h = threadIdx.x; h < tn.nh; h += NT) {
+                    const int pp = h == (int)threadIdx.x ? hp : __ldg(halo_n + h);
+                    cp_async16(sn.u + tn.no + h, tl.u[cur] + pp);
+                    cp_async16(sn.vf + tn.no + h, tl.vf[cur] + pp);
                 }
-            }
             __syncthreads();
-            if (s_fail) {
-                tile_abort(st, s_mbar, iss0 > uses0, uses0 & 1u, iss1 > uses1, uses1 & 1u, budget_ns);
-                return;
-            }
             /* gather of the own nodes, half kick, the next step's state */
             const unsigned short *iptr = reinterpret_cast<const unsigned short *>(rec + g.iptr);
             const unsigned short *ibe = reinterpret_cast<const unsigned short *>(rec + g.ibe);
             const unsigned short *inc = reinterpret_cast<const unsigned short *>(rec + g.inc);
+            const ushort2 *cnt = reinterpret_cast<const ushort2 *>(rec + g.cnt);
+            const unsigned *gq = reinterpret_cast<const unsigned *>(rec + g.gq);
             const unsigned char *fcode = rec + g.fcode;
             const int to_mag = (int)g.tref - (int)g.pk;
             for (int kk = threadIdx.x; (int)threadIdx.x < NG && kk < no; kk += NG) {
                 const unsigned fc = fcode[kk];
-                const int e0 = iptr[kk], eb = ibe[kk], e1 = iptr[kk + 1];
                 const float4 fa = sc_fa[kk];
                 const float2 ah = make_float2(fa.x, fa.y), al = make_float2(fa.z, fa.w);
                 float2 F = make_float2(0.f, 0.f);
@@ -544,42 +564,71 @@ __global__ void __launch_bounds__(NT, MINB)
                      * ordered by list lengths */
                     float2 dF = make_float2(0.f, 0.f);
                     float mag = 0.f;
-                    for (int e = e0; e < eb; e += 4) {
-                        float2 df[4];
-                        unsigned code[4];
+                    if (quads) {
+                        const ushort2 n = cnt[kk];
+                        const uint2 *qp = reinterpret_cast<const uint2 *>(inc) + gq[kk >> 5] + (kk & 31);
+                        const int nbe = n.x, nen = n.y;
+                        for (int e = 0; e < nen; e += 4, qp += 32) {
+                            const uint2 w = *qp;
+                            const unsigned code[4] = {w.x & 0xffffu, w.x >> 16, w.y & 0xffffu, w.y >> 16};
+                            float2 df[4];
+                            float mg[4];
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, eb - 1)];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) df[j] = *reinterpret_cast<const float2 *>(out + 8u * (code[j] & 0x7fffu));
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (e + j < eb) {
-                                df[j] = neg_if(df[j], code[j] >> 15);
-                                dF.x += df[j].x;
-                                dF.y += df[j].y;
-                                mag += fabsf(df[j].x) + fabsf(df[j].y);
+                            for (int j = 0; j < 4; ++j) {
+                                const unsigned char *at = out + 8u * (code[j] & 0x7fffu);
+                                const bool flag = (code[j] >> 15) != 0, bond = e + j < nbe;
+                                df[j] = neg_if(*reinterpret_cast<const float2 *>(at), flag && bond ? 1u : 0u);
+                                mg[j] = fabsf(df[j].x) + fabsf(df[j].y);
+                                if (flag && !bond) mg[j] = *reinterpret_cast<const float *>(at + to_mag);
                             }
-                    }
-                    for (int e = eb; e < e1; e += 4) {
-                        float2 df[4];
-                        float mg[4];
-                        unsigned code[4];
+                            /* the zeros that fill up the last quad change
+                             * nothing: no sum here is ever -0 */
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, e1 - 1)];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const unsigned char *at = out + 8u * (code[j] & 0x7fffu);
-                            df[j] = *reinterpret_cast<const float2 *>(at);
-                            mg[j] = fabsf(df[j].x) + fabsf(df[j].y);
-                            if (code[j] >> 15) mg[j] = *reinterpret_cast<const float *>(at + to_mag);
-                        }
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            if (e + j < e1) {
+                            for (int j = 0; j < 4; ++j) {
                                 dF.x += df[j].x;
                                 dF.y += df[j].y;
                                 mag += mg[j];
                             }
+                        }
+                    } else {
+                        const int e0 = iptr[kk], eb = ibe[kk], e1 = iptr[kk + 1];
+                        for (int e = e0; e < eb; e += 4) {
+                            float2 df[4];
+                            unsigned code[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, eb - 1)];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) df[j] = *reinterpret_cast<const float2 *>(out + 8u * (code[j] & 0x7fffu));
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (e + j < eb) {
+                                    df[j] = neg_if(df[j], code[j] >> 15);
+                                    dF.x += df[j].x;
+                                    dF.y += df[j].y;
+                                    mag += fabsf(df[j].x) + fabsf(df[j].y);
+                                }
+                        }
+                        for (int e = eb; e < e1; e += 4) {
+                            float2 df[4];
+                            float mg[4];
+                            unsigned code[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) code[j] = inc[min(e + j, e1 - 1)];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const unsigned char *at = out + 8u * (code[j] & 0x7fffu);
+                                df[j] = *reinterpret_cast<const float2 *>(at);
+                                mg[j] = fabsf(df[j].x) + fabsf(df[j].y);
+                                if (code[j] >> 15) mg[j] = *reinterpret_cast<const float *>(at + to_mag);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 4; ++j)
+                                if (e + j < e1) {
+                                    dF.x += df[j].x;
+                                    dF.y += df[j].y;
+                                    mag += mg[j];
+                                }
+                        }
                     }
                     A = fmaxf(A, mag);
                     F.x = ah.x + (al.x + dF.x);
@@ -602,9 +651,19 @@ __global__ void __launch_bounds__(NT, MINB)
                 M2f = fmaxf(M2f, f2);
             }
             /* the shared memory written here, before bulk copies (the async
-             * proxy) overwrite it; the next tile's first barrier orders the
-             * rest */
+             * proxy) overwrite it; the next tile's barrier orders the rest */
             if (!resident) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            if (more) {
+                if (mbar_wait(&s_mbar[b ^ 1], (b ? uses0 : uses1) & 1u, budget_ns)) {
+                    if (b) ++uses0;
+                    else ++uses1;
+                    tile_pass_range<NT>(c, sn, threadIdx.x, tn.no);
+                    cp_async_wait_all();
+                    tile_pass_range<NT>(c, sn, tn.no + threadIdx.x, tn.no + tn.nh);
+                } else {
+                    s_fail = 1;
+                }
+            }
         }
         /* the next state just written, before bulk copies read it */
         if (!resident) asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -717,32 +776,44 @@ __global__ void __launch_bounds__(NT, MINB)
 /* Host side: layout and launch                                         */
 /* ------------------------------------------------------------------ */
 
+/* Dynamic shared memory of a CTA: two record buffers and two node-state
+ * buffers. */
 size_t tile_smem(const NetTile &tl) {
-    return tile_smem_bytes(tl.max_ro, tl.max_nodes, tl.max_own, tl.max_bonds, tl.max_tris);
+    return 2 * (size_t)tl.max_ro + 2 * tile_state_bytes(tl.max_nodes, tl.max_own);
 }
 
 /* The kernel instantiation for `threads` per CTA (512, 768 or 256). */
-static const void *tile_kernel(int threads) {
-    if (threads == 256) return (const void *)k_fire_tile_mixed<256, 2>;
-    if (threads == 768) return (const void *)k_fire_tile_mixed<768, 1>;
-    return (const void *)k_fire_tile_mixed<512, 1>;
+template <bool resident, bool quads>
+static const void *tile_kernel_of(int threads) {
+    if (threads == 256) return (const void *)k_fire_tile_mixed<256, 2, resident, quads>;
+    if (threads == 768) return (const void *)k_fire_tile_mixed<768, 1, resident, quads>;
+    return (const void *)k_fire_tile_mixed<512, 1, resident, quads>;
+}
+static const void *tile_kernel(int threads, bool resident, bool quads) {
+    if (quads) return resident ? tile_kernel_of<true, true>(threads) : tile_kernel_of<false, true>(threads);
+    return resident ? tile_kernel_of<true, false>(threads) : tile_kernel_of<false, false>(threads);
 }
 
 /* CTAs of the cooperative launch: co-resident CTAs per SM times SMs (0 when
  * the kernel cannot launch with this shared memory). */
-int tile_grid_ctas(size_t smem, int threads) {
-    int dev = 0, sms = 0, per_sm = 0;
+int tile_grid_ctas(const NetTile &tl, int threads) {
+    const size_t smem = tile_smem(tl);
+    int dev = 0, sms = 0, least = 1 << 30;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
-    const void *k = tile_kernel(threads);
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) return 0;
-    return per_sm * sms;
+    for (const bool resident : {false, true}) {
+        const void *k = tile_kernel(threads, resident, tl.quads != 0);
+        int per_sm = 0;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) return 0;
+        least = std::min(least, per_sm);
+    }
+    return least * sms;
 }
 
 cudaError_t launch_mixed_tile(const NetDev &d, const NetTile &tl, const FireParamsDev &p, int ctas, int threads,
                               unsigned long long budget_ns, cudaStream_t stream) {
-    const void *k = tile_kernel(threads);
+    const void *k = tile_kernel(threads, tl.n_tiles <= ctas, tl.quads != 0);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(tl));
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(tl.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
@@ -760,7 +831,7 @@ cudaError_t launch_mixed_tile(const NetDev &d, const NetTile &tl, const FirePara
  * Returns NR_OK with the layout in `out` (host arrays), or NR_ERR_CAPACITY
  * when a tile exceeds the 16-bit local encoding. */
 int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
-                      bool use_triples, int ctas, int target_nodes, TileHost &out) {
+                      bool use_triples, int ctas, int target_nodes, bool quads, TileHost &out) {
     const int n = h.n_points, ne = h.n_edges(), nt = h.n_triples();
     const double W = h.offset, H = std::max(h.maxy - h.miny, 1e-300);
     if (n <= 0 || !(W > 0) || ctas < 1) return NR_ERR_INVALID;
@@ -875,7 +946,7 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
         /* incidence of the own nodes, canonical order: bonds, then triples;
          * an entry is where its result will lie in the record (these
          * segments' offsets do not depend on the incidence) */
-        const TileSegs at = tile_segs((int)bl.size(), (int)tlist.size(), (int)o.size(), 0, 0);
+        const TileSegs at = tile_segs((int)bl.size(), (int)tlist.size(), (int)o.size(), 0, 0, quads ? 0 : -1);
         iptr.clear();
         ibe.clear();
         incv.clear();
@@ -908,8 +979,20 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
         td.ni = (int)incv.size();
         td.bond_off = (int)out.bid.size();
         td.tri_off = (int)out.tid.size();
-        td.pad = 0;
-        const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
+        /* entries in quads: as many for each lane of a group of 32 nodes as
+         * its longest list takes */
+        const int no = td.no, groups = (no + 31) / 32;
+        std::vector<unsigned> gq(groups);
+        td.nq = quads ? 0 : -1;
+        if (quads)
+            for (int q = 0; q < groups; ++q) {
+                gq[q] = (unsigned)td.nq;
+                int most = 0;
+                for (int k = 32 * q; k < std::min(no, 32 * q + 32); ++k)
+                    most = std::max(most, (iptr[k + 1] - iptr[k] + 3) / 4);
+                td.nq += 32 * most;
+            }
+        const TileSegs g = tile_segs(td);
         out.ro.resize(out.ro.size() + g.total, 0);
         unsigned char *rec = out.ro.data() + td.ro_off;
         for (size_t k = 0; k < bl.size(); ++k) {
@@ -925,9 +1008,22 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
             memcpy(rec + g.tref + 8 * k, &r, 8);
             out.tid.push_back(qq);
         }
-        memcpy(rec + g.iptr, iptr.data(), 2 * iptr.size());
-        if (!ibe.empty()) memcpy(rec + g.ibe, ibe.data(), 2 * ibe.size());
-        if (!incv.empty()) memcpy(rec + g.inc, incv.data(), 2 * incv.size());
+        if (quads) {
+            const unsigned short none = (unsigned short)(g.zero / 8);
+            unsigned short *q = reinterpret_cast<unsigned short *>(rec + g.inc);
+            std::fill(q, q + 4 * (size_t)td.nq, none);
+            if (groups) memcpy(rec + g.gq, gq.data(), 4 * gq.size());
+            for (int k = 0; k < no; ++k) {
+                const unsigned short c[2] = {(unsigned short)(ibe[k] - iptr[k]), (unsigned short)(iptr[k + 1] - iptr[k])};
+                memcpy(rec + g.cnt + 4 * k, c, 4);
+                for (int e = 0; e < c[1]; ++e)
+                    q[4 * (gq[k >> 5] + 32 * (size_t)(e >> 2) + (k & 31)) + (e & 3)] = incv[iptr[k] + e];
+            }
+        } else {
+            memcpy(rec + g.iptr, iptr.data(), 2 * iptr.size());
+            if (!ibe.empty()) memcpy(rec + g.ibe, ibe.data(), 2 * ibe.size());
+            if (!incv.empty()) memcpy(rec + g.inc, incv.data(), 2 * incv.size());
+        }
         for (size_t k = 0; k < o.size(); ++k) rec[g.fcode + k] = fcodes[o[k]];
         for (size_t k = 0; k < halo.size(); ++k) {
             const int pp = pos_of[halo[k]];
@@ -939,6 +1035,7 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
         out.max_bonds = std::max(out.max_bonds, td.nb);
         out.max_tris = std::max(out.max_tris, td.nt);
         out.max_ro = std::max(out.max_ro, g.total);
+        out.max_plain = std::max(out.max_plain, tile_segs(td.nb, td.nt, td.no, td.ni, td.nh, -1).total);
         reset();
     }
     out.max_nodes = std::max(out.max_nodes, 1);
@@ -946,28 +1043,22 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
     out.max_bonds = std::max(out.max_bonds, 1);
     out.max_tris = std::max(out.max_tris, 1);
     out.max_ro = std::max(out.max_ro, 16u);
+    out.max_plain = std::max(out.max_plain, 16u);
     return NR_OK;
 }
 
-}  // namespace nr
-
-extern "C" int nr_tile_layout_check(const nr_host_network *h, int ctas, int target_nodes, long long stats[6]) {
-    using namespace nr;
-    if (!h || !stats || ctas < 1 || target_nodes < 1) return NR_ERR_INVALID;
-    for (int k = 0; k < 6; ++k) stats[k] = 0;
+/* Builds a layout and counts its violations (nr_tile_layout_check). */
+static int check_tile_layout(const nr_host_network *h, const Incidence &inc, const std::vector<unsigned char> &fc, int ctas,
+                             int target_nodes, bool quads, long long stats[6]) {
     const int n = h->n_points, ne = h->n_edges(), nt = h->n_triples();
-    Incidence inc;
-    build_incidence(n, h->edge_ij.data(), ne, h->tri_hjk.data(), nt, true, true, inc);
-    std::vector<unsigned char> fc(n);
-    nr_host_network_fcodes(h, fc.data());
     TileHost th;
-    const int rc = build_tile_layout(*h, inc, fc.data(), true, true, ctas, target_nodes, th);
+    const int rc = build_tile_layout(*h, inc, fc.data(), true, true, ctas, target_nodes, quads, th);
     if (rc != NR_OK) return rc;
     long long bad = 0, halo_total = 0;
     std::vector<int> owned(n, 0);
     for (int t = 0; t < th.n_tiles; ++t) {
         const TileDesc &td = th.desc[t];
-        const TileSegs g = tile_segs(td.nb, td.nt, td.no, td.ni, td.nh);
+        const TileSegs g = tile_segs(td);
         if (td.ro_off % 16 || g.total % 16 || td.ro_off + (long long)g.total > (long long)th.ro.size() ||
             g.total > th.max_ro) {
             ++bad;
@@ -1007,23 +1098,45 @@ extern "C" int nr_tile_layout_check(const nr_host_network *h, int ctas, int targ
             if (pp < 0 || pp >= th.n_pos || th.node_of_pos[pp] < 0) ++bad;
         }
         for (int k = 0; k < td.no; ++k) {
-            unsigned short a, b, e;
-            memcpy(&a, rec + g.iptr + 2 * k, 2);
-            memcpy(&e, rec + g.iptr + 2 * k + 2, 2);
-            memcpy(&b, rec + g.ibe + 2 * k, 2);
-            if (!(a <= b && b <= e && e <= td.ni)) {
+            /* the node's entries: bonds up to b, all up to e (quads: those
+             * that fill up, up to full) */
+            unsigned short a = 0, b, e;
+            unsigned q0 = 0, full = 0;
+            if (quads) {
+                const int groups = (td.no + 31) / 32;
+                unsigned q1 = (unsigned)td.nq;
+                memcpy(&q0, rec + g.gq + 4 * (k >> 5), 4);
+                if ((k >> 5) + 1 < groups) memcpy(&q1, rec + g.gq + 4 * (k >> 5) + 4, 4);
+                if (q0 > q1 || q1 > (unsigned)td.nq || (q1 - q0) % 32) {
+                    ++bad;
+                    continue;
+                }
+                full = (q1 - q0) / 32 * 4;
+                memcpy(&b, rec + g.cnt + 4 * k, 2);
+                memcpy(&e, rec + g.cnt + 4 * k + 2, 2);
+                if (e > full) {
+                    ++bad;
+                    continue;
+                }
+            } else {
+                memcpy(&a, rec + g.iptr + 2 * k, 2);
+                memcpy(&e, rec + g.iptr + 2 * k + 2, 2);
+                memcpy(&b, rec + g.ibe + 2 * k, 2);
+                full = e;
+            }
+            if (!(a <= b && b <= e && (quads || e <= td.ni))) {
                 ++bad;
                 continue;
             }
-            for (int x = a; x < e; ++x) {
+            for (int x = a; x < (int)full; ++x) {
                 unsigned short c;
-                memcpy(&c, rec + g.inc + 2 * x, 2);
+                memcpy(&c, rec + g.inc + 2 * (quads ? 4 * (q0 + 32 * (size_t)(x >> 2) + (k & 31)) + (x & 3) : (size_t)x), 2);
                 /* where the entry's result lies: sk, pk (hinges) or arms */
                 const unsigned at = c & 0x7fffu, flag = c >> 15;
-                const unsigned lo = x < b ? g.sk / 8 : flag ? g.pk / 8 : g.arms / 8;
-                const unsigned cnt = x < b ? td.nb : flag ? td.nt : 2 * td.nt;
+                const unsigned lo = x >= e ? g.zero / 8 : x < b ? g.sk / 8 : flag ? g.pk / 8 : g.arms / 8;
+                const unsigned cnt = x >= e ? 1 : x < b ? td.nb : flag ? td.nt : 2 * td.nt;
                 if (g.total > 8u * 0x8000u) continue; /* larger than any shared memory: never launched */
-                if (at < lo || at >= lo + cnt) ++bad;
+                if (at < lo || at >= lo + cnt || (x >= e && flag)) ++bad;
             }
         }
         halo_total += td.nh;
@@ -1033,9 +1146,23 @@ extern "C" int nr_tile_layout_check(const nr_host_network *h, int ctas, int targ
     stats[0] = th.n_tiles;
     stats[1] = th.n_pos;
     stats[2] = th.max_nodes;
-    stats[3] = th.max_ro;
+    stats[3] = th.max_plain;
     stats[4] = halo_total;
-    stats[5] = bad;
+    stats[5] += bad;
     return NR_OK;
+}
+
+}  // namespace nr
+
+extern "C" int nr_tile_layout_check(const nr_host_network *h, int ctas, int target_nodes, long long stats[6]) {
+    using namespace nr;
+    if (!h || !stats || ctas < 1 || target_nodes < 1) return NR_ERR_INVALID;
+    for (int k = 0; k < 6; ++k) stats[k] = 0;
+    Incidence inc;
+    build_incidence(h->n_points, h->edge_ij.data(), h->n_edges(), h->tri_hjk.data(), h->n_triples(), true, true, inc);
+    std::vector<unsigned char> fc(h->n_points);
+    nr_host_network_fcodes(h, fc.data());
+    const int rc = check_tile_layout(h, inc, fc, ctas, target_nodes, true, stats);
+    return rc != NR_OK ? rc : check_tile_layout(h, inc, fc, ctas, target_nodes, false, stats);
 }
 

@@ -197,6 +197,13 @@ struct NetDsm {
  *                       0x8000 | its pk for the hinge)
  *   fcode no x u8
  *   halo  nh x i32      tile-order position of each halo node
+ * With the entries in quads (NetTile.quads; 32 consecutive own nodes are a
+ * warp) iptr, ibe and inc give way to
+ *   zero  16 B          zeros, where the entries that fill up a quad point
+ *   cnt   no x u16 x 2  {bond entries, all entries}
+ *   gq    u32           first quad of every group of 32 own nodes
+ *   inc   nq x 4 x u16  quad q of a group's lane l at gq + 32 q + l: a warp
+ *                       loads four entries of each of its nodes side by side
  * (local node k < no: own node k; no + h: halo node h).  The anchor records
  * (mb, sk, arms, pk) are rewritten there at every anchor.  The state
  * (u, v, F) is double buffered: a step reads one copy and writes the other,
@@ -206,14 +213,14 @@ struct TileDesc {
     long long ro_off; /* byte offset of the tile's record in ro */
     int own_pos, no, nh, nb, nt, ni;
     int bond_off, tri_off; /* first entry of the tile in bid / tid */
-    int pad;
+    int nq;                /* quads of the entries; -1: not in quads */
 };
 struct TileSegs {
-    unsigned bref, mb, sk, tref, arms, pk, iptr, ibe, inc, fcode, halo, total; /* byte offsets in a tile record */
+    unsigned bref, mb, sk, tref, arms, pk, iptr, ibe, zero, cnt, gq, inc, fcode, halo, total; /* byte offsets in a tile record */
 };
 __host__ __device__ inline unsigned tile_pad16(unsigned b) { return (b + 15u) & ~15u; }
-__host__ __device__ inline TileSegs tile_segs(int nb, int nt, int no, int ni, int nh) {
-    TileSegs g;
+__host__ __device__ inline TileSegs tile_segs(int nb, int nt, int no, int ni, int nh, int nq) {
+    TileSegs g{};
     unsigned o = 0;
     g.bref = o;  o += tile_pad16(4u * nb);
     g.mb = o;    o += 16u * nb;
@@ -221,19 +228,30 @@ __host__ __device__ inline TileSegs tile_segs(int nb, int nt, int no, int ni, in
     g.tref = o;  o += tile_pad16(8u * nt);
     g.arms = o;  o += 16u * nt;
     g.pk = o;    o += tile_pad16(8u * nt);
-    g.iptr = o;  o += tile_pad16(2u * (no + 1));
-    g.ibe = o;   o += tile_pad16(2u * no);
-    g.inc = o;   o += tile_pad16(2u * ni);
+    if (nq >= 0) {
+        g.zero = o;  o += 16u;
+        g.cnt = o;   o += tile_pad16(4u * no);
+        g.gq = o;    o += tile_pad16(4u * ((no + 31) / 32));
+        g.inc = o;   o += 8u * nq;
+    } else {
+        g.iptr = o;  o += tile_pad16(2u * (no + 1));
+        g.ibe = o;   o += tile_pad16(2u * no);
+        g.inc = o;   o += tile_pad16(2u * ni);
+    }
     g.fcode = o; o += tile_pad16(1u * no);
     g.halo = o;  o += tile_pad16(4u * nh);
     g.total = o;
     return g;
+}
+__host__ __device__ inline TileSegs tile_segs(const TileDesc &t) {
+    return tile_segs(t.nb, t.nt, t.no, t.ni, t.nh, t.nq);
 }
 struct NetTile {
     int n_tiles, n_pos;                  /* tiles; tile-order positions (with padding) */
     int max_nodes, max_bonds, max_tris;  /* per tile: own + halo nodes, bond items, triple items */
     int max_own;                         /* per tile: own nodes */
     unsigned max_ro;                     /* largest tile record, bytes */
+    int quads;                           /* entries in quads */
     const TileDesc *desc;
     unsigned char *ro;                   /* tile records (anchor records rewritten in place) */
     const int *node_of_pos;              /* node id of each tile-order position (-1: padding) */
