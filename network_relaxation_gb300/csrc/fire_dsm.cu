@@ -22,13 +22,18 @@
  * host uses this kernel when the largest network of the batch fits.
  *
  * What bounds a step (8100 nodes on 4 CTAs, read-only data in global memory;
- * cycles): items 10 100, gather 10 000 to 13 500, pass A 2 200, three cluster
- * barriers with the wait for the slowest CTA 8 000, totals and scalars 4 500.
- * The gather took 16 200 while it decoded every entry and loaded it from L2 as
- * it went: entries are addresses now, a warp's lie in quads side by side, and
- * the next quad travels while one is added.  192-network batch of 600 steps:
- * 47.2 -> 36.8 ms, one network of 2491 nodes on 4 resident CTAs 7.5 -> 6.8 us
- * per step.
+ * cycles): items 10 100, gather 10 000, pass A 2 200, three cluster barriers
+ * with the wait for the slowest CTA 8 000, totals and scalars 4 500.  The gather
+ * took 16 200 while it decoded every entry and loaded it from L2 as it went:
+ * entries are addresses now, a warp's lie in quads side by side (one
+ * conflict-free 16-byte load for four entries; lists behind one another cost
+ * eight wavefronts for each 4-byte load), in shared memory where there is room,
+ * and the next quad travels while one is added.  192-network batch of 600
+ * steps 47.2 -> 36 ms, 30 networks of up to 30^2 nodes and 400 steps 2.2 -> 2.0;
+ * one network on 4 resident CTAs, us per step: 304 nodes 4.5 -> 3.5, 2491 nodes
+ * 7.5 -> 6.0.  Loads from other CTAs (94 clocks a warp against 5 to 9) are
+ * hidden: copying the boundary once a step and evaluating its items on both
+ * sides was 5 to 10 % slower.
  *
  * Compiled with --fmad=false; FP32 expressions use explicit fmaf().
  */
@@ -54,6 +59,7 @@ struct DsmSizes {
     int bmax, emax, tmax;   /* nodes, bonds, triples per CTA */
     int ebmax, etmax;       /* bond / triple incidence entries per CTA */
     int resident;
+    int extra; /* bytes behind the entries, for more of them (quads) */
 };
 struct DsmLayout {
     size_t u, tdf, mb, arms, tref, grec, v, f, bdf, fahi, falo, sk, pk, bref, bent, tent, total;
@@ -78,7 +84,7 @@ __host__ __device__ inline DsmLayout dsm_layout(const DsmSizes &z) {
     L.bref = o; o += R * 8 * em;
     L.bent = o; o += R * 4 * (size_t)z.ebmax;
     L.tent = o; o += R * 4 * (size_t)z.etmax;
-    L.total = o;
+    L.total = o + (size_t)z.extra;
     return L;
 }
 
@@ -180,16 +186,15 @@ struct GatherQuad {
             if (c[j] & 2u) b[j] = dsm_ld2((c[j] & ~3u) + 8u);
         }
     }
-    /* The first `n` entries; the product with the sign is exact. */
-    __device__ __forceinline__ void add(int n, float2 &dF, float &mag) const {
+    /* The product with the sign is exact. */
+    __device__ __forceinline__ void add(float2 &dF, float &mag) const {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (j < n) {
-                const float sg = (c[j] & 1u) ? -1.0f : 1.0f;
-                dF.x = fmaf(sg, a[j].x + b[j].x, dF.x);
-                dF.y = fmaf(sg, a[j].y + b[j].y, dF.y);
-                mag += ((fabsf(a[j].x) + fabsf(a[j].y)) + fabsf(b[j].x)) + fabsf(b[j].y);
-            }
+        for (int j = 0; j < 4; ++j) {
+            const float sg = (c[j] & 1u) ? -1.0f : 1.0f;
+            dF.x = fmaf(sg, a[j].x + b[j].x, dF.x);
+            dF.y = fmaf(sg, a[j].y + b[j].y, dF.y);
+            mag += ((fabsf(a[j].x) + fabsf(a[j].y)) + fabsf(b[j].x)) + fabsf(b[j].y);
+        }
     }
 };
 
@@ -215,8 +220,9 @@ __global__ void __launch_bounds__(NT, 1)
                      reinterpret_cast<float2 *>(dyn + L.fahi), reinterpret_cast<float2 *>(dyn + L.falo)};
     int4 *s_tref = reinterpret_cast<int4 *>(dyn + L.tref);
     int2 *s_bref = reinterpret_cast<int2 *>(dyn + L.bref);
-    int4 *s_grec = reinterpret_cast<int4 *>(dyn + L.grec);
-    unsigned *s_ent = reinterpret_cast<unsigned *>(dyn + L.bent); /* bond and triple entries: L.tent follows */
+    int4 *s_grec = reinterpret_cast<int4 *>(dyn + L.grec); /* NetDsm.xrec */
+    /* the entries' quads, from L.bent on, where they fit */
+    uint4 *s_quad = reinterpret_cast<uint4 *>(dyn + (L.bent + 15) / 16 * 16);
     __shared__ MixShared sh;
     __shared__ NetDev s_d;
     __shared__ NetDsm s_m;
@@ -276,10 +282,8 @@ __global__ void __launch_bounds__(NT, 1)
         const int n0 = rank * spr * bsub, nloc = max(0, min(spr * bsub, d.n - n0));
         const int b0 = m.bo[rank * spr], b1 = m.bo[(rank + 1) * spr];
         const int t0 = m.to[rank * spr], t1 = m.to[(rank + 1) * spr];
-        const int eb0 = m.be[rank * spr], eb1 = m.be[(rank + 1) * spr];
-        const int et0 = m.te[rank * spr], et1 = m.te[(rank + 1) * spr];
         if (R) /* the CTA's read-only slices into shared memory */
-            for (int k = threadIdx.x; k < nloc; k += NT) s_grec[k] = m.grec[n0 + k];
+            for (int k = threadIdx.x; k < nloc; k += NT) s_grec[k] = m.xrec[n0 + k];
         /* Node references and incidence entries resolved, once per network
          * and launch, to the shared::cluster addresses of this cluster size:
          * decoding owner, slot and role of every entry took two thirds of the
@@ -288,8 +292,8 @@ __global__ void __launch_bounds__(NT, 1)
          * bond, 16 B a triple):
          *   bond item    addresses of u_i, u_j
          *   triple item  addresses of u_h, u_j, u_k
-         * A node's entries, bonds then triples, lie together (shared copies:
-         * by node; else in the quads of NetDsm.xent, padded with s_zero):
+         * A node's entries, bonds then triples, lie in the quads of
+         * NetDsm.xent (or a shared copy), padded with s_zero:
          *   bond    address of the force change | 1 on the second node
          *   triple  address of {dF_j, dF_k}, for k of its second half, for
          *           the hinge | 3: minus the sum of both halves */
@@ -318,20 +322,21 @@ __global__ void __launch_bounds__(NT, 1)
                                   (int)u_addr(s_au, r.z, lg, bsub), r.w);
             }
         const unsigned zero_at = dsm_addr(&s_zero, (unsigned)rank);
+        /* the CTA's quads: first .. last of its groups of 32 nodes */
+        uint4 *quad = m.xent;
+        if (nloc > 0) {
+            const int4 x0 = __ldg(m.xrec + n0), x1 = __ldg(m.xrec + n0 + nloc - 1);
+            if ((size_t)(x1.y + 32 * x1.z - x0.y) * sizeof(uint4) + (size_t)((unsigned char *)s_quad - dyn) <= L.total)
+                quad = s_quad - x0.y;
+        }
         for (int k = threadIdx.x; k < nloc; k += NT) {
             const int4 g = __ldg(m.grec + n0 + k);
             const int nb = d.use_bonds ? g.z & 0xffff : 0, nt = d.use_triples ? (int)((unsigned)g.z >> 16) : 0;
-            if (R) {
-                unsigned *const p = s_ent + (g.y - eb0) + (g.w - et0);
-                for (int e = 0; e < nb; ++e) p[e] = bond_entry(g.y + e);
-                for (int e = 0; e < nt; ++e) p[nb + e] = triple_entry(g.w + e);
-            } else {
-                const int4 x = __ldg(m.xrec + n0 + k);
-                unsigned *const p = reinterpret_cast<unsigned *>(m.xent + x.y + (k & 31));
-                for (int e = 0; e < 4 * x.z; ++e)
-                    p[128 * (e >> 2) + (e & 3)] =
-                        e < nb ? bond_entry(g.y + e) : e < nb + nt ? triple_entry(g.w + e - nb) : zero_at;
-            }
+            const int4 x = __ldg(m.xrec + n0 + k);
+            unsigned *const p = reinterpret_cast<unsigned *>(quad + x.y + (k & 31));
+            for (int e = 0; e < 4 * x.z; ++e)
+                p[128 * (e >> 2) + (e & 3)] =
+                    e < nb ? bond_entry(g.y + e) : e < nb + nt ? triple_entry(g.w + e - nb) : zero_at;
         }
         /* item and node data for the step loops: shared copies or global */
         const uint2 *Bref = xb;
@@ -512,37 +517,16 @@ __global__ void __launch_bounds__(NT, 1)
                 float2 F = make_float2(0.f, 0.f);
                 float2 dF = make_float2(0.f, 0.f);
                 float mag = 0.f;
-                if constexpr (RES) {
-                    /* the entries' loads one quad ahead of their sums */
-                    const int cnt = (d.use_bonds ? g.z & 0xffff : 0) + (d.use_triples ? (int)((unsigned)g.z >> 16) : 0);
-                    const unsigned *const p = s_ent + (g.y - eb0) + (g.w - et0);
-                    if (fc != 0 && cnt > 0) {
-                        GatherQuad q, qn;
-                        q.load(make_uint4(p[0], p[min(1, cnt - 1)], p[min(2, cnt - 1)], p[min(3, cnt - 1)]));
-                        for (int e = 0;;) {
-                            const int en = e + 4;
-                            if (en < cnt)
-                                qn.load(make_uint4(p[en], p[min(en + 1, cnt - 1)], p[min(en + 2, cnt - 1)],
-                                                   p[min(en + 3, cnt - 1)]));
-                            q.add(cnt - e, dF, mag);
-                            if (en >= cnt) break;
-                            e = en;
-                            q = qn;
-                        }
-                    }
-                } else {
-                    /* quads of the whole group, the next one's addresses on
-                     * their way from L2 while this one is added; padding
-                     * entries add 0 */
-                    const uint4 *const p = m.xent + g.y + (k & 31);
-                    uint4 code = g.z > 0 ? p[0] : make_uint4(zero_at, zero_at, zero_at, zero_at);
-                    for (int i = 0; i < g.z; ++i) {
-                        const uint4 next = p[32 * min(i + 1, g.z - 1)];
-                        GatherQuad q;
-                        q.load(code);
-                        q.add(4, dF, mag);
-                        code = next;
-                    }
+                /* quads of the whole group, the next one's addresses on their
+                 * way while this one is added; padding entries add 0 */
+                const uint4 *const p = quad + g.y + (k & 31);
+                uint4 code = g.z > 0 ? p[0] : make_uint4(zero_at, zero_at, zero_at, zero_at);
+                for (int i = 0; i < g.z; ++i) {
+                    const uint4 next = p[32 * min(i + 1, g.z - 1)];
+                    GatherQuad q;
+                    q.load(code);
+                    q.add(dF, mag);
+                    code = next;
                 }
                 if (fc != 0) {
                     A = fmaxf(A, mag);
@@ -653,7 +637,7 @@ __global__ void __launch_bounds__(NT, 1)
 
 /* Dynamic shared memory of k_fire_dsm_mixed for the given per-CTA maxima. */
 size_t dsm_smem_bytes(int bmax, int emax, int tmax, int ebmax, int etmax, int resident) {
-    return dsm_layout(DsmSizes{bmax, emax, tmax, ebmax, etmax, resident}).total;
+    return dsm_layout(DsmSizes{bmax, emax, tmax, ebmax, etmax, resident, 0}).total;
 }
 
 constexpr int kDsmStatic = 3024;
@@ -668,6 +652,15 @@ size_t dsm_smem_limit() {
     if (cudaFuncGetAttributes(&fa, (const void *)k_fire_dsm_mixed<512, true>) != cudaSuccess) return 0;
     const int fixed = std::max((int)fa.sharedSizeBytes, kDsmStatic);
     return optin > fixed ? (size_t)(optin - fixed) : 0;
+}
+
+/* Shared memory for the entries filled up to quads, up to twice their size
+ * (4 bytes each; a resident CTA has the first half by its layout), as far as
+ * there is room. */
+static int dsm_extra(const DsmSizes &z) {
+    const size_t total = dsm_layout(z).total, limit = dsm_smem_limit();
+    if (limit <= total) return 0;
+    return (int)std::min<size_t>(limit - total, (z.resident ? 4 : 8) * (size_t)(z.ebmax + z.etmax) + 4096);
 }
 
 template <int NT, bool RES>
@@ -735,7 +728,8 @@ cudaError_t launch_mixed_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int 
                              const FireParamsDev &p, int *queue_dev, const int *order_dev, cudaStream_t stream,
                              const int *n_dev) {
     if (cluster < 1 || cluster > kDsmParts || (kDsmParts % cluster) != 0) return cudaErrorInvalidValue;
-    const DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident};
+    DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident, 0};
+    z.extra = dsm_extra(z);
     const bool wide = dsm_threads(resident != 0) == 1024;
     if (resident)
         return wide ? launch_dsm_nt<1024, true>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p,
@@ -782,7 +776,8 @@ cudaError_t launch_compact_yielded(const FireState *st, int n, int *order_out, i
 }
 
 cudaError_t dsm_max_active(int cluster, int bmax, int emax, int tmax, int ebmax, int etmax, int resident, int *out) {
-    const DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident};
+    DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident, 0};
+    z.extra = dsm_extra(z);
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     const bool wide = dsm_threads(resident != 0) == 1024;
