@@ -44,6 +44,7 @@
 #include <string>
 #include <vector>
 
+#include "canon_math.h"
 #include "nr_device.cuh"
 #include "nr_internal.h"
 
@@ -521,9 +522,11 @@ __device__ __forceinline__ double2 precond_row(double2 m, double o, double2 r, i
  * 152 CTAs) and the partials' and the halo's way through L2.
  * Measured per iteration, this kernel against k_spr_pcg (two barriers with a
  * last CTA working alone, all vectors through L2, 40 additions a warp for the
- * sums): 96 rows 7.0 us (31), 3 040 rows 8.1 (41), 50 560 rows 13.1 (46),
- * 124 000 rows 20.0 (48, matrix in global memory), 318 400 rows 39.6 (74,
- * mode 2). */
+ * sums): 96 rows 6.4 us (31), 3 040 rows 7.6 (41), 50 560 rows 12.6 (46),
+ * 124 000 rows 19.1 (48, matrix in global memory), 318 400 rows 39 (74, mode
+ * 2).  0.4 of it came from the scalars' quotients on the integer pipe
+ * (ieee_int.h, the same bits), 0.2 to 0.6 from dealing the slices evenly to the
+ * schedulers. */
 constexpr int kResSprThreads = 512;
 
 template <int MODE>
@@ -644,8 +647,11 @@ __global__ void __launch_bounds__(kResSprThreads, 1) k_spr_res(SprDev d, SprRes 
             }
         }
         __syncthreads();
-        /* s = K z */
-        for (int u = warp; u < nsl; u += NW) {
+        /* s = K z; the slices, longest first, to the four schedulers back
+         * and forth */
+        for (int n = warp; n < (nsl + 3) / 4 * 4; n += NW) {
+            const int u = n & 4 ? n ^ 3 : n;
+            if (u >= nsl) continue;
             const int2 sl = s_sl[u];
             const double *val = v_val + sl.x + lane;
             const unsigned short *col = v_col + sl.x + lane;
@@ -700,20 +706,20 @@ __global__ void __launch_bounds__(kResSprThreads, 1) k_spr_res(SprDev d, SprRes 
             if (it == 0) {
                 k_bb = k_rr = rr;
                 k_active = rr > 0 && rho != 0 && mu != 0;
-                if (k_active) alpha = rho / mu;
+                if (k_active) alpha = div_ieee(rho, mu);
                 k_rho = rho;
                 stop = max_iter <= 0;
             } else {
                 if (k_active) {
                     k_iters++;
                     k_rr = rr;
-                    beta = rho / k_rho;
-                    const double den = mu - beta * rho / k_alpha;
+                    beta = div_ieee(rho, k_rho);
+                    const double den = mu - div_ieee(beta * rho, k_alpha);
                     if (!(rr > tol * tol * k_bb) || rho == 0 || !(den != 0) || !isfinite(den)) {
                         k_active = 0;
                         beta = 0.0;
                     } else {
-                        alpha = rho / den;
+                        alpha = div_ieee(rho, den);
                         k_rho = rho;
                     }
                 }
