@@ -986,6 +986,16 @@ static int solo_ctas(int cap_clusters, int C) {
     return std::max(1, sms - cap_clusters * C);
 }
 
+/* The stream and events of a launch beside the caller's. */
+static int side_stream(DeviceSet &S) {
+    if (!S.side) {
+        NR_CUDA_TRY(cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking));
+        NR_CUDA_TRY(cudaEventCreateWithFlags(&S.ev_fork, cudaEventDisableTiming));
+        NR_CUDA_TRY(cudaEventCreateWithFlags(&S.ev_join, cudaEventDisableTiming));
+    }
+    return NR_OK;
+}
+
 static int relax_dsm_phases(DeviceSet &S, const nr_fire_params &prm, DsmPlan pl, cudaStream_t stream,
                             bool capture = false) {
     const double frac = escalate_fraction();
@@ -997,11 +1007,8 @@ static int relax_dsm_phases(DeviceSet &S, const nr_fire_params &prm, DsmPlan pl,
     int cap = 0;
     const int n_small = solo_split(S, pl, ps, cap);
     if (n_small > 0) {
-        if (!S.side) {
-            NR_CUDA_TRY(cudaStreamCreateWithFlags(&S.side, cudaStreamNonBlocking));
-            NR_CUDA_TRY(cudaEventCreateWithFlags(&S.ev_fork, cudaEventDisableTiming));
-            NR_CUDA_TRY(cudaEventCreateWithFlags(&S.ev_join, cudaEventDisableTiming));
-        }
+        const int rc = side_stream(S);
+        if (rc != NR_OK) return rc;
         n_run = S.n_nets - n_small;
     }
     /* Device-side escalation (the default; NR_ESCALATE_HOST=1 steers from
@@ -1099,6 +1106,53 @@ static int fp64_batch_cluster(int max_nodes) {
     return max_nodes <= 2304 ? 1 : 8;
 }
 
+/* The narrow teams beside an FP64 batch's wide ones.  Clusters of 16 leave SMs
+ * idle (14 of them, two CTAs an SM, take 112 of 152: a cluster stays within a
+ * part of the chip), and a team's step costs about 11 us however small its
+ * network.  So teams of 4 on the idle SMs work from the small end of the order
+ * while two networks are left for every wide team: a step of theirs takes up to
+ * twice as long, and the batch must not end with their last network.  FP64
+ * results do not depend on the team.  100 steps of 64 lattices of 16^2 to 96^2
+ * nodes 10.8 -> 9.5 ms, of 100 of 8^2 to 40^2 10.1 -> 8.0; run to convergence (up
+ * to 20 000 steps), 64 of 16^2 to 48^2 776 -> 672 ms, 40 of 24^2 to 64^2 675 ->
+ * 672 (892 with narrow teams until the end). */
+struct Fp64Back {
+    int n = 0, leave = 0, clusters = 0; /* networks they may take (the order's last), those left alone, teams */
+    int bmax = 0, emax = 0, tmax = 0;
+};
+constexpr int kFp64BackTeam = 4;
+static Fp64Back fp64_back(const DeviceSet &S, int C, int bmax, int emax, int tmax) {
+    Fp64Back b;
+    int dev = 0, sms = 0, per_sm = 0, wide = 0;
+    if (C <= kFp64BackTeam || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        dsm64_max_active(C, bmax, emax, tmax, &wide) != cudaSuccess) {
+        cudaGetLastError();
+        return b;
+    }
+    b.leave = 2 * wide;
+    if (S.n_nets - wide <= b.leave) return b;
+    const size_t half = (size_t)per_sm / 2 - 1024; /* two CTAs an SM, 1 KB of each reserved */
+    const int used = dsm64_cta_bytes(bmax, emax, tmax) <= half ? (wide * C + 1) / 2 : wide * C;
+    b.clusters = std::max(0, sms - used) * 2 / kFp64BackTeam;
+    const int spr = kDsmParts / kFp64BackTeam;
+    for (int k = S.n_nets - 1; k >= 0 && b.clusters > 0; --k) { /* the order's suffix that fits half an SM a CTA */
+        const int i = S.order_host[k];
+        const NetDsm &m = S.dsm[i];
+        Fp64Back t = b;
+        t.bmax = std::max(t.bmax, spr * m.bsub);
+        for (int r = 0; r < kFp64BackTeam; ++r) {
+            if (S.dev[i].use_bonds) t.emax = std::max(t.emax, m.bo[(r + 1) * spr] - m.bo[r * spr]);
+            if (S.dev[i].use_triples) t.tmax = std::max(t.tmax, m.to[(r + 1) * spr] - m.to[r * spr]);
+        }
+        if (dsm64_cta_bytes(t.bmax, t.emax, t.tmax) > half) break;
+        t.n = b.n + 1;
+        b = t;
+    }
+    return b;
+}
+
 /* Enqueues one relaxation of every network of S (FIRE states zeroed, the
  * kernels) without waiting for it.  capture: stream work only, as a stream
  * capture needs (fails when escalation would be steered from the host). */
@@ -1124,8 +1178,23 @@ static int enqueue_set_batch(DeviceSet &S, const nr_fire_params &prm, cudaStream
         const int c = fp64_batch_cluster(S.max_nodes);
         int bmax = 0, emax = 0, tmax = 0;
         if (c > 1 && fp64_kernel_choice() <= kFp64Dsm && fp64_dsm_plan(S, c, bmax, emax, tmax)) {
+            const Fp64Back b = fp64_back(S, c, bmax, emax, tmax);
+            if (b.n > 0) {
+                const int st = side_stream(S);
+                if (st != NR_OK) return st;
+            }
+            NR_CUDA_TRY(cudaMemsetAsync(S.queue, 0, 16, stream));
+            if (b.n > 0) NR_CUDA_TRY(cudaEventRecord(S.ev_fork, stream));
             NR_CUDA_TRY(launch_fp64_dsm(S.dev_array, S.dsm_array, S.n_nets, c, bmax, emax, tmax, to_dev(prm), S.queue,
-                                        S.order, stream));
+                                        S.order, stream, false));
+            if (b.n > 0) {
+                NR_CUDA_TRY(cudaStreamWaitEvent(S.side, S.ev_fork, 0));
+                NR_CUDA_TRY(launch_fp64_dsm(S.dev_array, S.dsm_array, S.n_nets, kFp64BackTeam, b.bmax, b.emax, b.tmax,
+                                            to_dev(prm), S.queue, S.order, S.side, false, b.n, b.leave, b.clusters));
+                S.launches++;
+                NR_CUDA_TRY(cudaEventRecord(S.ev_join, S.side));
+                NR_CUDA_TRY(cudaStreamWaitEvent(stream, S.ev_join, 0));
+            }
         } else if (c > 1) {
             NR_CUDA_TRY(launch_fp64_cluster(S.dev_array, S.n_nets, c, false, to_dev(prm), S.queue, S.order, stream));
         } else {
@@ -1726,7 +1795,13 @@ int nr_batch_plan(nr_batch *b, int precision, char *buf, size_t cap) {
         const int c = fp64_batch_cluster(S.max_nodes);
         int bmax = 0, emax = 0, tmax = 0;
         if (c > 1 && fp64_kernel_choice() <= kFp64Dsm && fp64_dsm_plan(S, c, bmax, emax, tmax))
-            snprintf(out, sizeof out, "k_fire_dsm64 cluster=%d", c);
+        {
+            const Fp64Back b = fp64_back(S, c, bmax, emax, tmax);
+            if (b.n > 0)
+                snprintf(out, sizeof out, "k_fire_dsm64 cluster=%d beside cluster=%d clusters=%d networks=%d", c,
+                         kFp64BackTeam, b.clusters, b.n);
+            else snprintf(out, sizeof out, "k_fire_dsm64 cluster=%d", c);
+        }
         else if (c > 1) snprintf(out, sizeof out, "k_fire_cluster cluster=%d", c);
         else snprintf(out, sizeof out, "k_fire_batch (one CTA per network)");
     }

@@ -40,6 +40,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cstdint>
 
 #include "fire_launch.h"
 #include "fp64_step.cuh"
@@ -95,10 +96,31 @@ __host__ __device__ inline Dsm64Layout dsm64_layout(const Dsm64Sizes &z) {
 
 constexpr int kDsm64Threads = 256;
 
+/* A second launch of narrow teams beside the wide ones: it takes networks from
+ * the back of the order, its last n at most (0: not such a launch), while more
+ * than `leave` are left for the wide teams. */
+struct Dsm64Back {
+    int n, leave;
+};
+
+/* The next network of a batch of n in its order: from the front (the largest
+ * first), or for narrow teams from the back.  *q: networks taken from the front
+ * | from the back << 32.  n when there is none for this launch. */
+__device__ __forceinline__ int take_network(unsigned long long *q, int n, Dsm64Back b) {
+    unsigned long long old = *(volatile unsigned long long *)q;
+    for (;;) { /* a failed exchange means that another team took one */
+        const int front = (int)(unsigned)old, back = (int)(unsigned)(old >> 32), left = n - front - back;
+        if (left <= (b.n > 0 ? b.leave : 0) || (b.n > 0 && back >= b.n)) return n;
+        const unsigned long long seen = atomicCAS(q, old, old + (b.n > 0 ? 1ULL << 32 : 1ULL));
+        if (seen == old) return b.n > 0 ? n - 1 - back : front;
+        old = seen;
+    }
+}
+
 template <bool kPairs>
 __global__ void __launch_bounds__(kDsm64Threads, 2)
-    k_fire_dsm64(const NetDev *nets, const NetDsm *dsms, int n_nets, FireParamsDev p, int *queue, const int *order,
-                 Dsm64Sizes z) {
+    k_fire_dsm64(const NetDev *nets, const NetDsm *dsms, int n_nets, FireParamsDev p, unsigned long long *queue,
+                 Dsm64Back back, const int *order, Dsm64Sizes z) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ double2 s_dyn64[];
@@ -129,7 +151,7 @@ __global__ void __launch_bounds__(kDsm64Threads, 2)
         s_apt[threadIdx.x] = cl_addr(s_part, threadIdx.x);
     }
     for (;;) {
-        if (rank == 0 && threadIdx.x == 0) s_slot = atomicAdd(queue, 1);
+        if (rank == 0 && threadIdx.x == 0) s_slot = take_network(queue, n_nets, back);
         cl.sync();
         const int slot = *cl.map_shared_rank(&s_slot, 0);
         cl.sync(); /* every CTA read rank 0's slot before any may exit */
@@ -436,7 +458,7 @@ cudaError_t dsm64_max_active(int cluster, int bmax, int emax, int tmax, int *out
 
 cudaError_t launch_fp64_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, int cluster, int bmax,
                             int emax, int tmax, const FireParamsDev &p, int *queue_dev, const int *order_dev,
-                            cudaStream_t stream) {
+                            cudaStream_t stream, bool reset, int back_n, int back_leave, int cap) {
     if (cluster < 1 || cluster > kDsmParts || (kDsmParts % cluster) != 0) return cudaErrorInvalidValue;
     Dsm64Sizes z{std::max(bmax, 1), std::max(emax, 1), std::max(tmax, 1), 0};
     cudaLaunchConfig_t cfg;
@@ -445,12 +467,22 @@ cudaError_t launch_fp64_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int n
     cudaError_t e = dsm64_config(cluster, z, cfg, attr, &max_clusters);
     if (e != cudaSuccess) return e;
     if (max_clusters < 1) return cudaErrorLaunchOutOfResources;
-    cfg.gridDim = dim3(std::max(1, std::min(n_nets, max_clusters)) * cluster);
+    if (cap > 0) max_clusters = std::min(max_clusters, cap);
+    cfg.gridDim = dim3(std::max(1, std::min(back_n > 0 ? back_n : n_nets, max_clusters)) * cluster);
     cfg.stream = stream;
-    if ((e = cudaMemsetAsync(queue_dev, 0, sizeof(int), stream)) != cudaSuccess) return e;
+    unsigned long long *q = reinterpret_cast<unsigned long long *>(queue_dev);
+    if (reset && (e = cudaMemsetAsync(q, 0, sizeof(*q), stream)) != cudaSuccess) return e;
     FireParamsDev pp = p;
-    void *args[] = {&nets_dev, &dsm_dev, &n_nets, &pp, &queue_dev, &order_dev, &z};
+    Dsm64Back back{back_n, back_leave};
+    void *args[] = {&nets_dev, &dsm_dev, &n_nets, &pp, &q, &back, &order_dev, &z};
     return cudaLaunchKernelExC(&cfg, dsm64_kernel(z.pairs != 0), args);
+}
+
+/* Shared memory of a CTA with three forces a triple, static arrays included. */
+size_t dsm64_cta_bytes(int bmax, int emax, int tmax) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, dsm64_kernel(false)) != cudaSuccess) return SIZE_MAX;
+    return dsm64_layout(Dsm64Sizes{std::max(bmax, 1), std::max(emax, 1), std::max(tmax, 1), 0}).total + fa.sharedSizeBytes;
 }
 
 }  // namespace nr

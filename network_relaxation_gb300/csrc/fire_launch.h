@@ -51,9 +51,14 @@ cudaError_t launch_fp64_cluster(const NetDev *nets_dev, int n_nets, int cluster,
  * NetDsm layout, per-CTA maxima of nodes, bond slots and triple slots.  The
  * same bits as launch_fp64_grid. */
 cudaError_t dsm64_max_active(int cluster, int bmax, int emax, int tmax, int *out);
+/* (reset: zero the queue first.  back_n > 0: a second launch beside the first,
+ * from the back of the order, its last back_n networks at most and while more
+ * than back_leave are left.  cap > 0 limits the clusters.) */
+size_t dsm64_cta_bytes(int bmax, int emax, int tmax);
 cudaError_t launch_fp64_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, int cluster, int bmax,
                             int emax, int tmax, const FireParamsDev &p, int *queue_dev, const int *order_dev,
-                            cudaStream_t stream);
+                            cudaStream_t stream, bool reset = true, int back_n = 0, int back_leave = 0,
+                            int cap = 0);
 /* Host arrays of a Res64 layout (fire_res64.cu) and the resident FP64
  * kernel: layout (eptr / eent: per-node element entries 3 e + vertex;
  * partner: duplicate vertex or -1), shared-memory limit, co-residency and

@@ -1,7 +1,8 @@
 """FP64 batches on the cluster kernel (k_fire_dsm64) against the oracle, bit
 for bit: teams of every width, networks of one chunk and with partly filled
-last chunks and CTAs, and networks whose triples' forces only fit in pairs
-(about 1 520 to 1 780 nodes a CTA)."""
+last chunks and CTAs, networks whose triples' forces only fit in pairs
+(about 1 520 to 1 780 nodes a CTA), and batches large enough for narrow teams
+beside the wide ones, also as a graph."""
 import numpy as np
 import pytest
 
@@ -44,3 +45,17 @@ def test_teams(cuda, monkeypatch, team, line):
 def test_pairs(cuda, monkeypatch, kb):
     hosts = [nr.HostNetwork.lattice(nx, ny, 0.65, 0.0, 3).get_triples() for nx, ny in ((81, 80), (83, 80), (12, 9))]
     run(hosts, monkeypatch, 4, 25, kb)
+
+
+def test_narrow_teams_beside_wide(cuda, monkeypatch):
+    monkeypatch.setenv("NR_FP64_BATCH_CLUSTER", "16")
+    hosts = [nr.HostNetwork.lattice(4 + k % 17, 3 + k % 13, 0.75, 0.0, 200 + k).get_triples() for k in range(70)]
+    assert "beside" in nr.Batch(hosts, ks=1.0, kb=1e-3).plan("fp64")
+    run(hosts, monkeypatch, 16, 30)
+    sweep = []
+    for graph in (False, True):
+        b = nr.Batch(hosts, ks=1.0, kb=1e-3)
+        sweep.append(b.sweep((0.0, 0.0, 0.0), (0.01, 0.02, 0.01), nr.fire_params(fcut=1e-13, max_steps=20), graph=graph))
+    key = lambda r: (r.curr_disp, r.e_stretch, r.e_bend, r.max_force, r.steps)  # noqa: E731
+    plain, graphed = ([[key(r) for r in one] for one in recs] for recs in sweep)
+    assert len(plain) == 2 and plain == graphed
