@@ -485,7 +485,7 @@ namespace {
  * work repay their start; every thread has its own Scratch. */
 template <class Scratch, class F>
 void parallel_for(int n, long items, F f) {
-    const int nt = std::max(1, std::min({n, (int)std::thread::hardware_concurrency(), 16, (int)(items / 20000)}));
+    const int nt = std::max(1, std::min({n, (int)std::thread::hardware_concurrency(), 16, (int)(items / 3000)}));
     std::atomic<int> next{0};
     auto work = [&] {
         Scratch s;
