@@ -34,8 +34,8 @@
  * thread per node and component.
  *
  * Measured per FIRE step (us): 1 024 nodes 22.5 (cluster of 16) -> 8.4; 9 991
- * nodes 40 (grid kernel) -> 10.9; 65 536 nodes 77 -> 23.1, 90 000 nodes 36.7;
- * Mikado of 50 306 nodes 26; gel of 27 792 nodes 67 -> 27.6.  Of the 23.1 us:
+ * nodes 40 (grid kernel) -> 10.0; 65 536 nodes 77 -> 23.0, 93 000 nodes 35.0;
+ * Mikado of 50 306 nodes 25; gel of 27 792 nodes 67 -> 25.6.  Of the 23.0 us:
  * items 10.7, passes over nodes and the gather 7.1, barrier and imbalance 1.7,
  * totals and scalars 3.9; the FP64 pipe is active for 17.  512 threads: 768
  * and 1024 measured 3 to 9 % slower.
@@ -575,16 +575,21 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
         }
     };
     /* FP64 slots of the largest tile's step (per warp of items: bonds 8,
-     * triples 33, elements 45; nodes 45 a chunk) and of the totals that every
-     * CTA takes from the unit partials */
+     * triples 33, elements 45; nodes 45 a chunk; 12 for the halo, about a node
+     * a cut bond) and of the totals that every CTA takes from the unit
+     * partials */
     auto cost = [&](Cand &q) {
         const int sh = __builtin_ctz((unsigned)(kChunk * q.sub)); /* a power of two */
-        std::vector<int> nb(q.T, 0), nt3(q.T, 0), ne3(q.T, 0), nu(q.T, 0);
+        std::vector<int> nb(q.T, 0), nt3(q.T, 0), ne3(q.T, 0), nu(q.T, 0), cut(q.T, 0);
         auto of = [&](int i) { return q.tile[i >> sh]; };
         for (int b = 0; b < ne; ++b) {
             const int x = of(h.edge_ij[2 * b]), y = of(h.edge_ij[2 * b + 1]);
             nb[x]++;
-            if (y != x) nb[y]++;
+            if (y != x) {
+                nb[y]++;
+                cut[x]++;
+                cut[y]++;
+            }
         }
         auto three = [&](const int *v, std::vector<int> &cnt) {
             const int x = of(v[0]), y = of(v[1]), z = of(v[2]);
@@ -598,7 +603,7 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
         double worst = 0.0;
         for (int t = 0; t < q.T; ++t)
             worst = std::max(worst, 8 * std::ceil(nb[t] / 32.0) + 33 * std::ceil(nt3[t] / 32.0) +
-                                        45 * std::ceil(ne3[t] / 32.0) + 45.0 * nu[t] * q.sub);
+                                        45 * std::ceil(ne3[t] / 32.0) + 45.0 * nu[t] * q.sub + 12 * std::ceil(cut[t] / 32.0));
         q.cost = worst + 3.0 * (8 / q.sub - 1) * ((n + kTile - 1) / kTile) / 32.0;
     };
     const long items = (long)ne + nt + nel;
@@ -612,12 +617,20 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
         ux.assign(U, 0.0);
         uy.assign(U, 0.0);
         for (int u = 0; u < U; ++u) {
+            /* x from the unit's first node on, the shorter way around the
+             * period: a unit that runs over a row's end lies at the seam
+             * (taken in the middle of the row it tore tiles apart: 181 x 181
+             * nodes 77 % more items than the network has instead of 42, 19.2 us
+             * a step instead of 17.4) */
             const int i0 = u * un, i1 = std::min(n, i0 + un);
+            const double x0 = h.points[2 * i0];
             for (int i = i0; i < i1; ++i) {
-                ux[u] += h.points[2 * i];
+                const double dx = h.points[2 * i] - x0;
+                ux[u] += dx - W * std::round(dx / W);
                 uy[u] += h.points[2 * i + 1];
             }
-            ux[u] /= i1 - i0;
+            ux[u] = x0 + ux[u] / (i1 - i0);
+            ux[u] -= W * std::floor(ux[u] / W);
             uy[u] /= i1 - i0;
         }
         std::vector<int> &o = order[sub];
