@@ -14,9 +14,10 @@ libnetrelax.so).  A JSON record of every measurement goes beside it
 (<PATH>.json); --merge starts from an earlier table and replaces only the
 classes tuned now.  Knobs and size classes:
 
-  FP64, one network      NR_FP64_KERNEL (dsm | l2), NR_FP64_CLUSTER (CTAs per
+  FP64, one network      NR_FP64_KERNEL (res: the whole GPU, on chip | dsm |
+                         l2: one cluster), NR_FP64_CLUSTER (CTAs per
                          cluster), NR_FP64_CLUSTER_NODES (largest network run
-                         on a cluster instead of the grid kernel): time per
+                         on that kernel instead of the grid kernel): time per
                          FIRE step on lattices of 32^2 .. 181^2 nodes
   mixed, one network     NR_TILE_MIN_NODES (smallest network run on the tiled
                          kernel), NR_TILE_THREADS (512 or 768: one CTA per
@@ -99,28 +100,34 @@ def per_step_us(nr, torch, h, kb, precision, steps, gamma=0.02, reps=2):
 
 def tune_fp64_single(nr, torch, log, quick):
     sides = [32, 64, 96, 128, 181] if not quick else [32, 96]
-    variants = [("dsm", 16), ("dsm", 8), ("l2", 16), ("grid", 0)]
+    variants = [("res", 0), ("dsm", 16), ("dsm", 8), ("l2", 16), ("grid", 0)]
     res = {}
     for L in sides:
         h = nr.HostNetwork.lattice(L, L, 0.7, 0.0, 3).get_triples()
         for kind, c in variants:
             kv = dict(NR_FP64_CLUSTER_NODES=0) if kind == "grid" else dict(
-                NR_FP64_CLUSTER_NODES=10 ** 9, NR_FP64_KERNEL=kind, NR_FP64_CLUSTER=c)
+                NR_FP64_CLUSTER_NODES=10 ** 9, NR_FP64_KERNEL=kind, NR_FP64_CLUSTER=c or None)
             with knobs(**kv):
                 us, plan = per_step_us(nr, torch, h, 1e-3, "fp64", 1500 if L < 128 else 600)
             res[(L, kind, c)] = us
             log.append({"class": "fp64 single", "nodes": L * L, "kernel": kind, "cluster": c, "us_per_step": us,
                         "plan": plan})
     out = {}
-    # cluster variant: the best summed over the classes where clusters run
-    cl = [v for v in variants if v[0] != "grid"]
-    best = min(cl, key=lambda v: sum(res[(L, v[0], v[1])] for L in sides))
-    out["NR_FP64_KERNEL"], out["NR_FP64_CLUSTER"] = best
+
+    def total(v):
+        return sum(res[(L, v[0], v[1])] for L in sides)
+
+    # the kernel: the best summed over the classes; clusters (which networks
+    # that do not fit the resident kernel fall back to): the best of theirs
+    best = min((v for v in variants if v[0] != "grid"), key=total)
+    out["NR_FP64_KERNEL"] = best[0]
+    out["NR_FP64_CLUSTER"] = min((v for v in variants if v[1] > 0), key=total)[1]
     # threshold: the largest class where that variant beats the grid kernel
+    # (none if it is the largest measured)
     thr = 0
     for L in sides:
         if res[(L, best[0], best[1])] < res[(L, "grid", 0)]:
-            thr = L * L
+            thr = L * L if L < sides[-1] else 10 ** 9
     out["NR_FP64_CLUSTER_NODES"] = thr
     return out, res
 
