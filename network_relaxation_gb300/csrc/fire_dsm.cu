@@ -671,9 +671,7 @@ static cudaError_t dsm_config(int cluster, const DsmSizes &z, cudaLaunchConfig_t
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     const size_t smem = dsm_layout(z).total;
-    if ((e = cudaFuncSetAttribute(k_fire_dsm_mixed<NT, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-        cudaSuccess)
-        return e;
+    if ((e = allow_dynamic_smem((const void *)k_fire_dsm_mixed<NT, RES>, smem)) != cudaSuccess) return e;
     if (cluster > 8 &&
         (e = cudaFuncSetAttribute(k_fire_dsm_mixed<NT, RES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) !=
             cudaSuccess)

@@ -433,7 +433,7 @@ static cudaError_t dsm64_config(int cluster, Dsm64Sizes &z, cudaLaunchConfig_t &
         y.pairs = pairs;
         cfg.dynamicSmemBytes = dsm64_layout(y).total;
         int n = 0;
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes);
+        e = allow_dynamic_smem(k, cfg.dynamicSmemBytes);
         if (e == cudaSuccess && cluster > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
         if (e != cudaSuccess) {

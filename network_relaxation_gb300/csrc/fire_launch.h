@@ -13,6 +13,19 @@ struct nr_host_network;
 
 namespace nr {
 
+/* Lets `kernel` be launched with `smem` bytes of dynamic shared memory. The
+ * limit set is always the device's, not smem: another thread may lie between
+ * this call and the launch and must find room for its own. */
+inline cudaError_t allow_dynamic_smem(const void *kernel, size_t smem) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes fa;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e != cudaSuccess) return e;
+    if (smem + fa.sharedSizeBytes > (size_t)optin) return cudaErrorInvalidValue;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+}
 /* A cooperative launch (all CTAs co-resident, as the grid barriers need),
  * expressed as a launch attribute so that stream capture records it as a
  * cooperative kernel node of a CUDA graph. */

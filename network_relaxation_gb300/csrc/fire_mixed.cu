@@ -286,8 +286,7 @@ static cudaError_t launch_batch_nt(const NetDev *nets_dev, int n_nets, int max_n
                                    int *queue_dev, const int *order_dev, cudaStream_t stream) {
     const int smem_nodes = mixed_smem_nodes(max_nodes);
     const size_t smem = (size_t)smem_nodes * 16;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_fire_batch_mixed<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem((const void *)k_fire_batch_mixed<NT>, smem);
     if (e != cudaSuccess) return e;
     int dev, sms, per_sm = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;

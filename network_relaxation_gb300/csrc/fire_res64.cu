@@ -453,7 +453,7 @@ bool res64_fits(int ctas, bool gel, int mode, size_t smem) {
     const void *k = res_kernel(gel, mode);
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        allow_dynamic_smem(k, smem) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResThreads, smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -464,7 +464,7 @@ bool res64_fits(int ctas, bool gel, int mode, size_t smem) {
 cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
                             unsigned long long budget_ns, cudaStream_t stream) {
     const void *k = res_kernel(d.use_gel != 0, r.mode);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(r.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
     NetDev dd = d;

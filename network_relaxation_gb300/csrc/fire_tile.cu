@@ -804,7 +804,7 @@ int tile_grid_ctas(const NetTile &tl, int threads) {
     for (const bool resident : {false, true}) {
         const void *k = tile_kernel(threads, resident, tl.quads != 0);
         int per_sm = 0;
-        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
+        if (allow_dynamic_smem(k, smem) != cudaSuccess) return 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess) return 0;
         least = std::min(least, per_sm);
     }
@@ -814,7 +814,7 @@ int tile_grid_ctas(const NetTile &tl, int threads) {
 cudaError_t launch_mixed_tile(const NetDev &d, const NetTile &tl, const FireParamsDev &p, int ctas, int threads,
                               unsigned long long budget_ns, cudaStream_t stream) {
     const void *k = tile_kernel(threads, tl.n_tiles <= ctas, tl.quads != 0);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem(tl));
+    cudaError_t e = allow_dynamic_smem(k, tile_smem(tl));
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(tl.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
     NetDev dd = d;
