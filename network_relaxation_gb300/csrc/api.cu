@@ -998,7 +998,8 @@ static int side_stream(DeviceSet &S) {
 
 static int relax_dsm_phases(DeviceSet &S, const nr_fire_params &prm, DsmPlan pl, cudaStream_t stream,
                             bool capture = false) {
-    const double frac = escalate_fraction();
+    /* one network never finds others idle */
+    const double frac = S.n_nets > 1 ? escalate_fraction() : 0.0;
     int n_run = S.n_nets;
     const int *order_dev = S.order;
     std::vector<FireState> st;

@@ -29,7 +29,8 @@
  * conflict-free 16-byte load for four entries; lists behind one another cost
  * eight wavefronts for each 4-byte load), in shared memory where there is room,
  * and the next quad travels while one is added.  192-network batch of 600
- * steps 47.2 -> 36 ms, 30 networks of up to 30^2 nodes and 400 steps 2.2 -> 2.0;
+ * steps without escalation 47.2 -> 36 ms (phases that may escalate run the
+ * earlier kernel, fire_dsm_escalate.cu), 30 networks of up to 30^2 nodes and 400 steps 2.2 -> 2.0;
  * one network on 4 resident CTAs, us per step: 304 nodes 4.5 -> 3.5, 2491 nodes
  * 7.5 -> 6.0.  Loads from other CTAs (94 clocks a warp against 5 to 9) are
  * hidden: copying the boundary once a step and evaluating its items on both
@@ -726,9 +727,12 @@ cudaError_t launch_mixed_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int 
                              const FireParamsDev &p, int *queue_dev, const int *order_dev, cudaStream_t stream,
                              const int *n_dev) {
     if (cluster < 1 || cluster > kDsmParts || (kDsmParts % cluster) != 0) return cudaErrorInvalidValue;
+    const bool wide = dsm_threads(resident != 0) == 1024;
+    if (escalate > 0) /* when they yield is a matter of timing: fire_dsm_escalate.cu */
+        return launch_mixed_dsm_escalate(nets_dev, dsm_dev, n_nets, cluster, bmax, emax, tmax, ebmax, etmax, resident,
+                                         wide, escalate, cap, p, queue_dev, order_dev, stream, n_dev);
     DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident, 0};
     z.extra = dsm_extra(z);
-    const bool wide = dsm_threads(resident != 0) == 1024;
     if (resident)
         return wide ? launch_dsm_nt<1024, true>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p,
                                                 queue_dev, order_dev, stream)

@@ -109,6 +109,11 @@ cudaError_t launch_mixed_cluster(const NetDev *nets_dev, int n_nets, int cluster
                                  int *queue_dev, const int *order_dev, cudaStream_t stream);
 size_t dsm_smem_bytes(int bmax, int emax, int tmax, int ebmax, int etmax, int resident);
 size_t dsm_smem_limit();
+/* A phase that may escalate (fire_dsm_escalate.cu; from launch_mixed_dsm). */
+cudaError_t launch_mixed_dsm_escalate(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, int cluster, int bmax,
+                                      int emax, int tmax, int ebmax, int etmax, int resident, bool wide, double escalate,
+                                      int cap, const FireParamsDev &p, int *queue_dev, const int *order_dev,
+                                      cudaStream_t stream, const int *n_dev);
 /* One launch of the distributed-shared-memory kernel over n_nets networks
  * (order_dev[0..n_nets)); per-CTA maxima of nodes, bonds, triples and
  * incidence entries; resident: the CTAs keep their read-only slices in
