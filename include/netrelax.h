@@ -567,7 +567,8 @@ int nr_tile_layout_check(const nr_host_network *net, int ctas, int target_nodes,
  * reference, incidence entry, wrap and rest length equal to the network's,
  * halo nodes published by their owners).  stats[0..5]: tiles, chunks per
  * unit, largest shared memory (bytes), items over all tiles, halo nodes over
- * all tiles, violations found.  Returns NR_OK or the builder's error. */
+ * all tiles, violations found.  Returns NR_OK or the builder's error
+ * (NR_ERR_CAPACITY, NR_ERR_OOM). */
 int nr_res64_layout_check(const nr_host_network *net, int ctas, long long smem_limit, long long stats[6]);
 
 /* No reference counterpart; host only: builds the sub-block layout of the

@@ -55,6 +55,8 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
+#include <new>
 #include <thread>
 #include <vector>
 
@@ -482,19 +484,33 @@ cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParams
 namespace {
 
 /* Runs f(k, scratch) for k < n, on a few host threads when `items` items of
- * work repay their start; every thread has its own Scratch. */
+ * work repay their start; every thread has its own Scratch. A thread that
+ * cannot be started is done without (the others take its share); an exception
+ * in a thread ends the work and is thrown here once all threads are joined. */
 template <class Scratch, class F>
 void parallel_for(int n, long items, F f) {
     const int nt = std::max(1, std::min({n, (int)std::thread::hardware_concurrency(), 16, (int)(items / 3000)}));
     std::atomic<int> next{0};
+    std::atomic<bool> thrown{false};
+    std::exception_ptr error;
     auto work = [&] {
-        Scratch s;
-        for (int k; (k = next.fetch_add(1)) < n;) f(k, s);
+        try {
+            Scratch s;
+            for (int k; (k = next.fetch_add(1)) < n;) f(k, s);
+        } catch (...) {
+            if (!thrown.exchange(true)) error = std::current_exception();
+            next = n;
+        }
     };
     std::vector<std::thread> ts;
-    for (int t = 1; t < nt; ++t) ts.emplace_back(work);
+    ts.reserve(nt);
+    try {
+        for (int t = 1; t < nt; ++t) ts.emplace_back(work);
+    } catch (...) { /* std::system_error: no thread; bad_alloc: no room for its state */
+    }
     work();
     for (auto &t : ts) t.join();
+    if (error) std::rethrow_exception(error);
 }
 
 struct NoScratch {};
@@ -513,10 +529,10 @@ struct TileScratch {
  * bands.  NR_ERR_CAPACITY when a tile exceeds the 16-bit local encoding or
  * smem_limit, or when boundary items make the largest tile's work more than
  * 2.5 times an even share (the numbering then has no locality, and the
- * kernels that evaluate every item once are faster). */
-int build_res64_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
-                       bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
-                       const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out) {
+ * kernels that evaluate every item once are faster). May throw. */
+static int build_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
+                        bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
+                        const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out) {
     const int n = h.n_points, ne = use_bonds ? h.n_edges() : 0, nt = use_triples ? h.n_triples() : 0;
     const int nel = h.n_facets();
     if (n <= 0 || max_ctas < 1) return NR_ERR_INVALID;
@@ -869,12 +885,19 @@ int build_res64_layout(const nr_host_network &h, const Incidence &inc, const uns
     return NR_OK;
 }
 
-}  // namespace nr
+int build_res64_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
+                       bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
+                       const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out) {
+    try {
+        return build_layout(h, inc, fcodes, use_bonds, use_triples, eptr, eent, partner, max_ctas, smem_limit, out);
+    } catch (...) { /* no memory: the network runs on the other kernels */
+        out = Res64Host();
+        return NR_ERR_OOM;
+    }
+}
 
-extern "C" int nr_res64_layout_check(const nr_host_network *h, int ctas, long long smem_limit, long long stats[6]) {
-    using namespace nr;
-    if (!h || !stats || ctas < 1 || smem_limit < 1) return NR_ERR_INVALID;
-    for (int k = 0; k < 6; ++k) stats[k] = 0;
+/* nr_res64_layout_check; may throw. */
+static int check_res64_layout(const nr_host_network *h, int ctas, long long smem_limit, long long stats[6]) {
     const int n = h->n_points;
     Incidence inc;
     build_incidence(n, h->edge_ij.data(), h->n_edges(), h->tri_hjk.data(), h->n_triples(), true, true, inc);
@@ -1007,4 +1030,16 @@ extern "C" int nr_res64_layout_check(const nr_host_network *h, int ctas, long lo
     stats[4] = halo;
     stats[5] = bad;
     return NR_OK;
+}
+
+}  // namespace nr
+
+extern "C" int nr_res64_layout_check(const nr_host_network *h, int ctas, long long smem_limit, long long stats[6]) {
+    if (!h || !stats || ctas < 1 || smem_limit < 1) return NR_ERR_INVALID;
+    for (int k = 0; k < 6; ++k) stats[k] = 0;
+    try {
+        return nr::check_res64_layout(h, ctas, smem_limit, stats);
+    } catch (...) {
+        return NR_ERR_OOM;
+    }
 }
