@@ -17,7 +17,7 @@ classes tuned now.  Knobs and size classes:
   FP64, one network      NR_FP64_KERNEL (res: the whole GPU, on chip | dsm |
                          l2: one cluster), NR_FP64_CLUSTER (CTAs per
                          cluster), NR_FP64_CLUSTER_NODES (largest network run
-                         on that kernel instead of the grid kernel): time per
+                         on a cluster instead of the grid kernel): time per
                          FIRE step on lattices of 32^2 .. 181^2 nodes
   mixed, one network     NR_TILE_MIN_NODES (smallest network run on the tiled
                          kernel), NR_TILE_THREADS (512 or 768: one CTA per
@@ -122,12 +122,12 @@ def tune_fp64_single(nr, torch, log, quick):
     best = min((v for v in variants if v[0] != "grid"), key=total)
     out["NR_FP64_KERNEL"] = best[0]
     out["NR_FP64_CLUSTER"] = min((v for v in variants if v[1] > 0), key=total)[1]
-    # threshold: the largest class where that variant beats the grid kernel
-    # (none if it is the largest measured)
+    # threshold: the largest class where both cluster kernels beat the grid
+    # kernel (the table is also read when NR_FP64_KERNEL asks for either)
     thr = 0
     for L in sides:
-        if res[(L, best[0], best[1])] < res[(L, "grid", 0)]:
-            thr = L * L if L < sides[-1] else 10 ** 9
+        if all(res[(L, k, 16)] < res[(L, "grid", 0)] for k in ("dsm", "l2")):
+            thr = L * L
     out["NR_FP64_CLUSTER_NODES"] = thr
     return out, res
 

@@ -350,17 +350,19 @@ static int fp64_kernel_choice() {
     return kFp64Res;
 }
 
-/* FP64, one network: networks of at most NR_FP64_CLUSTER_NODES nodes relax
- * on the on-chip kernels (NR_FP64_KERNEL), larger ones, and those that fit
- * none, on the cooperative grid kernel.  All give the same bits.  The
- * resident kernel takes whatever fits the SMs' shared memory in one of its
- * modes (about 200 000 nodes of a p = 0.65 lattice); a cluster of NR_FP64_CLUSTER CTAs (default
- * 16) has the FP64 pipes of 16 SMs and beats the grid kernel up to
- * kFp64DsmNodes. */
+/* FP64, one network.  All kernels give the same bits.  The resident kernel
+ * takes whatever fits the SMs' shared memory in one of its modes (about
+ * 200 000 nodes of a p = 0.65 lattice).  A cluster of NR_FP64_CLUSTER CTAs
+ * (default 16; NR_FP64_KERNEL=dsm or l2, and in the resident kernel's place up
+ * to kFp64DsmNodes where that does not fit) takes networks of at most
+ * NR_FP64_CLUSTER_NODES nodes: it has the FP64 pipes of 16 SMs, and past that
+ * line the cooperative grid kernel on all of them is faster (us a step, dsm /
+ * l2 / grid: 4 096 nodes 19 / 28 / 41, 9 216 nodes 37 / 55 / 46, 32 761 nodes
+ * 136 / 136 / 41).  0: the grid kernel alone. */
 constexpr int kFp64DsmNodes = 4096;
 static int fp64_cluster_nodes() {
     const char *env = knob("NR_FP64_CLUSTER_NODES");
-    return env ? std::max(0, atoi(env)) : 1 << 30;
+    return env ? std::max(0, atoi(env)) : 16384;
 }
 
 /* Offsets of the resident FP64 layout in a network's image. */
@@ -432,7 +434,7 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     S.gel.assign(n, NetGel{});
     std::vector<NetOff> off(n);
     const bool want_tile = n == 1 && nets[0]->n_points >= tile_min_nodes();
-    const bool want_res = n == 1 && fp64_kernel_choice() == kFp64Res && nets[0]->n_points <= fp64_cluster_nodes();
+    const bool want_res = n == 1 && fp64_kernel_choice() == kFp64Res && fp64_cluster_nodes() > 0;
     Incidence inc0;
     std::vector<unsigned char> fc0;
     bool have_res = false;
@@ -781,13 +783,13 @@ static int grid_plan(const DeviceSet &S, int i, bool mixed, GridPlan &g) {
         if ((size_t)5 * g.blocks > (size_t)4 * g.d.n_tiles * 8) return fail(NR_ERR_CAPACITY, "reduction scratch too small");
     } else {
         const int choice = fp64_kernel_choice();
-        const bool on_chip = g.d.n <= fp64_cluster_nodes() && choice != kFp64Grid;
-        if (on_chip && choice == kFp64Res && S.res.n_ctas > 0 && !(g.d.use_gel && g.d.n_elems == 0)) {
+        const int line = choice == kFp64Grid ? 0 : fp64_cluster_nodes();
+        if (line > 0 && choice == kFp64Res && S.res.n_ctas > 0 && !(g.d.use_gel && g.d.n_elems == 0)) {
             g.res = true;
             g.rd = S.res;
             g.res_smem = S.res_smem;
             g.blocks = S.res.n_ctas;
-        } else if (on_chip && (choice != kFp64Res || g.d.n <= kFp64DsmNodes)) {
+        } else if (g.d.n <= (choice == kFp64Res ? std::min(line, kFp64DsmNodes) : line)) {
             int c = fp64_cluster_ctas(), active = 0;
             const std::vector<int> one{i};
             if (choice != kFp64L2 && fp64_dsm_plan(S, c, g.bmax, g.emax, g.tmax, &one)) {
