@@ -384,8 +384,8 @@ static bool add_res_layout(const nr_host_network &h, const Incidence &inc, const
     if (build_res64_layout(h, inc, fcodes, use_bonds, use_triples, eptr, eent, partner, sms, res64_smem_limit(), L) !=
         NR_OK)
         return false;
-    if (!res64_fits(L.n_ctas, false, L.mode, L.max_smem) ||
-        (h.n_facets() > 0 && !res64_fits(L.n_ctas, true, L.mode, L.max_smem)))
+    if (!res64_fits(L.n_ctas, L.shape, false, L.mode, L.max_smem) ||
+        (h.n_facets() > 0 && !res64_fits(L.n_ctas, L.shape, true, L.mode, L.max_smem)))
         return false;
     o.desc = img.put(L.desc.data(), L.desc.size());
     o.ro = img.put(L.ro.data(), L.ro.size());
@@ -626,6 +626,7 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         r.sub = res_host.sub;
         r.n_units = res_host.n_units;
         r.mode = res_host.mode;
+        r.shape = res_host.shape;
         r.desc = (const Res64Desc *)(base + res_off.desc);
         r.ro = (const unsigned char *)(base + res_off.ro);
         for (int c = 0; c < 2; ++c) {

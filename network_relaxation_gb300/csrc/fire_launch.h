@@ -80,6 +80,7 @@ struct Res64Host {
     int n_ctas = 0, sub = 1, n_units = 0;
     size_t max_smem = 0;
     int mode = 0; /* res64_segs */
+    int shape = 0;
     std::vector<Res64Desc> desc;
     std::vector<unsigned char> ro;
 };
@@ -88,7 +89,7 @@ int build_res64_layout(const ::nr_host_network &h, const Incidence &inc, const u
                        bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
                        const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out);
 size_t res64_smem_limit();
-bool res64_fits(int ctas, bool gel, int mode, size_t smem);
+bool res64_fits(int ctas, int shape, bool gel, int mode, size_t smem);
 cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
                             unsigned long long budget_ns, cudaStream_t stream);
 cudaError_t launch_forces(const NetDev &d, cudaStream_t stream);

@@ -78,7 +78,23 @@ __device__ __forceinline__ double res_tile_sum(const double *p, int sub) {
     return ((a.x + a.y) + (b.x + b.y)) + ((c.x + c.y) + (e.x + e.y));
 }
 
-constexpr int kResThreads = 512;
+/* CTA shapes for tiles that are held whole. A large network fills the SMs'
+ * FP64 pipes; a step of a small one is a chain of latencies, and networks
+ * relaxed from several threads have to share an SM or they run one after the
+ * other (each takes 128 of the 152 SMs from 4 096 nodes on).
+ *   kResSmall   256 threads, 80 registers, three on an SM: at most 8 groups of
+ *               items a tile and 64 tiles in the sums
+ *   kResShared  512 threads, 64 registers, two on an SM: fewer than 64 tiles in
+ *               the sums (16 129 nodes)
+ *   kResAlone   512 threads, one on an SM
+ * us per step and network, one thread | 16 threads, against one 512-thread CTA
+ * on an SM for all sizes: 1 024 nodes 8.5 | 2.1 -> 8.5 | 1.3, 4 096
+ * 8.8 | 8.8 -> 8.9 | 4.0, 4 900 9.2 | 9.2 -> 9.4 | 5.7, 9 216 9.8 | 9.7 -> 9.9 | 6.4,
+ * 12 544 12.3 | 12.1 -> 12.5 | 8.0; at 16 384, 11.2 | 11.3, one thread
+ * would lose 2 %. */
+enum { kResSmall, kResShared, kResAlone };
+constexpr int kResSmallGroups = 8, kResSmallTiles = 64, kResSharedTiles = 63;
+__host__ __device__ constexpr int res_threads(int shape) { return shape == kResSmall ? 256 : 512; }
 
 /* One tile of the network per CTA (Res64Desc / Res64Segs, nr_device.cuh).
  * kGel: the network carries a gel; its elements, their reference inverses
@@ -86,20 +102,22 @@ constexpr int kResThreads = 512;
  * kResWhole: tiles too large to be held whole; topology, v and F are read from
  * L2 in order, and what is reached at random (x, the items' forces) is in
  * shared memory. */
-template <bool kGel, int kMode>
-__global__ void __launch_bounds__(kResThreads, 1)
+template <int kShape, bool kGel, int kMode>
+__global__ void __launch_bounds__(res_threads(kShape))
+    __maxnreg__(kShape == kResSmall ? 80 : kShape == kResShared ? 64 : 128)
     k_fire_res64(NetDev d, Res64Dev r, FireParamsDev p, unsigned long long budget_ns) {
     extern __shared__ __align__(16) unsigned char s_raw[];
     __shared__ Scal s_sc;
     __shared__ double s_tot[24];
-    __shared__ unsigned long long s_max[kResThreads / 32];
+    __shared__ unsigned long long s_max[res_threads(kShape) / 32];
     __shared__ unsigned long long s_m2;
     __shared__ int s_ok;
     const Res64Desc td = r.desc[blockIdx.x];
     const Res64Segs g = res64_segs(td, kMode);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr bool kStream = kMode != kResWhole, kPairs = kMode == kResPairs;
-    constexpr int NT = kResThreads, NW = kResThreads / 32;
+    constexpr int NT = res_threads(kShape), NW = NT / 32;
+    constexpr int kSplit = kShape == kResSmall ? 2 : 4; /* lane groups whose sums take a warp each */
     const int sub = r.sub, un = kChunk * sub; /* nodes of a unit, a power of two */
     const int lg_un = 31 - __clz(un);
     const int no = td.nu * un;                /* own local indices (the last unit may be padded) */
@@ -370,18 +388,18 @@ __global__ void __launch_bounds__(kResThreads, 1)
             hv = __ldcg(q);
             hf = __ldcg(q + 1);
         }
-        /* the canonical totals.  Up to four lane groups: a warp each for
-         * every sum (the shortest chain); more: warp k sums the tiles of lane
-         * group k for all three (the fewest FP64 slots) */
-        if (ng <= 4) {
+        /* the canonical totals.  Up to kSplit lane groups: a warp each for
+         * every sum (the shortest chain); more (not kResSmall): warp k sums the
+         * tiles of lane group k for all three (the fewest FP64 slots) */
+        if (kShape == kResSmall || ng <= kSplit) {
             if (warp < 3 * ng) {
                 const int q = warp / ng, grp = warp - q * ng, t = 32 * grp + lane;
                 double a = t < d.n_tiles ? res_tile_sum(pt + (size_t)q * n_units + (size_t)t * upt, sub) : 0.0;
                 a = warp_sum(a);
                 if (lane == 0) s_tot[8 * q + grp] = a;
-            } else if (warp == 12) {
+            } else if (warp == 3 * kSplit) {
                 if (lane < 24 && (lane & 7) >= ng) s_tot[lane] = 0.0;
-            } else if (warp == 13) {
+            } else if (warp == 3 * kSplit + 1) {
                 unsigned long long m = 0ULL;
                 for (unsigned b = lane; b < gridDim.x; b += 32) m = max(m, __ldcg(r.maxp[par] + b));
                 m = warp_max_bits(m);
@@ -428,11 +446,16 @@ __global__ void __launch_bounds__(kResThreads, 1)
     if (blockIdx.x == 0 && tid == 0) scal_store(d.st, s_sc);
 }
 
-static const void *res_kernel(bool gel, int mode) {
-    if (mode == kResPairs) return gel ? (const void *)k_fire_res64<true, kResPairs> : (const void *)k_fire_res64<false, kResPairs>;
-    if (mode == kResStream)
-        return gel ? (const void *)k_fire_res64<true, kResStream> : (const void *)k_fire_res64<false, kResStream>;
-    return gel ? (const void *)k_fire_res64<true, kResWhole> : (const void *)k_fire_res64<false, kResWhole>;
+template <int kShape, int kMode>
+static const void *res_kernel_of(bool gel) {
+    return gel ? (const void *)k_fire_res64<kShape, true, kMode> : (const void *)k_fire_res64<kShape, false, kMode>;
+}
+static const void *res_kernel(int shape, bool gel, int mode) {
+    if (mode == kResPairs) return res_kernel_of<kResAlone, kResPairs>(gel);
+    if (mode == kResStream) return res_kernel_of<kResAlone, kResStream>(gel);
+    if (shape == kResSmall) return res_kernel_of<kResSmall, kResWhole>(gel);
+    if (shape == kResShared) return res_kernel_of<kResShared, kResWhole>(gel);
+    return res_kernel_of<kResAlone, kResWhole>(gel);
 }
 
 /* Largest dynamic shared memory of the kernel on this device (NR_RES64_SMEM:
@@ -443,20 +466,20 @@ size_t res64_smem_limit() {
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return 0;
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, res_kernel(true, kResStream)) != cudaSuccess) return 0;
+    if (cudaFuncGetAttributes(&fa, res_kernel(kResAlone, true, kResStream)) != cudaSuccess) return 0;
     const size_t most = optin > (int)fa.sharedSizeBytes ? (size_t)(optin - (int)fa.sharedSizeBytes) : 0;
     const char *env = getenv("NR_RES64_SMEM");
     return env ? std::min(most, (size_t)std::max(0, atoi(env))) : most;
 }
 
 /* Whether `ctas` CTAs of the kernel are co-resident. */
-bool res64_fits(int ctas, bool gel, int mode, size_t smem) {
+bool res64_fits(int ctas, int shape, bool gel, int mode, size_t smem) {
     int dev = 0, sms = 0, per_sm = 0;
-    const void *k = res_kernel(gel, mode);
+    const void *k = res_kernel(shape, gel, mode);
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         allow_dynamic_smem(k, smem) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kResThreads, smem) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, res_threads(shape), smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -465,7 +488,7 @@ bool res64_fits(int ctas, bool gel, int mode, size_t smem) {
 
 cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParamsDev &p, size_t smem,
                             unsigned long long budget_ns, cudaStream_t stream) {
-    const void *k = res_kernel(d.use_gel != 0, r.mode);
+    const void *k = res_kernel(r.shape, d.use_gel != 0, r.mode);
     cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(r.bar, 0, sizeof(unsigned long long), stream)) != cudaSuccess) return e;
@@ -474,7 +497,7 @@ cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParams
     FireParamsDev pp = p;
     unsigned long long bb = budget_ns;
     void *args[] = {&dd, &rr, &pp, &bb};
-    return launch_cooperative(k, r.n_ctas, kResThreads, args, smem, stream);
+    return launch_cooperative(k, r.n_ctas, res_threads(r.shape), args, smem, stream);
 }
 
 /* ------------------------------------------------------------------ */
@@ -882,6 +905,12 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
         for (const Res64Desc &td : out.desc) out.max_smem = std::max(out.max_smem, (size_t)res64_segs(td, out.mode).total);
         if (out.max_smem <= smem_limit) break; /* at kResPairs at the latest (above) */
     }
+    unsigned groups = 0;
+    for (const Res64Desc &td : out.desc) groups = std::max(groups, res64_groups(td));
+    const int n_tiles = (n + kTile - 1) / kTile;
+    out.shape = kResAlone;
+    if (out.mode == kResWhole && n_tiles <= kResSharedTiles) out.shape = kResShared;
+    if (out.mode == kResWhole && n_tiles <= kResSmallTiles && groups <= kResSmallGroups) out.shape = kResSmall;
     return NR_OK;
 }
 

@@ -341,7 +341,7 @@ __host__ __device__ inline Res64Segs res64_segs(const Res64Desc &t, int mode) {
 }
 struct Res64Dev {
     int n_ctas, sub, n_units;       /* CTAs (tiles); chunks per unit; units, padded to whole 256-node tiles */
-    int mode;                       /* which k_fire_res64 (res64_segs) */
+    int mode, shape;                /* which k_fire_res64 (res64_segs; the CTA's shape) */
     const Res64Desc *desc;
     const unsigned char *ro;
     double2 *vf[2];                 /* published {v, F} per node, by step parity */
