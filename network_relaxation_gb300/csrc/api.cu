@@ -50,8 +50,18 @@ static unsigned barrier_stall() {
     return k > 0 && k < 1024 ? (unsigned)k : 0u;
 }
 
+/* A set's device memory: bytes that are uploaded, and behind them memory that
+ * starts as zeros (zeros(): offsets from zeros_at()). */
 struct Image {
     std::vector<char> bytes;
+    size_t n_zeros = 0;
+    size_t zeros(size_t nbytes) {
+        const size_t off = (n_zeros + 255) / 256 * 256;
+        n_zeros = off + nbytes;
+        return off;
+    }
+    size_t zeros_at() const { return (bytes.size() + 255) / 256 * 256; }
+    size_t total() const { return zeros_at() + n_zeros; }
     size_t add(size_t nbytes, size_t align = 256) {
         const size_t off = (bytes.size() + align - 1) / align * align;
         bytes.resize(off + nbytes);
@@ -70,7 +80,7 @@ struct NetOff {
     size_t dsm_bref, dsm_bidx, dsm_tref, dsm_bent, dsm_tent, dsm_grec, dsm_xrec, dsm_xent;
     size_t fcode, bond, bond_l0, bond_k, tri, tri_kb, tri_phi0, bptr, bent, tptr, tent, part, epart;
     size_t elem, elem_inv, elem_area, efrc, eptr, eent, partner;
-    bool has_bond_k, has_tri_kb, has_tri_phi0;
+    bool has_bond_k, has_tri_kb, has_tri_phi0, has_dsm_quads;
 };
 
 /* Device image of n networks (n = 1 for nr_network). */
@@ -131,7 +141,11 @@ struct DeviceSet {
  * bond's node i / the triple's hinge, in index order within a group; node
  * references and resolved incidence entries; per node, in gather order,
  * its gather record.  m.bsub = 0 when the network is too large for the
- * encoding (more than 2^20 nodes). */
+ * encoding (more than 2^20 nodes).  The mixed kernel's quads (xrec, xent) are
+ * left out where 32 B a node of 16 CTAs, the least it keeps in shared memory,
+ * exceed an SM's: a node of many entries has 31 others' lists filled up to its
+ * own. */
+constexpr int kDsmMaxSubBlock = 227 * 1024 / 32;
 static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, Image &img,
                              NetOff &o, NetDsm &m) {
     const int n = h.n_points, ne = h.n_edges(), nt = h.n_triples();
@@ -145,7 +159,8 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
     auto ref = [&](int v) { return (part(v) << 16) | (v % bsub); };
     std::vector<int2> bref(fits ? ne : 0);
     std::vector<int> bidx(fits ? ne : 0), bslot(fits ? ne : 0), dbent(fits ? inc.bent.size() : 0);
-    std::vector<int4> tref(fits ? nt : 0), grec(fits ? n : 0), xrec(fits ? n : 0);
+    const bool has_quads = fits && bsub <= kDsmMaxSubBlock;
+    std::vector<int4> tref(fits ? nt : 0), grec(fits ? n : 0), xrec(has_quads ? n : 0);
     size_t quads = 0;
     std::vector<int> tslot(fits ? nt : 0), dtent(fits ? inc.tent.size() : 0);
     if (fits) {
@@ -205,7 +220,7 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
             }
             /* bsub is a multiple of 32: the groups of a sub-block are the
              * groups a warp gathers */
-            for (int k0 = 0; k0 < v1 - v0; k0 += 32) {
+            for (int k0 = 0; has_quads && k0 < v1 - v0; k0 += 32) {
                 const int k1 = std::min(v1 - v0, k0 + 32);
                 int nq = 0;
                 for (int k = k0; k < k1; ++k) nq = std::max(nq, (nbe(ord[k]) + nte(ord[k]) + 3) / 4);
@@ -221,8 +236,9 @@ static void build_dsm_layout(const nr_host_network &h, const Incidence &inc, con
     o.dsm_bent = img.put(dbent.data(), dbent.size());
     o.dsm_tent = img.put(dtent.data(), dtent.size());
     o.dsm_grec = img.put(grec.data(), grec.size());
+    o.has_dsm_quads = has_quads;
     o.dsm_xrec = img.put(xrec.data(), xrec.size());
-    o.dsm_xent = img.add(sizeof(uint4) * quads);
+    o.dsm_xent = img.zeros(sizeof(uint4) * quads); /* written by the kernel */
 }
 
 /* Networks of at least NR_TILE_MIN_NODES nodes (default 131072) relaxed
@@ -514,14 +530,14 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         S.miny.push_back(h.miny);
         S.maxy.push_back(h.maxy);
     }
-    S.arena_bytes = img.bytes.size();
+    S.arena_bytes = img.total();
     cudaError_t e = cudaMalloc((void **)&S.arena, S.arena_bytes);
     if (e != cudaSuccess) {
         S.arena = nullptr;
         return fail(e == cudaErrorMemoryAllocation ? NR_ERR_OOM : NR_ERR_CUDA,
                     std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
-    char *base = S.arena;
+    char *base = S.arena, *zeros = S.arena + img.zeros_at();
     S.x_all = (double2 *)(base + x_off);
     S.v_all = (double2 *)(base + v_off);
     S.f_all = (double2 *)(base + f_off);
@@ -608,13 +624,14 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         m.bent = (const int *)(base + o.dsm_bent);
         m.tent = (const int *)(base + o.dsm_tent);
         m.grec = (const int4 *)(base + o.dsm_grec);
-        m.xrec = (const int4 *)(base + o.dsm_xrec);
-        m.xent = (uint4 *)(base + o.dsm_xent);
+        m.xrec = o.has_dsm_quads ? (const int4 *)(base + o.dsm_xrec) : nullptr;
+        m.xent = (uint4 *)(zeros + o.dsm_xent);
     }
     S.dsm_array = (NetDsm *)(base + dsm_off);
     memcpy(img.bytes.data() + dsm_off, S.dsm.data(), sizeof(NetDsm) * n);
     memcpy(img.bytes.data() + dev_off, S.dev.data(), sizeof(NetDev) * n);
-    NR_CUDA_TRY(cudaMemcpyAsync(S.arena, img.bytes.data(), S.arena_bytes, cudaMemcpyHostToDevice, stream));
+    NR_CUDA_TRY(cudaMemcpyAsync(S.arena, img.bytes.data(), img.bytes.size(), cudaMemcpyHostToDevice, stream));
+    NR_CUDA_TRY(cudaMemsetAsync(zeros, 0, img.n_zeros, stream));
     /* get_inv_mats on the positions as uploaded (network_mesh_relax.cu:1250
      * runs it before dilate) */
     for (int i = 0; i < n; ++i)
@@ -903,6 +920,7 @@ static bool dsm_plan(const DeviceSet &S, int forced, int least, DsmPlan &pl, con
             const int i = subset ? (*subset)[j] : j;
             const NetDsm &m = S.dsm[i];
             const NetDev &d = S.dev[i];
+            if (!m.xrec) return false;
             bm = std::max(bm, spr * m.bsub);
             for (int r = 0; r < C; ++r) {
                 if (d.use_bonds) {
@@ -2233,9 +2251,9 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
     const int *tent = (const int *)(base + o.dsm_tent);
     const int4 *grec = (const int4 *)(base + o.dsm_grec);
     const int4 *xrec = (const int4 *)(base + o.dsm_xrec);
-    const long long xquads = (long long)(img.bytes.size() - o.dsm_xent) / (long long)sizeof(uint4);
+    const long long xquads = (long long)(img.n_zeros / sizeof(uint4));
     const int bsub = m.bsub;
-    long long bad = 0;
+    long long bad = o.has_dsm_quads != (bsub <= kDsmMaxSubBlock) || (!o.has_dsm_quads && img.n_zeros > 0);
     auto ref_of = [&](int v) { return ((v / bsub) << 16) | (v % bsub); };
     std::vector<int> seen(n, 0);
     int parts = 0;
@@ -2247,10 +2265,13 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
             const int v = r.x & 0x0fffffff, f = (int)((unsigned)r.x >> 28);
             /* the group's record: the same node, room for its entries, the
              * same place for all 32 lanes and no other group's */
-            const int4 xr = xrec[k], x0 = xrec[k - (k - v0) % 32];
-            if (xr.x != r.x || xr.y != x0.y || xr.z != x0.z || 4 * xr.z < (r.z & 0xffff) + (int)((unsigned)r.z >> 16) ||
-                xr.y + 32LL * xr.z > xquads || (k > v0 && (k - v0) % 32 == 0 && xr.y < xrec[k - 1].y + 32 * xrec[k - 1].z))
-                ++bad;
+            if (o.has_dsm_quads) {
+                const int4 xr = xrec[k], x0 = xrec[k - (k - v0) % 32];
+                if (xr.x != r.x || xr.y != x0.y || xr.z != x0.z ||
+                    4 * xr.z < (r.z & 0xffff) + (int)((unsigned)r.z >> 16) || xr.y + 32LL * xr.z > xquads ||
+                    (k > v0 && (k - v0) % 32 == 0 && xr.y < xrec[k - 1].y + 32 * xrec[k - 1].z))
+                    ++bad;
+            }
             if (v < v0 || v >= v1) {
                 ++bad;
                 continue;
