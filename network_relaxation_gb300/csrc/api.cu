@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -52,27 +53,45 @@ static unsigned barrier_stall() {
 
 /* A set's device memory: bytes that are uploaded, and behind them memory that
  * starts as zeros (zeros(): offsets from zeros_at()). */
-struct Image {
-    std::vector<char> bytes;
-    size_t n_zeros = 0;
-    size_t zeros(size_t nbytes) {
-        const size_t off = (n_zeros + 255) / 256 * 256;
-        n_zeros = off + nbytes;
-        return off;
-    }
-    size_t zeros_at() const { return (bytes.size() + 255) / 256 * 256; }
-    size_t total() const { return zeros_at() + n_zeros; }
-    size_t add(size_t nbytes, size_t align = 256) {
-        const size_t off = (bytes.size() + align - 1) / align * align;
-        bytes.resize(off + nbytes);
+class Image {
+public:
+    Image() = default;
+    Image(const Image &) = delete;
+    Image &operator=(const Image &) = delete;
+    ~Image() { free(p_); }
+    char *data() { return p_; }
+    size_t size() const { return n_; }
+    size_t add(size_t nbytes) { /* to be written by the caller */
+        const size_t off = up(n_), end = off + nbytes;
+        if (end > cap_) {
+            cap_ = std::max(end, cap_ + cap_ / 2);
+            char *const q = (char *)realloc(p_, cap_);
+            if (!q) throw std::bad_alloc();
+            p_ = q;
+        }
+        memset(p_ + n_, 0, off - n_);
+        n_ = end;
         return off;
     }
     template <class T>
     size_t put(const T *src, size_t n) {
         const size_t off = add(n * sizeof(T));
-        if (n) memcpy(bytes.data() + off, src, n * sizeof(T));
+        if (n) memcpy(p_ + off, src, n * sizeof(T));
         return off;
     }
+    size_t zeros(size_t nbytes) {
+        const size_t off = up(n_zeros_);
+        n_zeros_ = off + nbytes;
+        return off;
+    }
+    size_t zeros_at() const { return up(n_); }
+    size_t zeros_size() const { return n_zeros_; }
+    size_t total() const { return zeros_at() + n_zeros_; }
+
+private:
+    static size_t up(size_t n) { return (n + 255) / 256 * 256; }
+    char *p_ = nullptr;
+    size_t n_ = 0, cap_ = 0, n_zeros_ = 0;
 };
 
 struct NetOff {
@@ -322,35 +341,36 @@ static int build_tile_set(const nr_host_network &h, const Incidence &inc, const 
     const size_t o_tid = img.put(th.tid.data(), th.tid.size());
     size_t o_u[2], o_vf[2];
     for (int c = 0; c < 2; ++c) {
-        o_u[c] = img.add(sizeof(float4) * np);
-        o_vf[c] = img.add(sizeof(float4) * np);
+        o_u[c] = img.zeros(sizeof(float4) * np);
+        o_vf[c] = img.zeros(sizeof(float4) * np);
     }
-    const size_t o_fa = img.add(sizeof(float4) * np);
-    const size_t o_cpart = img.add(sizeof(float) * 5 * 2 * (size_t)ctas);
-    const size_t o_dpart = img.add(sizeof(double) * 2 * (size_t)ctas);
-    const size_t o_bar = img.add(sizeof(unsigned long long));
-    cudaError_t e = cudaMalloc((void **)&S.tile_mem, img.bytes.size());
+    const size_t o_fa = img.zeros(sizeof(float4) * np);
+    const size_t o_cpart = img.zeros(sizeof(float) * 5 * 2 * (size_t)ctas);
+    const size_t o_dpart = img.zeros(sizeof(double) * 2 * (size_t)ctas);
+    const size_t o_bar = img.zeros(sizeof(unsigned long long));
+    cudaError_t e = cudaMalloc((void **)&S.tile_mem, img.total());
     if (e != cudaSuccess) {
         S.tile_mem = nullptr;
         return fail(e == cudaErrorMemoryAllocation ? NR_ERR_OOM : NR_ERR_CUDA,
                     std::string("cudaMalloc (tile layout): ") + cudaGetErrorString(e));
     }
-    NR_CUDA_TRY(cudaMemcpyAsync(S.tile_mem, img.bytes.data(), img.bytes.size(), cudaMemcpyHostToDevice, stream));
+    char *b = S.tile_mem, *zeros = S.tile_mem + img.zeros_at();
+    NR_CUDA_TRY(cudaMemcpyAsync(S.tile_mem, img.data(), img.size(), cudaMemcpyHostToDevice, stream));
+    NR_CUDA_TRY(cudaMemsetAsync(zeros, 0, img.zeros_size(), stream));
     NR_CUDA_TRY(cudaStreamSynchronize(stream));
-    char *b = S.tile_mem;
     tl.desc = (const TileDesc *)(b + o_desc);
     tl.ro = (unsigned char *)(b + o_ro);
     tl.node_of_pos = (const int *)(b + o_nop);
     tl.bid = (const int *)(b + o_bid);
     tl.tid = (const int *)(b + o_tid);
     for (int c = 0; c < 2; ++c) {
-        tl.u[c] = (float4 *)(b + o_u[c]);
-        tl.vf[c] = (float4 *)(b + o_vf[c]);
+        tl.u[c] = (float4 *)(zeros + o_u[c]);
+        tl.vf[c] = (float4 *)(zeros + o_vf[c]);
     }
-    tl.fa = (float4 *)(b + o_fa);
-    tl.cpart = (float *)(b + o_cpart);
-    tl.dpart = (double *)(b + o_dpart);
-    tl.bar = (unsigned long long *)(b + o_bar);
+    tl.fa = (float4 *)(zeros + o_fa);
+    tl.cpart = (float *)(zeros + o_cpart);
+    tl.dpart = (double *)(zeros + o_dpart);
+    tl.bar = (unsigned long long *)(zeros + o_bar);
     S.tile_ctas = ctas;
     S.tile_threads = threads;
     return NR_OK;
@@ -404,13 +424,14 @@ static bool add_res_layout(const nr_host_network &h, const Incidence &inc, const
         (h.n_facets() > 0 && !res64_fits(L.n_ctas, L.shape, true, L.mode, L.max_smem)))
         return false;
     o.desc = img.put(L.desc.data(), L.desc.size());
-    o.ro = img.put(L.ro.data(), L.ro.size());
+    o.ro = img.add((size_t)L.ro_bytes);
+    for (int t = 0; t < L.n_ctas; ++t) memcpy(img.data() + o.ro + L.desc[t].ro_off, L.rec[t].data(), L.rec[t].size());
     for (int c = 0; c < 2; ++c) {
-        o.vf[c] = img.add(sizeof(double2) * 2 * (size_t)h.n_points);
-        o.part[c] = img.add(sizeof(double) * 3 * (size_t)L.n_units);
-        o.maxp[c] = img.add(sizeof(unsigned long long) * (size_t)L.n_ctas);
+        o.vf[c] = img.zeros(sizeof(double2) * 2 * (size_t)h.n_points);
+        o.part[c] = img.zeros(sizeof(double) * 3 * (size_t)L.n_units);
+        o.maxp[c] = img.zeros(sizeof(unsigned long long) * (size_t)L.n_ctas);
     }
-    o.bar = img.add(sizeof(unsigned long long));
+    o.bar = img.zeros(sizeof(unsigned long long));
     return true;
 }
 
@@ -426,23 +447,23 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     }
     S.total_nodes = S.node_off[n];
     const size_t x_off = img.add(sizeof(double2) * S.total_nodes);
-    const size_t v_off = img.add(sizeof(double2) * S.total_nodes);
-    const size_t f_off = img.add(sizeof(double2) * S.total_nodes);
-    const size_t u_off = img.add(sizeof(float4) * S.total_nodes);
-    const size_t vf_off = img.add(sizeof(float2) * S.total_nodes);
-    const size_t ff_off = img.add(sizeof(float2) * S.total_nodes);
-    const size_t fah_off = img.add(sizeof(float2) * S.total_nodes);
-    const size_t fal_off = img.add(sizeof(float2) * S.total_nodes);
+    const size_t v_off = img.zeros(sizeof(double2) * S.total_nodes);
+    const size_t f_off = img.zeros(sizeof(double2) * S.total_nodes);
+    const size_t u_off = img.zeros(sizeof(float4) * S.total_nodes);
+    const size_t vf_off = img.zeros(sizeof(float2) * S.total_nodes);
+    const size_t ff_off = img.zeros(sizeof(float2) * S.total_nodes);
+    const size_t fah_off = img.zeros(sizeof(float2) * S.total_nodes);
+    const size_t fal_off = img.zeros(sizeof(float2) * S.total_nodes);
     std::vector<int> order(n);
     for (int i = 0; i < n; ++i) order[i] = i;
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return nets[a]->n_points > nets[b]->n_points; });
     const size_t order_off = img.put(order.data(), order.size());
     S.order_host = order;
-    const size_t order2_off = img.add(sizeof(int) * n);
-    const size_t st_off = img.add(sizeof(FireState) * n);
-    const size_t q_off = img.add(256);
-    const size_t aff_off = img.add(sizeof(double4) * n);
+    const size_t order2_off = img.zeros(sizeof(int) * n);
+    const size_t st_off = img.zeros(sizeof(FireState) * n);
+    const size_t q_off = img.zeros(256);
+    const size_t aff_off = img.zeros(sizeof(double4) * n);
     const size_t dev_off = img.add(sizeof(NetDev) * n);
     const size_t dsm_off = img.add(sizeof(NetDsm) * n);
     const size_t gel_off = img.add(sizeof(NetGel) * n);
@@ -458,7 +479,7 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     Res64Host res_host;
     for (int i = 0; i < n; ++i) {
         const nr_host_network &h = *nets[i];
-        memcpy(img.bytes.data() + x_off + sizeof(double2) * S.node_off[i], h.points.data(),
+        memcpy(img.data() + x_off + sizeof(double2) * S.node_off[i], h.points.data(),
                sizeof(double) * 2 * h.n_points);
         std::vector<unsigned char> fc(h.n_points);
         if (fcodes_in && fcodes_in[i]) memcpy(fc.data(), fcodes_in[i], h.n_points);
@@ -488,14 +509,14 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         o.tptr = img.put(inc.tptr.data(), inc.tptr.size());
         o.tent = img.put(inc.tent.data(), inc.tent.size());
         /* mixed precision: per-item anchor records and force changes */
-        o.mb_data = img.add(sizeof(float4) * (size_t)ne);
-        o.mb_sk = img.add(sizeof(float2) * (size_t)ne);
-        o.bdf = img.add(sizeof(float2) * (size_t)ne);
-        o.mt_arms = img.add(sizeof(float4) * (size_t)nt);
-        o.mt_pk = img.add(sizeof(float2) * (size_t)nt);
-        o.tdf = img.add(sizeof(float4) * (size_t)nt);
-        o.bfrc = img.add(sizeof(double2) * (size_t)ne);
-        o.tfrc = img.add(sizeof(double4) * (size_t)nt);
+        o.mb_data = img.zeros(sizeof(float4) * (size_t)ne);
+        o.mb_sk = img.zeros(sizeof(float2) * (size_t)ne);
+        o.bdf = img.zeros(sizeof(float2) * (size_t)ne);
+        o.mt_arms = img.zeros(sizeof(float4) * (size_t)nt);
+        o.mt_pk = img.zeros(sizeof(float2) * (size_t)nt);
+        o.tdf = img.zeros(sizeof(float4) * (size_t)nt);
+        o.bfrc = img.zeros(sizeof(double2) * (size_t)ne);
+        o.tfrc = img.zeros(sizeof(double4) * (size_t)nt);
         /* gel: triangles, inverse matrices (computed on the device after the
          * upload), element terms, per-node element incidence (3 e + role,
          * elements in index order) and duplicate partners */
@@ -507,9 +528,9 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         S.gel_ok.push_back(pairs_ok);
         S.minx.push_back(h.minx);
         o.elem = img.put(elem.data(), elem.size());
-        o.elem_inv = img.add(sizeof(double) * 6 * (size_t)nf);
+        o.elem_inv = img.zeros(sizeof(double) * 6 * (size_t)nf);
         o.elem_area = img.put(h.areas.data(), h.areas.size());
-        o.efrc = img.add(sizeof(double4) * 3 * (size_t)nf);
+        o.efrc = img.zeros(sizeof(double4) * 3 * (size_t)nf);
         o.eptr = img.put(eptr.data(), eptr.size());
         o.eent = img.put(eent.data(), eent.size());
         o.partner = img.put(partner.data(), partner.size());
@@ -524,9 +545,9 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         if (S.dsm[i].bsub <= 0) S.dsm_ok = false;
         S.max_nodes = std::max(S.max_nodes, h.n_points);
         const int tiles = (h.n_points + kTile - 1) / kTile;
-        o.part = img.add(sizeof(double) * 4 * (size_t)tiles * 8);
+        o.part = img.zeros(sizeof(double) * 4 * (size_t)tiles * 8);
         const int tb = (ne + kTile - 1) / kTile, tt = (nt + kTile - 1) / kTile, tg = (nf + kTile - 1) / kTile;
-        o.epart = img.add(sizeof(double) * kEpartLists * (size_t)std::max(1, std::max(tb, std::max(tt, tg))));
+        o.epart = img.zeros(sizeof(double) * kEpartLists * (size_t)std::max(1, std::max(tb, std::max(tt, tg))));
         S.miny.push_back(h.miny);
         S.maxy.push_back(h.maxy);
     }
@@ -539,18 +560,18 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     }
     char *base = S.arena, *zeros = S.arena + img.zeros_at();
     S.x_all = (double2 *)(base + x_off);
-    S.v_all = (double2 *)(base + v_off);
-    S.f_all = (double2 *)(base + f_off);
-    S.u_all = (float4 *)(base + u_off);
-    S.vf_all = (float2 *)(base + vf_off);
-    S.ff_all = (float2 *)(base + ff_off);
-    S.fa_hi_all = (float2 *)(base + fah_off);
-    S.fa_lo_all = (float2 *)(base + fal_off);
+    S.v_all = (double2 *)(zeros + v_off);
+    S.f_all = (double2 *)(zeros + f_off);
+    S.u_all = (float4 *)(zeros + u_off);
+    S.vf_all = (float2 *)(zeros + vf_off);
+    S.ff_all = (float2 *)(zeros + ff_off);
+    S.fa_hi_all = (float2 *)(zeros + fah_off);
+    S.fa_lo_all = (float2 *)(zeros + fal_off);
     S.order = (int *)(base + order_off);
-    S.order2 = (int *)(base + order2_off);
-    S.st = (FireState *)(base + st_off);
-    S.queue = (int *)(base + q_off);
-    S.affine_prm = (double4 *)(base + aff_off);
+    S.order2 = (int *)(zeros + order2_off);
+    S.st = (FireState *)(zeros + st_off);
+    S.queue = (int *)(zeros + q_off);
+    S.affine_prm = (double4 *)(zeros + aff_off);
     S.dev_array = (NetDev *)(base + dev_off);
     S.dev.resize(n);
     for (int i = 0; i < n; ++i) {
@@ -579,14 +600,14 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         d.ff = S.ff_all + S.node_off[i];
         d.fa_hi = S.fa_hi_all + S.node_off[i];
         d.fa_lo = S.fa_lo_all + S.node_off[i];
-        d.mb_data = (float4 *)(base + o.mb_data);
-        d.mb_sk = (float2 *)(base + o.mb_sk);
-        d.bdf = (float2 *)(base + o.bdf);
-        d.mt_arms = (float4 *)(base + o.mt_arms);
-        d.mt_pk = (float2 *)(base + o.mt_pk);
-        d.tdf = (float4 *)(base + o.tdf);
-        d.bfrc = (double2 *)(base + o.bfrc);
-        d.tfrc = (double4 *)(base + o.tfrc);
+        d.mb_data = (float4 *)(zeros + o.mb_data);
+        d.mb_sk = (float2 *)(zeros + o.mb_sk);
+        d.bdf = (float2 *)(zeros + o.bdf);
+        d.mt_arms = (float4 *)(zeros + o.mt_arms);
+        d.mt_pk = (float2 *)(zeros + o.mt_pk);
+        d.tdf = (float4 *)(zeros + o.tdf);
+        d.bfrc = (double2 *)(zeros + o.bfrc);
+        d.tfrc = (double4 *)(zeros + o.tfrc);
         d.fcode = (const unsigned char *)(base + o.fcode);
         d.bond = (const int4 *)(base + o.bond);
         d.bond_l0 = (const double *)(base + o.bond_l0);
@@ -598,23 +619,23 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         d.bent = (const int *)(base + o.bent);
         d.tptr = (const int *)(base + o.tptr);
         d.tent = (const int *)(base + o.tent);
-        d.part = (double *)(base + o.part);
-        d.epart = (double *)(base + o.epart);
+        d.part = (double *)(zeros + o.part);
+        d.epart = (double *)(zeros + o.epart);
         d.st = S.st + i;
         d.n_elems = h.n_facets();
         d.use_gel = 0;
         d.gel = (const NetGel *)(base + gel_off) + i;
         NetGel &g = S.gel[i];
         g.elem = (const int4 *)(base + o.elem);
-        g.elem_inv = (double *)(base + o.elem_inv);
+        g.elem_inv = (double *)(zeros + o.elem_inv);
         g.elem_area = (const double *)(base + o.elem_area);
-        g.efrc = (double4 *)(base + o.efrc);
+        g.efrc = (double4 *)(zeros + o.efrc);
         g.eptr = (const int *)(base + o.eptr);
         g.eent = (const int *)(base + o.eent);
         g.partner = (const int *)(base + o.partner);
     }
     S.gel_array = (NetGel *)(base + gel_off);
-    memcpy(img.bytes.data() + gel_off, S.gel.data(), sizeof(NetGel) * n);
+    memcpy(img.data() + gel_off, S.gel.data(), sizeof(NetGel) * n);
     for (int i = 0; i < n; ++i) {
         const NetOff &o = off[i];
         NetDsm &m = S.dsm[i];
@@ -628,10 +649,10 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         m.xent = (uint4 *)(zeros + o.dsm_xent);
     }
     S.dsm_array = (NetDsm *)(base + dsm_off);
-    memcpy(img.bytes.data() + dsm_off, S.dsm.data(), sizeof(NetDsm) * n);
-    memcpy(img.bytes.data() + dev_off, S.dev.data(), sizeof(NetDev) * n);
-    NR_CUDA_TRY(cudaMemcpyAsync(S.arena, img.bytes.data(), img.bytes.size(), cudaMemcpyHostToDevice, stream));
-    NR_CUDA_TRY(cudaMemsetAsync(zeros, 0, img.n_zeros, stream));
+    memcpy(img.data() + dsm_off, S.dsm.data(), sizeof(NetDsm) * n);
+    memcpy(img.data() + dev_off, S.dev.data(), sizeof(NetDev) * n);
+    NR_CUDA_TRY(cudaMemcpyAsync(S.arena, img.data(), img.size(), cudaMemcpyHostToDevice, stream));
+    NR_CUDA_TRY(cudaMemsetAsync(zeros, 0, img.zeros_size(), stream));
     /* get_inv_mats on the positions as uploaded (network_mesh_relax.cu:1250
      * runs it before dilate) */
     for (int i = 0; i < n; ++i)
@@ -647,11 +668,11 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
         r.desc = (const Res64Desc *)(base + res_off.desc);
         r.ro = (const unsigned char *)(base + res_off.ro);
         for (int c = 0; c < 2; ++c) {
-            r.vf[c] = (double2 *)(base + res_off.vf[c]);
-            r.part[c] = (double *)(base + res_off.part[c]);
-            r.maxp[c] = (unsigned long long *)(base + res_off.maxp[c]);
+            r.vf[c] = (double2 *)(zeros + res_off.vf[c]);
+            r.part[c] = (double *)(zeros + res_off.part[c]);
+            r.maxp[c] = (unsigned long long *)(zeros + res_off.maxp[c]);
         }
-        r.bar = (unsigned long long *)(base + res_off.bar);
+        r.bar = (unsigned long long *)(zeros + res_off.bar);
         S.res_smem = res_host.max_smem;
         r.n_ctas = res_host.n_ctas;
     }
@@ -2243,7 +2264,7 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
     NetDsm m;
     build_dsm_layout(*h, inc, fc.data(), img, o, m);
     if (m.bsub <= 0) return NR_ERR_CAPACITY;
-    const char *base = img.bytes.data();
+    const char *base = img.data();
     const int2 *bref = (const int2 *)(base + o.dsm_bref);
     const int *bidx = (const int *)(base + o.dsm_bidx);
     const int4 *tref = (const int4 *)(base + o.dsm_tref);
@@ -2251,9 +2272,9 @@ extern "C" int nr_dsm_layout_check(const nr_host_network *h, long long stats[4])
     const int *tent = (const int *)(base + o.dsm_tent);
     const int4 *grec = (const int4 *)(base + o.dsm_grec);
     const int4 *xrec = (const int4 *)(base + o.dsm_xrec);
-    const long long xquads = (long long)(img.n_zeros / sizeof(uint4));
+    const long long xquads = (long long)(img.zeros_size() / sizeof(uint4));
     const int bsub = m.bsub;
-    long long bad = o.has_dsm_quads != (bsub <= kDsmMaxSubBlock) || (!o.has_dsm_quads && img.n_zeros > 0);
+    long long bad = o.has_dsm_quads != (bsub <= kDsmMaxSubBlock) || (!o.has_dsm_quads && img.zeros_size() > 0);
     auto ref_of = [&](int v) { return ((v / bsub) << 16) | (v % bsub); };
     std::vector<int> seen(n, 0);
     int parts = 0;

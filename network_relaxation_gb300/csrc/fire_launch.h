@@ -82,7 +82,8 @@ struct Res64Host {
     int mode = 0; /* res64_segs */
     int shape = 0;
     std::vector<Res64Desc> desc;
-    std::vector<unsigned char> ro;
+    std::vector<std::vector<unsigned char>> rec; /* the tiles' records, one behind the other on the device */
+    long long ro_bytes = 0;
 };
 struct Incidence;
 int build_res64_layout(const ::nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,

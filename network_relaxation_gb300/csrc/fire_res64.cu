@@ -57,7 +57,9 @@
 #include <cstring>
 #include <exception>
 #include <new>
+#include <numeric>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "fire_launch.h"
@@ -537,22 +539,37 @@ void parallel_for(int n, long items, F f) {
 }
 
 struct NoScratch {};
-/* Local index of every node, slot of every item in the tile at hand (-1). */
+/* Halo index of every node in the tile at hand (-1). */
 struct TileScratch {
-    std::vector<int> loc, bslot, tslot, eslot;
+    std::vector<int> loc;
+};
+
+/* The items of every tile in index order (item[off[t] .. off[t + 1])) and the
+ * slot of each in the tile of each of its k nodes (slot[k q + r]). */
+struct TileItems {
+    std::vector<int> off, item, slot;
 };
 
 }  // namespace
 
-/* Tiles of whole reduction units (Res64Host).  Units are dealt to tiles in
- * strips of y and columns of x; of several unit sizes and column counts the
- * one whose largest tile takes the fewest FP64 slots is taken: row-ordered
- * lattices get blocks (256 x 256: 152 tiles of 32 x 13 or 14 nodes that
- * evaluate 12 % more items than the network has), networks numbered by y
- * bands.  NR_ERR_CAPACITY when a tile exceeds the 16-bit local encoding or
- * smem_limit, or when boundary items make the largest tile's work more than
- * 2.5 times an even share (the numbering then has no locality, and the
- * kernels that evaluate every item once are faster). May throw. */
+/* Tiles of whole reduction units (Res64Host).  A network of no more chunks than
+ * there are CTAs gets a chunk a tile.  Else units are dealt to tiles in strips
+ * of y and columns of x; of several unit sizes and column counts the one whose
+ * largest tile takes the fewest FP64 slots is taken: row-ordered lattices get
+ * blocks (256 x 256: 152 tiles of 32 x 13 or 14 nodes that evaluate 12 % more
+ * items than the network has), networks numbered by y bands.  NR_ERR_CAPACITY
+ * when a tile exceeds the 16-bit local encoding or smem_limit, or when boundary
+ * items make the largest tile's work more than 2.5 times an even share (the
+ * numbering then has no locality, and the kernels that evaluate every item once
+ * are faster). May throw.
+ *
+ * Every network's creation pays for it, so the tiles' item lists come from one
+ * walk over the items in index order, without sorting and without a search for
+ * slots, and the records go to the image tile by tile.  Creating a network (us,
+ * without a layout | with): 1 024 nodes 183 | 420, 2 500 333 | 810, 10 000
+ * 1 309 | 3 030 (600, 1 350 and 3 400 when each tile gathered, sorted and
+ * numbered its items itself).  A host thread takes 25 to 40 us to start there:
+ * fewer than 3 000 items do not repay it. */
 static int build_layout(const nr_host_network &h, const Incidence &inc, const unsigned char *fcodes, bool use_bonds,
                         bool use_triples, const std::vector<int> &eptr, const std::vector<int> &eent,
                         const std::vector<int> &partner, int max_ctas, size_t smem_limit, Res64Host &out) {
@@ -649,45 +666,51 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
     std::vector<Cand> cand;
     std::vector<std::vector<double>> uxs(9), uys(9);
     std::vector<std::vector<int>> order(9);
-    for (int sub : {1, 2, 4, 8}) {
-        const int U = units_of(sub), un = kChunk * sub;
-        if (sub > 1 && (U < max_ctas || n < 16 * kTile)) break; /* fewer partials only matter when there are many */
-        std::vector<double> &ux = uxs[sub], &uy = uys[sub];
-        ux.assign(U, 0.0);
-        uy.assign(U, 0.0);
-        for (int u = 0; u < U; ++u) {
-            /* x from the unit's first node on, the shorter way around the
-             * period: a unit that runs over a row's end lies at the seam
-             * (taken in the middle of the row it tore tiles apart: 181 x 181
-             * nodes 77 % more items than the network has instead of 42, 19.2 us
-             * a step instead of 17.4) */
-            const int i0 = u * un, i1 = std::min(n, i0 + un);
-            const double x0 = h.points[2 * i0];
-            for (int i = i0; i < i1; ++i) {
-                const double dx = h.points[2 * i] - x0;
-                ux[u] += dx - W * std::round(dx / W);
-                uy[u] += h.points[2 * i + 1];
+    if (units_of(1) <= max_ctas) { /* a chunk a tile: nothing to choose */
+        cand.push_back(Cand{1, 1, units_of(1), std::vector<int>(units_of(1)), 0.0});
+        std::iota(cand[0].tile.begin(), cand[0].tile.end(), 0);
+        cost(cand[0]);
+    } else {
+        for (int sub : {1, 2, 4, 8}) {
+            const int U = units_of(sub), un = kChunk * sub;
+            if (sub > 1 && (U < max_ctas || n < 16 * kTile)) break; /* fewer partials only matter when there are many */
+            std::vector<double> &ux = uxs[sub], &uy = uys[sub];
+            ux.assign(U, 0.0);
+            uy.assign(U, 0.0);
+            for (int u = 0; u < U; ++u) {
+                /* x from the unit's first node on, the shorter way around the
+                 * period: a unit that runs over a row's end lies at the seam
+                 * (taken in the middle of the row it tore tiles apart: 181 x
+                 * 181 nodes 77 % more items than the network has instead of
+                 * 42, 19.2 us a step instead of 17.4) */
+                const int i0 = u * un, i1 = std::min(n, i0 + un);
+                const double x0 = h.points[2 * i0];
+                for (int i = i0; i < i1; ++i) {
+                    const double dx = h.points[2 * i] - x0;
+                    ux[u] += std::fabs(dx) < 0.499 * W ? dx : dx - W * std::round(dx / W);
+                    uy[u] += h.points[2 * i + 1];
+                }
+                ux[u] = x0 + ux[u] / (i1 - i0);
+                ux[u] -= W * std::floor(ux[u] / W);
+                uy[u] /= i1 - i0;
             }
-            ux[u] = x0 + ux[u] / (i1 - i0);
-            ux[u] -= W * std::floor(ux[u] / W);
-            uy[u] /= i1 - i0;
+            std::vector<int> &o = order[sub];
+            o.resize(U);
+            for (int u = 0; u < U; ++u) o[u] = u;
+            std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return uy[a] < uy[b]; });
+            /* columns: bands (c = 1), and around square tiles */
+            const int G = std::min(U, max_ctas), sq = std::max(1, (int)std::lround(std::sqrt(G * W / H)));
+            std::vector<int> cs{1};
+            for (int c : {sq / 3, sq / 2, 2 * sq / 3, 3 * sq / 4, sq}) cs.push_back(std::max(1, std::min(G, c)));
+            std::sort(cs.begin(), cs.end());
+            cs.erase(std::unique(cs.begin(), cs.end()), cs.end());
+            for (int c : cs) cand.push_back(Cand{sub, c, 0, {}, 1e300});
         }
-        std::vector<int> &o = order[sub];
-        o.resize(U);
-        for (int u = 0; u < U; ++u) o[u] = u;
-        std::stable_sort(o.begin(), o.end(), [&](int a, int b) { return uy[a] < uy[b]; });
-        /* columns: bands (c = 1), and around square tiles */
-        const int G = std::min(U, max_ctas), sq = std::max(1, (int)std::lround(std::sqrt(G * W / H)));
-        std::vector<int> cs{1};
-        for (int c : {sq / 3, sq / 2, 2 * sq / 3, 3 * sq / 4, sq}) cs.push_back(std::max(1, std::min(G, c)));
-        std::sort(cs.begin(), cs.end());
-        cs.erase(std::unique(cs.begin(), cs.end()), cs.end());
-        for (int c : cs) cand.push_back(Cand{sub, c, 0, {}, 1e300});
+        parallel_for<NoScratch>((int)cand.size(), items, [&](int k, NoScratch &) {
+            deal(cand[k], uxs[cand[k].sub], uys[cand[k].sub], order[cand[k].sub]);
+            cost(cand[k]);
+        });
     }
-    parallel_for<NoScratch>((int)cand.size(), items, [&](int k, NoScratch &) {
-        deal(cand[k], uxs[cand[k].sub], uys[cand[k].sub], order[cand[k].sub]);
-        cost(cand[k]);
-    });
     const Cand &best = *std::min_element(cand.begin(), cand.end(),
                                          [](const Cand &a, const Cand &b) { return a.cost < b.cost; });
     const int sub = best.sub, un = kChunk * sub, U = units_of(sub), T = best.T;
@@ -700,65 +723,113 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
      * networks are bound by latency and may do more) */
     if (best.cost > 2.5 * (8.0 * ne + 33.0 * nt + 45.0 * nel + 45.0 * n) / 32.0 / max_ctas + 2000.0)
         return NR_ERR_CAPACITY;
+    const int lg_un = __builtin_ctz((unsigned)un); /* a power of two */
     std::vector<std::vector<int>> tu(T);
-    for (int u = 0; u < U; ++u) tu[tile[u]].push_back(u);
+    std::vector<int> uslot(U);
+    for (int u = 0; u < U; ++u) {
+        uslot[u] = (int)tu[tile[u]].size();
+        tu[tile[u]].push_back(u);
+    }
+    auto tile_of = [&](int i) { return tile[i >> lg_un]; };
+    /* the tile besides its own that gathers a node, its duplicate's (-1) */
+    std::vector<int> other;
+    if (nel > 0) {
+        other.assign(n, -1);
+        for (int i = 0; i < n; ++i)
+            if (partner[i] >= 0 && tile_of(partner[i]) != tile_of(i)) other[i] = tile_of(partner[i]);
+    }
+    /* the items that touch a node gathered by a tile: bonds, triples, elements */
+    TileItems its[3];
+    auto list = [&](auto nodes, int count, const int *v, TileItems &L) {
+        constexpr int k = decltype(nodes)::value;
+        L.off.assign(T + 1, 0);
+        L.slot.resize((size_t)k * count);
+        /* f(tile) for each of an item's tiles once */
+        auto tiles = [&](const int *w, auto f) {
+            int ts[2 * k], m = 0;
+            auto add = [&](int t) {
+                for (int r = 0; r < m; ++r)
+                    if (ts[r] == t) return;
+                ts[m++] = t;
+                f(t);
+            };
+            for (int r = 0; r < k; ++r) add(tile_of(w[r]));
+            if (!other.empty())
+                for (int r = 0; r < k; ++r)
+                    if (other[w[r]] >= 0) add(other[w[r]]);
+        };
+        for (int q = 0; q < count; ++q) tiles(v + (size_t)k * q, [&](int t) { L.off[t + 1]++; });
+        for (int t = 0; t < T; ++t) L.off[t + 1] += L.off[t];
+        L.item.resize(L.off[T]);
+        std::vector<int> fill(L.off.begin(), L.off.end() - 1);
+        for (int q = 0; q < count; ++q) {
+            const int *const w = v + (size_t)k * q;
+            tiles(w, [&](int t) { L.item[fill[t]++] = q; });
+            for (int r = 0; r < k; ++r) L.slot[(size_t)k * q + r] = fill[tile_of(w[r])] - 1 - L.off[tile_of(w[r])];
+        }
+    };
+    parallel_for<NoScratch>(3, items, [&](int kind, NoScratch &) {
+        if (kind == 0) list(std::integral_constant<int, 3>(), nt, h.tri_hjk.data(), its[1]);
+        if (kind == 1) list(std::integral_constant<int, 2>(), ne, h.edge_ij.data(), its[0]);
+        if (kind == 2) list(std::integral_constant<int, 3>(), nel, h.facets.data(), its[2]);
+    });
     out.desc.assign(T, Res64Desc{});
-    std::vector<std::vector<unsigned char>> rec(T);
+    out.rec.resize(T);
     std::vector<std::vector<int>> halos(T);
     std::vector<char> failed(T, 0);
     const bool has_k = !h.bond_k.empty(), has_kb = !h.tri_kb.empty(), has_phi = !h.tri_phi0.empty();
     parallel_for<TileScratch>(T, items, [&](int t, TileScratch &sc) {
-        if (sc.loc.empty()) {
-            sc.loc.assign(n, -1);
-            sc.bslot.assign(ne, -1);
-            sc.tslot.assign(nt, -1);
-            sc.eslot.assign(nel, -1);
-        }
+        if (sc.loc.empty()) sc.loc.assign(n, -1);
         const std::vector<int> &un_of = tu[t];
         const int no = (int)un_of.size() * un;
+        struct Span {
+            const int *b, *e;
+            const int *begin() const { return b; }
+            const int *end() const { return e; }
+            size_t size() const { return (size_t)(e - b); }
+        };
+        auto span = [&](int kind) {
+            return Span{its[kind].item.data() + its[kind].off[t], its[kind].item.data() + its[kind].off[t + 1]};
+        };
+        const Span bl = span(0), tl = span(1), el = span(2);
         /* nodes gathered here: the own ones and other tiles' duplicate
-         * partners of own ones */
-        std::vector<int> gn, ghosts;
+         * partners of own ones; the longest lists first, so that the lanes of a
+         * warp gather equally many */
+        auto nbe = [&](int i) { return use_bonds ? inc.bptr[i + 1] - inc.bptr[i] : 0; };
+        auto nte = [&](int i) { return use_triples ? inc.tptr[i + 1] - inc.tptr[i] : 0; };
+        auto nee = [&](int i) { return eptr[i + 1] - eptr[i]; };
+        std::vector<std::pair<unsigned, int>> gn; /* (descending lists, place), later (.., node) */
+        std::vector<int> gather, ghosts, hal;
+        gather.reserve(no);
         for (int u : un_of)
             for (int i = u * un; i < std::min(n, (u + 1) * un); ++i) {
-                gn.push_back(i);
-                if (partner[i] >= 0 && tile[partner[i] / un] != t) ghosts.push_back(partner[i]);
+                gather.push_back(i);
+                if (!other.empty() && other[i] >= 0) ghosts.push_back(partner[i]);
             }
         std::sort(ghosts.begin(), ghosts.end());
         ghosts.erase(std::unique(ghosts.begin(), ghosts.end()), ghosts.end());
-        gn.insert(gn.end(), ghosts.begin(), ghosts.end());
-        std::vector<int> bl, tl, el, hal(ghosts);
-        /* the items of the gathered nodes, each once, in index order */
-        auto add = [](std::vector<int> &list, std::vector<int> &slot, int q) {
-            if (slot[q] < 0) {
-                slot[q] = 0;
-                list.push_back(q);
+        gather.insert(gather.end(), ghosts.begin(), ghosts.end());
+        gn.reserve(gather.size());
+        size_t ni = 0;
+        for (size_t k = 0; k < gather.size(); ++k) {
+            const int i = gather[k], a = nbe(i), b = nte(i), c = nee(i);
+            if (a > 255 || b > 255 || c > 255) {
+                failed[t] = 1;
+                return;
             }
-        };
-        for (int i : gn) {
-            if (use_bonds)
-                for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e) add(bl, sc.bslot, inc.bent[e] >> 1);
-            if (use_triples)
-                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e) add(tl, sc.tslot, inc.tent[e] >> 2);
-            for (int e = eptr[i]; e < eptr[i + 1]; ++e) add(el, sc.eslot, eent[e] / 3);
+            gn.push_back({0xffffffu - ((unsigned)c << 16 | (unsigned)b << 8 | (unsigned)a), (int)k});
+            ni += (size_t)a + b + c;
         }
-        auto number = [](std::vector<int> &list, std::vector<int> &slot) {
-            std::sort(list.begin(), list.end());
-            for (size_t k = 0; k < list.size(); ++k) slot[list[k]] = (int)k;
-        };
-        number(bl, sc.bslot);
-        number(tl, sc.tslot);
-        number(el, sc.eslot);
-        for (size_t u = 0; u < un_of.size(); ++u)
-            for (int i = un_of[u] * un; i < std::min(n, (un_of[u] + 1) * un); ++i)
-                sc.loc[i] = (int)u * un + i % un;
-        for (int i : ghosts) sc.loc[i] = 0;
+        std::sort(gn.begin(), gn.end());
+        for (auto &g : gn) g.second = gather[g.second];
+        hal.reserve(4 * (size_t)kChunk * un_of.size());
         auto touch = [&](int i) {
-            if (sc.loc[i] < 0) {
+            if (tile_of(i) != t && sc.loc[i] < 0) {
                 sc.loc[i] = 0;
                 hal.push_back(i);
             }
         };
+        for (int i : ghosts) touch(i);
         for (int b : bl) {
             touch(h.edge_ij[2 * b]);
             touch(h.edge_ij[2 * b + 1]);
@@ -771,45 +842,18 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
         for (size_t k = 0; k < hal.size(); ++k) sc.loc[hal[k]] = no + (int)k;
         struct Reset {
             TileScratch &sc;
-            const std::vector<int> &gn, &hal, &bl, &tl, &el;
+            const std::vector<int> &hal;
             ~Reset() {
-                for (int i : gn) sc.loc[i] = -1;
                 for (int i : hal) sc.loc[i] = -1;
-                for (int q : bl) sc.bslot[q] = -1;
-                for (int q : tl) sc.tslot[q] = -1;
-                for (int q : el) sc.eslot[q] = -1;
             }
-        } reset{sc, gn, hal, bl, tl, el};
-        auto local = [&](int i) { return sc.loc[i]; };
+        } reset{sc, hal};
+        auto local = [&](int i) {
+            const int u = i >> lg_un;
+            return tile[u] == t ? (uslot[u] << lg_un) + (i & (un - 1)) : sc.loc[i];
+        };
         if (no + hal.size() > 0xffff || bl.size() > 0x7fff || 3 * tl.size() > 0xffff || 3 * el.size() > 0xffff) {
             failed[t] = 1;
             return;
-        }
-        /* the longest lists first: the lanes of a warp gather equally many */
-        auto nbe = [&](int i) { return use_bonds ? inc.bptr[i + 1] - inc.bptr[i] : 0; };
-        auto nte = [&](int i) { return use_triples ? inc.tptr[i + 1] - inc.tptr[i] : 0; };
-        auto nee = [&](int i) { return eptr[i + 1] - eptr[i]; };
-        std::stable_sort(gn.begin(), gn.end(), [&](int a, int b) {
-            if (nee(a) != nee(b)) return nee(a) > nee(b);
-            return nte(a) != nte(b) ? nte(a) > nte(b) : nbe(a) > nbe(b);
-        });
-        std::vector<unsigned short> incv;
-        std::vector<uint2> grec;
-        for (int i : gn) {
-            if (nbe(i) > 255 || nte(i) > 255 || nee(i) > 255 || incv.size() > 0xffff) {
-                failed[t] = 1;
-                return;
-            }
-            grec.push_back(make_uint2((unsigned)local(i) | (unsigned)nbe(i) << 16 | (unsigned)nte(i) << 24,
-                                      (unsigned)incv.size() | (unsigned)nee(i) << 16 | (unsigned)(fcodes[i] & 3u) << 24));
-            if (use_bonds)
-                for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e)
-                    incv.push_back((unsigned short)(sc.bslot[inc.bent[e] >> 1] << 1 | (inc.bent[e] & 1)));
-            if (use_triples)
-                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e)
-                    incv.push_back((unsigned short)(3 * sc.tslot[inc.tent[e] >> 2] + (inc.tent[e] & 3)));
-            for (int e = eptr[i]; e < eptr[i + 1]; ++e)
-                incv.push_back((unsigned short)(3 * sc.eslot[eent[e] / 3] + eent[e] % 3));
         }
         Res64Desc &td = out.desc[t];
         td.nu = (int)un_of.size();
@@ -819,7 +863,7 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
         td.nt = (int)tl.size();
         td.nel = (int)el.size();
         td.ngather = (int)gn.size();
-        td.ni = (int)incv.size();
+        td.ni = (int)ni;
         td.has_k = has_k;
         td.has_kb = has_kb;
         td.has_phi = has_phi;
@@ -829,38 +873,68 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
             failed[t] = 1;
             return;
         }
-        std::vector<unsigned char> &o = rec[t];
+        std::vector<unsigned char> &o = out.rec[t];
         o.assign(g.rec, 0);
+        unsigned char *const rec = o.data();
         auto put = [&](unsigned off, const void *src, size_t bytes) {
-            if (bytes) memcpy(o.data() + off, src, bytes);
+            if (bytes) memcpy(rec + off, src, bytes);
         };
         put(g.units, un_of.data(), 4 * un_of.size());
         put(g.halo, hal.data(), 4 * hal.size());
         for (size_t k = 0; k < bl.size(); ++k) {
-            const int b = bl[k];
+            const int b = bl.b[k];
             const unsigned q = (unsigned)local(h.edge_ij[2 * b]) | (unsigned)local(h.edge_ij[2 * b + 1]) << 16;
-            put(g.bref + 4 * k, &q, 4);
-            put(g.bl0 + 8 * k, &h.edge_l0[b], 8);
-            if (has_k) put(g.bk + 8 * k, &h.bond_k[b], 8);
-            o[g.bwrap + k] = (unsigned char)h.edge_wrap[b];
+            memcpy(rec + g.bref + 4 * k, &q, 4);
+            memcpy(rec + g.bl0 + 8 * k, &h.edge_l0[b], 8);
+            if (has_k) memcpy(rec + g.bk + 8 * k, &h.bond_k[b], 8);
+            rec[g.bwrap + k] = (unsigned char)h.edge_wrap[b];
         }
         for (size_t k = 0; k < tl.size(); ++k) {
-            const int q = tl[k];
+            const int q = tl.b[k];
             const uint2 w = make_uint2((unsigned)local(h.tri_hjk[3 * q]) | (unsigned)local(h.tri_hjk[3 * q + 1]) << 16,
                                        (unsigned)local(h.tri_hjk[3 * q + 2]) |
                                            (unsigned)(unsigned char)h.tri_wrap[2 * q] << 16 |
                                            (unsigned)(unsigned char)h.tri_wrap[2 * q + 1] << 24);
-            put(g.tref + 8 * k, &w, 8);
-            if (has_kb) put(g.tkb + 8 * k, &h.tri_kb[q], 8);
-            if (has_phi) put(g.tphi + 8 * k, &h.tri_phi0[q], 8);
+            memcpy(rec + g.tref + 8 * k, &w, 8);
+            if (has_kb) memcpy(rec + g.tkb + 8 * k, &h.tri_kb[q], 8);
+            if (has_phi) memcpy(rec + g.tphi + 8 * k, &h.tri_phi0[q], 8);
         }
         for (size_t k = 0; k < el.size(); ++k) {
-            const int *f = &h.facets[3 * (size_t)el[k]];
+            const int *f = &h.facets[3 * (size_t)el.b[k]];
             const uint2 w = make_uint2((unsigned)local(f[0]) | (unsigned)local(f[1]) << 16, (unsigned)local(f[2]));
-            put(g.eref + 8 * k, &w, 8);
-            put(g.eid + 4 * k, &el[k], 4);
+            memcpy(rec + g.eref + 8 * k, &w, 8);
+            memcpy(rec + g.eid + 4 * k, &el.b[k], 4);
         }
-        put(g.grec, grec.data(), 8 * grec.size());
+        /* gather records and entries; a ghost's items by their place in the
+         * tile's lists */
+        auto slot = [&](int kind, int k, int q, int r, bool ghost) -> int {
+            if (!ghost) return its[kind].slot[(size_t)k * q + r];
+            const Span l = kind == 0 ? bl : kind == 1 ? tl : el;
+            return (int)(std::lower_bound(l.b, l.e, q) - l.b);
+        };
+        size_t at = 0;
+        for (size_t k = 0; k < gn.size(); ++k) {
+            const int i = gn[k].second;
+            const bool ghost = tile_of(i) != t;
+            if (at > 0xffff) {
+                failed[t] = 1;
+                return;
+            }
+            const uint2 w = make_uint2((unsigned)local(i) | (unsigned)nbe(i) << 16 | (unsigned)nte(i) << 24,
+                                       (unsigned)at | (unsigned)nee(i) << 16 | (unsigned)(fcodes[i] & 3u) << 24);
+            memcpy(rec + g.grec + 8 * k, &w, 8);
+            auto entry = [&](int v) {
+                const unsigned short c = (unsigned short)v;
+                memcpy(rec + g.inc + 2 * at++, &c, 2);
+            };
+            if (use_bonds)
+                for (int e = inc.bptr[i]; e < inc.bptr[i + 1]; ++e)
+                    entry(slot(0, 2, inc.bent[e] >> 1, inc.bent[e] & 1, ghost) << 1 | (inc.bent[e] & 1));
+            if (use_triples)
+                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e)
+                    entry(3 * slot(1, 3, inc.tent[e] >> 2, inc.tent[e] & 3, ghost) + (inc.tent[e] & 3));
+            for (int e = eptr[i]; e < eptr[i + 1]; ++e) entry(3 * slot(2, 3, eent[e] / 3, eent[e] % 3, ghost) + eent[e] % 3);
+        }
         /* groups of 32 items in the order the warps take them: four of one
          * kind (one for each scheduler), then four of the other, so that a
          * scheduler's warps are not all in their FP64 or all in their integer
@@ -874,7 +948,6 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
             for (int k = 0; k < 4 && b < light.size(); ++k) grp.push_back(light[b++]);
         }
         put(g.grp, grp.data(), 2 * grp.size());
-        put(g.inc, incv.data(), 2 * incv.size());
         if (td.has_gel)
             for (int u = 0; u < td.nu; ++u)
                 for (int k = 0; k < un; ++k) {
@@ -895,10 +968,10 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
         for (int u = 0; u < out.desc[t].nu; ++u)
             for (int k = 0; k < un; ++k) {
                 const int i = tu[t][u] * un + k;
-                rec[t][g.pub + (unsigned)(u * un + k)] = i < n ? wanted[i] : 0;
+                out.rec[t][g.pub + (unsigned)(u * un + k)] = i < n ? wanted[i] : 0;
             }
-        out.desc[t].ro_off = (long long)out.ro.size();
-        out.ro.insert(out.ro.end(), rec[t].begin(), rec[t].end());
+        out.desc[t].ro_off = out.ro_bytes; /* a multiple of 16 */
+        out.ro_bytes += (long long)out.rec[t].size();
     }
     for (out.mode = kResWhole;; ++out.mode) {
         out.max_smem = 0;
@@ -941,14 +1014,18 @@ static int check_res64_layout(const nr_host_network *h, int ctas, long long smem
     long long bad = 0, items = 0, halo = 0;
     std::vector<int> owned(n, 0), wanted(n, 0), published(n, 0);
     if (L.n_ctas > ctas || (int)L.desc.size() != L.n_ctas) ++bad;
+    long long ro_end = 0;
     for (const Res64Desc &td : L.desc) {
         const Res64Segs g = res64_segs(td, L.mode);
-        if (td.ro_off % 16 || td.ro_off + (long long)g.rec > (long long)L.ro.size() || g.total > (unsigned)smem_limit ||
+        const std::vector<unsigned char> &record = L.rec[&td - L.desc.data()];
+        const bool placed = td.ro_off % 16 == 0 && td.ro_off == ro_end && record.size() == res64_segs(td, kResWhole).rec;
+        ro_end = td.ro_off + (long long)record.size();
+        if (!placed || ro_end > L.ro_bytes || g.total > (unsigned)smem_limit ||
             g.total > L.max_smem || td.no != td.nu * un) {
             ++bad;
             continue;
         }
-        const unsigned char *rec = L.ro.data() + td.ro_off;
+        const unsigned char *rec = record.data();
         auto at = [&](unsigned off, auto &v) { memcpy(&v, rec + off, sizeof v); };
         /* node id of a local index, -1 when it is none */
         auto node = [&](unsigned l) -> int {
