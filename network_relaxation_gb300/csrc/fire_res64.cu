@@ -666,14 +666,17 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
     std::vector<Cand> cand;
     std::vector<std::vector<double>> uxs(9), uys(9);
     std::vector<std::vector<int>> order(9);
-    if (units_of(1) <= max_ctas) { /* a chunk a tile: nothing to choose */
+    const char *env = getenv("NR_RES64_SUB"); /* units of so many chunks alone (tests) */
+    const int only = env ? atoi(env) : 0;
+    if (units_of(1) <= max_ctas && !only) { /* a chunk a tile: nothing to choose */
         cand.push_back(Cand{1, 1, units_of(1), std::vector<int>(units_of(1)), 0.0});
         std::iota(cand[0].tile.begin(), cand[0].tile.end(), 0);
         cost(cand[0]);
     } else {
         for (int sub : {1, 2, 4, 8}) {
             const int U = units_of(sub), un = kChunk * sub;
-            if (sub > 1 && (U < max_ctas || n < 16 * kTile)) break; /* fewer partials only matter when there are many */
+            if (only && sub != only) continue;
+            if (!only && sub > 1 && (U < max_ctas || n < 16 * kTile)) break; /* fewer partials only matter when there are many */
             std::vector<double> &ux = uxs[sub], &uy = uys[sub];
             ux.assign(U, 0.0);
             uy.assign(U, 0.0);
@@ -711,6 +714,7 @@ static int build_layout(const nr_host_network &h, const Incidence &inc, const un
             cost(cand[k]);
         });
     }
+    if (cand.empty()) return NR_ERR_INVALID;
     const Cand &best = *std::min_element(cand.begin(), cand.end(),
                                          [](const Cand &a, const Cand &b) { return a.cost < b.cost; });
     const int sub = best.sub, un = kChunk * sub, U = units_of(sub), T = best.T;
