@@ -64,7 +64,7 @@ NR_IHD double ii_double(uint64_t u) {
 }
 #if !defined(__CUDA_ARCH__)
 /* Host: the FP32 estimate moved by this many units in the last place (the
- * tests sweep it over the device's error bound). */
+ * tests sweep it over the device's error: one for rcp, two for rsqrt). */
 inline int &ii_nudge() {
     static thread_local int n = 0;
     return n;
@@ -74,7 +74,9 @@ inline int &ii_nudge() {
 /* FP32 estimates of 1 / f, f in [1, 2], and 1 / sqrt(f), f in [1, 4], as
  * Q32 fixed point in [2^31, 2^32).  f is the significand rounded to 24 bits;
  * with it the relative error e0 is below 2^-22 (rcp.approx: 1 ulp;
- * rsqrt.approx: 2^-22.9). */
+ * rsqrt.approx: 2^-22.9, at most 2.1 units of 2^-24).  Over all f on GB300:
+ * within one unit and two units of the rounded value.  (Estimates moved by three
+ * units break the bound for values near 1/2, and quotients come out wrong.) */
 NR_IHD uint32_t ii_q32(uint32_t fbits) {
     /* kept within [1/2, 1): the ends of the range by a step */
     fbits = fbits > 0x3f7fffffu ? 0x3f7fffffu : fbits < 0x3f000000u ? 0x3f000000u : fbits;
