@@ -30,7 +30,7 @@
  * eight wavefronts for each 4-byte load), in shared memory where there is room,
  * and the next quad travels while one is added.  192-network batch of 600
  * steps without escalation 47.2 -> 36 ms (phases that may escalate run the
- * earlier kernel, fire_dsm_escalate.cu), 30 networks of up to 30^2 nodes and 400 steps 2.2 -> 2.0;
+ * earlier kernel, fire_dsm_escalate.cu; this one takes up what yielded there),
  * one network on 4 resident CTAs, us per step: 304 nodes 4.5 -> 3.5, 2491 nodes
  * 7.5 -> 6.0.  Loads from other CTAs (94 clocks a warp against 5 to 9) are
  * hidden: copying the boundary once a step and evaluating its items on both
@@ -202,7 +202,7 @@ struct GatherQuad {
 template <int NT, bool RES>
 __global__ void __launch_bounds__(NT, 1)
     k_fire_dsm_mixed(const NetDev *nets, const NetDsm *dsms, int n_nets, const int *n_dev, FireParamsDev p,
-                     int *queue, const int *order, DsmSizes z, int yield_at, int yield_pm) {
+                     int *queue, const int *order, DsmSizes z) {
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     extern __shared__ float4 s_dyn[];
@@ -229,13 +229,12 @@ __global__ void __launch_bounds__(NT, 1)
     __shared__ NetDsm s_m;
     __shared__ int s_slot;
     __shared__ float4 s_zero; /* what padding entries add */
-    /* every CTA's step totals and rank 0's escalation flag, pushed into
-     * every CTA of the cluster before the barrier that ends the step: each
-     * CTA then reads them from its own shared memory */
+    /* every CTA's step totals, pushed into every CTA of the cluster before
+     * the barrier that ends the step: each CTA then reads them from its own
+     * shared memory */
     __shared__ float s_parts[kDsmParts][5];
-    __shared__ int s_yield_all;
     __shared__ double s_ancs[kDsmParts][2]; /* every CTA's FP64 anchor totals (pushed) */
-    __shared__ int s_flag;  /* network start: resume a yielded network; in the loop: leave after this anchor */
+    __shared__ int s_resume; /* the network yielded in an earlier phase (fire_dsm_escalate.cu) */
     __shared__ unsigned s_au[kDsmParts], s_ab[kDsmParts], s_at[kDsmParts];
     const int rank = (int)cl.block_rank(), C = (int)cl.num_blocks();
     const int spr = kDsmParts / C, lg = __ffs(spr) - 1; /* sub-blocks per CTA, log2 */
@@ -246,13 +245,7 @@ __global__ void __launch_bounds__(NT, 1)
         s_at[threadIdx.x] = dsm_addr(s_tdf, threadIdx.x);
     }
     /* n_dev: the count of this launch's networks, written on the device by
-     * an earlier kernel (device-side escalation); the escalation threshold
-     * is then yield_pm / 1000 of the clusters that get a network */
-    if (n_dev && yield_pm > 0) {
-        const int n_eff = *(volatile const int *)n_dev, clusters = (int)(gridDim.x / C);
-        yield_at = max(1, yield_pm * min(clusters, n_eff) / 1000);
-    }
-    bool ran = false; /* this cluster relaxed a network in this launch */
+     * an earlier kernel (device-side escalation) */
     for (;;) {
         if (rank == 0 && threadIdx.x == 0) {
             const int sl = atomicAdd(queue, 1);
@@ -264,13 +257,7 @@ __global__ void __launch_bounds__(NT, 1)
          * shared memory must not be read remotely after it exits) or rank 0
          * overwrites it for the next network */
         cl.sync();
-        if (slot >= n_nets) {
-            /* one more idle cluster (one that never got a network does not
-             * count: it was never busy) */
-            if (rank == 0 && threadIdx.x == 0 && (ran || !n_dev)) atomicAdd(queue + 1, 1);
-            return;
-        }
-        ran = true;
+        if (slot >= n_nets) return;
         if (threadIdx.x == 0) {
             const int idx = order ? order[slot] : slot;
             s_d = nets[idx];
@@ -349,7 +336,7 @@ __global__ void __launch_bounds__(NT, 1)
         const int4 *Gr = R ? s_grec : m.xrec + n0;
         const float2 *FaH = R ? res.fahi : d.fa_hi + n0;
         const float2 *FaL = R ? res.falo : d.fa_lo + n0;
-        if (threadIdx.x == 0) s_flag = ((volatile FireState *)d.st)->yielded;
+        if (threadIdx.x == 0) s_resume = ((volatile FireState *)d.st)->yielded;
         __syncthreads();
         /* the FIRE scalars, advanced by thread 0 of every CTA (identical
          * copies), in shared memory: registers stay free for the passes */
@@ -358,7 +345,7 @@ __global__ void __launch_bounds__(NT, 1)
         MixScal &s = s_mix;
         MixParams &q = s_mq;
         double F2, M2, tF2, tM2;
-        if (s_flag) {
+        if (s_resume) {
             /* resume a network a smaller cluster left at an anchor: u = 0,
              * v and the FIRE scalars saved, F = F(X) and the anchor records
              * in global memory (slot-indexed: the layout does not depend on
@@ -504,11 +491,6 @@ __global__ void __launch_bounds__(NT, 1)
              * kick; the nodes in gather-record order (lanes of a warp take
              * nodes with equally long entry lists) */
             float P = 0.f, V2 = 0.f, Fs = 0.f, M2f = 0.f, A = 0.f;
-            /* rank 0 reads the idle-cluster count now; its global-memory
-             * latency passes during the gather instead of before the
-             * cluster barrier */
-            int idle = 0;
-            if (rank == 0 && threadIdx.x == 0 && yield_at > 0) idle = *(volatile int *)(queue + 1);
             for (int k = threadIdx.x; k < nloc; k += NT) {
                 /* one record load gives the node, its fcode and its entries */
                 const int4 g = ldro<RES>(Gr + k);
@@ -551,10 +533,6 @@ __global__ void __launch_bounds__(NT, 1)
             __syncthreads();
             if (threadIdx.x < 32) {
                 const Part t = block_totals(sh.slots);
-                /* rank 0's escalation flag: thread 0 read the idle count, so
-                 * lane 0's decision goes to every lane before any is pushed
-                 * (every CTA must take the same branch) */
-                const int yv = __shfl_sync(kFull, (int)(yield_at > 0 && idle >= yield_at), 0);
                 /* lane r pushes this CTA's totals into CTA r (remote stores
                  * complete before the cluster barrier releases) */
                 if ((int)threadIdx.x < C) {
@@ -564,7 +542,6 @@ __global__ void __launch_bounds__(NT, 1)
                     dsm_st1(a + 8u, t.F2);
                     dsm_st1(a + 12u, t.M2);
                     dsm_st1(a + 16u, t.A);
-                    if (rank == 0) dsm_st1i(dsm_addr(&s_yield_all, threadIdx.x), yv);
                 }
             }
             cl.sync();
@@ -576,11 +553,8 @@ __global__ void __launch_bounds__(NT, 1)
                              s_parts[threadIdx.x][3], s_parts[threadIdx.x][4]};
                 t = warp_reduce(t);
                 if (threadIdx.x == 0) {
-                    /* rank 0's escalation flag, the same in every CTA */
-                    const int y = s_yield_all;
                     mix_step(s, q, t);
-                    sh.coef = coef_of(s, need_anchor(s, q, t) || y);
-                    s_flag = y;
+                    sh.coef = coef_of(s, need_anchor(s, q, t));
                 }
             }
             __syncthreads();
@@ -605,20 +579,9 @@ __global__ void __launch_bounds__(NT, 1)
                     anchor_totals(s_ancs, C, t);
                     mix_certify(s, p, d.sqrt_dof, t[0], t[1]);
                     sh.coef = coef_of(s, 0);
-                    s_flag = s_flag && !s.done;
                 }
                 __syncthreads();
-                if (s_flag) break;
             }
-        }
-        if (s_flag) {
-            /* escalate: keep v and the FIRE scalars for the relaunch */
-            for (int li = threadIdx.x; li < nloc; li += NT) d.vf[n0 + li] = s_v[li];
-            if (rank == 0 && threadIdx.x == 0) {
-                d.st->mix = s;
-                d.st->yielded = 1;
-            }
-            continue;
         }
         for (int li = threadIdx.x; li < nloc; li += NT) {
             const float2 v = s_v[li];
@@ -693,8 +656,8 @@ static cudaError_t dsm_config(int cluster, const DsmSizes &z, cudaLaunchConfig_t
 
 template <int NT, bool RES>
 static cudaError_t launch_dsm_nt(const NetDev *nets_dev, const NetDsm *dsm_dev, int n_nets, const int *n_dev,
-                                 int cluster, const DsmSizes &z, double escalate, int cap, const FireParamsDev &p,
-                                 int *queue_dev, const int *order_dev, cudaStream_t stream) {
+                                 int cluster, const DsmSizes &z, int cap, const FireParamsDev &p, int *queue_dev,
+                                 const int *order_dev, cudaStream_t stream) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
     int max_clusters = 0;
@@ -705,11 +668,9 @@ static cudaError_t launch_dsm_nt(const NetDev *nets_dev, const NetDsm *dsm_dev, 
     if (cap > 0) clusters = std::min(clusters, cap);
     cfg.gridDim = dim3(clusters * cluster);
     cfg.stream = stream;
-    const int yield_at = escalate > 0 ? std::max(1, (int)(escalate * clusters)) : 0;
-    const int yield_pm = escalate > 0 ? std::max(1, (int)(1000.0 * escalate)) : 0;
-    if ((e = cudaMemsetAsync(queue_dev, 0, 2 * sizeof(int), stream)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(queue_dev, 0, sizeof(int), stream)) != cudaSuccess) return e;
     return cudaLaunchKernelEx(&cfg, k_fire_dsm_mixed<NT, RES>, nets_dev, dsm_dev, n_nets, n_dev, p, queue_dev,
-                              order_dev, z, yield_at, n_dev ? yield_pm : 0);
+                              order_dev, z);
 }
 
 /* Threads per CTA: NR_MIX_THREADS (512 or 1024), else 1024 when the state
@@ -733,15 +694,9 @@ cudaError_t launch_mixed_dsm(const NetDev *nets_dev, const NetDsm *dsm_dev, int 
                                          wide, escalate, cap, p, queue_dev, order_dev, stream, n_dev);
     DsmSizes z{bmax, emax, tmax, ebmax, etmax, resident, 0};
     z.extra = dsm_extra(z);
-    if (resident)
-        return wide ? launch_dsm_nt<1024, true>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p,
-                                                queue_dev, order_dev, stream)
-                    : launch_dsm_nt<512, true>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p,
-                                               queue_dev, order_dev, stream);
-    return wide ? launch_dsm_nt<1024, false>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p, queue_dev,
-                                             order_dev, stream)
-                : launch_dsm_nt<512, false>(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, escalate, cap, p, queue_dev,
-                                            order_dev, stream);
+    auto launch = resident ? (wide ? launch_dsm_nt<1024, true> : launch_dsm_nt<512, true>)
+                           : (wide ? launch_dsm_nt<1024, false> : launch_dsm_nt<512, false>);
+    return launch(nets_dev, dsm_dev, n_nets, n_dev, cluster, z, cap, p, queue_dev, order_dev, stream);
 }
 
 /* Device-side escalation: the networks of a batch that left their last
