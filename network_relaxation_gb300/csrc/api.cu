@@ -15,7 +15,6 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
-#include <new>
 #include <string>
 #include <vector>
 
@@ -50,49 +49,6 @@ static unsigned barrier_stall() {
     const int k = env ? atoi(env) : 0;
     return k > 0 && k < 1024 ? (unsigned)k : 0u;
 }
-
-/* A set's device memory: bytes that are uploaded, and behind them memory that
- * starts as zeros (zeros(): offsets from zeros_at()). */
-class Image {
-public:
-    Image() = default;
-    Image(const Image &) = delete;
-    Image &operator=(const Image &) = delete;
-    ~Image() { free(p_); }
-    char *data() { return p_; }
-    size_t size() const { return n_; }
-    size_t add(size_t nbytes) { /* to be written by the caller */
-        const size_t off = up(n_), end = off + nbytes;
-        if (end > cap_) {
-            cap_ = std::max(end, cap_ + cap_ / 2);
-            char *const q = (char *)realloc(p_, cap_);
-            if (!q) throw std::bad_alloc();
-            p_ = q;
-        }
-        memset(p_ + n_, 0, off - n_);
-        n_ = end;
-        return off;
-    }
-    template <class T>
-    size_t put(const T *src, size_t n) {
-        const size_t off = add(n * sizeof(T));
-        if (n) memcpy(p_ + off, src, n * sizeof(T));
-        return off;
-    }
-    size_t zeros(size_t nbytes) {
-        const size_t off = up(n_zeros_);
-        n_zeros_ = off + nbytes;
-        return off;
-    }
-    size_t zeros_at() const { return up(n_); }
-    size_t zeros_size() const { return n_zeros_; }
-    size_t total() const { return zeros_at() + n_zeros_; }
-
-private:
-    static size_t up(size_t n) { return (n + 255) / 256 * 256; }
-    char *p_ = nullptr;
-    size_t n_ = 0, cap_ = 0, n_zeros_ = 0;
-};
 
 struct NetOff {
     size_t mb_data, mb_sk, bdf, mt_arms, mt_pk, tdf, bfrc, tfrc;

@@ -2,7 +2,11 @@
 #ifndef NR_INTERNAL_H
 #define NR_INTERNAL_H
 
+#include <algorithm>
 #include <cstdint>
+#include <cstdlib>
+#include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -38,14 +42,57 @@ namespace nr {
 int fail(int status, const std::string &msg);
 void clear_error();
 
-/* Per-node incidence lists in canonical order: every bond (in index order,
- * first endpoint before second) and every triple (in index order, hinge, j,
- * k) touching the node.  Entry encodings: bond (b << 1) | role,
- * triple (t << 2) | role. */
+/* An object's device memory: bytes that are uploaded, and behind them memory
+ * that starts as zeros (zeros(): offsets from zeros_at()). */
+class Image {
+public:
+    Image() = default;
+    Image(const Image &) = delete;
+    Image &operator=(const Image &) = delete;
+    ~Image() { std::free(p_); }
+    char *data() { return p_; }
+    size_t size() const { return n_; }
+    size_t add(size_t nbytes) { /* to be written by the caller */
+        const size_t off = up(n_), end = off + nbytes;
+        if (end > cap_) {
+            cap_ = std::max(end, cap_ + cap_ / 2);
+            char *const q = (char *)std::realloc(p_, cap_);
+            if (!q) throw std::bad_alloc();
+            p_ = q;
+        }
+        std::memset(p_ + n_, 0, off - n_);
+        n_ = end;
+        return off;
+    }
+    template <class T>
+    size_t put(const T *src, size_t n) {
+        const size_t off = add(n * sizeof(T));
+        if (n) std::memcpy(p_ + off, src, n * sizeof(T));
+        return off;
+    }
+    size_t zeros(size_t nbytes) {
+        const size_t off = up(n_zeros_);
+        n_zeros_ = off + nbytes;
+        return off;
+    }
+    size_t zeros_at() const { return up(n_); }
+    size_t zeros_size() const { return n_zeros_; }
+    size_t total() const { return zeros_at() + n_zeros_; }
+
+private:
+    static size_t up(size_t n) { return (n + 255) / 256 * 256; }
+    char *p_ = nullptr;
+    size_t n_ = 0, cap_ = 0, n_zeros_ = 0;
+};
+
 /* A launch-policy knob: the environment variable `name`, else the tuning
  * table's entry of that name (tuning.cu), else null. */
 const char *knob(const char *name);
 
+/* Per-node incidence lists in canonical order: every bond (in index order,
+ * first endpoint before second) and every triple (in index order, hinge, j,
+ * k) touching the node.  Entry encodings: bond (b << 1) | role,
+ * triple (t << 2) | role. */
 struct Incidence {
     std::vector<int> bptr, bent, tptr, tent;
 };

@@ -994,21 +994,6 @@ void unit_rhs(nr_spr &S, int affine, std::vector<double> &rhs2) {
     }
 }
 
-struct Img {
-    std::vector<char> bytes;
-    size_t add(size_t nb) {
-        const size_t off = (bytes.size() + 255) / 256 * 256;
-        bytes.resize(off + nb);
-        return off;
-    }
-    template <class T>
-    size_t put(const T *src, size_t cnt) {
-        const size_t off = add(cnt * sizeof(T));
-        if (cnt) memcpy(bytes.data() + off, src, cnt * sizeof(T));
-        return off;
-    }
-};
-
 /* Cuts nodes idx[b, e) into parts [g0, g0 + P) by recursive coordinate
  * bisection along the longer side, in whole units of 16 nodes (a slice of 32
  * rows); start[g]: a part's first node. */
@@ -1302,48 +1287,48 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     }
     const int tb = (S->n_edges + kTile - 1) / kTile, tt = (S->n_triples + kTile - 1) / kTile;
     S->e_stride = std::max(1, std::max(tb, tt));
-    Img img;
+    Image img;
     const size_t o_sp = img.put(slice_ptr.data(), slice_ptr.size());
     const size_t o_sw = img.put(slice_w.data(), slice_w.size());
     const size_t o_col = img.put(scol.data(), scol.size());
     const size_t o_val = img.put(sval.data(), sval.size());
     const size_t o_md = img.put(mdiag.data(), mdiag.size());
     const size_t o_mo = img.put(moff.data(), moff.size());
-    const size_t o_b = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_x = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_r = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_p = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_q = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_z = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_s = img.add(sizeof(double2) * (nrp + 1));
-    const size_t o_part = img.add(sizeof(double) * kParts * (size_t)std::max(blocks, 2 * P));
+    const size_t o_b = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_x = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_r = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_p = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_q = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_z = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_s = img.zeros(sizeof(double2) * (nrp + 1));
+    const size_t o_part = img.zeros(sizeof(double) * kParts * (size_t)std::max(blocks, 2 * P));
     S->pcg_blocks = blocks;
     S->rpart_blocks = 4 * sm_count_spr(); /* k_spr_residual's largest grid */
-    const size_t o_rpart = img.add(sizeof(double) * kParts * (size_t)S->rpart_blocks);
-    const size_t o_sc = img.add(sizeof(SprScal));
-    const size_t o_bar = img.add(sizeof(SprBar));
+    const size_t o_rpart = img.zeros(sizeof(double) * kParts * (size_t)S->rpart_blocks);
+    const size_t o_sc = img.zeros(sizeof(SprScal));
+    const size_t o_bar = img.zeros(sizeof(SprBar));
     const size_t o_sl0 = img.put(sl0.data(), sl0.size());
     const size_t o_h0 = img.put(h0.data(), h0.size());
     const size_t o_hn = img.put(hnode.data(), hnode.size());
     const size_t o_lcol = img.put(lcol.data(), lcol.size());
     const size_t o_map = img.put(dof_dev.data(), dof_dev.size());
     const size_t o_top = img.put(S->top.data(), S->top.size());
-    const size_t o_ured = img.add(sizeof(double) * (nrp + 1));
-    const size_t o_uf = img.add(sizeof(double2) * (size_t)S->n);
+    const size_t o_ured = img.zeros(sizeof(double) * (nrp + 1));
+    const size_t o_uf = img.zeros(sizeof(double2) * (size_t)S->n);
     const size_t o_pos = img.put((const double2 *)h.points.data(), (size_t)S->n);
     const size_t o_bond = img.put(bond.data(), bond.size());
     const size_t o_l0 = img.put(h.edge_l0.data(), h.edge_l0.size());
     const size_t o_tri = img.put(tri.data(), tri.size());
-    const size_t o_ep = img.add(sizeof(double) * 2 * (size_t)S->e_stride);
-    const size_t o_scalar = img.add(sizeof(double) * 4);
-    cudaError_t e = cudaMalloc((void **)&S->arena, img.bytes.size());
+    const size_t o_ep = img.zeros(sizeof(double) * 2 * (size_t)S->e_stride);
+    const size_t o_scalar = img.zeros(sizeof(double) * 4);
+    cudaError_t e = cudaMalloc((void **)&S->arena, img.total());
     if (e != cudaSuccess) {
         S->arena = nullptr;
         delete S;
         return fail(e == cudaErrorMemoryAllocation ? NR_ERR_OOM : NR_ERR_CUDA,
                     std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
-    char *base = S->arena;
+    char *base = S->arena, *zeros = S->arena + img.zeros_at();
     SprDev &d = S->dev;
     d.nr = nrp;
     d.n_slices = S->n_slices;
@@ -1353,16 +1338,16 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     d.val = (const double *)(base + o_val);
     d.mdiag = (const double2 *)(base + o_md);
     d.moff = (const double *)(base + o_mo);
-    d.b = (const double2 *)(base + o_b);
-    d.x = (double2 *)(base + o_x);
-    d.r = (double2 *)(base + o_r);
-    d.p = (double2 *)(base + o_p);
-    d.q = (double2 *)(base + o_q);
-    d.z = (double2 *)(base + o_z);
-    d.s = (double2 *)(base + o_s);
-    d.part = (double *)(base + o_part);
-    d.sc = (SprScal *)(base + o_sc);
-    d.bar = &((SprBar *)(base + o_bar))->st;
+    d.b = (const double2 *)(zeros + o_b);
+    d.x = (double2 *)(zeros + o_x);
+    d.r = (double2 *)(zeros + o_r);
+    d.p = (double2 *)(zeros + o_p);
+    d.q = (double2 *)(zeros + o_q);
+    d.z = (double2 *)(zeros + o_z);
+    d.s = (double2 *)(zeros + o_s);
+    d.part = (double *)(zeros + o_part);
+    d.sc = (SprScal *)(zeros + o_sc);
+    d.bar = &((SprBar *)(zeros + o_bar))->st;
     S->res.sl0 = (const int *)(base + o_sl0);
     S->res.h0 = (const int *)(base + o_h0);
     S->res.hnode = (const int *)(base + o_hn);
@@ -1370,14 +1355,14 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     S->res.pub[0] = d.s;
     S->res.pub[1] = d.z;
     S->res.part = d.part;
-    S->res.count = &((SprBar *)(base + o_bar))->count;
-    S->d_rpart = (double *)(base + o_rpart);
+    S->res.count = &((SprBar *)(zeros + o_bar))->count;
+    S->d_rpart = (double *)(zeros + o_rpart);
     S->d_dof_map = (int *)(base + o_map);
     S->d_top = (unsigned char *)(base + o_top);
-    S->d_u_red = (double *)(base + o_ured);
-    S->d_u_final = (double2 *)(base + o_uf);
-    S->d_epart = (double *)(base + o_ep);
-    S->d_scalar = (double *)(base + o_scalar);
+    S->d_u_red = (double *)(zeros + o_ured);
+    S->d_u_final = (double2 *)(zeros + o_uf);
+    S->d_epart = (double *)(zeros + o_ep);
+    S->d_scalar = (double *)(zeros + o_scalar);
     SprEnergyDev &ed = S->edev;
     ed.n_edges = S->n_edges;
     ed.n_triples = S->n_triples;
@@ -1390,7 +1375,8 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     ed.l0 = (const double *)(base + o_l0);
     ed.tri = (const int4 *)(base + o_tri);
     ed.u = S->d_u_final;
-    e = cudaMemcpyAsync(S->arena, img.bytes.data(), img.bytes.size(), cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(S->arena, img.data(), img.size(), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(zeros, 0, img.zeros_size(), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         delete S;
