@@ -391,8 +391,9 @@ static bool add_res_layout(const nr_host_network &h, const Incidence &inc, const
     return true;
 }
 
-static int build_set(int n, const nr_host_network *const *nets, const double *ks, const double *kb,
-                     const unsigned char *const *fcodes_in, cudaStream_t stream, DeviceSet &S) {
+/* May throw. */
+static int fill_set(int n, const nr_host_network *const *nets, const double *ks, const double *kb,
+                    const unsigned char *const *fcodes_in, cudaStream_t stream, DeviceSet &S) {
     if (n <= 0) return fail(NR_ERR_INVALID, "network count must be positive");
     Image img;
     S.n_nets = n;
@@ -634,6 +635,10 @@ static int build_set(int n, const nr_host_network *const *nets, const double *ks
     }
     if (want_tile) return build_tile_set(*nets[0], inc0, fc0.data(), S, stream);
     return NR_OK;
+}
+static int build_set(int n, const nr_host_network *const *nets, const double *ks, const double *kb,
+                     const unsigned char *const *fcodes_in, cudaStream_t stream, DeviceSet &S) {
+    return no_throw([&] { return fill_set(n, nets, ks, kb, fcodes_in, stream, S); });
 }
 
 /* Energy launch width for network d. */

@@ -53,14 +53,8 @@ void parallel_ranges(long n, int threads, F &&f) {
         f(0L, n);
         return;
     }
-    std::vector<std::thread> pool;
     const long per = (n + t - 1) / t;
-    for (int k = 1; k < t; ++k) {
-        const long b = std::min(n, k * per), e = std::min(n, (k + 1) * per);
-        pool.emplace_back([=, &f] { f(b, e); });
-    }
-    f(0L, std::min(n, per));
-    for (auto &th : pool) th.join();
+    run_threads(t, [&](int k) { f(std::min(n, k * per), std::min(n, (k + 1) * per)); });
 }
 
 inline bool is_space(char c) { return c == ' ' || c == '\t' || c == '\n' || c == '\v' || c == '\f' || c == '\r'; }

@@ -55,8 +55,6 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
-#include <exception>
-#include <new>
 #include <numeric>
 #include <thread>
 #include <type_traits>
@@ -509,33 +507,15 @@ cudaError_t launch_fp64_res(const NetDev &d, const Res64Dev &r, const FireParams
 namespace {
 
 /* Runs f(k, scratch) for k < n, on a few host threads when `items` items of
- * work repay their start; every thread has its own Scratch. A thread that
- * cannot be started is done without (the others take its share); an exception
- * in a thread ends the work and is thrown here once all threads are joined. */
+ * work repay their start; every thread has its own Scratch. */
 template <class Scratch, class F>
 void parallel_for(int n, long items, F f) {
     const int nt = std::max(1, std::min({n, (int)std::thread::hardware_concurrency(), 16, (int)(items / 3000)}));
     std::atomic<int> next{0};
-    std::atomic<bool> thrown{false};
-    std::exception_ptr error;
-    auto work = [&] {
-        try {
-            Scratch s;
-            for (int k; (k = next.fetch_add(1)) < n;) f(k, s);
-        } catch (...) {
-            if (!thrown.exchange(true)) error = std::current_exception();
-            next = n;
-        }
-    };
-    std::vector<std::thread> ts;
-    ts.reserve(nt);
-    try {
-        for (int t = 1; t < nt; ++t) ts.emplace_back(work);
-    } catch (...) { /* std::system_error: no thread; bad_alloc: no room for its state */
-    }
-    work();
-    for (auto &t : ts) t.join();
-    if (error) std::rethrow_exception(error);
+    run_threads(nt, [&](int) {
+        Scratch s;
+        for (int k; (k = next.fetch_add(1)) < n;) f(k, s);
+    });
 }
 
 struct NoScratch {};

@@ -98,8 +98,7 @@ int nr_abi_version(void) { return NR_ABI_VERSION; }
  * order (forward wrap for the first endpoint, negated for the second),
  * hinges ascending, pairs i < j in list order, accepted when dot < 0 and
  * |dot^2 - |a|^2 |b|^2| < 1e-10. */
-int nr_get_triples(nr_host_network *net) {
-    if (!net) return fail(NR_ERR_INVALID, "nr_get_triples: null network");
+static int get_triples(nr_host_network *net) {
     const int n = net->n_points, ne = net->n_edges();
     std::vector<int> start((size_t)n + 1, 0);
     for (int e = 0; e < ne; ++e) {
@@ -156,15 +155,16 @@ int nr_get_triples(nr_host_network *net) {
             }
         }
     };
-    std::vector<std::thread> pool;
-    for (int t = 1; t < threads; ++t) pool.emplace_back(work, t);
-    work(0);
-    for (auto &th : pool) th.join();
+    nr::run_threads(threads, work);
     for (int t = 0; t < threads; ++t) {
         net->tri_hjk.insert(net->tri_hjk.end(), hjk[t].begin(), hjk[t].end());
         net->tri_wrap.insert(net->tri_wrap.end(), tw[t].begin(), tw[t].end());
     }
     return NR_OK;
+}
+int nr_get_triples(nr_host_network *net) {
+    if (!net) return fail(NR_ERR_INVALID, "nr_get_triples: null network");
+    return nr::no_throw([&] { return get_triples(net); });
 }
 
 int nr_host_network_from_arrays(int n_points, const double *points, int n_edges, const int *edge_ij,

@@ -3,11 +3,14 @@
 #define NR_INTERNAL_H
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/netrelax.h"
@@ -41,6 +44,44 @@ namespace nr {
 /* Thread-local error message + status helper. */
 int fail(int status, const std::string &msg);
 void clear_error();
+
+/* f()'s status; NR_ERR_OOM when host memory runs out in it (an exception must
+ * not leave a C function). */
+template <class F>
+int no_throw(F f) {
+    try {
+        return f();
+    } catch (const std::bad_alloc &) {
+        return fail(NR_ERR_OOM, "no host memory"); /* fits a string without memory of its own */
+    }
+}
+
+/* work(k) for every k < n, on n host threads (the caller's is one).  A thread
+ * that cannot be started leaves its part to the caller's; an exception in one is
+ * thrown here once all have ended. */
+template <class F>
+void run_threads(int n, F work) {
+    std::atomic<bool> thrown{false};
+    std::exception_ptr error;
+    auto guarded = [&](int k) {
+        try {
+            work(k);
+        } catch (...) {
+            if (!thrown.exchange(true)) error = std::current_exception();
+        }
+    };
+    std::vector<std::thread> ts;
+    int started = 1;
+    try {
+        ts.reserve(n);
+        for (; started < n; ++started) ts.emplace_back(guarded, started);
+    } catch (...) { /* std::system_error: no thread; bad_alloc: no room for its state */
+    }
+    guarded(0);
+    for (int k = started; k < n; ++k) guarded(k);
+    for (auto &t : ts) t.join();
+    if (error) std::rethrow_exception(error);
+}
 
 /* An object's device memory: bytes that are uploaded, and behind them memory
  * that starts as zeros (zeros(): offsets from zeros_at()). */

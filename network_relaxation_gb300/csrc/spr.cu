@@ -41,6 +41,7 @@
 #include <cfloat>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -167,7 +168,7 @@ void assemble_upper(const nr_host_network &h, double ks, double kb, double mu, U
         copy.edge_ij = h.edge_ij;
         copy.edge_l0 = h.edge_l0;
         copy.edge_wrap = h.edge_wrap;
-        nr_get_triples(&copy);
+        if (nr_get_triples(&copy) != NR_OK) throw std::bad_alloc();
         tri_hjk.swap(copy.tri_hjk);
         tri_wrap.swap(copy.tri_wrap);
     }
@@ -1073,12 +1074,14 @@ long nr_spr_assemble(const nr_host_network *net, double ks, double kb, double mu
     return (long)K.col.size();
 }
 
-int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, void *stream, nr_spr **out) {
+/* May throw. */
+static int spr_create(const nr_host_network *net, double ks, double kb, double mu, void *stream, nr_spr **out) {
     if (!net || !out || net->n_points <= 0 || !(ks >= 0) || !(kb >= 0) || !(mu >= 0))
         return fail(NR_ERR_INVALID, "nr_spr_create: bad arguments");
     *out = nullptr;
     cudaStream_t s = (cudaStream_t)stream;
-    auto *S = new nr_spr();
+    std::unique_ptr<nr_spr> owner(new nr_spr());
+    nr_spr *const S = owner.get();
     const nr_host_network &h = *net;
     S->n = h.n_points;
     S->ks = ks;
@@ -1266,7 +1269,7 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
         copy.edge_ij = h.edge_ij;
         copy.edge_l0 = h.edge_l0;
         copy.edge_wrap = h.edge_wrap;
-        nr_get_triples(&copy);
+        if (nr_get_triples(&copy) != NR_OK) throw std::bad_alloc();
         for (int t = 0; t < copy.n_triples(); ++t)
             tri.push_back(make_int4(copy.tri_hjk[3 * t], copy.tri_hjk[3 * t + 1], copy.tri_hjk[3 * t + 2],
                                     copy.tri_wrap[2 * t]));
@@ -1275,16 +1278,10 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     S->n_triples = (int)tri.size();
     int blocks = 0;
     int rc = spr_blocks(&blocks);
-    if (rc != NR_OK) {
-        delete S;
-        return rc;
-    }
+    if (rc != NR_OK) return rc;
     S->parts = P;
     rc = spr_res_mode(rz, narrow, &S->mode);
-    if (rc != NR_OK) {
-        delete S;
-        return rc;
-    }
+    if (rc != NR_OK) return rc;
     const int tb = (S->n_edges + kTile - 1) / kTile, tt = (S->n_triples + kTile - 1) / kTile;
     S->e_stride = std::max(1, std::max(tb, tt));
     Image img;
@@ -1324,7 +1321,6 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     cudaError_t e = cudaMalloc((void **)&S->arena, img.total());
     if (e != cudaSuccess) {
         S->arena = nullptr;
-        delete S;
         return fail(e == cudaErrorMemoryAllocation ? NR_ERR_OOM : NR_ERR_CUDA,
                     std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
@@ -1378,13 +1374,14 @@ int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, v
     e = cudaMemcpyAsync(S->arena, img.data(), img.size(), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(zeros, 0, img.zeros_size(), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        delete S;
-        return fail(NR_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
-    }
+    if (e != cudaSuccess) return fail(NR_ERR_CUDA, std::string("upload: ") + cudaGetErrorString(e));
     S->points = h.points;
-    *out = S;
+    *out = owner.release();
     return NR_OK;
+}
+
+int nr_spr_create(const nr_host_network *net, double ks, double kb, double mu, void *stream, nr_spr **out) {
+    return no_throw([&] { return spr_create(net, ks, kb, mu, stream, out); });
 }
 
 int nr_spr_destroy(nr_spr *s) {
