@@ -85,13 +85,14 @@ __device__ __forceinline__ double res_tile_sum(const double *p, int sub) {
  *   kResSmall   256 threads, 80 registers, three on an SM: at most 8 groups of
  *               items a tile and 64 tiles in the sums
  *   kResShared  512 threads, 64 registers, two on an SM: fewer than 64 tiles in
- *               the sums (16 129 nodes)
+ *               the sums (up to 16 128 nodes)
  *   kResAlone   512 threads, one on an SM
  * us per step and network, one thread | 16 threads, against one 512-thread CTA
- * on an SM for all sizes: 1 024 nodes 8.5 | 2.1 -> 8.5 | 1.3, 4 096
- * 8.8 | 8.8 -> 8.9 | 4.0, 4 900 9.2 | 9.2 -> 9.4 | 5.7, 9 216 9.8 | 9.7 -> 9.9 | 6.4,
- * 12 544 12.3 | 12.1 -> 12.5 | 8.0; at 16 384, 11.2 | 11.3, one thread
- * would lose 2 %. */
+ * on an SM for all sizes: 1 024 nodes 8.5 | 2.1 -> 8.45 | 1.25, 4 096 8.8 | 8.8
+ * -> 8.85 | 4.0, 4 900 9.2 | 9.2 -> 9.3 | 5.7, 9 216 9.8 | 9.7 -> 9.9 | 6.4,
+ * 12 544 12.3 | 12.1 -> 12.35 | 7.9; at 16 384, 11.2 | 11.3, one thread would
+ * lose 2 %.  (By __maxnreg__: with a minimum of CTAs an SM the compiler goes
+ * below the registers it may use, 4 % slower for one thread.) */
 enum { kResSmall, kResShared, kResAlone };
 constexpr int kResSmallGroups = 8, kResSmallTiles = 64, kResSharedTiles = 63;
 __host__ __device__ constexpr int res_threads(int shape) { return shape == kResSmall ? 256 : 512; }
@@ -263,7 +264,9 @@ __global__ void __launch_bounds__(res_threads(kShape))
             }
         }
         __syncthreads();
-        /* gather in canonical order, one thread per node and component */
+        /* gather in canonical order, one thread per node and component, two
+         * entries in flight (four take registers: 65 536 nodes 23.1 us a step
+         * against 22.9, 9 216 nodes 9.95 against 9.88) */
         {
             const double *bfd = reinterpret_cast<const double *>(s_bf);
             const double *tfd = reinterpret_cast<const double *>(s_tf);
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(res_threads(kShape))
                 if ((q.y >> (24 + c)) & 1u) {
                     if (d.use_bonds) {
                         const int m = (int)((q.x >> 16) & 0xffu);
-#pragma unroll 4
+#pragma unroll 2
                         for (int a = 0; a < m; ++a) {
                             const unsigned code = e[a];
                             f = f + ii_flip(bfd[(code & ~1u) + c], (code & 1u) != 0);
@@ -285,7 +288,7 @@ __global__ void __launch_bounds__(res_threads(kShape))
                     }
                     if (d.use_triples) {
                         const int m = (int)(q.x >> 24);
-#pragma unroll 4
+#pragma unroll 2
                         for (int a = 0; a < m; ++a) {
                             if (kPairs) {
                                 const unsigned code = e[a], t = code / 3u, role = code - 3u * t;
