@@ -5,7 +5,8 @@
  * Every network (or batch of networks) lives in ONE device allocation built
  * from a host staging image: node state first (x, v, f of all networks
  * contiguous, so a batch's positions are one array), then the FIRE states,
- * then per network its topology, incidence lists and reduction scratch.
+ * then per network its topology, incidence lists and reduction scratch; what
+ * starts as zeros lies behind the uploaded part, in the same order.
  */
 #include <cuda_runtime.h>
 

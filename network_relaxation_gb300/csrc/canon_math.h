@@ -74,9 +74,6 @@ NR_HD double inv_sqrt_ieee(double q) {
 #endif
 }
 
-/* Quadrant/octant reduction, then atan(t) = pi/4 + atan((t-1)/(t+1)) above
- * tan(pi/8), then the polynomial; pi/4, pi/2 and pi are added as two-part
- * constants.  About one ulp for finite non-zero arguments; (0,0) -> 0. */
 /* Rare cases as functions of their own, called, not inlined: an inlined
  * branch becomes predicated instructions, and a predicated-off FP64
  * instruction takes its slot all the same (measured). */
@@ -98,7 +95,10 @@ NR_RARE double wrap_gap(double x1, double x2, double wW) { return (x1 - x2) - wW
 /* (x2 + wW) - x1 */
 NR_RARE double wrap_reach(double x1, double x2, double wW) { return (x2 + wW) - x1; }
 
-/* atan2 from the operands' magnitudes and signs (negative: below zero). */
+/* atan2 from the operands' magnitudes and signs (negative: below zero).
+ * Quadrant/octant reduction, then atan(t) = pi/4 + atan((t-1)/(t+1)) above
+ * tan(pi/8), then the polynomial; pi/4, pi/2 and pi are added as two-part
+ * constants.  About one ulp for finite non-zero arguments; (0,0) -> 0. */
 NR_HD double atan2_parts(double ay, double ax, bool yneg, bool xneg) {
     /* the comparisons on the operands' bits: an FP64 comparison takes an FP64
      * slot, and the magnitudes order like their bits (a NaN gives NaN either

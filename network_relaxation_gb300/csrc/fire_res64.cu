@@ -33,12 +33,13 @@
  * entries, and the nodes are gathered in the order of their list lengths, one
  * thread per node and component.
  *
- * Measured per FIRE step (us): 1 024 nodes 22.5 (cluster of 16) -> 8.4; 9 991
- * nodes 40 (grid kernel) -> 10.0; 65 536 nodes 77 -> 23.0, 93 000 nodes 35.0;
- * Mikado of 50 306 nodes 25; gel of 27 792 nodes 67 -> 25.6.  Of the 23.0 us:
- * items 10.7, passes over nodes and the gather 7.1, barrier and imbalance 1.7,
- * totals and scalars 3.9; the FP64 pipe is active for 17.  512 threads: 768
- * and 1024 measured 3 to 9 % slower.
+ * Measured per FIRE step (us): 1 024 nodes 22.5 (cluster of 16) -> 8.5; 9 991
+ * nodes 40 (grid kernel) -> 10.1; 65 536 nodes 77 -> 22.9; gel of 27 648 nodes
+ * 67 -> 25.7.  Of 23 us: items 10.7, passes over nodes and the gather 7.1,
+ * barrier and imbalance 1.7, totals and scalars 3.9; the FP64 pipe is active for
+ * 17 (62 % of a peak of a warp instruction in 16 clocks, of which FP64
+ * instructions reach 84 %).  512 threads: 768 and 1024 measured 3 to 9 % slower;
+ * smaller networks: the CTA shapes below.
  *
  * Tiles that do not fit whole (from about 125 000 nodes of a p = 0.65 lattice) are
  * still twice as fast as the grid kernel with their topology, v and F in L2

@@ -38,7 +38,7 @@
  * gather selected its share, and the item loops ended in nearly empty rounds.
  * 16 384 nodes 6.7 -> 4.8, 262 144 nodes 19.1 -> 15.6, 1 048 576 nodes 58.2 ->
  * 50.8 us: there 14 tiles a step pass through the SM, whose warps issue on
- * 45 % of the cycles and wait for shared memory (3.3 wavefronts a load) and at
+ * 45 % of the cycles (360 000 nodes: 42 %) and wait for shared memory and at
  * the barriers between the phases.  Of the last 5.8 us, 2.4 came from the
  * gather's entries in quads (four 2-byte loads of scattered addresses before),
  * 3.4 from pass A following the previous tile's gather without a barrier.  Two
@@ -957,8 +957,7 @@ int build_tile_layout(const nr_host_network &h, const Incidence &inc, const unsi
                     incv.push_back((unsigned short)(((inc.bent[e] & 1) << 15) | (at.sk / 8 + bslot[inc.bent[e] >> 1])));
             ibe.push_back((unsigned short)incv.size());
             if (use_triples)
-                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e)
-{
+                for (int e = inc.tptr[i]; e < inc.tptr[i + 1]; ++e) {
                     const int sl = tslot[inc.tent[e] >> 2], role = inc.tent[e] & 3;
                     incv.push_back((unsigned short)(role == 0 ? 0x8000 | (at.pk / 8 + sl)
                                                               : at.arms / 8 + 2 * sl + (role == 2)));

@@ -36,10 +36,6 @@ struct MeshPointLess {
 };
 }  // namespace
 
-/* The reader keeps the points in a std::map under PointComp (a point
- * equivalent to an earlier one is not inserted) and pairs every map entry
- * with x < minx + 1e-10, in map order, with the entry found at
- * (x + offset, y). */
 bool element_incidence(const nr_host_network &h, std::vector<int> &eptr, std::vector<int> &eent,
                        std::vector<int> &partner) {
     const int n = h.n_points, nf = h.n_facets();
@@ -64,6 +60,10 @@ bool element_incidence(const nr_host_network &h, std::vector<int> &eptr, std::ve
     return ok;
 }
 
+/* The reader keeps the points in a std::map under PointComp (a point
+ * equivalent to an earlier one is not inserted) and pairs every map entry
+ * with x < minx + 1e-10, in map order, with the entry found at
+ * (x + offset, y). */
 void find_mesh_pairs(const std::vector<double> &points, double offset, double minx, std::vector<int> &pairs) {
     /* The same red-black tree as std::map (hence the same answers on
      * near-duplicates, where PointComp is not a strict order), with its
